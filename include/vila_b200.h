@@ -334,7 +334,8 @@ int vila_gated_norm_residual(float* x, const void* part, int part_dtype, int64_t
                              int bias_dtype, const void* w, int w_dtype, float w_offset, float eps,
                              int rows, int cols, void* stream);
 
-/* vila_glinear — any-shape (grouped) linear layer on the CUDA cores with fp32 accumulation:
+/* vila_glinear — any-shape (grouped) linear layer with fp32 accumulation (bf16 operands on 16-byte boundaries and
+ * N >= 128: tcgen05, otherwise CUDA cores):
  *   out = act(a · w[g]^T + bias[g]) (* row_scale)
  * mode 0 (batched): every group g sees all M rows; its A columns start at g * a_group_off and its
  *   output columns at g * o_group_off (per-head projections); groups == 1 is a plain linear layer.
@@ -360,6 +361,9 @@ typedef struct vila_glinear_params {
   int32_t M, N, K, groups, mode, a_row_div, act, flags;
 } vila_glinear_params;
 int vila_glinear(const vila_glinear_params* p, void* stream);
+/* Waits inside vila_glinear's tensor-core kernel that ran out of tries since the process started on the current
+ * device (0 in a correct run; the launch's output is then incomplete).  Synchronises; -1: could not be read. */
+int vila_stalled_waits(void);
 
 /* vila_latent_attention — causal attention of H query heads over ONE shared latent per token
  * (keys and values are both the cached latent c_j of width R; the per-head key/value expansions

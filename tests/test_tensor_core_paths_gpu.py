@@ -1,0 +1,78 @@
+"""Tensor-core forms of the token-id models' kernels at the sizes where they can go wrong (tile edges, remainders, the
+smallest and largest of their ranges), against float64 on the device.  Sums of bf16 products are exact per product and
+accumulated in fp32: the bound on fp32 results is a few fp32 roundings per accumulated partial, 2e-6 relative in norm."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+BF, F32 = torch.bfloat16, torch.float32
+
+
+@pytest.fixture(scope="module")
+def ops():
+    from vila_b200 import ops
+    return ops
+
+
+def rel(a, b):
+    return float((a.double() - b).norm() / b.norm().clamp_min(1e-30))
+
+
+def gen(seed):
+    return torch.Generator(device="cuda").manual_seed(seed)
+
+
+def randn(g, *shape, dtype=BF):
+    return torch.randn(*shape, generator=g, device="cuda").to(dtype)
+
+
+@pytest.mark.parametrize("M,N,K", [(1, 128, 8), (8, 1000, 512), (15, 129, 72), (16, 256, 64), (17, 384, 136), (64, 130, 2048),
+                                   (65, 257, 448), (128, 128, 200), (129, 640, 1000), (300, 1408, 2048)])
+def test_glinear_plain(ops, M, N, K):
+    g = gen(M * 7 + N)
+    a, w, b = randn(g, M, K + 8)[:, :K], randn(g, N, K), randn(g, N)
+    ref = a.double() @ w.double().T
+    assert rel(ops.glinear(a, w, out_dtype=F32), ref) < 2e-6
+    assert rel(ops.glinear(a, w, bias=b, act=ops.ACT_RELU2, out_dtype=F32), torch.relu(ref + b.double()) ** 2) < 4e-6
+    assert rel(ops.glinear(a, w), ref) < 2.0 ** -8
+    if N % 2 == 0:
+        z = ref / K ** 0.5
+        want = torch.nn.functional.silu(z[:, 0::2]) * z[:, 1::2]
+        assert rel(ops.glinear((a.float() / K ** 0.5).to(BF), w, swiglu=True, out_dtype=F32), want) < 2.0 ** -7   # a is rounded once more
+    from vila_b200 import _lib
+    assert _lib.load().vila_stalled_waits() == 0
+
+
+@pytest.mark.parametrize("T,E,top,W,ff", [(3, 8, 2, 128, 128), (8, 32, 4, 256, 192), (40, 5, 3, 136, 200), (200, 33, 2, 256, 264), (520, 4, 2, 320, 136)])
+@pytest.mark.parametrize("skew", [False, True])
+def test_glinear_routed(ops, T, E, top, W, ff, skew):
+    """experts with no rows, with one and with more than a tile; scattered output rows, routing weights, input scales"""
+    g = gen(T + E)
+    x, up, down = randn(g, T, W), randn(g, E, 2 * ff, W), randn(g, E, W, ff)
+    score = torch.rand(T, E, generator=g, device="cuda")
+    if skew:
+        score[:, 1] += 1.0
+        score[:, E - 1] -= 2.0
+    idx = score.topk(top, 1).indices.to(torch.int32)
+    wt = torch.rand(T, top, generator=g, device="cuda")
+    seg, srt = ops.moe_group(idx, E)
+    act = ops.glinear(x, up, groups=E, seg=seg, a_rows=srt, a_row_div=top, glu_clamp=(1.702, 7.0), out_dtype=F32)
+    part = ops.glinear(act.to(BF), down, groups=E, seg=seg, o_rows=srt, row_scale=wt.view(-1), out_dtype=F32, out_rows_total=T * top)
+    scaled = ops.glinear(x, up, groups=E, seg=seg, a_rows=srt, a_row_div=top, in_scale=wt.view(-1), out_dtype=F32)
+    e, pair = idx.view(-1)[srt.long()].long(), srt.long()
+    z = torch.einsum("rk,rnk->rn", x.double()[pair // top], up.double()[e])
+    gt, u = z[:, 0::2].clamp_max(7.0), z[:, 1::2].clamp(-7.0, 7.0)
+    assert rel(act, gt * torch.sigmoid(1.702 * gt) * (u + 1)) < 4e-6
+    assert rel(scaled, z * wt.view(-1)[pair].double()[:, None]) < 2e-6
+    want = torch.empty(T * top, W, device="cuda", dtype=torch.float64)
+    want[pair] = torch.einsum("rk,rnk->rn", act.to(BF).double(), down.double()[e]) * wt.view(-1)[pair].double()[:, None]
+    assert rel(part, want) < 2e-6
+
+
+@pytest.mark.parametrize("M", [1, 20, 150])
+def test_glinear_batched(ops, M):
+    """per-head projections: column groups of A and of the output"""
+    g, H, K, N = gen(M), 6, 136, 128
+    a, w = randn(g, M, H * K), randn(g, H, N, K)
+    ref = torch.einsum("mhk,hnk->mhn", a.double().view(M, H, K), w.double()).reshape(M, H * N)
+    assert rel(ops.glinear(a, w, groups=H, a_group_off=K, o_group_off=N, out_dtype=F32), ref) < 2e-6

@@ -32,6 +32,7 @@ SOURCES = [
     "decode_mega.cu",
     "ragged_lm.cu",
     "glinear.cu",
+    "glinear_tcgen05.cu",
     "latent_attn.cu",
     "hgrn2.cu",
     "short_conv.cu",
@@ -39,7 +40,7 @@ SOURCES = [
     "ssm.cu",
     "outer_scan.cu",
 ]
-HEADERS = ["common.cuh", "kernels.h", "dtype_any.cuh", "../../include/vila_b200.h"]
+HEADERS = ["common.cuh", "kernels.h", "dtype_any.cuh", "glinear_epi.cuh", "../../include/vila_b200.h"]
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",

@@ -367,6 +367,8 @@ int vila_gated_norm_residual(float* x, const void* part, int part_dtype, int64_t
                                  bias_dtype, w, w_dtype, w_offset, eps, rows, cols, st(stream));
 }
 
+int vila_stalled_waits(void) { return static_cast<int>(vb::stalled_waits()); }
+
 int vila_glinear(const vila_glinear_params* p, void* stream) {
   VB_REQUIRE_DEVICE();
   return vb::glinear(*p, st(stream));

@@ -297,6 +297,10 @@ int rope_append(const vila_rope_append_params& p, cudaStream_t stream);
 int paged_attention(const vila_paged_attn_params& p, cudaStream_t stream);
 int sink_attention(const vila_sink_attn_params& p, cudaStream_t stream);
 int gather_rows(const void* src, const int32_t* rows, void* dst, int n_rows, int row_bytes, cudaStream_t stream);
+// bf16 operands on 16-byte boundaries with at least 128 weight rows: tcgen05 tiles (glinear_tcgen05.cu)
+bool glinear_tc_takes(const vila_glinear_params& p);
+unsigned int stalled_waits();
+int glinear_tc(const vila_glinear_params& p, cudaStream_t stream, const vila_glinear_ext& x);
 int glinear(const vila_glinear_params& p, cudaStream_t stream, const vila_glinear_ext* ext = nullptr);
 int latent_attention(const vila_latent_attn_params& p, cudaStream_t stream);
 int latent_rope_append(const vila_latent_rope_params& p, cudaStream_t stream);
