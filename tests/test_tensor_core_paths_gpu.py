@@ -1,6 +1,7 @@
 """Tensor-core forms of the token-id models' kernels at the sizes where they can go wrong (tile edges, remainders, the
-smallest and largest of their ranges), against float64 on the device.  Sums of bf16 products are exact per product and
-accumulated in fp32: the bound on fp32 results is a few fp32 roundings per accumulated partial, 2e-6 relative in norm."""
+smallest and largest of their ranges), against float64 on the device.  Products of bf16 numbers are exact, their sums are
+fp32: the tensor core truncates after every step of 16 products, at most 2^-23 of the running sum each time, and the
+truncations of a sum all go one way, half that much on average."""
 import pytest
 import torch
 
@@ -18,6 +19,11 @@ def rel(a, b):
     return float((a.double() - b).norm() / b.norm().clamp_min(1e-30))
 
 
+def acc(K):
+    """relative error of fp32 sums over K products that are truncated every 16, and of an epilogue's few roundings"""
+    return K / 16 * 2.0 ** -24 + 1e-6
+
+
 def gen(seed):
     return torch.Generator(device="cuda").manual_seed(seed)
 
@@ -27,13 +33,14 @@ def randn(g, *shape, dtype=BF):
 
 
 @pytest.mark.parametrize("M,N,K", [(1, 128, 8), (8, 1000, 512), (15, 129, 72), (16, 256, 64), (17, 384, 136), (64, 130, 2048),
-                                   (65, 257, 448), (128, 128, 200), (129, 640, 1000), (300, 1408, 2048)])
+                                   (65, 257, 448), (128, 128, 200), (129, 640, 1000), (257, 130, 64),
+                                   (300, 1408, 2048)])
 def test_glinear_plain(ops, M, N, K):
     g = gen(M * 7 + N)
     a, w, b = randn(g, M, K + 8)[:, :K], randn(g, N, K), randn(g, N)
     ref = a.double() @ w.double().T
-    assert rel(ops.glinear(a, w, out_dtype=F32), ref) < 2e-6
-    assert rel(ops.glinear(a, w, bias=b, act=ops.ACT_RELU2, out_dtype=F32), torch.relu(ref + b.double()) ** 2) < 4e-6
+    assert rel(ops.glinear(a, w, out_dtype=F32), ref) < acc(K)
+    assert rel(ops.glinear(a, w, bias=b, act=ops.ACT_RELU2, out_dtype=F32), torch.relu(ref + b.double()) ** 2) < 2 * acc(K)
     assert rel(ops.glinear(a, w), ref) < 2.0 ** -8
     if N % 2 == 0:
         z = ref / K ** 0.5
@@ -62,11 +69,11 @@ def test_glinear_routed(ops, T, E, top, W, ff, skew):
     e, pair = idx.view(-1)[srt.long()].long(), srt.long()
     z = torch.einsum("rk,rnk->rn", x.double()[pair // top], up.double()[e])
     gt, u = z[:, 0::2].clamp_max(7.0), z[:, 1::2].clamp(-7.0, 7.0)
-    assert rel(act, gt * torch.sigmoid(1.702 * gt) * (u + 1)) < 4e-6
-    assert rel(scaled, z * wt.view(-1)[pair].double()[:, None]) < 2e-6
+    assert rel(act, gt * torch.sigmoid(1.702 * gt) * (u + 1)) < 2 * acc(W)
+    assert rel(scaled, z * wt.view(-1)[pair].double()[:, None]) < acc(W)
     want = torch.empty(T * top, W, device="cuda", dtype=torch.float64)
     want[pair] = torch.einsum("rk,rnk->rn", act.to(BF).double(), down.double()[e]) * wt.view(-1)[pair].double()[:, None]
-    assert rel(part, want) < 2e-6
+    assert rel(part, want) < acc(ff)
 
 
 @pytest.mark.parametrize("M", [1, 20, 150])
@@ -75,4 +82,4 @@ def test_glinear_batched(ops, M):
     g, H, K, N = gen(M), 6, 136, 128
     a, w = randn(g, M, H * K), randn(g, H, N, K)
     ref = torch.einsum("mhk,hnk->mhn", a.double().view(M, H, K), w.double()).reshape(M, H * N)
-    assert rel(ops.glinear(a, w, groups=H, a_group_off=K, o_group_off=N, out_dtype=F32), ref) < 2e-6
+    assert rel(ops.glinear(a, w, groups=H, a_group_off=K, o_group_off=N, out_dtype=F32), ref) < acc(K)
