@@ -83,3 +83,40 @@ def test_glinear_batched(ops, M):
     a, w = randn(g, M, H * K), randn(g, H, N, K)
     ref = torch.einsum("mhk,hnk->mhn", a.double().view(M, H, K), w.double()).reshape(M, H * N)
     assert rel(ops.glinear(a, w, groups=H, a_group_off=K, o_group_off=N, out_dtype=F32), ref) < acc(K)
+
+
+@pytest.mark.parametrize("pairs,E", [(1, 1), (31, 5), (256, 32), (257, 7), (8192, 32), (8191, 300), (20000, 64), (600, 1500), (9000, 1100)])
+def test_moe_group_is_a_stable_sort(ops, pairs, E):
+    """expert segments in pair order; indices of no expert (identity choices) belong to no segment"""
+    g = gen(pairs)
+    idx = torch.randint(0, E + 3, (pairs,), generator=g, device="cuda", dtype=torch.int32)
+    seg, srt = ops.moe_group(idx, E)
+    want = [torch.nonzero(idx == e).view(-1) for e in range(E)]
+    assert seg.tolist() == [0] + torch.tensor([w.numel() for w in want]).cumsum(0).tolist()
+    assert torch.equal(srt[:int(seg[-1])].long(), torch.cat(want))
+
+
+@pytest.mark.parametrize("rows", [1, 256, 257, 1184, 1191])
+@pytest.mark.parametrize("cols", [256, 1030])
+def test_moe_route_forms_agree(ops, rows, cols):
+    """however many tokens and outputs a CTA takes, a token's choice and weights are the same bits"""
+    g = gen(rows)
+    x, w, c = randn(g, rows, cols), randn(g, 37, cols, dtype=F32) * cols ** -0.5, randn(g, 36, dtype=F32) * 0.05
+    kw = dict(score=ops.SCORE_SOFTMAX, groups=4, keep=2, group_top=2, scale=2.0, gate_w=w[36].contiguous())
+    idx, wt, gate = ops.moe_route_scores(x, w[:36].contiguous(), c, 5, **kw)
+    for r in sorted({0, rows // 2, rows - 1}):
+        one = ops.moe_route_scores(x[r:r + 1].contiguous(), w[:36].contiguous(), c, 5, **kw)
+        assert torch.equal(one[0][0], idx[r]) and torch.equal(one[1][0], wt[r]) and torch.equal(one[2][0], gate[r])
+
+
+@pytest.mark.parametrize("rows,cols,np_", [(1, 4, 1), (3, 1028, 2), (300, 2048, 4), (5, 136, 7)])
+@pytest.mark.parametrize("a_dt", [None, BF, F32])
+def test_residual_add_vec_equals_the_general_form(ops, rows, cols, np_, a_dt):
+    """four columns a thread against one: the same sums in the same order (the general form is forced by an odd stride)"""
+    g = gen(rows + np_)
+    x, part = randn(g, rows, cols, dtype=F32), randn(g, rows * np_, cols + 1, dtype=F32)[:, :cols]
+    a = None if a_dt is None else randn(g, rows, cols, dtype=a_dt)
+    y = x.clone()
+    c0 = ops.residual_add_rows(x, a, part, n_partials=np_, mult=0.5, copy_dtype=BF)
+    c1 = ops.residual_add_rows(y, a, part.contiguous(), n_partials=np_, mult=0.5, copy_dtype=BF)
+    assert torch.equal(x, y) and torch.equal(c0, c1)

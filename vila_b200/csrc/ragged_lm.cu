@@ -226,6 +226,99 @@ moe_group_kernel(const int32_t* __restrict__ idx, int32_t* __restrict__ seg, int
   }
 }
 
+// The same grouping with the pairs dealt to the warps instead of the experts: every pair is read twice in all, not once
+// per expert and pass.  A warp owns a run of consecutive pairs; the lanes of one expert find each other with a ballot per
+// bit of the index, so the ranks stay those of the pairs' order (__match_any_sync does the same in one instruction, but
+// its 512 uses were 10 of 16 us).  cnt_s [warps][experts]: first the counts, then the warp's next position.
+// 8192 pairs, 32 experts: 59 -> 12 us; the loop over experts is kept for few pairs (32: 1.9 against 5.1 us) and for
+// tables that do not fit shared memory.
+__global__ void __launch_bounds__(1024)
+moe_group_pairs_kernel(const int32_t* __restrict__ idx, int32_t* __restrict__ seg, int32_t* __restrict__ sorted,
+                       int pairs, int experts) {
+  extern __shared__ int cnt_s[];
+  __shared__ int carry_s[32];
+  const int wid = threadIdx.x >> 5, lane = lane_id(), nw = blockDim.x >> 5;
+  const int per = (pairs + 32 * nw - 1) / (32 * nw) * 32, p_begin = wid * per, p_end = min(pairs, p_begin + per);
+  for (int i = threadIdx.x; i < nw * experts; i += blockDim.x) cnt_s[i] = 0;
+  __syncthreads();
+  int* mine = cnt_s + wid * experts;
+  const int bits = 32 - __clz(experts);
+  auto peers = [&](int e) {                           // lanes with the same e in -1 .. experts - 1
+    unsigned m = 0xffffffffu;
+    for (int b = 0; b < bits; ++b) {
+      const bool on = ((e + 1) >> b) & 1;
+      const unsigned v = __ballot_sync(0xffffffffu, on);
+      m &= on ? v : ~v;
+    }
+    return m;
+  };
+  constexpr int kBatch = 8;                           // steps whose indices are in flight together
+  int ev[kBatch];
+  auto fetch = [&](int p0) {
+#pragma unroll
+    for (int j = 0; j < kBatch; ++j) {
+      const int p = p0 + 32 * j + lane, e = p < p_end ? idx[p] : -1;
+      ev[j] = e >= 0 && e < experts ? e : -1;         // -1: belongs to no expert
+    }
+  };
+  for (int p0 = p_begin; p0 < p_end; p0 += 32 * kBatch) {
+    fetch(p0);
+#pragma unroll
+    for (int j = 0; j < kBatch; ++j) {
+      const unsigned m = peers(ev[j]);
+      if (ev[j] >= 0 && lane == __ffs(m) - 1) mine[ev[j]] += __popc(m);
+      __syncwarp();
+    }
+  }
+  __syncthreads();
+  // exclusive prefix over (expert, warp): a thread per expert, then over the threads of the CTA
+  int at = 0;
+  for (int e0 = 0; e0 < experts; e0 += blockDim.x) {
+    const int e = e0 + threadIdx.x;
+    int n = 0;
+    if (e < experts)
+      for (int w = 0; w < nw; ++w) n += cnt_s[w * experts + e];
+    int end = n;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int v = __shfl_up_sync(0xffffffffu, end, o);
+      if (lane >= o) end += v;
+    }
+    if (lane == 31) carry_s[wid] = end;
+    __syncthreads();
+    int before = at, all = 0;
+    for (int w = 0; w < nw; ++w) {
+      if (w < wid) before += carry_s[w];
+      all += carry_s[w];
+    }
+    if (e < experts) {
+      int pos = before + end - n;
+      seg[e] = pos;
+      for (int w = 0; w < nw; ++w) {
+        const int c = cnt_s[w * experts + e];
+        cnt_s[w * experts + e] = pos;
+        pos += c;
+      }
+      if (e == experts - 1) seg[experts] = pos;
+    }
+    at += all;
+    __syncthreads();
+  }
+  for (int p0 = p_begin; p0 < p_end; p0 += 32 * kBatch) {
+    if (per > 32 * kBatch) fetch(p0);                 // otherwise they are still there
+#pragma unroll
+    for (int j = 0; j < kBatch; ++j) {
+      const int e = ev[j];
+      const unsigned m = peers(e);
+      const int pos = e >= 0 ? mine[e] : 0;
+      __syncwarp();
+      if (e >= 0) sorted[pos + __popc(m & ((1u << lane) - 1u))] = p0 + 32 * j + lane;
+      if (e >= 0 && lane == __ffs(m) - 1) mine[e] = pos + __popc(m);
+      __syncwarp();
+    }
+  }
+}
+
 inline int row_grid(int rows) { return (rows + kRowsPerCta - 1) / kRowsPerCta; }
 
 // ---- word row + hashed (previous, current) pair row ------------------------------------------------
@@ -268,6 +361,37 @@ residual_add_rows_kernel(float* __restrict__ x, const void* __restrict__ a, int 
     const float v = x[i] + mult * y;
     x[i] = v;
     if (copy) st_any(copy, c_dt, i, v);
+  }
+}
+
+// The same for rows of four-element pieces whose partials are fp32: the loads of a piece are in flight together (the
+// branches on dtypes kept them apart: 24.5 us for 2048 x 2048 and four partials, now 13.2).  A: 0 no a, 1 bf16, 2 fp32.
+template <int A>
+__global__ void __launch_bounds__(kRowThreads)
+residual_add_vec_kernel(float* __restrict__ x, const void* __restrict__ a, int64_t lda, const float* __restrict__ part,
+                        int64_t ldp, int np, float mult, void* __restrict__ copy, int c_dt, int cols) {
+  const size_t r = blockIdx.y;
+  const int c = 4 * (blockIdx.x * kRowThreads + threadIdx.x);
+  if (c >= cols) return;
+  const float4 v = *reinterpret_cast<const float4*>(x + r * cols + c);
+  float4 y = make_float4(0.f, 0.f, 0.f, 0.f);
+  if (A == 1) {
+    const uint2 u = __ldg(reinterpret_cast<const uint2*>(static_cast<const __nv_bfloat16*>(a) + r * lda + c));
+    y = make_float4(bf_lo(u.x), bf_hi(u.x), bf_lo(u.y), bf_hi(u.y));
+  } else if (A == 2) {
+    y = __ldg(reinterpret_cast<const float4*>(static_cast<const float*>(a) + r * lda + c));
+  }
+  const float* pr = part + r * np * ldp + c;
+#pragma unroll 4
+  for (int j = 0; j < np; ++j) {
+    const float4 q = __ldg(reinterpret_cast<const float4*>(pr + j * ldp));
+    y.x += q.x; y.y += q.y; y.z += q.z; y.w += q.w;
+  }
+  const float o[4] = {v.x + mult * y.x, v.y + mult * y.y, v.z + mult * y.z, v.w + mult * y.w};
+  *reinterpret_cast<float4*>(x + r * cols + c) = make_float4(o[0], o[1], o[2], o[3]);
+  if (copy) {
+#pragma unroll
+    for (int e = 0; e < 4; ++e) st_any(copy, c_dt, r * cols + c + e, o[e]);
   }
 }
 
@@ -318,10 +442,13 @@ __device__ __forceinline__ void st4_any(void* p, int dt, size_t i, float4 v) {
   *reinterpret_cast<uint2*>(static_cast<__nv_bfloat16*>(p) + i) = u;
 }
 
-// A CTA takes NT tokens; its warps split the outputs, four at a time and for all the tokens (every weight is read once per
+// A CTA takes NT tokens; its warps split the outputs, NU at a time and for all the tokens (every weight is read once per
 // CTA, the dot products overlap); the shared expert's gate, if there is one, is the output after the last.  Then a warp
-// per token chooses.  A token's sums run in the same order whatever NT is.
-template <int NT, int THREADS, bool VEC>
+// per token chooses.  A token's sums run in the same order whatever NT and NU are.
+// The dtype of x is a template parameter: a branch around every load kept the loads of a step from being in flight
+// together (2048 x 2048, 32 experts: 41.8 -> 28 us; 8 tokens, where a warp also takes one output and has eight of its
+// pieces in flight: 20.5 -> 11.5 us).  Eight tokens per CTA are no faster than four.
+template <int NT, int NU, int THREADS, bool VEC, bool F32>
 __global__ void __launch_bounds__(THREADS) moe_route_scores_kernel(const vila_moe_route_params p) {
   extern __shared__ float z_s[];  // per token: s [experts] | c [experts] | group score [groups]
   const int wid = threadIdx.x >> 5, lane = lane_id(), row0 = blockIdx.x * NT;
@@ -330,27 +457,37 @@ __global__ void __launch_bounds__(THREADS) moe_route_scores_kernel(const vila_mo
   size_t xb[NT];
 #pragma unroll
   for (int t = 0; t < NT; ++t) xb[t] = static_cast<size_t>(min(row0 + t, p.rows - 1)) * p.ldx;
-  for (int e0 = 4 * wid; e0 < outs; e0 += 4 * (THREADS / 32)) {
-    const float* we[4];
-    float a[NT][4];
+  for (int e0 = NU * wid; e0 < outs; e0 += NU * (THREADS / 32)) {
+    const float* we[NU];
+    float a[NT][NU];
 #pragma unroll
-    for (int u = 0; u < 4; ++u) {
+    for (int u = 0; u < NU; ++u) {
       const int e = min(e0 + u, outs - 1);
       we[u] = e < experts ? p.w + static_cast<size_t>(e) * cols : p.gate_w;
 #pragma unroll
       for (int t = 0; t < NT; ++t) a[t][u] = 0.f;
     }
     if (VEC) {
-#pragma unroll 2
+#pragma unroll (NU == 1 ? 8 : 2)
       for (int k = 4 * lane; k < cols; k += 128) {
-        float4 wv[4];
+        float4 wv[NU];
+        uint4 xr[NT];   // raw bits: the loads of all tokens are in flight before the first is converted
 #pragma unroll
-        for (int u = 0; u < 4; ++u) wv[u] = __ldg(reinterpret_cast<const float4*>(we[u] + k));
+        for (int u = 0; u < NU; ++u) wv[u] = __ldg(reinterpret_cast<const float4*>(we[u] + k));
 #pragma unroll
         for (int t = 0; t < NT; ++t) {
-          const float4 xv = ld4_any(p.x, p.x_dtype, xb[t] + k);
+          if (F32) {
+            xr[t] = __ldg(reinterpret_cast<const uint4*>(static_cast<const float*>(p.x) + xb[t] + k));
+          } else {
+            const uint2 h = __ldg(reinterpret_cast<const uint2*>(static_cast<const __nv_bfloat16*>(p.x) + xb[t] + k));
+            xr[t] = make_uint4(h.x << 16, h.x & 0xffff0000u, h.y << 16, h.y & 0xffff0000u);
+          }
+        }
 #pragma unroll
-          for (int u = 0; u < 4; ++u) {
+        for (int t = 0; t < NT; ++t) {
+          const float4 xv = make_float4(__uint_as_float(xr[t].x), __uint_as_float(xr[t].y), __uint_as_float(xr[t].z), __uint_as_float(xr[t].w));
+#pragma unroll
+          for (int u = 0; u < NU; ++u) {
             a[t][u] = fmaf(xv.x, wv[u].x, a[t][u]); a[t][u] = fmaf(xv.y, wv[u].y, a[t][u]);
             a[t][u] = fmaf(xv.z, wv[u].z, a[t][u]); a[t][u] = fmaf(xv.w, wv[u].w, a[t][u]);
           }
@@ -362,7 +499,7 @@ __global__ void __launch_bounds__(THREADS) moe_route_scores_kernel(const vila_mo
         for (int t = 0; t < NT; ++t) {
           const float xv = ld_any(p.x, p.x_dtype, xb[t] + k);
 #pragma unroll
-          for (int u = 0; u < 4; ++u) a[t][u] = fmaf(xv, we[u][k], a[t][u]);
+          for (int u = 0; u < NU; ++u) a[t][u] = fmaf(xv, we[u][k], a[t][u]);
         }
       }
     }
@@ -371,12 +508,12 @@ __global__ void __launch_bounds__(THREADS) moe_route_scores_kernel(const vila_mo
 #pragma unroll
       for (int t = 0; t < NT; ++t)
 #pragma unroll
-        for (int u = 0; u < 4; ++u) a[t][u] += __shfl_xor_sync(0xffffffffu, a[t][u], o);
+        for (int u = 0; u < NU; ++u) a[t][u] += __shfl_xor_sync(0xffffffffu, a[t][u], o);
     if (lane == 0) {
 #pragma unroll
       for (int t = 0; t < NT; ++t)
 #pragma unroll
-        for (int u = 0; u < 4; ++u) {
+        for (int u = 0; u < NU; ++u) {
           const int e = e0 + u;
           if (e < experts) z_s[t * per_tok + e] = a[t][u];
           else if (e < outs && row0 + t < p.rows) p.gate[row0 + t] = sigmoid_f(a[t][u]);
@@ -874,6 +1011,17 @@ int residual_add_rows(float* x, const void* a, int a_dt, int64_t lda, const void
                       int np, float mult, void* copy, int c_dt, int rows, int cols, cudaStream_t stream) {
   if (rows <= 0 || cols <= 0) return 0;
   VB_CHECK(part == nullptr || np >= 1, "residual_add_rows: n_partials=%d", np);
+  if (part != nullptr && p_dt == VILA_DT_F32 && cols % 4 == 0 && rows <= 65535 && aligned_to(x, 16) && rows4(part, ldp, p_dt) &&
+      (a == nullptr || rows4(a, lda, a_dt))) {
+    const dim3 grid((cols / 4 + kRowThreads - 1) / kRowThreads, rows);
+    const float* fp = static_cast<const float*>(part);
+#define VB_RES(A) VB_CUDA(launch_serial(residual_add_vec_kernel<A>, grid, dim3(kRowThreads), 0, stream, x, a, lda, fp, ldp, np, mult, copy, c_dt, cols))
+    if (a == nullptr) VB_RES(0);
+    else if (a_dt == VILA_DT_BF16) VB_RES(1);
+    else VB_RES(2);
+#undef VB_RES
+    return 0;
+  }
   VB_CUDA(launch_serial(residual_add_rows_kernel, dim3(flat_grid(static_cast<size_t>(rows) * cols)),
                         dim3(kRowThreads), 0, stream, x, a, a_dt, lda, part, p_dt, ldp, np, mult, copy, c_dt, rows, cols));
   return 0;
@@ -897,16 +1045,19 @@ int moe_route_scores(const vila_moe_route_params& p, cudaStream_t stream) {
            "moe_route_scores: score=%d group_top=%d", p.score, p.group_top);
   const size_t per_tok = sizeof(float) * (2 * p.experts + p.groups);
   const bool vec = p.cols % 4 == 0 && rows4(p.x, p.ldx, p.x_dtype) && aligned_to(p.w, 16) && (!p.gate_w || aligned_to(p.gate_w, 16));
-#define VB_ROUTE(NT, TH, VEC)                                                                                       \
-  VB_CUDA(launch_serial(moe_route_scores_kernel<NT, TH, VEC>, dim3((p.rows + NT - 1) / NT), dim3(TH), NT * per_tok, \
-                        stream, p))
-  if (p.rows <= 256 || 4 * per_tok > 48 * 1024) {   // few tokens (or very many experts): one per CTA of 32 warps
-    if (vec) VB_ROUTE(1, 1024, true);
-    else VB_ROUTE(1, 1024, false);
-  } else {
-    if (vec) VB_ROUTE(4, 256, true);
-    else VB_ROUTE(4, 256, false);
-  }
+#define VB_ROUTE_K(NT, NU, TH, VEC, F32)                                                                                \
+  VB_CUDA(launch_serial(moe_route_scores_kernel<NT, NU, TH, VEC, F32>, dim3((p.rows + NT - 1) / NT), dim3(TH),          \
+                        NT * per_tok, stream, p))
+#define VB_ROUTE(NT, NU, TH)                                                                                            \
+  do {                                                                                                                  \
+    if (!vec) VB_ROUTE_K(NT, NU, TH, false, false);                                                                     \
+    else if (p.x_dtype == VILA_DT_F32) VB_ROUTE_K(NT, NU, TH, true, true);                                              \
+    else VB_ROUTE_K(NT, NU, TH, true, false);                                                                           \
+  } while (0)
+  // Few tokens (or very many experts): one per CTA of 32 warps, otherwise four
+  if (p.rows <= 256 || 4 * per_tok > 48 * 1024) VB_ROUTE(1, 1, 1024);
+  else VB_ROUTE(4, 4, 256);
+#undef VB_ROUTE_K
 #undef VB_ROUTE
   return 0;
 }
@@ -914,8 +1065,13 @@ int moe_route_scores(const vila_moe_route_params& p, cudaStream_t stream) {
 int moe_group(const int32_t* idx, int32_t* seg, int32_t* sorted, int pairs, int experts,
               cudaStream_t stream) {
   VB_CHECK(experts >= 1 && experts <= 8192 && pairs >= 0, "moe_group: experts=%d pairs=%d", experts, pairs);
-  VB_CUDA(launch_serial(moe_group_kernel, dim3(1), dim3(1024), sizeof(int) * (experts + 1), stream, idx, seg,
-                     sorted, pairs, experts));
+  const int warps = pairs >= 32 * 256 ? 32 : (pairs + 255) / 256;   // a warp per 256 pairs up to 32
+  const size_t table = sizeof(int) * static_cast<size_t>(warps) * experts;
+  if (warps > 1 && table <= 32 * 1024)
+    VB_CUDA(launch_serial(moe_group_pairs_kernel, dim3(1), dim3(32 * warps), table, stream, idx, seg, sorted, pairs, experts));
+  else
+    VB_CUDA(launch_serial(moe_group_kernel, dim3(1), dim3(1024), sizeof(int) * (experts + 1), stream, idx, seg,
+                       sorted, pairs, experts));
   return 0;
 }
 
