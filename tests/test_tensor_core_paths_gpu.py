@@ -120,3 +120,104 @@ def test_residual_add_vec_equals_the_general_form(ops, rows, cols, np_, a_dt):
     c0 = ops.residual_add_rows(x, a, part, n_partials=np_, mult=0.5, copy_dtype=BF)
     c1 = ops.residual_add_rows(y, a, part.contiguous(), n_partials=np_, mult=0.5, copy_dtype=BF)
     assert torch.equal(x, y) and torch.equal(c0, c1)
+
+
+# ---- paged attention of prompt portions ---------------------------------------------------------------------
+ATT_FORMS = {"plain": {}, "capped": dict(softcap=5.0, gate=True), "sink": dict(sink=True, head_scale=True), "window": dict(window=21, keep_first=3),
+             "narrow": dict(window=5, gate=True), "chunk": dict(chunk=24, dist_bias=30, sink=True, gate=True),
+             "diff": dict(diff=(0.4, 0.6, 1e-5), window=37, gate=True), "diff_plain": dict(diff=(0.3, 0.7, 1e-5))}
+
+
+def attention_reference(q, pool, tables, seqs, H, G, D, V, page, scale, o):
+    """float64, row by row of positions; seqs: (row0, rows, pos0, slot)"""
+    maps = 2 if "diff" in o else 1
+    out = torch.empty(q.shape[0], H, V, device="cuda", dtype=torch.float64)
+    for row0, n, pos0, slot in seqs:
+        j = torch.arange(pos0 + n, device="cuda")
+        rows = tables[slot, j // page].long() * page + j % page
+        k, v = pool[rows, :G * maps * D].double().view(-1, G, maps, D), pool[rows, G * maps * D:].double().view(-1, G, V)
+        i = pos0 + torch.arange(n, device="cuda")
+        back = i[:, None] - j[None]
+        see = back >= 0
+        if "window" in o:
+            see &= (back < o["window"]) | (j[None] < o.get("keep_first", 0))
+        if "chunk" in o:
+            see &= j[None] >= (i[:, None] // o["chunk"]) * o["chunk"]
+        s = torch.einsum("ihmd,jhmd->hmij", q[row0:row0 + n].double().view(n, H, maps, D), k.repeat_interleave(H // G, 1)) * scale
+        if "head_scale" in o:
+            s = s * o["head_scale"].double()[:, None, None, None]
+        if "softcap" in o:
+            s = o["softcap"] * torch.tanh(s / o["softcap"])
+        if "talk" in o and not o.get("talk_after"):
+            s = torch.einsum("hg,gmij->hmij", o["talk"].double(), s)
+        if "dist_bias" in o:
+            s = s + o["dist_bias"].double()[back.clamp(0, o["dist_bias"].shape[0] - 1)].permute(2, 0, 1)[:, None]
+        s = s.masked_fill(~see, float("-inf"))
+        if "sink" in o:
+            s = torch.cat([s, o["sink"].double()[:, None, None, None].expand(H, maps, n, 1)], -1)
+        w = torch.softmax(s, -1)[..., :pos0 + n]
+        if o.get("talk_after"):
+            w = torch.einsum("hg,gmij->hmij", o["talk"].double(), w)
+        a = torch.einsum("hmij,jhd->ihmd", w, v.repeat_interleave(H // G, 1))
+        if maps == 2:
+            lam, sc, eps = o["diff"]
+            a = a[:, :, 0] - lam * a[:, :, 1]
+            a = a / torch.sqrt(a.pow(2).mean(-1, keepdim=True) + eps) * sc
+        else:
+            a = a[:, :, 0]
+        if "gate" in o:
+            a = a * torch.sigmoid(o["gate"][row0:row0 + n].double())[..., None]
+        out[row0:row0 + n] = a
+    return out.view(q.shape[0], -1)
+
+
+def attention_case(ops, form, H, G, D, V, page, seqs, seed, q_scale=1.0, scale=0.1, **call):
+    g, o = gen(seed), dict(form)
+    maps = 2 if "diff" in o else 1
+    T, slots = sum(n for n, _ in seqs), len(seqs)
+    pages = max((p + n + page - 1) // page for n, p in seqs)
+    pool = randn(g, slots * pages * page, G * (maps * D + V))
+    tables = torch.randperm(slots * pages, generator=g, device="cuda").to(torch.int32).view(slots, pages)
+    q = torch.randn(T, H * maps * D, generator=g, device="cuda") * q_scale
+    for k, shape in (("gate", (T, H)), ("sink", (H,)), ("head_scale", (H,))):
+        if o.get(k) is True:
+            o[k] = torch.randn(shape, generator=g, device="cuda") * 0.5 + (1.0 if k == "head_scale" else 0.0)
+    if isinstance(o.get("dist_bias"), int):
+        o["dist_bias"] = torch.randn(o["dist_bias"], H, generator=g, device="cuda")
+    if o.get("talk") is True:
+        o["talk"] = torch.eye(H, device="cuda") + 0.3 * torch.randn(H, H, generator=g, device="cuda")
+    at, spans = 0, []
+    for s, (n, p) in enumerate(seqs):
+        spans.append((at, n, p, s))
+        at += n
+    step = call.get("max_rows", 16)
+    tiles = torch.tensor([(r + i, min(step, n - i), p + i, s) for r, n, p, s in spans for i in range(0, n, step)], dtype=torch.int32, device="cuda")
+    call.setdefault("max_rows", 16)
+    got = ops.paged_attention(q, pool, tables, tiles, heads=H, kv_heads=G, dim=D, vdim=V, page=page, scale=scale, out_dtype=F32, **call, **o)
+    return got, attention_reference(q, pool, tables, spans, H, G, D, V, page, scale, o), (q, pool, tables, tiles, o)
+
+
+@pytest.mark.parametrize("form", list(ATT_FORMS))
+@pytest.mark.parametrize("rep", [1, 2, 3, 4])
+@pytest.mark.parametrize("seqs", [[(2, 0)], [(16, 0), (17, 63), (3, 128)], [(200, 0)], [(33, 300), (64, 1)]])
+def test_paged_attention_prompt(ops, form, rep, seqs):
+    """fp32 results of bf16 caches: a score sums 128 products of three parts, a row up to 333 weights; 3e-6 of the norm.
+    Capped, biased and masked forms, tiles of 1 to 16 rows, several sequences in one launch, page sizes 16 and 64."""
+    o = ATT_FORMS[form]
+    D, V = (64, 128) if "diff" in o else (128, 128)
+    got, want, _ = attention_case(ops, o, 2 * rep, 2, D, V, 16 if rep % 2 else 64, seqs, seed=rep)
+    assert rel(got, want) < 3e-6
+    if form == "plain":
+        got, want, _ = attention_case(ops, o, 2 * rep, 2, 64, 64, 48, seqs, seed=rep)
+        assert rel(got, want) < 3e-6
+
+
+def test_paged_attention_prompt_extremes(ops):
+    """large scores (one key takes a row), and a row whose result does not depend on what else is in the launch"""
+    got, want, (q, pool, tables, tiles, o) = attention_case(ops, {}, 8, 2, 128, 128, 64, [(40, 90), (25, 0)], seed=5, q_scale=30.0, scale=1.0)
+    assert torch.isfinite(got).all() and rel(got, want) < 1e-4   # scores of several hundred: their last bits are 3e-5 of a weight
+    kw = dict(heads=8, kv_heads=2, dim=128, vdim=128, page=64, scale=1.0, out_dtype=F32, max_rows=16)
+    alone = ops.paged_attention(q, pool, tables, tiles[1:2].contiguous(), **kw)
+    assert torch.equal(alone[16:32], got[16:32])
+    q[3, 7] = float("nan")
+    assert torch.isnan(ops.paged_attention(q, pool, tables, tiles, **kw)[3, :128]).all()

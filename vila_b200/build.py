@@ -37,10 +37,11 @@ SOURCES = [
     "hgrn2.cu",
     "short_conv.cu",
     "paged_attn.cu",
+    "paged_attn_mma.cu",
     "ssm.cu",
     "outer_scan.cu",
 ]
-HEADERS = ["common.cuh", "kernels.h", "dtype_any.cuh", "glinear_epi.cuh", "../../include/vila_b200.h"]
+HEADERS = ["common.cuh", "kernels.h", "dtype_any.cuh", "glinear_epi.cuh", "paged_attn_common.cuh", "../../include/vila_b200.h"]
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",

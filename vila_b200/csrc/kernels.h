@@ -294,6 +294,9 @@ int ssd_scan(const vila_ssd_scan_params& p, cudaStream_t stream);
 int selective_scan(const vila_selective_scan_params& p, cudaStream_t stream);
 int norm_conv_rows(const vila_norm_conv_params& p, cudaStream_t stream);
 int rope_append(const vila_rope_append_params& p, cudaStream_t stream);
+// prompt portions over a bf16 pool, head sizes 64 / 128, heads not mixed: tensor cores (paged_attn_mma.cu)
+bool paged_attention_mma_takes(const vila_paged_attn_params& p);
+int paged_attention_mma(const vila_paged_attn_params& p, cudaStream_t stream);
 int paged_attention(const vila_paged_attn_params& p, cudaStream_t stream);
 int sink_attention(const vila_sink_attn_params& p, cudaStream_t stream);
 int gather_rows(const void* src, const int32_t* rows, void* dst, int n_rows, int row_bytes, cudaStream_t stream);

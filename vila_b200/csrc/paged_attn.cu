@@ -36,13 +36,13 @@
 #include "common.cuh"
 #include "kernels.h"
 #include "dtype_any.cuh"
+#include "paged_attn_common.cuh"
 
 namespace vb {
 namespace {
 
 constexpr int kThreads = 256;
 constexpr int kWarps = kThreads / 32;
-constexpr float kNegBig = -1e30f;
 
 __host__ __device__ __forceinline__ int round4(int r) { return (r + 3) & ~3; }
 // Floats between the K rows of consecutive keys in shared memory: all G heads of a key (G * DS, DS = D4 + 4)
@@ -50,7 +50,6 @@ __host__ __device__ __forceinline__ int round4(int r) { return (r + 3) & ~3; }
 // column) fall into 8 different bank groups.
 __host__ __device__ __forceinline__ int key_stride(int G, int DS) { return G * DS + ((36 - (G * DS) % 32) % 32); }
 
-__host__ __device__ __forceinline__ int maps_of(int maps) { return maps > 1 ? maps : 1; }
 
 // ---- rotary + unit norm + append ---------------------------------------------------------------------
 // One CTA per token; warp w takes the heads w, w + 8, ... of q then k; v is copied by all threads.
@@ -129,54 +128,6 @@ struct AttnShape {
                // leaves every CTA's running (max, sum) in its partial record, 1 = this launch merges those records and
                // adds its share of the values; -1 = one CTA does both passes itself
 };
-
-__device__ __forceinline__ size_t pool_row(const int32_t* pt, int page, int j) {
-  return static_cast<size_t>(pt[j / page]) * page + (j % page);
-}
-
-// first key a query at position pos can see
-__device__ __forceinline__ int first_key(const vila_paged_attn_params& p, int pos) {
-  return p.chunk > 0 ? (pos / p.chunk) * p.chunk : 0;
-}
-// may the query at position pos see key j?
-__device__ __forceinline__ bool sees(const vila_paged_attn_params& p, int pos, int j) {
-  return j <= pos && j >= first_key(p, pos) && (p.window <= 0 || pos - j < p.window || j < p.keep_first);
-}
-// Key blocks of BK keys a tile visits, in order: [0, kb) then [wb, nblocks).
-struct BlockList {
-  int kb, wb, count;
-  __device__ __forceinline__ int block(int v) const { return v < kb ? v : wb + (v - kb); }
-};
-__device__ __forceinline__ BlockList visible_blocks(const vila_paged_attn_params& p, int pos0, int nkeys, int BK) {
-  BlockList b;
-  const int nblocks = (nkeys + BK - 1) / BK;
-  if (p.window <= 0) {
-    b.kb = 0;
-    b.wb = first_key(p, pos0) / BK;
-  } else {
-    b.kb = min((min(p.keep_first, nkeys) + BK - 1) / BK, nblocks);
-    b.wb = max(b.kb, max(max(pos0 - p.window + 1, 0), first_key(p, pos0)) / BK);
-  }
-  b.count = b.kb + max(nblocks - b.wb, 0);
-  return b;
-}
-__device__ __forceinline__ float head_scale(const vila_paged_attn_params& p, int h) {
-  return p.head_scale ? p.scale * p.head_scale[h] : p.scale;
-}
-// a head's own scaled score, bounded to (-softcap, softcap) when a cap is set
-__device__ __forceinline__ float capped(const vila_paged_attn_params& p, float s) {
-  return p.softcap > 0.f ? p.softcap * tanhf(s / p.softcap) : s;
-}
-__device__ __forceinline__ float dist_bias(const vila_paged_attn_params& p, int dist, int h) {
-  return __ldg(p.dist_bias + static_cast<size_t>(min(dist, p.dist_rows - 1)) * p.H + h);
-}
-// Score head h counts the maps singly: model head h / maps, map h % maps.  Its key head (also counted with maps) and
-// value head; rep = query heads per key / value head.
-__device__ __forceinline__ int key_head(int h, int maps, int rep) { return maps == 1 ? h / rep : ((h >> 1) / rep) * 2 + (h & 1); }
-__device__ __forceinline__ int value_head(int h, int maps, int rep) { return maps == 1 ? h / rep : (h >> 1) / rep; }
-__device__ __forceinline__ float out_gate(const vila_paged_attn_params& p, int row, int h) {
-  return p.gate ? sigmoid_f(ld_any(p.gate, p.gate_dtype, static_cast<size_t>(row) * p.ldg + h)) : 1.0f;
-}
 
 // K | V rows of a key block, widened to fp32.  16-byte loads when the head sizes allow (bf16: multiples of 8, fp32:
 // multiples of 4; the pool row is then 16-byte aligned as well): the block's pieces are dealt to all threads (a warp per
@@ -901,6 +852,7 @@ int paged_attention(const vila_paged_attn_params& p, cudaStream_t stream) {
            "paged_attention: maps=%d (two maps per head take no head mixing, sink, distance bias or head scale)", p.maps);
   VB_CHECK(p.max_rows >= 1 && p.max_rows <= 16 && (p.nsplit == 1 || p.max_rows == 1),
            "paged_attention: max_rows=%d nsplit=%d (key splitting serves one-row tiles)", p.max_rows, p.nsplit);
+  if (paged_attention_mma_takes(p)) return paged_attention_mma(p, stream);
   AttnShape sh;
   sh.phase = -1;
   // Without head mixing the K/V-head groups are independent: a CTA then serves ONE K/V head and its query heads, holds

@@ -1,0 +1,61 @@
+// Masks, block lists and score options of vila_paged_attention, shared by its CUDA-core and its tensor-core kernels.
+#pragma once
+#include "../../include/vila_b200.h"
+#include "common.cuh"
+#include "dtype_any.cuh"
+
+namespace vb {
+
+constexpr float kNegBig = -1e30f;
+
+__host__ __device__ __forceinline__ int maps_of(int maps) { return maps > 1 ? maps : 1; }
+
+__device__ __forceinline__ size_t pool_row(const int32_t* pt, int page, int j) {
+  return static_cast<size_t>(pt[j / page]) * page + (j % page);
+}
+
+// first key a query at position pos can see
+__device__ __forceinline__ int first_key(const vila_paged_attn_params& p, int pos) {
+  return p.chunk > 0 ? (pos / p.chunk) * p.chunk : 0;
+}
+// may the query at position pos see key j?
+__device__ __forceinline__ bool sees(const vila_paged_attn_params& p, int pos, int j) {
+  return j <= pos && j >= first_key(p, pos) && (p.window <= 0 || pos - j < p.window || j < p.keep_first);
+}
+// Key blocks of BK keys a tile visits, in order: [0, kb) then [wb, nblocks).
+struct BlockList {
+  int kb, wb, count;
+  __device__ __forceinline__ int block(int v) const { return v < kb ? v : wb + (v - kb); }
+};
+__device__ __forceinline__ BlockList visible_blocks(const vila_paged_attn_params& p, int pos0, int nkeys, int BK) {
+  BlockList b;
+  const int nblocks = (nkeys + BK - 1) / BK;
+  if (p.window <= 0) {
+    b.kb = 0;
+    b.wb = first_key(p, pos0) / BK;
+  } else {
+    b.kb = min((min(p.keep_first, nkeys) + BK - 1) / BK, nblocks);
+    b.wb = max(b.kb, max(max(pos0 - p.window + 1, 0), first_key(p, pos0)) / BK);
+  }
+  b.count = b.kb + max(nblocks - b.wb, 0);
+  return b;
+}
+__device__ __forceinline__ float head_scale(const vila_paged_attn_params& p, int h) {
+  return p.head_scale ? p.scale * p.head_scale[h] : p.scale;
+}
+// a head's own scaled score, bounded to (-softcap, softcap) when a cap is set
+__device__ __forceinline__ float capped(const vila_paged_attn_params& p, float s) {
+  return p.softcap > 0.f ? p.softcap * tanhf(s / p.softcap) : s;
+}
+__device__ __forceinline__ float dist_bias(const vila_paged_attn_params& p, int dist, int h) {
+  return __ldg(p.dist_bias + static_cast<size_t>(min(dist, p.dist_rows - 1)) * p.H + h);
+}
+// Score head h counts the maps singly: model head h / maps, map h % maps.  Its key head (also counted with maps) and
+// value head; rep = query heads per key / value head.
+__device__ __forceinline__ int key_head(int h, int maps, int rep) { return maps == 1 ? h / rep : ((h >> 1) / rep) * 2 + (h & 1); }
+__device__ __forceinline__ int value_head(int h, int maps, int rep) { return maps == 1 ? h / rep : (h >> 1) / rep; }
+__device__ __forceinline__ float out_gate(const vila_paged_attn_params& p, int row, int h) {
+  return p.gate ? sigmoid_f(ld_any(p.gate, p.gate_dtype, static_cast<size_t>(row) * p.ldg + h)) : 1.0f;
+}
+
+}  // namespace vb
