@@ -4,14 +4,19 @@
 // three bf16 parts (8 + 8 + 8 bits) whose products with a bf16 number are exact, and the three products are summed
 // in fp32.  Three bf16 products are cheaper than two tf32 ones and need no range assumptions.
 //
-// A warp owns 16 rows of one sequence x one score head (mma.sync m16n8k16: rows x 8 keys, then rows x 8 value columns),
-// its queries' parts in registers (96 of them at 128 columns) for the whole key loop, scores and sums never leave
-// registers.  A CTA serves one key / value head: the score heads that share it x as many consecutive 16-row tiles as make
-// four warps.  Blocks of 64 keys come by cp.async into a double buffer of 16-byte pieces swizzled over 8 rows (the
-// ldmatrix reads of 8 keys fall into different banks).  CTAs of late positions, which see most keys, start first.
+// A warp owns 16 rows of one sequence x one score head (mma.sync m16n8k16: rows x 8 keys, then rows x 8 value columns);
+// scores and sums never leave its registers, the queries' parts lie in shared memory in fragment order.  A CTA serves
+// one key / value head: the score heads that share it x as many consecutive 16-row tiles as make four warps, twice: one
+// set of warps takes the even blocks of 64 keys, the other the odd ones (by position, so that a row's sums do not depend
+// on its tile), and the two are merged at the end.  The sets run freely against each other, one's softmax under the
+// other's products, and the longest chain of blocks is half as long.  Blocks come by cp.async into double buffers of
+// 16-byte pieces swizzled over 8 rows (the ldmatrix reads of 8 keys fall into different banks).  CTAs of late
+// positions, which see most keys, start first.
 //
-// Bound by the tensor pipe: six products where bf16 attention issues two.  Tiled on the CUDA cores the same
-// attention ran at 10 TFLOP/s (two shared-memory reads per 16 multiply-adds): MEASURED_ATTN.
+// Bound by the tensor pipe (mma.sync: 1024 multiply-adds per clock and SM measured), six products where bf16 attention
+// issues two.  Tiled on the CUDA cores the same attention ran at 10 TFLOP/s (two shared-memory reads per 16
+// multiply-adds).  2048 causal rows, 16 heads over 4, 128 columns: 1560 us there with capped scores, 221 here (165 without the
+// cap's tanh; one set of warps with the queries in registers: 351 and 263, tensor pipe 37 % of the time).
 #include "../../include/vila_b200.h"
 #include "common.cuh"
 #include "kernels.h"
@@ -23,6 +28,7 @@ namespace {
 
 constexpr int kBK = 64;      // keys of a block
 constexpr int kMaxWarps = 8;
+constexpr float kLog2e = 1.44269504f;   // 1 / ln 2
 
 __device__ __forceinline__ void ldsm4(uint32_t addr, uint32_t (&r)[4]) {
   asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
@@ -48,6 +54,13 @@ __device__ __forceinline__ void cp16(uint32_t dst, const void* src, bool ok) {
   const uint32_t n = ok ? 16u : 0u;   // 0: zeros
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(n) : "memory");
 }
+__device__ __forceinline__ float ex2(float x) {
+  float y;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+// log2(e) x, rounded (never fused into what follows: a maximum's value has to be the same wherever it is used)
+__device__ __forceinline__ float log2_units(float x) { return __fmul_rn(x, kLog2e); }
 __device__ __forceinline__ float quad_max(float v) {
   v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, 1));
   return fmaxf(v, __shfl_xor_sync(0xffffffffu, v, 2));
@@ -57,13 +70,19 @@ __device__ __forceinline__ float quad_sum(float v) {
   return v + __shfl_xor_sync(0xffffffffu, v, 2);
 }
 
-// D: columns of a map, MAPS: maps of a head, V: value columns.  A key's row in shared memory: MAPS * D columns.
-template <int D, int MAPS, int V>
-__global__ void __launch_bounds__(32 * kMaxWarps) paged_attn_mma_kernel(const vila_paged_attn_params p, int tiles_per_cta) {
+// D: columns of a map, MAPS: maps of a head, V: value columns, SETS: sets of warps that share the key blocks.  A key's row
+// in shared memory has MAPS * D columns.
+// exp(s - m) is taken as 2^(s log2 e - m log2 e) with one fused multiply-add: the rounded m log2 e is common to a row's
+// weights and cancels in their quotient, which leaves the rounding of the difference, as in exp(s - m).
+template <int D, int MAPS, int V, int SETS>
+__global__ void __launch_bounds__(32 * (SETS == 2 ? 8 : kMaxWarps), 1)
+paged_attn_mma_kernel(const vila_paged_attn_params p, int tiles_per_cta) {
   constexpr int KB = MAPS * D * 2, VB = V * 2;             // bytes of a key's / value's row
-  constexpr int kBuf = kBK * (KB + VB);                     // one of two buffers: keys, then values
+  constexpr int kBuf = kBK * (KB + VB);                     // one of a set's two buffers: keys, then values
+  constexpr int kQ = 3 * (D / 16) * 512;                    // bytes of a warp's query parts
   extern __shared__ __align__(128) uint8_t sm[];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarps = blockDim.x >> 5;
+  const int lane = threadIdx.x & 31, W = (blockDim.x >> 5) / SETS;   // warps of a set
+  const int set = (threadIdx.x >> 5) / W, warp = (threadIdx.x >> 5) - set * W;
   const int rep = p.H / p.G, SH = rep * MAPS, g = blockIdx.y;
   const int tile0 = (gridDim.x - 1 - blockIdx.x) * tiles_per_cta, ntile = min(tiles_per_cta, p.ntiles - tile0);
   const int my_tile = warp / SH, sh = warp - my_tile * SH;  // this warp's tile and score head
@@ -72,25 +91,31 @@ __global__ void __launch_bounds__(32 * kMaxWarps) paged_attn_mma_kernel(const vi
   const int* tile = p.tiles + 4 * (tile0 + (active ? my_tile : 0));
   const int row0 = tile[0], n = active ? tile[1] : 0, pos0 = tile[2];
   const int gid = lane >> 2, tig = lane & 3;                // rows gid, gid + 8; columns 2 tig, 2 tig + 1 of an 8-column tile
-  const uint32_t sm0 = smem_u32(sm);
+  uint4* q_s = reinterpret_cast<uint4*>(sm + warp * kQ) + lane;      // [part][D / 16] fragments, 32 lanes apart
+  uint8_t* buf = sm + W * kQ + set * 2 * kBuf;
+  const uint32_t buf0 = smem_u32(buf);
 
-  // queries, scaled, in three parts
-  uint32_t q[3][D / 16][4];
+  // queries, scaled, in three parts (the sets share them: set s brings every SETS-th fragment)
   {
     const float sc = head_scale(p, h);
 #pragma unroll
-    for (int k = 0; k < D / 16; ++k)
+    for (int k0 = 0; k0 < D / 16; k0 += SETS) {
+      const int k = k0 + set;
+      uint32_t q[3][4];
 #pragma unroll
       for (int e = 0; e < 4; ++e) {
         const int i = gid + 8 * (e & 1), c = 16 * k + 8 * (e >> 1) + 2 * tig;
         float2 v = make_float2(0.f, 0.f);
         if (active && i < n)
           v = *reinterpret_cast<const float2*>(p.q + (static_cast<size_t>(row0 + i) * p.H * MAPS + h * MAPS + map) * D + c);
-        split3(v.x * sc, v.y * sc, q[0][k][e], q[1][k][e], q[2][k][e]);
+        split3(v.x * sc, v.y * sc, q[0][e], q[1][e], q[2][e]);
         // the parts of an infinite query are itself and zeros
-        if (isinf(v.x * sc)) q[1][k][e] &= 0xffff0000u, q[2][k][e] &= 0xffff0000u;
-        if (isinf(v.y * sc)) q[1][k][e] &= 0xffffu, q[2][k][e] &= 0xffffu;
+        if (isinf(v.x * sc)) q[1][e] &= 0xffff0000u, q[2][e] &= 0xffff0000u;
+        if (isinf(v.y * sc)) q[1][e] &= 0xffffu, q[2][e] &= 0xffffu;
       }
+#pragma unroll
+      for (int part = 0; part < 3; ++part) q_s[(part * (D / 16) + k) * 32] = make_uint4(q[part][0], q[part][1], q[part][2], q[part][3]);
+    }
   }
   float o[V / 8][4];
 #pragma unroll
@@ -98,10 +123,11 @@ __global__ void __launch_bounds__(32 * kMaxWarps) paged_attn_mma_kernel(const vi
 #pragma unroll
     for (int e = 0; e < 4; ++e) o[t][e] = 0.f;
   float m[2], l[2];
+  const bool sink = p.sink != nullptr && set == 0;
 #pragma unroll
   for (int r = 0; r < 2; ++r) {
-    m[r] = p.sink ? p.sink[h] : kNegBig;
-    l[r] = p.sink ? 1.0f : 0.0f;
+    m[r] = sink ? p.sink[h] : kNegBig;
+    l[r] = sink ? ex2(fmaf(m[r], kLog2e, -log2_units(m[r]))) : 0.0f;
   }
   // positions of this thread's two rows and what they see: keys lo .. pos, and of those the last `window` or the first keep_first
   int pos[2], lo[2], wlo[2];
@@ -112,10 +138,11 @@ __global__ void __launch_bounds__(32 * kMaxWarps) paged_attn_mma_kernel(const vi
     wlo[r] = p.window > 0 ? pos[r] - p.window + 1 : 0;
   }
   const int keep = p.window > 0 ? p.keep_first : 0;
-  const int row_max = pos0 + n - 1;
+  const int row_max = pos0 + n - 1, lo_min = first_key(p, pos0), lo_max = first_key(p, max(row_max, 0));
   const size_t prow = static_cast<size_t>(p.G) * (MAPS * D + V);   // elements of a pool row
   const __nv_bfloat16* pool = static_cast<const __nv_bfloat16*>(p.pool);
   const size_t koff = static_cast<size_t>(g) * MAPS * D, voff = static_cast<size_t>(p.G) * MAPS * D + static_cast<size_t>(g) * V;
+  __syncthreads();   // queries
 
   // the CTA's tiles in runs of one sequence (nearly always a single run)
   for (int run = 0; run < ntile;) {
@@ -130,19 +157,24 @@ __global__ void __launch_bounds__(32 * kMaxWarps) paged_attn_mma_kernel(const vi
     run = end;
     const int32_t* pt = p.page_tables + static_cast<size_t>(slot) * p.pt_stride;
     const BlockList bl = visible_blocks(p, first_pos, nkeys, kBK);
-
-    // block v to buffer b: a warp takes every nwarps-th key, its lanes the row's pieces
+    auto next_block = [&](int v) {   // the first of this set's blocks from v on
+      while (SETS == 2 && v < bl.count && (bl.block(v) & 1) != set) ++v;
+      return v;
+    };
+    // block v to buffer b: a warp takes every W-th run of 32 keys, its lanes the rows' pieces
     auto fetch = [&](int v, int b) {
       const int j0 = bl.block(v) * kBK;
       constexpr int kPieces = (KB + VB) / 16;
-      const uint32_t base = sm0 + b * kBuf;
-      for (int k0 = warp * 32; k0 < kBK; k0 += 32 * nwarps) {       // rows of 32 keys, a lane each
-        const int j = j0 + k0 + lane;
+      const uint32_t base = buf0 + b * kBuf;
+      for (int k0 = warp * 16; k0 < kBK; k0 += 16 * W) {             // rows of 16 keys, a lane each
+        const int j = j0 + k0 + (lane & 15);
         const unsigned long long at = j < nkeys ? pool_row(pt, p.page, j) * prow : 0ull;
-        for (int jj = 0; jj < 32; ++jj) {
+#pragma unroll 4
+        for (int jj = 0; jj < 16; ++jj) {
           const unsigned long long row = __shfl_sync(0xffffffffu, at, jj);
           const int key = k0 + jj;
           const bool ok = j0 + key < nkeys;
+#pragma unroll
           for (int x = lane; x < kPieces; x += 32) {
             const bool is_k = x < KB / 16;
             const int c = is_k ? x : x - KB / 16;
@@ -153,22 +185,24 @@ __global__ void __launch_bounds__(32 * kMaxWarps) paged_attn_mma_kernel(const vi
       }
       asm volatile("cp.async.commit_group;" ::: "memory");
     };
-    if (bl.count > 0) fetch(0, 0);
-    for (int v = 0; v < bl.count; ++v) {
-      if (v + 1 < bl.count) {
-        fetch(v + 1, (v + 1) & 1);
+    auto set_sync = [&]() { asm volatile("bar.sync %0, %1;" ::"r"(1 + set), "r"(32 * W) : "memory"); };
+    int v = next_block(0), b = 0;
+    if (v < bl.count) fetch(v, 0);
+    while (v < bl.count) {
+      const int after = next_block(v + 1);
+      if (after < bl.count) {
+        fetch(after, b ^ 1);
         asm volatile("cp.async.wait_group 1;" ::: "memory");
       } else {
         asm volatile("cp.async.wait_group 0;" ::: "memory");
       }
-      __syncthreads();
+      set_sync();
       const int j0 = bl.block(v) * kBK, j1 = j0 + kBK - 1;
       // does any row of this warp see a key of the block; do all of them see all of its keys
-      const bool some = mine && j0 <= row_max && j1 >= first_key(p, pos0) &&
-                        (p.window <= 0 || j1 > pos0 - p.window || j0 < keep);
-      const bool all = j1 <= pos0 && n == 16 && j0 >= first_key(p, row_max) && (p.window <= 0 || j0 > row_max - p.window || j1 < keep);
+      const bool some = mine && j0 <= row_max && j1 >= lo_min && (p.window <= 0 || j1 > pos0 - p.window || j0 < keep);
+      const bool all = j1 <= pos0 && n == 16 && j0 >= lo_max && (p.window <= 0 || j0 > row_max - p.window || j1 < keep);
       if (some) {
-        const uint32_t kb = sm0 + (v & 1) * kBuf, vb = kb + kBK * KB;
+        const uint32_t kb = buf0 + b * kBuf, vb = kb + kBK * KB;
         float s[kBK / 8][4];
 #pragma unroll
         for (int t = 0; t < kBK / 8; ++t)
@@ -178,19 +212,22 @@ __global__ void __launch_bounds__(32 * kMaxWarps) paged_attn_mma_kernel(const vi
         const int lkey = (lane & 7) + ((lane >> 4) << 3), lc = (lane >> 3) & 1;
 #pragma unroll
         for (int k = 0; k < D / 16; ++k) {
+          // eight independent sums between two uses of the same one: the products' latency is covered
+          uint32_t kf[kBK / 16][4];
 #pragma unroll
-          for (int t = 0; t < kBK / 16; ++t) {
-            uint32_t b[4];
-            ldsm4(kb + (16 * t + lkey) * KB + (((map * D / 8 + 2 * k + lc) ^ (lkey & 7)) << 4), b);
+          for (int t = 0; t < kBK / 16; ++t) ldsm4(kb + (16 * t + lkey) * KB + (((map * D / 8 + 2 * k + lc) ^ (lkey & 7)) << 4), kf[t]);
 #pragma unroll
-            for (int part = 2; part >= 0; --part) {
-              mma_bf16(s[2 * t], q[part][k], b[0], b[1]);
-              mma_bf16(s[2 * t + 1], q[part][k], b[2], b[3]);
+          for (int part = 2; part >= 0; --part) {
+            const uint4 qv = q_s[(part * (D / 16) + k) * 32];
+            const uint32_t qf[4] = {qv.x, qv.y, qv.z, qv.w};
+#pragma unroll
+            for (int t = 0; t < kBK / 16; ++t) {
+              mma_bf16(s[2 * t], qf, kf[t][0], kf[t][1]);
+              mma_bf16(s[2 * t + 1], qf, kf[t][2], kf[t][3]);
             }
           }
         }
         // cap, bias, mask; the block's maximum per row
-        float mn[2] = {m[0], m[1]};
         if (p.softcap > 0.f) {
 #pragma unroll
           for (int t = 0; t < kBK / 8; ++t)
@@ -212,31 +249,43 @@ __global__ void __launch_bounds__(32 * kMaxWarps) paged_attn_mma_kernel(const vi
               if (!(j <= pos[r] && j >= lo[r] && (j >= wlo[r] || j < keep))) s[t][e] = kNegBig;
             }
         }
+        float mn[2] = {m[0], m[1]};
 #pragma unroll
         for (int t = 0; t < kBK / 8; ++t)
 #pragma unroll
           for (int e = 0; e < 4; ++e) mn[e >> 1] = fmaxf(mn[e >> 1], s[t][e]);
-        float ps[2] = {0.f, 0.f}, alpha[2];
+        float ps[2] = {0.f, 0.f}, alpha[2], ml[2];
 #pragma unroll
         for (int r = 0; r < 2; ++r) {
           mn[r] = quad_max(mn[r]);
-          alpha[r] = expf(m[r] - mn[r]);
+          ml[r] = log2_units(mn[r]);
+          alpha[r] = ex2(__fsub_rn(log2_units(m[r]), ml[r]));
           m[r] = mn[r];
+        }
+        if (all) {
+#pragma unroll
+          for (int t = 0; t < kBK / 8; ++t)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) s[t][e] = ex2(fmaf(s[t][e], kLog2e, -ml[e >> 1]));
+        } else {
+          // a hidden key weighs nothing, also while its row has seen no key at all (maximum still kNegBig)
+#pragma unroll
+          for (int t = 0; t < kBK / 8; ++t)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) s[t][e] = s[t][e] == kNegBig ? 0.f : ex2(fmaf(s[t][e], kLog2e, -ml[e >> 1]));
         }
 #pragma unroll
         for (int t = 0; t < kBK / 8; ++t)
 #pragma unroll
-          for (int e = 0; e < 4; ++e) {
-            // a hidden key weighs nothing, also while its row has seen no key at all (maximum still kNegBig)
-            s[t][e] = s[t][e] == kNegBig ? 0.f : expf(s[t][e] - mn[e >> 1]);
-            ps[e >> 1] += s[t][e];
-          }
+          for (int e = 0; e < 4; ++e) ps[e >> 1] += s[t][e];
 #pragma unroll
         for (int r = 0; r < 2; ++r) l[r] = l[r] * alpha[r] + quad_sum(ps[r]);
+        if (__any_sync(0xffffffffu, alpha[0] != 1.f || alpha[1] != 1.f)) {
 #pragma unroll
-        for (int t = 0; t < V / 8; ++t)
+          for (int t = 0; t < V / 8; ++t)
 #pragma unroll
-          for (int e = 0; e < 4; ++e) o[t][e] *= alpha[e >> 1];
+            for (int e = 0; e < 4; ++e) o[t][e] *= alpha[e >> 1];
+        }
         // weights (three parts) x values: 16 keys x 16 columns per ldmatrix
         const int vkey = (lane & 7) + (((lane >> 3) & 1) << 3), vc = lane >> 4;
 #pragma unroll
@@ -248,32 +297,74 @@ __global__ void __launch_bounds__(32 * kMaxWarps) paged_attn_mma_kernel(const vi
             split3(w[0], w[1], a[0][e], a[1][e], a[2][e]);
           }
 #pragma unroll
-          for (int t = 0; t < V / 16; ++t) {
-            uint32_t b[4];
-            ldsm4_t(vb + (16 * k + vkey) * VB + (((2 * t + vc) ^ (vkey & 7)) << 4), b);
+          for (int t0 = 0; t0 < V / 16; t0 += 4) {
+            uint32_t vf[4][4];
 #pragma unroll
-            for (int part = 2; part >= 0; --part) {
-              mma_bf16(o[2 * t], a[part], b[0], b[1]);
-              mma_bf16(o[2 * t + 1], a[part], b[2], b[3]);
-            }
+            for (int t = 0; t < 4; ++t) ldsm4_t(vb + (16 * k + vkey) * VB + (((2 * (t0 + t) + vc) ^ (vkey & 7)) << 4), vf[t]);
+#pragma unroll
+            for (int part = 2; part >= 0; --part)
+#pragma unroll
+              for (int t = 0; t < 4; ++t) {
+                mma_bf16(o[2 * (t0 + t)], a[part], vf[t][0], vf[t][1]);
+                mma_bf16(o[2 * (t0 + t) + 1], a[part], vf[t][2], vf[t][3]);
+              }
           }
         }
       }
-      __syncthreads();   // everyone has read the buffer that the next block but one overwrites
+      set_sync();   // the set has read the buffer that its next block but one overwrites
+      v = after;
+      b ^= 1;
     }
   }
 
+  float* xch = reinterpret_cast<float*>(sm + W * kQ + (SETS - 1) * 2 * kBuf);   // the last set's buffers: rows handed over
+  if (SETS == 2) {
+    // the odd blocks' sums join the even blocks'
+    constexpr int kRec = 16 * V + 64;
+    float* rec = xch + warp * kRec;
+    if (set == 1) {
+#pragma unroll
+      for (int t = 0; t < V / 8; ++t)
+#pragma unroll
+        for (int r = 0; r < 2; ++r)
+          *reinterpret_cast<float2*>(rec + (gid + 8 * r) * V + 8 * t + 2 * tig) = make_float2(o[t][2 * r], o[t][2 * r + 1]);
+#pragma unroll
+      for (int r = 0; r < 2; ++r)
+        if (tig == 0) {
+          rec[16 * V + gid + 8 * r] = m[r];
+          rec[16 * V + 16 + gid + 8 * r] = l[r];
+        }
+    }
+    __syncthreads();
+    if (set == 0) {
+#pragma unroll
+      for (int r = 0; r < 2; ++r) {
+        const float m1 = rec[16 * V + gid + 8 * r], l1 = rec[16 * V + 16 + gid + 8 * r], mx = fmaxf(m[r], m1);
+        const float ml = log2_units(mx), f0 = ex2(__fsub_rn(log2_units(m[r]), ml));
+        const float f1 = l1 == 0.f ? 0.f : ex2(__fsub_rn(log2_units(m1), ml));   // l1 == 0: no odd block was seen
+        l[r] = l[r] * f0 + l1 * f1;
+#pragma unroll
+        for (int t = 0; t < V / 8; ++t) {
+          const float2 x = *reinterpret_cast<const float2*>(rec + (gid + 8 * r) * V + 8 * t + 2 * tig);
+          o[t][2 * r] = o[t][2 * r] * f0 + x.x * f1;
+          o[t][2 * r + 1] = o[t][2 * r + 1] * f0 + x.y * f1;
+        }
+      }
+    }
+    if (MAPS == 2) __syncthreads();   // the records have been read
+  }
+  const bool writes = active && set == 0;
   if (MAPS == 2) {
     // the second map's rows through shared memory to the warp of the first, which combines, norms and gates them
-    float* a2 = reinterpret_cast<float*>(sm) + (warp >> 1) * 16 * V;
-    if (active && map == 1) {
+    float* a2 = xch + (warp >> 1) * 16 * V;
+    if (writes && map == 1) {
 #pragma unroll
       for (int t = 0; t < V / 8; ++t)
 #pragma unroll
         for (int e = 0; e < 4; ++e) a2[(gid + 8 * (e >> 1)) * V + 8 * t + 2 * tig + (e & 1)] = o[t][e] * (1.0f / l[e >> 1]);
     }
     __syncthreads();
-    if (!active || map == 1) return;
+    if (!writes || map == 1) return;
     float ss[2] = {0.f, 0.f};
 #pragma unroll
     for (int t = 0; t < V / 8; ++t)
@@ -286,7 +377,7 @@ __global__ void __launch_bounds__(32 * kMaxWarps) paged_attn_mma_kernel(const vi
 #pragma unroll
     for (int r = 0; r < 2; ++r) l[r] = sqrtf(quad_sum(ss[r]) / static_cast<float>(V) + p.diff_eps) / p.diff_scale;
   }
-  if (!active) return;
+  if (!writes) return;
 #pragma unroll
   for (int r = 0; r < 2; ++r) {
     const int i = gid + 8 * r;
@@ -302,15 +393,19 @@ __global__ void __launch_bounds__(32 * kMaxWarps) paged_attn_mma_kernel(const vi
   }
 }
 
+template <int D, int MAPS, int V, int SETS>
+int launch_sets(const vila_paged_attn_params& p, int warps, int tpc, cudaStream_t stream) {
+  auto kernel = paged_attn_mma_kernel<D, MAPS, V, SETS>;
+  const int smem = warps * 3 * (D / 16) * 512 + SETS * 2 * kBK * (MAPS * D + V) * 2;
+  static PerDeviceOnce once;
+  if (once.first()) VB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 224 * 1024));
+  VB_CUDA(launch_serial(kernel, dim3((p.ntiles + tpc - 1) / tpc, p.G), dim3(32 * warps * SETS), smem, stream, p, tpc));
+  return 0;
+}
 template <int D, int MAPS, int V>
 int launch(const vila_paged_attn_params& p, cudaStream_t stream) {
-  constexpr int smem = 2 * kBK * (MAPS * D + V) * 2;
   const int SH = p.H / p.G * MAPS, tpc = SH >= 4 ? 1 : 4 / SH;   // four warps, or one tile of all the heads
-  static PerDeviceOnce once;
-  if (once.first())
-    VB_CUDA(cudaFuncSetAttribute(paged_attn_mma_kernel<D, MAPS, V>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-  VB_CUDA(launch_serial(paged_attn_mma_kernel<D, MAPS, V>, dim3((p.ntiles + tpc - 1) / tpc, p.G), dim3(32 * SH * tpc), smem, stream, p, tpc));
-  return 0;
+  return SH * tpc <= 4 ? launch_sets<D, MAPS, V, 2>(p, SH * tpc, tpc, stream) : launch_sets<D, MAPS, V, 1>(p, SH * tpc, tpc, stream);
 }
 
 bool aligned(const void* p, size_t n) { return reinterpret_cast<uintptr_t>(p) % n == 0; }
