@@ -221,3 +221,29 @@ def test_paged_attention_prompt_extremes(ops):
     assert torch.equal(alone[16:32], got[16:32])
     q[3, 7] = float("nan")
     assert torch.isnan(ops.paged_attention(q, pool, tables, tiles, **kw)[3, :128]).all()
+
+
+@pytest.mark.parametrize("dim,rot,halves", [(2, 2, False), (64, 64, True), (96, 32, False), (128, 64, True), (130, 128, False), (256, 256, True)])
+@pytest.mark.parametrize("dtype", [BF, F32])
+def test_rope_append_pairs(ops, dim, rot, halves, dtype):
+    """a lane's pairs of columns at head sizes below, at and past its 32: against float64 angles, unit norm with weights, value mixing"""
+    g, T, H, G, V = gen(dim), 5, 3, 2, 24
+    qkv, vf = randn(g, T, (H + G) * dim + G * V, dtype=dtype), randn(g, T, G * V, dtype=dtype)
+    pos = torch.tensor([0, 1, 77, 5000, 100000], dtype=torch.int32, device="cuda")
+    rows, pool = torch.tensor([4, 0, 3, 1, 2], dtype=torch.int32, device="cuda"), torch.zeros(5, G * (dim + V), device="cuda", dtype=F32)
+    inv = 10000.0 ** (-2.0 * torch.arange(rot // 2, device="cuda", dtype=torch.float64) / rot)
+    w = [1 + 0.1 * torch.randn(dim, generator=g, device="cuda") for _ in range(2)]
+    q = ops.rope_append(qkv, pos, rows, pool, heads=H, kv_heads=G, dim=dim, vdim=V, inv_freq=inv, unit_norm=True, eps=1e-5, q_norm_w=w[0],
+                        k_norm_w=w[1], halves=halves, mscale=1.25, v_first=vf, v_mix=0.3)
+    x = qkv.double()[:, :(H + G) * dim].reshape(T, H + G, dim)
+    ang = pos.double()[:, None] * inv
+    c, s = 1.25 * torch.cos(ang)[:, None], 1.25 * torch.sin(ang)[:, None]
+    i = torch.arange(rot // 2, device="cuda")
+    i0, i1 = (i, i + rot // 2) if halves else (2 * i, 2 * i + 1)
+    y = x.clone()
+    y[..., i0], y[..., i1] = x[..., i0] * c - x[..., i1] * s, x[..., i1] * c + x[..., i0] * s
+    y = y / torch.sqrt(y.pow(2).mean(-1, keepdim=True) + 1e-5)
+    want_q, want_k = y[:, :H] * w[0].double(), y[:, H:] * w[1].double()
+    assert rel(q, want_q.reshape(T, -1)) < 5e-7
+    want_v = 0.7 * qkv.double()[:, (H + G) * dim:] + 0.3 * vf.double()
+    assert rel(pool[rows.long()], torch.cat([want_k.reshape(T, -1), want_v], 1)) < 5e-7

@@ -120,7 +120,7 @@ __global__ void __launch_bounds__(kThreads) rope_append_kernel(const vila_rope_a
 // The same for even head sizes, a pair of columns (rotated together, or neighbours past the rotated part) at a time: a lane
 // loads its NP pairs of a head once, all in flight, and keeps them over the norm; the first head's are on their way while
 // the angles are evaluated.  The general form reads every element twice, one after the other (2048 tokens of 24 heads:
-// 33 us, here MEASURED_ROPE).
+// 33 us, here 13.8; 8 tokens 7.2 and 3.3).
 template <bool BF16, int NP>
 __global__ void __launch_bounds__(kThreads) rope_append_pairs_kernel(const vila_rope_append_params p) {
   extern __shared__ float cs[];   // cos [rot/2] | sin [rot/2]
