@@ -9,12 +9,18 @@
 //                  S <- diag(alpha) S + k v^T;  o = S^T (q_scale q),   alpha = sigmoid(z + z_bias)^(1 / tau)
 //   decay_scan   linear attention with one constant decay per head (lightning attention):
 //                  S <- g S + k v^T;  o = S^T (q_scale q);  optionally SiLU on q, k and v as they are read
+//   ssd_scan     one decay per head and token (state-space duality form):
+//                  S <- g S + B (dt x)^T;  y = S^T C + D x;  out = y silu(z),   g = exp(-exp(A_log) dt),
+//                  dt = softplus(dt_raw + dt_bias);  heads share the B / C of their group
+//   hgrn2_scan   one decay per key channel, which also sets the input gate:
+//                  S <- diag(f) S + (1 - f) v^T;  o = S^T q,   f = lower + (1 - lower) sigmoid(zf + bias), q = silu(zq);
+//                  its state is stored [.., dim, vdim] and passes through shared memory once at either end
 //
 // The read-outs are taken from the state BEFORE the token's write, which is the same number and shortens the chain
 // of dependent steps to one pass over the state per token:
 //   delta:  S_new^T q = g (S^T q) + (k . q) u        so S^T k and S^T q are reduced together
 //   gla:    S_new^T q = S^T (alpha q) + (k . q) v    so the state update does not wait for the reduction
-//   decay:  S_new^T q = g (S^T q) + (k . q) v        likewise
+//   decay, ssd:  S_new^T q = g (S^T q) + (k . q) v   likewise;  hgrn2 as gla
 //
 // Grid (sequence, head, COLS columns of vdim).  Warps 0-3 own the state: R lanes share CPT columns, lane r
 // keeps the float4 pieces r, r + R, .. of a column in registers (state layout [.., vdim, dim]: coalesced loads, and
@@ -22,8 +28,12 @@
 // sums are reduced over the R lanes with a transposing tree: every step halves the number of values a lane carries.
 // The other 4 or 8 warps stage the next 16 tokens (load, unit norms or decays, k . q, fp32 into the other shared-memory buffer)
 // and write the previous 16 tokens' outputs while the owners run; one barrier per 16 tokens.
-// A column's sum runs in the same order whatever CPT is, and time runs in order: a row's result depends neither on
+// Only the delta rule needs a token's sums before its write.  The others take kBatch tokens at a time: every owner keeps
+// the batch's partial sums and one tree reduces them together (half the shuffles, and the tree's latency under the next
+// tokens' products).
+// A column's sum runs in the same order whatever CPT and the batch are, and time runs in order: a row's result depends neither on
 // the batch nor on how its sequence was cut into steps.
+#include <type_traits>
 #include "../../include/vila_b200.h"
 #include "common.cuh"
 #include "kernels.h"
@@ -34,6 +44,7 @@ namespace {
 
 constexpr int kOwnerWarps = 4;
 constexpr int kChunk = 16;   // tokens per stage
+constexpr int kBatch = 4;    // tokens whose sums are reduced together
 
 __device__ __forceinline__ float softplus_f(float z) { return z > 20.0f ? z : log1pf(expf(z)); }
 
@@ -95,18 +106,23 @@ __device__ __forceinline__ void transpose_sum(float (&v)[NV], int r) {
   }
 }
 
-enum Mode : int { kDelta, kGla, kDecay };
+enum Mode : int { kDelta, kGla, kDecay, kSsd, kHgrn2 };
 
 struct ScanArgs {
   const void *q, *k, *v;        // rows of the step; head offsets are added by the kernel
   int64_t ldq, ldk, ldv;
-  const void *a, *b;            // delta: decay / step-size pre-activations, column h;  gla: a = z, H * dim columns
+  const void *a, *b;            // delta: decay / step-size pre-activations, column h;  gla: a = z, H * dim columns;  ssd: a = dt
   int64_t lda, ldb;
   const float *A_log, *bias;    // delta: A_log [H], dt_bias [H];  gla: bias [H * dim] or NULL
   float* state;                 // [slots, H, vdim, dim]
   const int32_t* seqs;
-  float* out;
+  void* out;
   int64_t ldo;
+  int out_dt;                   // fp32 but for ssd
+  const void* z;                // ssd: gate [rows, H * vdim], or NULL
+  int64_t ldz;
+  const float* D;               // ssd: [H]
+  const float* lower;           // hgrn2: [H * dim], or NULL
   int in_dt, a_dt, H, G, dim, vdim;
   float q_scale, eps, inv_tau;
   const float* decay;           // decay: [H]
@@ -117,12 +133,13 @@ struct ScanArgs {
 template <int MODE, int R, int KPT, int CPT, int kStageWarps>
 __global__ void __launch_bounds__(32 * (kOwnerWarps + kStageWarps)) outer_scan_kernel(const ScanArgs p) {
   extern __shared__ __align__(16) float sm[];
-  constexpr bool DELTA = MODE == kDelta, GLA = MODE == kGla;
+  constexpr bool DELTA = MODE == kDelta, SSD = MODE == kSsd, HGRN = MODE == kHgrn2;
+  constexpr bool GLA = MODE == kGla || HGRN;        // a decay per key channel
   constexpr int NP = R * KPT;                       // key channels the owners cover
   constexpr int NQ = KPT / 4;                       // float4 pieces per lane
   constexpr int GPW = 32 / R;                       // column groups per warp
   constexpr int COLS = kOwnerWarps * GPW * CPT;
-  constexpr int NV = DELTA ? 2 * CPT : CPT;
+  constexpr int NV = DELTA ? 2 * CPT : CPT;         // sums per token
   constexpr int NVEC = GLA ? 3 : 2;                 // staged vectors per token: k, q (, alpha)
   constexpr int TOK = NVEC * NP;
   constexpr int NG = NP > 128 ? NP / 128 : 1;       // four-element pieces a staging lane handles per vector
@@ -140,14 +157,30 @@ __global__ void __launch_bounds__(32 * (kOwnerWarps + kStageWarps)) outer_scan_k
   const int col0 = blockIdx.z * COLS;
   const int nchunks = (n + kChunk - 1) / kChunk;
 
+  // hgrn2: the state's columns through shared memory (coalesced rows of vdim in global memory), padded rows
+  float* tr_s = vec_s;
+  constexpr int TS = NP + 4;
+  auto state_at = [&](int i, int c) {
+    return p.state + ((static_cast<size_t>(slot) * p.H + h) * dim + i) * vdim + col0 + c;
+  };
+  if (HGRN) {
+    static_assert(!HGRN || COLS * TS <= 2 * kChunk * TOK, "the transposed state fits the staging buffers");
+    for (int idx = threadIdx.x; idx < COLS * dim; idx += blockDim.x) {
+      const int i = idx / COLS, c = idx - i * COLS;
+      tr_s[c * TS + i] = pos0 > 0 && col0 + c < vdim ? *state_at(i, c) : 0.f;
+    }
+    __syncthreads();
+  }
+
   if (warp >= kOwnerWarps) {
     // ---------------- staging warps ----------------
+    if (HGRN) __syncthreads();                       // the owners have taken their columns
     const int sw = warp - kOwnerWarps, st = threadIdx.x - kOwnerWarps * 32;
     const int dt = p.in_dt, adt = p.a_dt;
     const size_t qoff = static_cast<size_t>(kh) * dim, voff = static_cast<size_t>(h) * vdim;
     const size_t zoff = static_cast<size_t>(h) * dim;
-    const float neg_a = DELTA ? -expf(p.A_log[h]) : 0.f, dbias = DELTA ? p.bias[h] : 0.f;
-    float4 zb[NG];
+    const float neg_a = DELTA || SSD ? -expf(p.A_log[h]) : 0.f, dbias = DELTA || SSD ? p.bias[h] : 0.f;
+    float4 zb[NG], lw[NG];
 #pragma unroll
     for (int j = 0; j < NG; ++j) {
       zb[j] = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -157,6 +190,14 @@ __global__ void __launch_bounds__(32 * (kOwnerWarps + kStageWarps)) outer_scan_k
 #pragma unroll
         for (int k = 0; k < 4; ++k) e[k] = i + k < dim ? p.bias[zoff + i + k] : 0.f;
         zb[j] = make_float4(e[0], e[1], e[2], e[3]);
+      }
+      lw[j] = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (HGRN && p.lower) {
+        const int i = 4 * (lane + 32 * j);
+        float e[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) e[k] = i + k < dim ? p.lower[zoff + i + k] : 0.f;
+        lw[j] = make_float4(e[0], e[1], e[2], e[3]);
       }
     }
     auto stage = [&](int ch) {
@@ -170,9 +211,9 @@ __global__ void __launch_bounds__(32 * (kOwnerWarps + kStageWarps)) outer_scan_k
         const int idx = st + k * kStageWarps * 32, t = idx / COLS, c = col0 + idx % COLS;
         rv[k] = (t < nt && c < vdim) ? ld_raw(p.v, dt, static_cast<size_t>(row0 + t0 + t) * p.ldv + voff + c) : 0u;
       }
-      if (DELTA && st < nt) {
+      if ((DELTA || SSD) && st < nt) {
         ra = ld_raw(p.a, adt, static_cast<size_t>(row0 + t0 + st) * p.lda + h);
-        rb = ld_raw(p.b, adt, static_cast<size_t>(row0 + t0 + st) * p.ldb + h);
+        if (DELTA) rb = ld_raw(p.b, adt, static_cast<size_t>(row0 + t0 + st) * p.ldb + h);
       }
 #pragma unroll 1
       for (int tb = 0; tb < TPW; tb += TB) {
@@ -186,7 +227,7 @@ __global__ void __launch_bounds__(32 * (kOwnerWarps + kStageWarps)) outer_scan_k
             const int i = t < nt ? 4 * (lane + 32 * j) : dim;
             rk[u][j] = ld_raw4(p.k, dt, row * p.ldk + qoff, i, dim, p.vec_qk != 0);
             rq[u][j] = ld_raw4(p.q, dt, row * p.ldq + qoff, i, dim, p.vec_qk != 0);
-            if (GLA) rz[u][j] = ld_raw4(p.a, adt, row * p.lda + zoff, i, dim, p.vec_a != 0);
+            if (MODE == kGla) rz[u][j] = ld_raw4(p.a, adt, row * p.lda + zoff, i, dim, p.vec_a != 0);
           }
         }
 #pragma unroll
@@ -194,11 +235,19 @@ __global__ void __launch_bounds__(32 * (kOwnerWarps + kStageWarps)) outer_scan_k
           const int t = sw + (tb + u) * kStageWarps;
           if (t >= nt) break;
           float kq = 0.f, kk = 0.f, qq = 0.f;
-          float4 kv[NG], qv[NG];
+          float4 kv[NG], qv[NG], fv[NG];
 #pragma unroll
           for (int j = 0; j < NG; ++j) {
             kv[j] = raw4_to_float(rk[u][j], dt);
             qv[j] = raw4_to_float(rq[u][j], dt);
+            if (HGRN) {
+              const bool in = 4 * (lane + 32 * j) < dim;   // past the key channels everything is zero
+              const float4 z = kv[j], b = zb[j], l = lw[j];
+              fv[j] = make_float4(l.x + (1.0f - l.x) * sigmoid_f(z.x + b.x), l.y + (1.0f - l.y) * sigmoid_f(z.y + b.y),
+                                  l.z + (1.0f - l.z) * sigmoid_f(z.z + b.z), l.w + (1.0f - l.w) * sigmoid_f(z.w + b.w));
+              kv[j] = in ? make_float4(1.0f - fv[j].x, 1.0f - fv[j].y, 1.0f - fv[j].z, 1.0f - fv[j].w) : make_float4(0.f, 0.f, 0.f, 0.f);
+              qv[j] = silu4(qv[j]);
+            }
             if (MODE == kDecay && p.silu) {
               kv[j] = silu4(kv[j]);
               qv[j] = silu4(qv[j]);
@@ -227,11 +276,14 @@ __global__ void __launch_bounds__(32 * (kOwnerWarps + kStageWarps)) outer_scan_k
               float4 q4 = make_float4(qv[j].x * qs, qv[j].y * qs, qv[j].z * qs, qv[j].w * qs);
               *reinterpret_cast<float4*>(kd + i) = make_float4(kv[j].x * ks, kv[j].y * ks, kv[j].z * ks, kv[j].w * ks);
               if (GLA) {
-                const float4 z = raw4_to_float(rz[u][j], adt);
-                const float4 al = make_float4(expf(-softplus_f(-(z.x + zb[j].x)) * p.inv_tau),
-                                              expf(-softplus_f(-(z.y + zb[j].y)) * p.inv_tau),
-                                              expf(-softplus_f(-(z.z + zb[j].z)) * p.inv_tau),
-                                              expf(-softplus_f(-(z.w + zb[j].w)) * p.inv_tau));
+                float4 al;
+                if (HGRN) {
+                  al = fv[j];
+                } else {
+                  const float4 z = raw4_to_float(rz[u][j], adt);
+                  al = make_float4(expf(-softplus_f(-(z.x + zb[j].x)) * p.inv_tau), expf(-softplus_f(-(z.y + zb[j].y)) * p.inv_tau),
+                                   expf(-softplus_f(-(z.z + zb[j].z)) * p.inv_tau), expf(-softplus_f(-(z.w + zb[j].w)) * p.inv_tau));
+                }
                 q4 = make_float4(q4.x * al.x, q4.y * al.y, q4.z * al.z, q4.w * al.w);
                 *reinterpret_cast<float4*>(kd + 2 * NP + i) = al;
               }
@@ -247,10 +299,11 @@ __global__ void __launch_bounds__(32 * (kOwnerWarps + kStageWarps)) outer_scan_k
         const float v = raw_to_float(rv[k], dt);
         if (idx < kChunk * COLS) v_s[bf * kChunk * COLS + idx] = MODE == kDecay && p.silu ? silu_exact_f(v) : v;
       }
-      if (DELTA && st < nt) {
+      if ((DELTA || SSD) && st < nt) {
         float* s = reinterpret_cast<float*>(sc_s + bf * kChunk + st);
-        s[0] = expf(neg_a * softplus_f(raw_to_float(ra, adt) + dbias));
-        s[1] = sigmoid_f(raw_to_float(rb, adt));
+        const float step = softplus_f(raw_to_float(ra, adt) + dbias);
+        s[0] = expf(neg_a * step);
+        s[1] = SSD ? step : sigmoid_f(raw_to_float(rb, adt));
       }
     };
     auto flush = [&](int ch) {
@@ -258,7 +311,10 @@ __global__ void __launch_bounds__(32 * (kOwnerWarps + kStageWarps)) outer_scan_k
       const float* y = y_s + (ch & 1) * kChunk * COLS;
       for (int idx = st; idx < nt * COLS; idx += kStageWarps * 32) {
         const int t = idx / COLS, c = col0 + idx % COLS;
-        if (c < vdim) p.out[static_cast<size_t>(row0 + t0 + t) * p.ldo + voff + c] = y[idx];
+        if (c >= vdim) continue;
+        const size_t row = static_cast<size_t>(row0 + t0 + t), at = row * p.ldo + voff + c;
+        if (SSD) st_any(p.out, p.out_dt, at, p.z ? y[idx] * silu_exact_f(ld_any(p.z, dt, row * p.ldz + voff + c)) : y[idx]);
+        else static_cast<float*>(p.out)[at] = y[idx];
       }
     };
     stage(0);
@@ -269,9 +325,7 @@ __global__ void __launch_bounds__(32 * (kOwnerWarps + kStageWarps)) outer_scan_k
       __syncthreads();
     }
     if (nchunks > 0) flush(nchunks - 1);
-    return;
-  }
-
+  } else {
   // ---------------- owners of the state ----------------
   const int r = lane & (R - 1), cg = (warp * GPW + lane / R) * CPT;   // first column of this lane's group
   float* stp = p.state + ((static_cast<size_t>(slot) * p.H + h) * vdim + col0 + cg) * dim;
@@ -283,7 +337,12 @@ __global__ void __launch_bounds__(32 * (kOwnerWarps + kStageWarps)) outer_scan_k
     for (int j = 0; j < NQ; ++j) {
       S[c][j] = make_float4(0.f, 0.f, 0.f, 0.f);
       const int i = 4 * (r + R * j);
-      if (pos0 > 0 && col0 + cg + c < vdim && i < dim) {
+      if (HGRN) {
+        if (i < dim) S[c][j] = *reinterpret_cast<const float4*>(tr_s + (cg + c) * TS + i);   // rows past dim are never stored
+        if (i + 1 >= dim) S[c][j].y = 0.f;
+        if (i + 2 >= dim) S[c][j].z = 0.f;
+        if (i + 3 >= dim) S[c][j].w = 0.f;
+      } else if (pos0 > 0 && col0 + cg + c < vdim && i < dim) {
         const float* s = stp + static_cast<size_t>(c) * dim + i;
         if (vec_s4) S[c][j] = *reinterpret_cast<const float4*>(s);
         else {
@@ -298,7 +357,8 @@ __global__ void __launch_bounds__(32 * (kOwnerWarps + kStageWarps)) outer_scan_k
   const int mine = r / kSpan;                      // which of the NV sums this lane ends up with
   const int my_col = DELTA ? mine - CPT : mine;    // its column, if it is a read-out
   const bool writes = my_col >= 0 && (r % kSpan) == 0;
-  const float gh = MODE == kDecay ? p.decay[h] : 0.f;
+  const float gh = MODE == kDecay ? p.decay[h] : 0.f, Dh = SSD ? p.D[h] : 0.f;
+  if (HGRN) __syncthreads();
   __syncthreads();
   for (int ch = 0; ch < nchunks; ++ch) {
     const int nt = min(kChunk, n - ch * kChunk), bf = ch & 1;
@@ -306,15 +366,66 @@ __global__ void __launch_bounds__(32 * (kOwnerWarps + kStageWarps)) outer_scan_k
     const float* vv = v_s + bf * kChunk * COLS;
     float* yy = y_s + bf * kChunk * COLS;
     const float4* sc = sc_s + bf * kChunk;
-    float4 kn[NQ], qn[NQ], an[NQ];
+    if (!DELTA) {
+      // `count` tokens from t0 on: every token's sums over the state before its write, then its write
+      auto tokens = [&](int t0, auto count) {
+        constexpr int NT = decltype(count)::value, NS = NT * CPT, SPAN = R / NS;
+        float d[NS];
+#pragma unroll
+        for (int u = 0; u < NT; ++u) {
+          const float* tk = tok + (t0 + u) * TOK;
+          const float4 s4 = sc[t0 + u];
+          const float g = SSD ? s4.x : gh;
+          float w[CPT];
+#pragma unroll
+          for (int c = 0; c < CPT; ++c) w[c] = SSD ? s4.y * vv[(t0 + u) * COLS + cg + c] : vv[(t0 + u) * COLS + cg + c];
+          float4 eq[CPT];
+#pragma unroll
+          for (int c = 0; c < CPT; ++c) eq[c] = make_float4(0.f, 0.f, 0.f, 0.f);   // four partial sums: short chains
+#pragma unroll
+          for (int j = 0; j < NQ; ++j) {
+            const float4 kc = reinterpret_cast<const float4*>(tk)[r + R * j], qc = reinterpret_cast<const float4*>(tk + NP)[r + R * j];
+            float4 al = make_float4(g, g, g, g);
+            if (GLA) al = reinterpret_cast<const float4*>(tk + 2 * NP)[r + R * j];
+#pragma unroll
+            for (int c = 0; c < CPT; ++c) {
+              eq[c].x = fmaf(S[c][j].x, qc.x, eq[c].x); eq[c].y = fmaf(S[c][j].y, qc.y, eq[c].y);
+              eq[c].z = fmaf(S[c][j].z, qc.z, eq[c].z); eq[c].w = fmaf(S[c][j].w, qc.w, eq[c].w);
+              S[c][j].x = fmaf(al.x, S[c][j].x, kc.x * w[c]);
+              S[c][j].y = fmaf(al.y, S[c][j].y, kc.y * w[c]);
+              S[c][j].z = fmaf(al.z, S[c][j].z, kc.z * w[c]);
+              S[c][j].w = fmaf(al.w, S[c][j].w, kc.w * w[c]);
+            }
+          }
+#pragma unroll
+          for (int c = 0; c < CPT; ++c) d[u * CPT + c] = (eq[c].x + eq[c].y) + (eq[c].z + eq[c].w);
+        }
+        transpose_sum<R, NS>(d, r);
+        const int own = r / SPAN, tt = t0 + own / CPT, cc = cg + own % CPT;   // the sum this lane ends up with
+        const float4 s4 = sc[tt];
+        const float x = vv[tt * COLS + cc], g = SSD ? s4.x : gh;
+        if (r % SPAN == 0) {
+          float y = fmaf(s4.z, SSD ? s4.y * x : x, GLA ? d[0] : g * d[0]);
+          if (SSD) y = fmaf(Dh, x, y);
+          yy[tt * COLS + cc] = y;
+        }
+      };
+      int t0 = 0;
+      constexpr int NB = R / CPT < kBatch ? R / CPT : kBatch;   // a lane ends up with one sum at most
+      for (; t0 + NB <= nt; t0 += NB) tokens(t0, std::integral_constant<int, NB>());
+      for (; t0 < nt; ++t0) tokens(t0, std::integral_constant<int, 1>());
+      __syncthreads();
+      continue;
+    }
+    // delta rule: token by token
+    float4 kn[NQ], qn[NQ];
 #pragma unroll
     for (int j = 0; j < NQ; ++j) {
       kn[j] = reinterpret_cast<const float4*>(tok)[r + R * j];
       qn[j] = reinterpret_cast<const float4*>(tok + NP)[r + R * j];
-      if (GLA) an[j] = reinterpret_cast<const float4*>(tok + 2 * NP)[r + R * j];
     }
     for (int t = 0; t < nt; ++t) {
-      float4 kc[NQ], qc[NQ], ac[NQ];
+      float4 kc[NQ], qc[NQ];
       float vc[CPT];
       const float4 s4 = sc[t];
 #pragma unroll
@@ -323,7 +434,6 @@ __global__ void __launch_bounds__(32 * (kOwnerWarps + kStageWarps)) outer_scan_k
       for (int j = 0; j < NQ; ++j) {
         kc[j] = kn[j];
         qc[j] = qn[j];
-        if (GLA) ac[j] = an[j];
       }
       // the next token's vectors (row kChunk of a buffer does not exist: the last token reads its own again)
       const float* nx = tok + (t + 1 < nt ? t + 1 : t) * TOK;
@@ -331,7 +441,6 @@ __global__ void __launch_bounds__(32 * (kOwnerWarps + kStageWarps)) outer_scan_k
       for (int j = 0; j < NQ; ++j) {
         kn[j] = reinterpret_cast<const float4*>(nx)[r + R * j];
         qn[j] = reinterpret_cast<const float4*>(nx + NP)[r + R * j];
-        if (GLA) an[j] = reinterpret_cast<const float4*>(nx + 2 * NP)[r + R * j];
       }
       float d[NV];
 #pragma unroll
@@ -339,51 +448,33 @@ __global__ void __launch_bounds__(32 * (kOwnerWarps + kStageWarps)) outer_scan_k
         float4 ek = make_float4(0.f, 0.f, 0.f, 0.f), eq = ek;   // four partial sums: short chains
 #pragma unroll
         for (int j = 0; j < NQ; ++j) {
-          if (DELTA) {
-            ek.x = fmaf(S[c][j].x, kc[j].x, ek.x); ek.y = fmaf(S[c][j].y, kc[j].y, ek.y);
-            ek.z = fmaf(S[c][j].z, kc[j].z, ek.z); ek.w = fmaf(S[c][j].w, kc[j].w, ek.w);
-          }
+          ek.x = fmaf(S[c][j].x, kc[j].x, ek.x); ek.y = fmaf(S[c][j].y, kc[j].y, ek.y);
+          ek.z = fmaf(S[c][j].z, kc[j].z, ek.z); ek.w = fmaf(S[c][j].w, kc[j].w, ek.w);
           eq.x = fmaf(S[c][j].x, qc[j].x, eq.x); eq.y = fmaf(S[c][j].y, qc[j].y, eq.y);
           eq.z = fmaf(S[c][j].z, qc[j].z, eq.z); eq.w = fmaf(S[c][j].w, qc[j].w, eq.w);
         }
-        if (DELTA) d[c] = (ek.x + ek.y) + (ek.z + ek.w);
+        d[c] = (ek.x + ek.y) + (ek.z + ek.w);
         d[NV - CPT + c] = (eq.x + eq.y) + (eq.z + eq.w);
       }
       transpose_sum<R, NV>(d, r);
-      if (DELTA) {
-        const float g = s4.x, beta = s4.y;
-        float u[CPT], um = 0.f;
+      const float g = s4.x, beta = s4.y;
+      float u[CPT], um = 0.f;
 #pragma unroll
-        for (int c = 0; c < CPT; ++c) {
-          const float dk = __shfl_sync(0xffffffffu, d[0], c * kSpan, R);
-          u[c] = beta * (vc[c] - g * dk);
-          if (c == my_col) um = u[c];
-        }
-        if (writes) yy[t * COLS + cg + my_col] = fmaf(g, d[0], s4.z * um);
-#pragma unroll
-        for (int c = 0; c < CPT; ++c)
-#pragma unroll
-          for (int j = 0; j < NQ; ++j) {
-            S[c][j].x = fmaf(g, S[c][j].x, kc[j].x * u[c]);
-            S[c][j].y = fmaf(g, S[c][j].y, kc[j].y * u[c]);
-            S[c][j].z = fmaf(g, S[c][j].z, kc[j].z * u[c]);
-            S[c][j].w = fmaf(g, S[c][j].w, kc[j].w * u[c]);
-          }
-      } else {
-        float vm = 0.f;
-#pragma unroll
-        for (int c = 0; c < CPT; ++c) {
-          if (c == my_col) vm = vc[c];
-#pragma unroll
-          for (int j = 0; j < NQ; ++j) {
-            S[c][j].x = fmaf(GLA ? ac[j].x : gh, S[c][j].x, kc[j].x * vc[c]);
-            S[c][j].y = fmaf(GLA ? ac[j].y : gh, S[c][j].y, kc[j].y * vc[c]);
-            S[c][j].z = fmaf(GLA ? ac[j].z : gh, S[c][j].z, kc[j].z * vc[c]);
-            S[c][j].w = fmaf(GLA ? ac[j].w : gh, S[c][j].w, kc[j].w * vc[c]);
-          }
-        }
-        if (writes) yy[t * COLS + cg + my_col] = fmaf(s4.z, vm, GLA ? d[0] : gh * d[0]);
+      for (int c = 0; c < CPT; ++c) {
+        const float dk = __shfl_sync(0xffffffffu, d[0], c * kSpan, R);
+        u[c] = beta * (vc[c] - g * dk);
+        if (c == my_col) um = u[c];
       }
+      if (writes) yy[t * COLS + cg + my_col] = fmaf(g, d[0], s4.z * um);
+#pragma unroll
+      for (int c = 0; c < CPT; ++c)
+#pragma unroll
+        for (int j = 0; j < NQ; ++j) {
+          S[c][j].x = fmaf(g, S[c][j].x, kc[j].x * u[c]);
+          S[c][j].y = fmaf(g, S[c][j].y, kc[j].y * u[c]);
+          S[c][j].z = fmaf(g, S[c][j].z, kc[j].z * u[c]);
+          S[c][j].w = fmaf(g, S[c][j].w, kc[j].w * u[c]);
+        }
     }
     __syncthreads();
   }
@@ -392,7 +483,9 @@ __global__ void __launch_bounds__(32 * (kOwnerWarps + kStageWarps)) outer_scan_k
 #pragma unroll
     for (int j = 0; j < NQ; ++j) {
       const int i = 4 * (r + R * j);
-      if (col0 + cg + c < vdim && i < dim) {
+      if (HGRN) {
+        *reinterpret_cast<float4*>(tr_s + (cg + c) * TS + i) = S[c][j];
+      } else if (col0 + cg + c < vdim && i < dim) {
         float* s = stp + static_cast<size_t>(c) * dim + i;
         if (vec_s4) *reinterpret_cast<float4*>(s) = S[c][j];
         else {
@@ -403,12 +496,20 @@ __global__ void __launch_bounds__(32 * (kOwnerWarps + kStageWarps)) outer_scan_k
         }
       }
     }
+  }
+  if (HGRN) {
+    __syncthreads();
+    for (int idx = threadIdx.x; idx < COLS * dim; idx += blockDim.x) {
+      const int i = idx / COLS, c = idx - i * COLS;
+      if (col0 + c < vdim) *state_at(i, c) = tr_s[c * TS + i];
+    }
+  }
 }
 
 template <int MODE, int R, int KPT, int CPT>
 int launch_scan(const ScanArgs& p, int nseq, cudaStream_t stream) {
   constexpr int NP = R * KPT, COLS = kOwnerWarps * (32 / R) * CPT;
-  constexpr size_t smem = sizeof(float) * (2 * kChunk * (MODE == kGla ? 3 : 2) * NP + 4 * kChunk * COLS + 2 * kChunk * 4);
+  constexpr size_t smem = sizeof(float) * (2 * kChunk * (MODE == kGla || MODE == kHgrn2 ? 3 : 2) * NP + 4 * kChunk * COLS + 2 * kChunk * 4);
   static_assert(smem <= 224 * 1024, "outer_scan: shared memory");
   // the staging work of a token is the same for 2 as for 4 columns per group: twice the warps for the narrow form,
   // where an SM holds one or two CTAs, fewer for the wide one, where CTAs share it
@@ -503,6 +604,48 @@ int decay_scan(const vila_decay_scan_params& p, cudaStream_t stream) {
   a.q_scale = p.q_scale;
   a.vec_qk = p.dim % 4 == 0 && rows_aligned4(a.q, p.ld_q, p.in_dtype) && rows_aligned4(a.k, p.ld_k, p.in_dtype);
   return scan_by_dim<kDecay>(a, p.nseq, stream);
+}
+
+int ssd_scan(const vila_ssd_scan_params& p, cudaStream_t stream) {
+  if (p.nseq <= 0) return 0;
+  VB_CHECK(p.H >= 1 && p.G >= 1 && p.H % p.G == 0 && p.P >= 1 && p.N >= 1 && p.N <= 256,
+           "ssd_scan: H=%d G=%d P=%d N=%d (<= 256)", p.H, p.G, p.P, p.N);
+  const size_t es = p.in_dtype ? 4 : 2;
+  const char* base = static_cast<const char*>(p.xbc);
+  ScanArgs a = {};
+  a.v = base;
+  a.k = base + static_cast<size_t>(p.H) * p.P * es;                                       // B
+  a.q = base + (static_cast<size_t>(p.H) * p.P + static_cast<size_t>(p.G) * p.N) * es;    // C
+  a.ldq = a.ldk = a.ldv = p.ld_xbc;
+  a.a = p.dt; a.lda = p.ld_dt;
+  a.z = p.z; a.ldz = p.ld_z;
+  a.A_log = p.A_log; a.bias = p.dt_bias; a.D = p.D;
+  a.state = p.state; a.seqs = p.seqs; a.out = p.out; a.ldo = p.ld_out; a.out_dt = p.out_dtype;
+  a.in_dt = a.a_dt = p.in_dtype;
+  a.H = p.H; a.G = p.G; a.dim = p.N; a.vdim = p.P;
+  a.q_scale = 1.0f;
+  a.vec_qk = p.N % 4 == 0 && rows_aligned4(a.q, p.ld_xbc, p.in_dtype) && rows_aligned4(a.k, p.ld_xbc, p.in_dtype);
+  return scan_by_dim<kSsd>(a, p.nseq, stream);
+}
+
+int hgrn2_scan(const vila_hgrn2_params& p, cudaStream_t stream) {
+  if (p.nseq <= 0) return 0;
+  VB_CHECK(p.dim >= 1 && p.dim <= 256 && p.vdim >= 1 && p.H >= 1, "hgrn2_scan: H=%d dim=%d (<= 256) vdim=%d",
+           p.H, p.dim, p.vdim);
+  const size_t es = p.proj_dtype ? 4 : 2;
+  const char* base = static_cast<const char*>(p.proj);
+  ScanArgs a = {};
+  a.q = base + p.q_off * es;
+  a.k = base + p.f_off * es;
+  a.v = base + p.v_off * es;
+  a.ldq = a.ldk = a.ldv = p.ldp;
+  a.bias = p.f_bias; a.lower = p.lower;
+  a.state = p.state; a.seqs = p.seqs; a.out = p.out; a.ldo = static_cast<int64_t>(p.H) * p.vdim; a.out_dt = VILA_DT_F32;
+  a.in_dt = p.proj_dtype;
+  a.H = a.G = p.H; a.dim = p.dim; a.vdim = p.vdim;
+  a.q_scale = 1.0f;
+  a.vec_qk = p.dim % 4 == 0 && rows_aligned4(a.q, p.ldp, p.proj_dtype) && rows_aligned4(a.k, p.ldp, p.proj_dtype);
+  return scan_by_dim<kHgrn2>(a, p.nseq, stream);
 }
 
 }  // namespace vb
