@@ -200,12 +200,29 @@ __global__ void __launch_bounds__(32 * (kOwnerWarps + kStageWarps)) outer_scan_k
         lw[j] = make_float4(e[0], e[1], e[2], e[3]);
       }
     }
-    auto stage = [&](int ch) {
-      const int t0 = ch * kChunk, nt = min(kChunk, n - t0), bf = ch & 1;
-      float* vb_ = vec_s + bf * kChunk * TOK;
-      // the value columns and (delta) the head's two scalars of every token: loads first
-      constexpr int VN = (kChunk * COLS + kStageWarps * 32 - 1) / (kStageWarps * 32);
-      uint32_t rv[VN], ra = 0u, rb = 0u;
+    // raw bits of a stage: value columns, (delta, ssd) the head's scalars, and, where a warp's tokens fit its registers,
+    // the vectors.  They are requested one stage ahead: nothing waits for them before the next barrier.
+    constexpr int VN = (kChunk * COLS + kStageWarps * 32 - 1) / (kStageWarps * 32);
+    constexpr bool AHEAD = TB == TPW;
+    uint32_t rv[VN], ra = 0u, rb = 0u, rg[VN];
+    uint4 rk[TB][NG], rq[TB][NG], rz[TB][NG];
+    auto fetch_vectors = [&](int ch, int tb) {
+      const int t0 = ch * kChunk, nt = min(kChunk, n - t0);
+#pragma unroll
+      for (int u = 0; u < TB; ++u) {
+        const int t = sw + (tb + u) * kStageWarps;
+        const size_t row = static_cast<size_t>(row0 + t0 + t);
+#pragma unroll
+        for (int j = 0; j < NG; ++j) {
+          const int i = t < nt ? 4 * (lane + 32 * j) : dim;
+          rk[u][j] = ld_raw4(p.k, dt, row * p.ldk + qoff, i, dim, p.vec_qk != 0);
+          rq[u][j] = ld_raw4(p.q, dt, row * p.ldq + qoff, i, dim, p.vec_qk != 0);
+          if (MODE == kGla) rz[u][j] = ld_raw4(p.a, adt, row * p.lda + zoff, i, dim, p.vec_a != 0);
+        }
+      }
+    };
+    auto fetch = [&](int ch) {
+      const int t0 = ch * kChunk, nt = min(kChunk, n - t0);
 #pragma unroll
       for (int k = 0; k < VN; ++k) {
         const int idx = st + k * kStageWarps * 32, t = idx / COLS, c = col0 + idx % COLS;
@@ -215,21 +232,23 @@ __global__ void __launch_bounds__(32 * (kOwnerWarps + kStageWarps)) outer_scan_k
         ra = ld_raw(p.a, adt, static_cast<size_t>(row0 + t0 + st) * p.lda + h);
         if (DELTA) rb = ld_raw(p.b, adt, static_cast<size_t>(row0 + t0 + st) * p.ldb + h);
       }
+      if (AHEAD) fetch_vectors(ch, 0);
+    };
+    auto fetch_gates = [&](int ch) {   // ssd: of a stage's outputs
+      if (!SSD || p.z == nullptr) return;
+      const int t0 = ch * kChunk, nt = min(kChunk, n - t0);
+#pragma unroll
+      for (int k = 0; k < VN; ++k) {
+        const int idx = st + k * kStageWarps * 32, t = idx / COLS, c = col0 + idx % COLS;
+        rg[k] = (t < nt && c < vdim) ? ld_raw(p.z, dt, static_cast<size_t>(row0 + t0 + t) * p.ldz + voff + c) : 0u;
+      }
+    };
+    auto stage = [&](int ch) {
+      const int t0 = ch * kChunk, nt = min(kChunk, n - t0), bf = ch & 1;
+      float* vb_ = vec_s + bf * kChunk * TOK;
 #pragma unroll 1
       for (int tb = 0; tb < TPW; tb += TB) {
-        uint4 rk[TB][NG], rq[TB][NG], rz[TB][NG];
-#pragma unroll
-        for (int u = 0; u < TB; ++u) {
-          const int t = sw + (tb + u) * kStageWarps;
-          const size_t row = static_cast<size_t>(row0 + t0 + t);
-#pragma unroll
-          for (int j = 0; j < NG; ++j) {
-            const int i = t < nt ? 4 * (lane + 32 * j) : dim;
-            rk[u][j] = ld_raw4(p.k, dt, row * p.ldk + qoff, i, dim, p.vec_qk != 0);
-            rq[u][j] = ld_raw4(p.q, dt, row * p.ldq + qoff, i, dim, p.vec_qk != 0);
-            if (MODE == kGla) rz[u][j] = ld_raw4(p.a, adt, row * p.lda + zoff, i, dim, p.vec_a != 0);
-          }
-        }
+        if (!AHEAD) fetch_vectors(ch, tb);
 #pragma unroll
         for (int u = 0; u < TB; ++u) {
           const int t = sw + (tb + u) * kStageWarps;
@@ -309,19 +328,26 @@ __global__ void __launch_bounds__(32 * (kOwnerWarps + kStageWarps)) outer_scan_k
     auto flush = [&](int ch) {
       const int t0 = ch * kChunk, nt = min(kChunk, n - t0);
       const float* y = y_s + (ch & 1) * kChunk * COLS;
-      for (int idx = st; idx < nt * COLS; idx += kStageWarps * 32) {
-        const int t = idx / COLS, c = col0 + idx % COLS;
-        if (c >= vdim) continue;
-        const size_t row = static_cast<size_t>(row0 + t0 + t), at = row * p.ldo + voff + c;
-        if (SSD) st_any(p.out, p.out_dt, at, p.z ? y[idx] * silu_exact_f(ld_any(p.z, dt, row * p.ldz + voff + c)) : y[idx]);
+#pragma unroll
+      for (int k = 0; k < VN; ++k) {
+        const int idx = st + k * kStageWarps * 32, t = idx / COLS, c = col0 + idx % COLS;
+        if (idx >= nt * COLS || c >= vdim) continue;
+        const size_t at = static_cast<size_t>(row0 + t0 + t) * p.ldo + voff + c;
+        if (SSD) st_any(p.out, p.out_dt, at, p.z ? y[idx] * silu_exact_f(raw_to_float(rg[k], dt)) : y[idx]);
         else static_cast<float*>(p.out)[at] = y[idx];
       }
     };
-    stage(0);
+    if (nchunks > 0) {
+      fetch(0);
+      stage(0);
+      if (nchunks > 1) fetch(1);
+    }
     __syncthreads();
     for (int ch = 0; ch < nchunks; ++ch) {
-      if (ch + 1 < nchunks) stage(ch + 1);
       if (ch > 0) flush(ch - 1);
+      fetch_gates(ch);
+      if (ch + 1 < nchunks) stage(ch + 1);
+      if (ch + 2 < nchunks) fetch(ch + 2);
       __syncthreads();
     }
     if (nchunks > 0) flush(nchunks - 1);
