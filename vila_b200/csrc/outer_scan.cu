@@ -16,11 +16,10 @@
 //                  S <- diag(f) S + (1 - f) v^T;  o = S^T q,   f = lower + (1 - lower) sigmoid(zf + bias), q = silu(zq);
 //                  its state is stored [.., dim, vdim] and passes through shared memory once at either end
 //
-// The read-outs are taken from the state BEFORE the token's write, which is the same number and shortens the chain
-// of dependent steps to one pass over the state per token:
-//   delta:  S_new^T q = g (S^T q) + (k . q) u        so S^T k and S^T q are reduced together
-//   gla:    S_new^T q = S^T (alpha q) + (k . q) v    so the state update does not wait for the reduction
-//   decay, ssd:  S_new^T q = g (S^T q) + (k . q) v   likewise;  hgrn2 as gla
+// The delta rule's read-outs are taken from the state BEFORE the token's write, which is the same number and shortens the
+// chain of dependent steps to one pass over the state per token:
+//   S_new^T q = g (S^T q) + (k . q) u        so S^T k and S^T q are reduced together
+// The others read the state after its write; nothing that follows waits for their sums.
 //
 // Grid (sequence, head, COLS columns of vdim).  Warps 0-3 own the state: R lanes share CPT columns, lane r
 // keeps the float4 pieces r, r + R, .. of a column in registers (state layout [.., vdim, dim]: coalesced loads, and
@@ -30,7 +29,7 @@
 // and write the previous 16 tokens' outputs while the owners run; one barrier per 16 tokens.
 // Only the delta rule needs a token's sums before its write.  The others take kBatch tokens at a time: every owner keeps
 // the batch's partial sums and one tree reduces them together (half the shuffles, and the tree's latency under the next
-// tokens' products).
+// tokens' products), two state entries per instruction (fma.rn.f32x2).  They are bound by instruction issue: MEASURED_SCAN
 // A column's sum runs in the same order whatever CPT and the batch are, and time runs in order: a row's result depends neither on
 // the batch nor on how its sequence was cut into steps.
 #include <type_traits>
@@ -80,6 +79,29 @@ __device__ __forceinline__ float dot4(float4 a, float4 b, float s) {
   s = fmaf(a.y, b.y, s);
   s = fmaf(a.z, b.z, s);
   return fmaf(a.w, b.w, s);
+}
+
+// two fp32 numbers in one register pair
+using f2 = unsigned long long;
+__device__ __forceinline__ f2 pair(float x, float y) {
+  f2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(x), "f"(y));
+  return r;
+}
+__device__ __forceinline__ float2 unpair(f2 v) {
+  float2 r;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+  return r;
+}
+__device__ __forceinline__ f2 mul2(f2 a, f2 b) {
+  f2 r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ f2 fma2(f2 a, f2 b, f2 c) {
+  f2 r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
 }
 
 // Sum NV values per lane over the R lanes of a group.  Afterwards v[0] of lane r is the complete sum of value
@@ -177,6 +199,7 @@ __global__ void __launch_bounds__(32 * (kOwnerWarps + kStageWarps)) outer_scan_k
     if (HGRN) __syncthreads();                       // the owners have taken their columns
     const int sw = warp - kOwnerWarps, st = threadIdx.x - kOwnerWarps * 32;
     const int dt = p.in_dt, adt = p.a_dt;
+    const bool bf16_vec = dt == VILA_DT_BF16 && p.vec_qk && (MODE != kGla || (adt == VILA_DT_BF16 && p.vec_a));
     const size_t qoff = static_cast<size_t>(kh) * dim, voff = static_cast<size_t>(h) * vdim;
     const size_t zoff = static_cast<size_t>(h) * dim;
     const float neg_a = DELTA || SSD ? -expf(p.A_log[h]) : 0.f, dbias = DELTA || SSD ? p.bias[h] : 0.f;
@@ -208,6 +231,28 @@ __global__ void __launch_bounds__(32 * (kOwnerWarps + kStageWarps)) outer_scan_k
     uint4 rk[TB][NG], rq[TB][NG], rz[TB][NG];
     auto fetch_vectors = [&](int ch, int tb) {
       const int t0 = ch * kChunk, nt = min(kChunk, n - t0);
+      if (bf16_vec) {   // one branch around all loads
+#pragma unroll
+        for (int u = 0; u < TB; ++u) {
+          const int t = sw + (tb + u) * kStageWarps;
+          const size_t row = static_cast<size_t>(row0 + t0 + t);
+#pragma unroll
+          for (int j = 0; j < NG; ++j) {
+            const int i = 4 * (lane + 32 * j);
+            const bool in = t < nt && i < dim;
+            const uint2 z = make_uint2(0u, 0u);
+            const uint2 k2 = in ? __ldg(reinterpret_cast<const uint2*>(static_cast<const __nv_bfloat16*>(p.k) + row * p.ldk + qoff + i)) : z;
+            const uint2 q2 = in ? __ldg(reinterpret_cast<const uint2*>(static_cast<const __nv_bfloat16*>(p.q) + row * p.ldq + qoff + i)) : z;
+            rk[u][j] = make_uint4(k2.x, k2.y, 0u, 0u);
+            rq[u][j] = make_uint4(q2.x, q2.y, 0u, 0u);
+            if (MODE == kGla) {
+              const uint2 a2 = in ? __ldg(reinterpret_cast<const uint2*>(static_cast<const __nv_bfloat16*>(p.a) + row * p.lda + zoff + i)) : z;
+              rz[u][j] = make_uint4(a2.x, a2.y, 0u, 0u);
+            }
+          }
+        }
+        return;
+      }
 #pragma unroll
       for (int u = 0; u < TB; ++u) {
         const int t = sw + (tb + u) * kStageWarps;
@@ -271,28 +316,29 @@ __global__ void __launch_bounds__(32 * (kOwnerWarps + kStageWarps)) outer_scan_k
               kv[j] = silu4(kv[j]);
               qv[j] = silu4(qv[j]);
             }
-            kq = dot4(kv[j], qv[j], kq);
             if (DELTA) {
+              kq = dot4(kv[j], qv[j], kq);
               kk = dot4(kv[j], kv[j], kk);
               qq = dot4(qv[j], qv[j], qq);
             }
           }
+          float ks = 1.0f, qs = 1.0f;
+          if (DELTA) {
 #pragma unroll
-          for (int o = 16; o > 0; o >>= 1) {
-            kq += __shfl_xor_sync(0xffffffffu, kq, o);
-            if (DELTA) {
+            for (int o = 16; o > 0; o >>= 1) {
+              kq += __shfl_xor_sync(0xffffffffu, kq, o);
               kk += __shfl_xor_sync(0xffffffffu, kk, o);
               qq += __shfl_xor_sync(0xffffffffu, qq, o);
             }
+            ks = 1.0f / sqrtf(kk + p.eps);
+            qs = 1.0f / sqrtf(qq + p.eps) * p.q_scale;
           }
-          const float ks = DELTA ? 1.0f / sqrtf(kk + p.eps) : 1.0f;
-          const float qs = (DELTA ? 1.0f / sqrtf(qq + p.eps) : 1.0f) * p.q_scale;
           float* kd = vb_ + t * TOK;
 #pragma unroll
           for (int j = 0; j < NG; ++j) {
             const int i = 4 * (lane + 32 * j);
             if (i < NP) {
-              float4 q4 = make_float4(qv[j].x * qs, qv[j].y * qs, qv[j].z * qs, qv[j].w * qs);
+              const float4 q4 = make_float4(qv[j].x * qs, qv[j].y * qs, qv[j].z * qs, qv[j].w * qs);
               *reinterpret_cast<float4*>(kd + i) = make_float4(kv[j].x * ks, kv[j].y * ks, kv[j].z * ks, kv[j].w * ks);
               if (GLA) {
                 float4 al;
@@ -303,13 +349,12 @@ __global__ void __launch_bounds__(32 * (kOwnerWarps + kStageWarps)) outer_scan_k
                   al = make_float4(expf(-softplus_f(-(z.x + zb[j].x)) * p.inv_tau), expf(-softplus_f(-(z.y + zb[j].y)) * p.inv_tau),
                                    expf(-softplus_f(-(z.z + zb[j].z)) * p.inv_tau), expf(-softplus_f(-(z.w + zb[j].w)) * p.inv_tau));
                 }
-                q4 = make_float4(q4.x * al.x, q4.y * al.y, q4.z * al.z, q4.w * al.w);
                 *reinterpret_cast<float4*>(kd + 2 * NP + i) = al;
               }
               *reinterpret_cast<float4*>(kd + NP + i) = q4;
             }
           }
-          if (lane == 0) reinterpret_cast<float*>(sc_s + bf * kChunk + t)[2] = kq * ks * qs;
+          if (DELTA && lane == 0) reinterpret_cast<float*>(sc_s + bf * kChunk + t)[2] = kq * ks * qs;
         }
       }
 #pragma unroll
@@ -379,6 +424,14 @@ __global__ void __launch_bounds__(32 * (kOwnerWarps + kStageWarps)) outer_scan_k
         }
       }
     }
+  f2 P[CPT][NQ][2];                                // the state in pairs (all but the delta rule)
+#pragma unroll
+  for (int c = 0; c < CPT; ++c)
+#pragma unroll
+    for (int j = 0; j < NQ; ++j) {
+      P[c][j][0] = pair(S[c][j].x, S[c][j].y);
+      P[c][j][1] = pair(S[c][j].z, S[c][j].w);
+    }
   constexpr int kSpan = R / NV;                    // neighbouring lanes that end up with the same sum
   const int mine = r / kSpan;                      // which of the NV sums this lane ends up with
   const int my_col = DELTA ? mine - CPT : mine;    // its column, if it is a read-out
@@ -400,41 +453,42 @@ __global__ void __launch_bounds__(32 * (kOwnerWarps + kStageWarps)) outer_scan_k
 #pragma unroll
         for (int u = 0; u < NT; ++u) {
           const float* tk = tok + (t0 + u) * TOK;
-          const float4 s4 = sc[t0 + u];
-          const float g = SSD ? s4.x : gh;
-          float w[CPT];
+          const float2 s2 = SSD ? *reinterpret_cast<const float2*>(sc + t0 + u) : make_float2(0.f, 0.f);   // decay, step
+          const float g = SSD ? s2.x : gh;
+          f2 w[CPT], eq[CPT][2];
 #pragma unroll
-          for (int c = 0; c < CPT; ++c) w[c] = SSD ? s4.y * vv[(t0 + u) * COLS + cg + c] : vv[(t0 + u) * COLS + cg + c];
-          float4 eq[CPT];
-#pragma unroll
-          for (int c = 0; c < CPT; ++c) eq[c] = make_float4(0.f, 0.f, 0.f, 0.f);   // four partial sums: short chains
-#pragma unroll
-          for (int j = 0; j < NQ; ++j) {
-            const float4 kc = reinterpret_cast<const float4*>(tk)[r + R * j], qc = reinterpret_cast<const float4*>(tk + NP)[r + R * j];
-            float4 al = make_float4(g, g, g, g);
-            if (GLA) al = reinterpret_cast<const float4*>(tk + 2 * NP)[r + R * j];
-#pragma unroll
-            for (int c = 0; c < CPT; ++c) {
-              eq[c].x = fmaf(S[c][j].x, qc.x, eq[c].x); eq[c].y = fmaf(S[c][j].y, qc.y, eq[c].y);
-              eq[c].z = fmaf(S[c][j].z, qc.z, eq[c].z); eq[c].w = fmaf(S[c][j].w, qc.w, eq[c].w);
-              S[c][j].x = fmaf(al.x, S[c][j].x, kc.x * w[c]);
-              S[c][j].y = fmaf(al.y, S[c][j].y, kc.y * w[c]);
-              S[c][j].z = fmaf(al.z, S[c][j].z, kc.z * w[c]);
-              S[c][j].w = fmaf(al.w, S[c][j].w, kc.w * w[c]);
-            }
+          for (int c = 0; c < CPT; ++c) {
+            const float x = SSD ? s2.y * vv[(t0 + u) * COLS + cg + c] : vv[(t0 + u) * COLS + cg + c];
+            w[c] = pair(x, x);
+            eq[c][0] = eq[c][1] = 0ull;                // four partial sums: short chains
           }
 #pragma unroll
-          for (int c = 0; c < CPT; ++c) d[u * CPT + c] = (eq[c].x + eq[c].y) + (eq[c].z + eq[c].w);
+          for (int j = 0; j < NQ; ++j) {
+            const ulonglong2 k4 = reinterpret_cast<const ulonglong2*>(tk)[r + R * j], q4 = reinterpret_cast<const ulonglong2*>(tk + NP)[r + R * j];
+            const f2 kp[2] = {k4.x, k4.y}, qp[2] = {q4.x, q4.y};
+            f2 al[2] = {pair(g, g), pair(g, g)};
+            if (GLA) {
+              const ulonglong2 a4 = reinterpret_cast<const ulonglong2*>(tk + 2 * NP)[r + R * j];
+              al[0] = a4.x;
+              al[1] = a4.y;
+            }
+#pragma unroll
+            for (int c = 0; c < CPT; ++c)
+#pragma unroll
+              for (int e = 0; e < 2; ++e) {
+                P[c][j][e] = fma2(al[e], P[c][j][e], mul2(kp[e], w[c]));
+                eq[c][e] = fma2(P[c][j][e], qp[e], eq[c][e]);
+              }
+          }
+#pragma unroll
+          for (int c = 0; c < CPT; ++c) {
+            const float2 lo = unpair(eq[c][0]), hi = unpair(eq[c][1]);
+            d[u * CPT + c] = (lo.x + lo.y) + (hi.x + hi.y);
+          }
         }
         transpose_sum<R, NS>(d, r);
         const int own = r / SPAN, tt = t0 + own / CPT, cc = cg + own % CPT;   // the sum this lane ends up with
-        const float4 s4 = sc[tt];
-        const float x = vv[tt * COLS + cc], g = SSD ? s4.x : gh;
-        if (r % SPAN == 0) {
-          float y = fmaf(s4.z, SSD ? s4.y * x : x, GLA ? d[0] : g * d[0]);
-          if (SSD) y = fmaf(Dh, x, y);
-          yy[tt * COLS + cc] = y;
-        }
+        if (r % SPAN == 0) yy[tt * COLS + cc] = SSD ? fmaf(Dh, vv[tt * COLS + cc], d[0]) : p.q_scale * d[0];
       };
       int t0 = 0;
       constexpr int NB = R / CPT < kBatch ? R / CPT : kBatch;   // a lane ends up with one sum at most
@@ -509,6 +563,10 @@ __global__ void __launch_bounds__(32 * (kOwnerWarps + kStageWarps)) outer_scan_k
 #pragma unroll
     for (int j = 0; j < NQ; ++j) {
       const int i = 4 * (r + R * j);
+      if (!DELTA) {
+        const float2 lo = unpair(P[c][j][0]), hi = unpair(P[c][j][1]);
+        S[c][j] = make_float4(lo.x, lo.y, hi.x, hi.y);
+      }
       if (HGRN) {
         *reinterpret_cast<float4*>(tr_s + (cg + c) * TS + i) = S[c][j];
       } else if (col0 + cg + c < vdim && i < dim) {
