@@ -435,6 +435,8 @@ typedef struct vila_hgrn2_params {
   int32_t proj_dtype, q_off, f_off, v_off, nseq, H, dim, vdim;
 } vila_hgrn2_params;
 int vila_hgrn2_scan(const vila_hgrn2_params* p, void* stream);
+/* The same where every sequence brings one row (decoded tokens). */
+int vila_hgrn2_step(const vila_hgrn2_params* p, void* stream);
 
 /* Router of a mixture of experts: z = w_router x + bias in fp32, the `top` largest logits (ties: the
  * lower index), weights = softmax over the chosen logits.  idx / weight are [rows, top]. */

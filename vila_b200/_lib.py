@@ -294,6 +294,7 @@ SIGNATURES = {
     "vila_latent_attention": [C.POINTER(LatentAttnParams), c_void_p],
     "vila_latent_rope_append": [C.POINTER(LatentRopeParams), c_void_p],
     "vila_hgrn2_scan": [C.POINTER(Hgrn2Params), c_void_p],
+    "vila_hgrn2_step": [C.POINTER(Hgrn2Params), c_void_p],
     "vila_sink_attention": [C.POINTER(SinkAttnParams), c_void_p],
     "vila_gather_rows": [c_void_p, c_void_p, c_void_p, c_int, c_int, c_void_p],
     "vila_moe_route": [c_void_p, c_int, c_i64, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int,

@@ -34,6 +34,7 @@ SOURCES = [
     "glinear.cu",
     "glinear_tcgen05.cu",
     "latent_attn.cu",
+    "hgrn2.cu",
     "short_conv.cu",
     "paged_attn.cu",
     "paged_attn_mma.cu",

@@ -400,6 +400,11 @@ int vila_hgrn2_scan(const vila_hgrn2_params* p, void* stream) {
   return vb::hgrn2_scan(*p, st(stream));
 }
 
+int vila_hgrn2_step(const vila_hgrn2_params* p, void* stream) {
+  VB_REQUIRE_DEVICE();
+  return vb::hgrn2_step(*p, st(stream));
+}
+
 int vila_moe_route(const void* x, int x_dtype, int64_t ldx, const float* w_router, const float* bias,
                    int32_t* idx, float* weight, int rows, int cols, int experts, int top, void* stream) {
   VB_REQUIRE_DEVICE();

@@ -308,5 +308,6 @@ int glinear(const vila_glinear_params& p, cudaStream_t stream, const vila_glinea
 int latent_attention(const vila_latent_attn_params& p, cudaStream_t stream);
 int latent_rope_append(const vila_latent_rope_params& p, cudaStream_t stream);
 int hgrn2_scan(const vila_hgrn2_params& p, cudaStream_t stream);
+int hgrn2_step(const vila_hgrn2_params& p, cudaStream_t stream);
 
 }  // namespace vb

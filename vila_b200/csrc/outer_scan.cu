@@ -14,7 +14,7 @@
 //                  dt = softplus(dt_raw + dt_bias);  heads share the B / C of their group
 //   hgrn2_scan   one decay per key channel, which also sets the input gate:
 //                  S <- diag(f) S + (1 - f) v^T;  o = S^T q,   f = lower + (1 - lower) sigmoid(zf + bias), q = silu(zq);
-//                  its state is stored [.., dim, vdim] and passes through shared memory once at either end
+//                  its state is stored [.., dim, vdim]
 //
 // The delta rule's read-outs are taken from the state BEFORE the token's write, which is the same number and shortens the
 // chain of dependent steps to one pass over the state per token:
@@ -29,7 +29,9 @@
 // and write the previous 16 tokens' outputs while the owners run; one barrier per 16 tokens.
 // Only the delta rule needs a token's sums before its write.  The others take kBatch tokens at a time: every owner keeps
 // the batch's partial sums and one tree reduces them together (half the shuffles, and the tree's latency under the next
-// tokens' products), two state entries per instruction (fma.rn.f32x2).  They are bound by instruction issue: MEASURED_SCAN
+// tokens' products), two state entries per instruction (fma.rn.f32x2).  They are bound by
+// instruction issue (2.9 of 4 per clock).  2048 rows of one sequence, 16 heads of 128 x 128: decay 329 -> 238 us, gla 327 -> 243,
+// hgrn2 1208 -> 242 and ssd (64 heads of 64 x 128) 785 -> 304 from the forms that kept one column per thread group.
 // A column's sum runs in the same order whatever CPT and the batch are, and time runs in order: a row's result depends neither on
 // the batch nor on how its sequence was cut into steps.
 #include <type_traits>
@@ -179,24 +181,8 @@ __global__ void __launch_bounds__(32 * (kOwnerWarps + kStageWarps)) outer_scan_k
   const int col0 = blockIdx.z * COLS;
   const int nchunks = (n + kChunk - 1) / kChunk;
 
-  // hgrn2: the state's columns through shared memory (coalesced rows of vdim in global memory), padded rows
-  float* tr_s = vec_s;
-  constexpr int TS = NP + 4;
-  auto state_at = [&](int i, int c) {
-    return p.state + ((static_cast<size_t>(slot) * p.H + h) * dim + i) * vdim + col0 + c;
-  };
-  if (HGRN) {
-    static_assert(!HGRN || COLS * TS <= 2 * kChunk * TOK, "the transposed state fits the staging buffers");
-    for (int idx = threadIdx.x; idx < COLS * dim; idx += blockDim.x) {
-      const int i = idx / COLS, c = idx - i * COLS;
-      tr_s[c * TS + i] = pos0 > 0 && col0 + c < vdim ? *state_at(i, c) : 0.f;
-    }
-    __syncthreads();
-  }
-
   if (warp >= kOwnerWarps) {
     // ---------------- staging warps ----------------
-    if (HGRN) __syncthreads();                       // the owners have taken their columns
     const int sw = warp - kOwnerWarps, st = threadIdx.x - kOwnerWarps * 32;
     const int dt = p.in_dt, adt = p.a_dt;
     const bool bf16_vec = dt == VILA_DT_BF16 && p.vec_qk && (MODE != kGla || (adt == VILA_DT_BF16 && p.vec_a));
@@ -408,12 +394,7 @@ __global__ void __launch_bounds__(32 * (kOwnerWarps + kStageWarps)) outer_scan_k
     for (int j = 0; j < NQ; ++j) {
       S[c][j] = make_float4(0.f, 0.f, 0.f, 0.f);
       const int i = 4 * (r + R * j);
-      if (HGRN) {
-        if (i < dim) S[c][j] = *reinterpret_cast<const float4*>(tr_s + (cg + c) * TS + i);   // rows past dim are never stored
-        if (i + 1 >= dim) S[c][j].y = 0.f;
-        if (i + 2 >= dim) S[c][j].z = 0.f;
-        if (i + 3 >= dim) S[c][j].w = 0.f;
-      } else if (pos0 > 0 && col0 + cg + c < vdim && i < dim) {
+      if (!HGRN && pos0 > 0 && col0 + cg + c < vdim && i < dim) {
         const float* s = stp + static_cast<size_t>(c) * dim + i;
         if (vec_s4) S[c][j] = *reinterpret_cast<const float4*>(s);
         else {
@@ -424,6 +405,33 @@ __global__ void __launch_bounds__(32 * (kOwnerWarps + kStageWarps)) outer_scan_k
         }
       }
     }
+  // hgrn2's state: key channel i of the lane's CPT columns in one access where they are aligned (the four owner warps
+  // use the 64 or 128 bytes of a channel together)
+  auto hgrn_rows = [&](auto access) {
+#pragma unroll
+    for (int j = 0; j < NQ; ++j)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const int i = 4 * (r + R * j) + e;
+        if (i < dim) access(p.state + ((static_cast<size_t>(slot) * p.H + h) * dim + i) * vdim + col0 + cg, j, e);
+      }
+  };
+  auto entry = [&](int c, int j, int e) -> float& { return e == 0 ? S[c][j].x : e == 1 ? S[c][j].y : e == 2 ? S[c][j].z : S[c][j].w; };
+  const bool wide = vdim % CPT == 0 && col0 + cg < vdim;
+  if (HGRN && pos0 > 0)
+    hgrn_rows([&](const float* s, int j, int e) {
+      if (wide) {
+        float v[CPT];
+        if (CPT == 4) *reinterpret_cast<float4*>(v) = *reinterpret_cast<const float4*>(s);
+        else *reinterpret_cast<float2*>(v) = *reinterpret_cast<const float2*>(s);
+#pragma unroll
+        for (int c = 0; c < CPT; ++c) entry(c, j, e) = v[c];
+      } else {
+#pragma unroll
+        for (int c = 0; c < CPT; ++c)
+          if (col0 + cg + c < vdim) entry(c, j, e) = s[c];
+      }
+    });
   f2 P[CPT][NQ][2];                                // the state in pairs (all but the delta rule)
 #pragma unroll
   for (int c = 0; c < CPT; ++c)
@@ -437,7 +445,6 @@ __global__ void __launch_bounds__(32 * (kOwnerWarps + kStageWarps)) outer_scan_k
   const int my_col = DELTA ? mine - CPT : mine;    // its column, if it is a read-out
   const bool writes = my_col >= 0 && (r % kSpan) == 0;
   const float gh = MODE == kDecay ? p.decay[h] : 0.f, Dh = SSD ? p.D[h] : 0.f;
-  if (HGRN) __syncthreads();
   __syncthreads();
   for (int ch = 0; ch < nchunks; ++ch) {
     const int nt = min(kChunk, n - ch * kChunk), bf = ch & 1;
@@ -567,9 +574,7 @@ __global__ void __launch_bounds__(32 * (kOwnerWarps + kStageWarps)) outer_scan_k
         const float2 lo = unpair(P[c][j][0]), hi = unpair(P[c][j][1]);
         S[c][j] = make_float4(lo.x, lo.y, hi.x, hi.y);
       }
-      if (HGRN) {
-        *reinterpret_cast<float4*>(tr_s + (cg + c) * TS + i) = S[c][j];
-      } else if (col0 + cg + c < vdim && i < dim) {
+      if (!HGRN && col0 + cg + c < vdim && i < dim) {
         float* s = stp + static_cast<size_t>(c) * dim + i;
         if (vec_s4) *reinterpret_cast<float4*>(s) = S[c][j];
         else {
@@ -580,13 +585,20 @@ __global__ void __launch_bounds__(32 * (kOwnerWarps + kStageWarps)) outer_scan_k
         }
       }
     }
-  }
-  if (HGRN) {
-    __syncthreads();
-    for (int idx = threadIdx.x; idx < COLS * dim; idx += blockDim.x) {
-      const int i = idx / COLS, c = idx - i * COLS;
-      if (col0 + c < vdim) *state_at(i, c) = tr_s[c * TS + i];
-    }
+  if (HGRN)
+    hgrn_rows([&](float* s, int j, int e) {
+      if (wide) {
+        float v[CPT];
+#pragma unroll
+        for (int c = 0; c < CPT; ++c) v[c] = entry(c, j, e);
+        if (CPT == 4) *reinterpret_cast<float4*>(s) = *reinterpret_cast<const float4*>(v);
+        else *reinterpret_cast<float2*>(s) = *reinterpret_cast<const float2*>(v);
+      } else {
+#pragma unroll
+        for (int c = 0; c < CPT; ++c)
+          if (col0 + cg + c < vdim) s[c] = entry(c, j, e);
+      }
+    });
   }
 }
 
@@ -608,8 +620,8 @@ int launch_scan(const ScanArgs& p, int nseq, cudaStream_t stream) {
   return 0;
 }
 
-// columns per lane group: four where the launch still fills the machine twice over, else fewer, so that one long
-// prompt spreads over more CTAs
+// columns per lane group: four where the launch still fills the machine twice over, else two, so that one long
+// prompt spreads over more CTAs (ssd, 64 heads of 64 columns, 2048 rows: 128 CTAs of four 337 us, 256 of two 304)
 template <int MODE, int R, int KPT>
 int pick_columns(const ScanArgs& p, int nseq, cudaStream_t stream) {
   const long groups = static_cast<long>(nseq) * p.H * ((p.vdim + 4 * (32 / R) - 1) / (4 * (32 / R)));   // CTAs at CPT = 1

@@ -625,7 +625,10 @@ def hgrn2_scan(proj: torch.Tensor, state: torch.Tensor, seqs: torch.Tensor, *, h
     p.state, p.seqs, p.out = _p(state), _i32(seqs, "seqs"), _p(out)
     p.q_off, p.f_off, p.v_off = q_off, f_off, v_off
     p.nseq, p.H, p.dim, p.vdim = seqs.shape[0], heads, dim, vdim
-    check(_lib.load().vila_hgrn2_scan(C.byref(p), _stream()), "vila_hgrn2_scan")
+    if proj.shape[0] == p.nseq:   # one row per sequence (decoded tokens)
+        check(_lib.load().vila_hgrn2_step(C.byref(p), _stream()), "vila_hgrn2_step")
+    else:
+        check(_lib.load().vila_hgrn2_scan(C.byref(p), _stream()), "vila_hgrn2_scan")
     return out
 
 
