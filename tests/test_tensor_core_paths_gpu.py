@@ -247,3 +247,15 @@ def test_rope_append_pairs(ops, dim, rot, halves, dtype):
     assert rel(q, want_q.reshape(T, -1)) < 5e-7
     want_v = 0.7 * qkv.double()[:, (H + G) * dim:] + 0.3 * vf.double()
     assert rel(pool[rows.long()], torch.cat([want_k.reshape(T, -1), want_v], 1)) < 5e-7
+
+
+@pytest.mark.parametrize("form", list(ATT_FORMS))
+@pytest.mark.parametrize("rep", [1, 2, 4, 8])
+@pytest.mark.parametrize("nsplit", [1, 3, 16])
+def test_paged_attention_decode(ops, form, rep, nsplit):
+    """one row per sequence: contexts below, at and past a group of 16 keys and past all the warps of a cluster"""
+    o = ATT_FORMS[form]
+    D = 64 if "diff" in o else 128
+    seqs = [(1, p) for p in (0, 15, 16, 130, 1500)]
+    got, want, _ = attention_case(ops, o, 2 * rep, 2, D, 128, 64 if rep % 2 else 48, seqs, seed=rep, max_rows=1, nsplit=nsplit)
+    assert rel(got, want) < 2e-6

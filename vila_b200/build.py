@@ -38,6 +38,7 @@ SOURCES = [
     "short_conv.cu",
     "paged_attn.cu",
     "paged_attn_mma.cu",
+    "paged_attn_decode.cu",
     "ssm.cu",
     "outer_scan.cu",
 ]

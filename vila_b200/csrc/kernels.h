@@ -297,6 +297,9 @@ int rope_append(const vila_rope_append_params& p, cudaStream_t stream);
 // prompt portions over a bf16 pool, head sizes 64 / 128, heads not mixed: tensor cores (paged_attn_mma.cu)
 bool paged_attention_mma_takes(const vila_paged_attn_params& p);
 int paged_attention_mma(const vila_paged_attn_params& p, cudaStream_t stream);
+// decoded tokens over a bf16 pool, 128 key and value columns, heads not mixed (paged_attn_decode.cu)
+bool paged_attention_decode_takes(const vila_paged_attn_params& p);
+int paged_attention_decode(const vila_paged_attn_params& p, cudaStream_t stream);
 int paged_attention(const vila_paged_attn_params& p, cudaStream_t stream);
 int sink_attention(const vila_sink_attn_params& p, cudaStream_t stream);
 int gather_rows(const void* src, const int32_t* rows, void* dst, int n_rows, int row_bytes, cudaStream_t stream);

@@ -958,6 +958,7 @@ int paged_attention(const vila_paged_attn_params& p, cudaStream_t stream) {
   VB_CHECK(p.max_rows >= 1 && p.max_rows <= 16 && (p.nsplit == 1 || p.max_rows == 1),
            "paged_attention: max_rows=%d nsplit=%d (key splitting serves one-row tiles)", p.max_rows, p.nsplit);
   if (paged_attention_mma_takes(p)) return paged_attention_mma(p, stream);
+  if (paged_attention_decode_takes(p)) return paged_attention_decode(p, stream);
   AttnShape sh;
   sh.phase = -1;
   // Without head mixing the K/V-head groups are independent: a CTA then serves ONE K/V head and its query heads, holds
