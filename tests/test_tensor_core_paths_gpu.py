@@ -259,3 +259,29 @@ def test_paged_attention_decode(ops, form, rep, nsplit):
     seqs = [(1, p) for p in (0, 15, 16, 130, 1500)]
     got, want, _ = attention_case(ops, o, 2 * rep, 2, D, 128, 64 if rep % 2 else 48, seqs, seed=rep, max_rows=1, nsplit=nsplit)
     assert rel(got, want) < 2e-6
+
+
+@pytest.mark.parametrize("M", [1, 2, 3, 4, 5, 8])
+@pytest.mark.parametrize("N,K", [(8, 8), (40, 264), (64, 1024), (136, 1032), (1000, 2720)])
+def test_linear_few_rows(ops, M, N, K):
+    """weight rows and columns below, at and past a warp's four and a pass's 1024; every epilogue; bf16 results: half an ulp,
+    one more for every rounding in between, of values of the size of their row's norm"""
+    g = gen(M * N + K)
+    x, w = randn(g, M, K + 8)[:, :K], (randn(g, N, K).float() * K ** -0.5).to(BF)
+    b, res = randn(g, N), randn(g, M, N)
+    ref = x.double() @ w.double().T
+    bf = lambda t: t.to(BF).double()
+    assert rel(ops.linear(x, w, static_w=True), ref) < 2.0 ** -8
+    z = bf(ref + b.double())
+    assert rel(ops.linear(x, w, b, residual=res), z + res.double()) < 2.0 ** -7
+    for act, fn in ((ops.ACT_GELU_TANH, lambda t: torch.nn.functional.gelu(t, approximate="tanh")), (ops.ACT_GELU_ERF, torch.nn.functional.gelu),
+                    (ops.ACT_SILU, torch.nn.functional.silu), (ops.ACT_RELU2, lambda t: torch.relu(t) ** 2)):
+        assert rel(ops.linear(x, w, b, act=act), fn(z)) < 2.0 ** -7
+    if N % 32 == 0:
+        gt, u = ref[:, 0::2], ref[:, 1::2]
+        assert rel(ops.linear(x, w, swiglu=True), torch.nn.functional.silu(gt) * u) < 2.0 ** -6
+        assert rel(ops.linear(x, w, geglu=True), torch.nn.functional.gelu(gt, approximate="tanh") * u) < 2.0 ** -7
+        c = gt.clamp_max(0.5)
+        assert rel(ops.linear(x, w, glu_clamp=(1.702, 0.5)), c * torch.sigmoid(1.702 * c) * (u.clamp(-0.5, 0.5) + 1)) < 2.0 ** -7
+    many = ops.linear(torch.cat([x] * 3)[:8].contiguous(), w, static_w=True)
+    assert torch.equal(many[:min(M, 8)], ops.linear(x, w, static_w=True))   # a row's result does not depend on how many there are

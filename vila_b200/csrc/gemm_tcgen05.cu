@@ -679,6 +679,8 @@ int gemm_bf16(const __nv_bfloat16* A, int lda, const __nv_bfloat16* W, int ldw, 
               int ldc, int M, int N, int K, const GemmEpilogue& epi, cudaStream_t stream) {
   if (check_args(A, lda, W, ldw, C, ldc, M, N, K, epi)) return 1;
   VB_CHECK(epi.rope_table == nullptr, "gemm: the fused RoPE epilogue is only available through gemm_qkv_rope_bf16");
+  // decoded tokens: the weight stream alone
+  if (gemm_rows_takes(A, lda, W, ldw, M, N, K, epi)) return gemm_rows(A, lda, W, ldw, C, ldc, M, N, K, epi, stream);
   // Tile-shape heuristic. N=256 tiles keep the MMA (not shared-memory bandwidth) the limiter when
   // there is enough work; N=128 otherwise; stream-K (inside launch_gemm) fixes SM under-fill.
   // Measured on B200 (tools/bench_gemm.py): 128x256 tiles win as soon as they fill ~70 % of the

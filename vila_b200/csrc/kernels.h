@@ -39,6 +39,10 @@ int set_workspace(void* ptr, size_t bytes);
 void get_workspace(void** ptr, size_t* bytes);
 int gemm_skinny_bf16(const __nv_bfloat16* A, int lda, const __nv_bfloat16* W, int ldw, __nv_bfloat16* C,
                      int ldc, int M, int N, int K, const GemmEpilogue& epi, int pair, cudaStream_t stream);  // -1: not handled
+// up to 8 rows: fp32 FMA over the streamed weights (gemm_rows.cu)
+bool gemm_rows_takes(const __nv_bfloat16* A, int lda, const __nv_bfloat16* W, int ldw, int M, int N, int K, const GemmEpilogue& epi);
+int gemm_rows(const __nv_bfloat16* A, int lda, const __nv_bfloat16* W, int ldw, __nv_bfloat16* C, int ldc, int M, int N, int K,
+              const GemmEpilogue& epi, cudaStream_t stream);
 int gemm_bf16(const __nv_bfloat16* A, int lda, const __nv_bfloat16* W, int ldw, __nv_bfloat16* C,
               int ldc, int M, int N, int K, const GemmEpilogue& epi, cudaStream_t stream);
 int gemm_qkv_rope_bf16(const __nv_bfloat16* A, int lda, const __nv_bfloat16* W, int ldw, __nv_bfloat16* C,
