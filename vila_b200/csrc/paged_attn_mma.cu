@@ -2,7 +2,9 @@
 //
 // The keys and values are bf16 numbers; the queries and the softmax weights are fp32 and stay so: each is cut into
 // three bf16 parts (8 + 8 + 8 bits) whose products with a bf16 number are exact, and the three products are summed
-// in fp32.  Three bf16 products are cheaper than two tf32 ones and need no range assumptions.
+// in fp32.  Three bf16 products are cheaper than two tf32 ones and need no range assumptions.  (An infinite key or value
+// meets the zero parts of a number that one part holds: the row becomes NaN, as an infinite score or a hidden infinite
+// value makes it in the CUDA-core kernels too.)
 //
 // A warp owns 16 rows of one sequence x one score head (mma.sync m16n8k16: rows x 8 keys, then rows x 8 value columns);
 // scores and sums never leave its registers, the queries' parts lie in shared memory in fragment order.  A CTA serves
