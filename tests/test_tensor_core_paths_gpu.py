@@ -223,6 +223,15 @@ def test_paged_attention_prompt_extremes(ops):
     assert torch.isnan(ops.paged_attention(q, pool, tables, tiles, **kw)[3, :128]).all()
 
 
+@pytest.mark.parametrize("max_rows,nsplit", [(16, 1), (1, 1), (1, 8)])
+def test_paged_attention_sink_switched_off(ops, max_rows, nsplit):
+    """a sink of -inf (or below every score) adds nothing to a head's sum; the other heads keep theirs"""
+    sink = torch.tensor([float("-inf"), 0.5, -2e30, 1.5], device="cuda")
+    seqs = [(40, 90), (17, 0)] if max_rows > 1 else [(1, 130), (1, 0)]
+    got, want, _ = attention_case(ops, {"sink": sink}, 4, 2, 128, 128, 64, seqs, seed=9, max_rows=max_rows, nsplit=nsplit)
+    assert rel(got, want) < 3e-6
+
+
 @pytest.mark.parametrize("dim,rot,halves", [(2, 2, False), (64, 64, True), (96, 32, False), (128, 64, True), (130, 128, False), (256, 256, True)])
 @pytest.mark.parametrize("dtype", [BF, F32])
 def test_rope_append_pairs(ops, dim, rot, halves, dtype):

@@ -128,8 +128,11 @@ paged_attn_mma_kernel(const vila_paged_attn_params p, int tiles_per_cta) {
   const bool sink = p.sink != nullptr && set == 0;
 #pragma unroll
   for (int r = 0; r < 2; ++r) {
-    m[r] = sink ? p.sink[h] : kNegBig;
-    l[r] = sink ? ex2(fmaf(m[r], kLog2e, -log2_units(m[r]))) : 0.0f;
+    // a sink below every score (-inf: switched off) weighs nothing
+    const float z = sink ? p.sink[h] : kNegBig;
+    const bool none = !sink || z < kNegBig;
+    m[r] = none ? kNegBig : z;
+    l[r] = none ? 0.0f : ex2(fmaf(z, kLog2e, -log2_units(z)));
   }
   // positions of this thread's two rows and what they see: keys lo .. pos, and of those the last `window` or the first keep_first
   int pos[2], lo[2], wlo[2];
