@@ -232,6 +232,17 @@ def test_paged_attention_sink_switched_off(ops, max_rows, nsplit):
     assert rel(got, want) < 3e-6
 
 
+def test_paged_attention_decode_skips_empty_tiles(ops):
+    """a tile of no rows names an output row but has nothing to write"""
+    for nsplit in (1, 4):
+        got, _, (q, pool, tables, tiles, o) = attention_case(ops, {}, 8, 2, 128, 128, 64, [(1, 100), (1, 30), (1, 5)], seed=2, max_rows=1, nsplit=nsplit)
+        tiles = tiles.clone()
+        tiles[1, 1] = 0
+        out = torch.full_like(got, 7.0)
+        ops.paged_attention(q, pool, tables, tiles, heads=8, kv_heads=2, dim=128, vdim=128, page=64, scale=0.1, max_rows=1, nsplit=nsplit, out=out)
+        assert bool((out[1] == 7.0).all()) and torch.equal(out[0], got[0]) and torch.equal(out[2], got[2])
+
+
 @pytest.mark.parametrize("dim,rot,halves", [(2, 2, False), (64, 64, True), (96, 32, False), (128, 64, True), (130, 128, False), (256, 256, True)])
 @pytest.mark.parametrize("dtype", [BF, F32])
 def test_rope_append_pairs(ops, dim, rot, halves, dtype):

@@ -35,6 +35,7 @@ __global__ void __launch_bounds__(kThreads, HM * MAPS <= 4 ? 2 : 1) paged_attn_d
   const int map = l16 / R, r = l16 - map * R;
   const int C = gridDim.z, rank = blockIdx.z, g = blockIdx.y;
   const int* tile = p.tiles + 4 * blockIdx.x;
+  if (tile[1] < 1) return;                                       // the same for the whole cluster
   const int row0 = tile[0], pos = tile[2];
   const int32_t* pt = p.page_tables + static_cast<size_t>(tile[3]) * p.pt_stride;
   const size_t prow = static_cast<size_t>(p.G) * (128 + kV);
