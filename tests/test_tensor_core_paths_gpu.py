@@ -232,6 +232,40 @@ def test_paged_attention_sink_switched_off(ops, max_rows, nsplit):
     assert rel(got, want) < 3e-6
 
 
+@pytest.mark.parametrize("form", ["plain", "capped", "window", "chunk", "diff_plain"])
+@pytest.mark.parametrize("rep", [1, 4, 8])
+def test_paged_attention_prompt_infinite_entries(ops, form, rep):
+    """an infinite value reaches the rows that see it and nothing else (earlier rows of its tile and of its CTA keep their
+    numbers); a score of -inf weighs nothing"""
+    o, H = ATT_FORMS[form], 2 * min(rep, 4 if "diff" in ATT_FORMS[form] else 8)
+    D, V, maps, page, T, j = (64, 128, 2, 64, 90, 37) if "diff" in o else (128, 128, 1, 64, 90, 37)
+    got, want, (q, pool, tables, tiles, o) = attention_case(ops, o, H, 2, D, V, page, [(T, 0)], seed=rep)
+    kw = dict(heads=H, kv_heads=2, dim=D, vdim=V, page=page, scale=0.1, out_dtype=F32, max_rows=16, **o)
+    row = int(tables[0, j // page]) * page + j % page
+    bad = pool.clone()
+    bad[row, 2 * maps * D + 5] = float("inf")                       # value column 5 of the first key head
+    inf = ops.paged_attention(q, bad, tables, tiles, **kw)
+    assert rel(inf[:j], want[:j]) < 3e-6
+    heads = inf.view(T, H, V)[:, :H // 2]                           # of that key head
+    assert rel(inf.view(T, H, V)[:, H // 2:], want.view(T, H, V)[:, H // 2:]) < 3e-6
+    reach = min(T, j + o.get("window", T), (j // o["chunk"] + 1) * o["chunk"] if "chunk" in o else T)
+    if "diff" in o:
+        assert not torch.isfinite(heads[j:reach, :, 5]).any()       # inf - lambda inf
+    else:
+        assert torch.isinf(heads[j:reach, :, 5]).all()
+        others = [c for c in range(V) if c != 5]
+        assert rel(heads[:, :, others], want.view(T, H, V)[:, :H // 2][:, :, others]) < 3e-6
+        q = q.clone()
+        q.view(T, H, D)[:, :, 3] = q.view(T, H, D)[:, :, 3].abs() + 0.1
+        bad = pool.clone()
+        bad[row, 3] = float("-inf")
+        if "softcap" not in o:                                      # a capped score is finite
+            ref = attention_reference(q, bad, tables, [(0, T, 0, 0)], H, 2, D, V, page, 0.1, o)
+            got = ops.paged_attention(q, bad, tables, tiles, **kw)
+            seen = torch.isfinite(ref).all(1)                       # (a row that sees no other key has no number)
+            assert int(seen.sum()) > T - 3 and rel(got[seen], ref[seen]) < 3e-6
+
+
 def test_paged_attention_decode_skips_empty_tiles(ops):
     """a tile of no rows names an output row but has nothing to write"""
     for nsplit in (1, 4):

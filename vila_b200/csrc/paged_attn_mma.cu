@@ -2,9 +2,9 @@
 //
 // The keys and values are bf16 numbers; the queries and the softmax weights are fp32 and stay so: each is cut into
 // three bf16 parts (8 + 8 + 8 bits) whose products with a bf16 number are exact, and the three products are summed
-// in fp32.  Three bf16 products are cheaper than two tf32 ones and need no range assumptions.  (An infinite key or value
-// meets the zero parts of a number that one part holds: the row becomes NaN, as an infinite score or a hidden infinite
-// value makes it in the CUDA-core kernels too.)
+// in fp32.  Three bf16 products are cheaper than two tf32 ones and need no range assumptions.  Only an infinite key or
+// value cannot be taken so (it meets the zero parts of a number that one part holds): rows that come out infinite or NaN
+// are computed again key by key.
 //
 // A warp owns 16 rows of one sequence x one score head (mma.sync m16n8k16: rows x 8 keys, then rows x 8 value columns);
 // scores and sums never leave its registers, the queries' parts lie in shared memory in fragment order.  A CTA serves
@@ -72,13 +72,49 @@ __device__ __forceinline__ float quad_sum(float v) {
   return v + __shfl_xor_sync(0xffffffffu, v, 2);
 }
 
+// A row of one score head again, key by key in fp32 multiply-adds, into dst (V numbers, divided by their weights' sum): what
+// the CUDA-core kernels compute.  Rows that met an infinite or NaN number come here, because the parts of a finite number
+// hold zeros and zero times infinity is NaN where the whole number times infinity is not.  A warp per row.
+template <int D, int MAPS, int V>
+__device__ __noinline__ void row_again(const vila_paged_attn_params& p, int row, int pos, int slot, int h, int map, float* dst) {
+  constexpr int DL = D / 32, VL = V / 32;                 // columns of a lane
+  const int lane = threadIdx.x & 31, g = h / (p.H / p.G);
+  const int32_t* pt = p.page_tables + static_cast<size_t>(slot) * p.pt_stride;
+  const size_t prow = static_cast<size_t>(p.G) * (MAPS * D + V);
+  const __nv_bfloat16* pool = static_cast<const __nv_bfloat16*>(p.pool);
+  const size_t koff = static_cast<size_t>(g * MAPS + map) * D + DL * lane, voff = static_cast<size_t>(p.G) * MAPS * D + static_cast<size_t>(g) * V + VL * lane;
+  const float sc = head_scale(p, h);
+  float q[DL], acc[VL];
+#pragma unroll
+  for (int e = 0; e < DL; ++e) q[e] = p.q[((static_cast<size_t>(row) * p.H + h) * MAPS + map) * D + DL * lane + e] * sc;
+#pragma unroll
+  for (int e = 0; e < VL; ++e) acc[e] = 0.f;
+  float m = p.sink ? p.sink[h] : kNegBig, l = p.sink ? 1.0f : 0.0f;
+  for (int j = 0; j <= pos; ++j) {
+    if (!sees(p, pos, j)) continue;
+    const __nv_bfloat16* at = pool + pool_row(pt, p.page, j) * prow;
+    float s = 0.f;
+#pragma unroll
+    for (int e = 0; e < DL; ++e) s = fmaf(q[e], __bfloat162float(at[koff + e]), s);
+    s = capped(p, warp_sum(s));
+    if (p.dist_bias) s += dist_bias(p, pos - j, h);
+    const float mn = fmaxf(m, s), w = expf(s - mn), alpha = expf(m - mn);
+    l = fmaf(l, alpha, w);
+    m = mn;
+#pragma unroll
+    for (int e = 0; e < VL; ++e) acc[e] = fmaf(w, __bfloat162float(at[voff + e]), acc[e] * alpha);
+  }
+#pragma unroll
+  for (int e = 0; e < VL; ++e) dst[VL * lane + e] = acc[e] * (1.0f / l);
+}
+
 // D: columns of a map, MAPS: maps of a head, V: value columns, SETS: sets of warps that share the key blocks.  A key's row
 // in shared memory has MAPS * D columns.
 // exp(s - m) is taken as 2^(s log2 e - m log2 e) with one fused multiply-add: the rounded m log2 e is common to a row's
 // weights and cancels in their quotient, which leaves the rounding of the difference, as in exp(s - m).
 template <int D, int MAPS, int V, int SETS>
 __global__ void __launch_bounds__(32 * (SETS == 2 ? 8 : kMaxWarps), 1)
-paged_attn_mma_kernel(const vila_paged_attn_params p, int tiles_per_cta) {
+paged_attn_mma_kernel(const __grid_constant__ vila_paged_attn_params p, int tiles_per_cta) {
   constexpr int KB = MAPS * D * 2, VB = V * 2;             // bytes of a key's / value's row
   constexpr int kBuf = kBK * (KB + VB);                     // one of a set's two buffers: keys, then values
   constexpr int kQ = 3 * (D / 16) * 512;                    // bytes of a warp's query parts
@@ -356,9 +392,39 @@ paged_attn_mma_kernel(const vila_paged_attn_params p, int tiles_per_cta) {
         }
       }
     }
-    if (MAPS == 2) __syncthreads();   // the records have been read
   }
   const bool writes = active && set == 0;
+  if (writes) {
+    unsigned odd[2];   // rows gid and gid + 8 that are not finite, a bit per lane
+#pragma unroll
+    for (int r = 0; r < 2; ++r) {
+      float z = l[r] * 0.f;
+#pragma unroll
+      for (int t = 0; t < V / 8; ++t) z = fmaf(o[t][2 * r], 0.f, fmaf(o[t][2 * r + 1], 0.f, z));
+      odd[r] = __ballot_sync(0xffffffffu, !(z == 0.f));
+    }
+    if (odd[0] | odd[1]) {
+      float* rows = xch + warp * (SETS == 2 ? 16 * V + 64 : 16 * V);   // SETS == 2: this warp's record, already read
+      __syncwarp();
+      for (int i = 0; i < n; ++i) {
+        const bool again = (odd[i >> 3] >> (4 * (i & 7))) & 15u;
+        if (again) row_again<D, MAPS, V>(p, row0 + i, pos0 + i, tile[3], h, map, rows + i * V);
+      }
+      __syncwarp();
+#pragma unroll
+      for (int r = 0; r < 2; ++r) {
+        if (gid + 8 * r >= n || ((odd[r] >> (4 * gid)) & 15u) == 0u) continue;
+        l[r] = 1.f;
+#pragma unroll
+        for (int t = 0; t < V / 8; ++t) {
+          const float2 x = *reinterpret_cast<const float2*>(rows + (gid + 8 * r) * V + 8 * t + 2 * tig);
+          o[t][2 * r] = x.x;
+          o[t][2 * r + 1] = x.y;
+        }
+      }
+    }
+  }
+  if (MAPS == 2) __syncthreads();   // the records and rows have been read
   if (MAPS == 2) {
     // the second map's rows through shared memory to the warp of the first, which combines, norms and gates them
     float* a2 = xch + (warp >> 1) * 16 * V;
