@@ -232,6 +232,15 @@ def test_paged_attention_sink_switched_off(ops, max_rows, nsplit):
     assert rel(got, want) < 3e-6
 
 
+@pytest.mark.parametrize("keys", [64, 333, 2048, 4096, 16384])
+@pytest.mark.parametrize("D,G", [(64, 2), (128, 2), (128, 8)])
+def test_paged_attention_prompt_long(ops, keys, D, G):
+    """the error does not grow with the keys as it would in one truncating sum (8e-6 at 2048 keys): 32 keys are summed on
+    the tensor core, two truncations of that size, and the keys / 32 parts by rounded additions, whose errors go both ways"""
+    got, want, _ = attention_case(ops, {}, 8, G, D, D, 64, [(40, keys - 40)], seed=keys, scale=0.05)
+    assert rel(got, want) < 4e-7 + (keys / 32) ** 0.5 * 2.0 ** -25
+
+
 @pytest.mark.parametrize("form", ["plain", "capped", "window", "chunk", "diff_plain"])
 @pytest.mark.parametrize("rep", [1, 4, 8])
 def test_paged_attention_prompt_infinite_entries(ops, form, rep):

@@ -17,8 +17,14 @@
 //
 // Bound by the tensor pipe (mma.sync: 1024 multiply-adds per clock and SM measured), six products where bf16 attention
 // issues two.  Tiled on the CUDA cores the same attention ran at 10 TFLOP/s (two shared-memory reads per 16
-// multiply-adds).  2048 causal rows, 16 heads over 4, 128 columns: 1560 us there with capped scores, 221 here (165 without the
-// cap's tanh; one set of warps with the queries in registers: 351 and 263, tensor pipe 37 % of the time).
+// multiply-adds).  2048 causal rows, 16 heads over 4, 128 columns: 1560 us there with capped scores, 247 here (174 without the
+// cap's tanh).
+//
+// The tensor core truncates as it accumulates, and the truncations of a sum all go one way: with running sums over all keys
+// the rows were 2.8e-6 off at 2048 keys and 2.6e-5 at 16384, where fp32 multiply-adds are 8e-7 and 2.3e-6 off.  So a block's
+// products go into fresh sums, the parts in ascending size (four additions of full size for 64 keys), and join the row's
+// sums by rounded additions; the first parts of a score's products (eight additions) are summed apart from the others.
+// Error 7e-8 at 64 keys, 1.4e-7 at 2048, 2.6e-7 at 16384; the running sums took 219 and 153 us.
 #include "../../include/vila_b200.h"
 #include "common.cuh"
 #include "kernels.h"
@@ -44,6 +50,30 @@ __device__ __forceinline__ void mma_bf16(float (&c)[4], const uint32_t (&a)[4], 
   asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
                : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
                : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+// the same into fresh sums
+__device__ __forceinline__ void mma_bf16_first(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};"
+               : "=f"(c[0]), "=f"(c[1]), "=f"(c[2]), "=f"(c[3])
+               : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1), "f"(0.f));
+}
+// two of a fragment's sums at a time: c0, c1 (or c2, c3) belong to one row
+using f2 = unsigned long long;
+__device__ __forceinline__ f2 pair(float x, float y) {
+  f2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(x), "f"(y));
+  return r;
+}
+__device__ __forceinline__ void unpair(f2 v, float& x, float& y) { asm("mov.b64 {%0, %1}, %2;" : "=f"(x), "=f"(y) : "l"(v)); }
+__device__ __forceinline__ void fma2(float& ax, float& ay, float m, float cx, float cy) {   // a = a m + c
+  f2 r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(pair(ax, ay)), "l"(pair(m, m)), "l"(pair(cx, cy)));
+  unpair(r, ax, ay);
+}
+__device__ __forceinline__ void add2(float& ax, float& ay, float cx, float cy) {
+  f2 r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(pair(ax, ay)), "l"(pair(cx, cy)));
+  unpair(r, ax, ay);
 }
 // two fp32 numbers -> three packed pairs of bf16 that add up to them (the last part takes what 16 bits leave)
 __device__ __forceinline__ void split3(float x, float y, uint32_t& hi, uint32_t& mid, uint32_t& lo) {
@@ -245,15 +275,12 @@ paged_attn_mma_kernel(const __grid_constant__ vila_paged_attn_params p, int tile
       if (some) {
         const uint32_t kb = buf0 + b * kBuf, vb = kb + kBK * KB;
         float s[kBK / 8][4];
-#pragma unroll
-        for (int t = 0; t < kBK / 8; ++t)
-#pragma unroll
-          for (int e = 0; e < 4; ++e) s[t][e] = 0.f;
         // lanes 0-7 / 8-15 / 16-23 / 24-31 address the matrices (keys 0-7, d 0-7), (same keys, d 8-15), (keys 8-15, ..)
         const int lkey = (lane & 7) + ((lane >> 4) << 3), lc = (lane >> 3) & 1;
+        // the queries' first parts in sums of their own: eight truncating additions of full size (four for 64 columns)
+        float sl[kBK / 8][4];
 #pragma unroll
         for (int k = 0; k < D / 16; ++k) {
-          // eight independent sums between two uses of the same one: the products' latency is covered
           uint32_t kf[kBK / 16][4];
 #pragma unroll
           for (int t = 0; t < kBK / 16; ++t) ldsm4(kb + (16 * t + lkey) * KB + (((map * D / 8 + 2 * k + lc) ^ (lkey & 7)) << 4), kf[t]);
@@ -262,12 +289,17 @@ paged_attn_mma_kernel(const __grid_constant__ vila_paged_attn_params p, int tile
             const uint4 qv = q_s[(part * (D / 16) + k) * 32];
             const uint32_t qf[4] = {qv.x, qv.y, qv.z, qv.w};
 #pragma unroll
-            for (int t = 0; t < kBK / 16; ++t) {
-              mma_bf16(s[2 * t], qf, kf[t][0], kf[t][1]);
-              mma_bf16(s[2 * t + 1], qf, kf[t][2], kf[t][3]);
+            for (int t = 0; t < kBK / 8; ++t) {
+              float (&c)[4] = part == 0 ? s[t] : sl[t];
+              if (k == 0 && part != 1) mma_bf16_first(c, qf, kf[t / 2][2 * (t & 1)], kf[t / 2][2 * (t & 1) + 1]);
+              else mma_bf16(c, qf, kf[t / 2][2 * (t & 1)], kf[t / 2][2 * (t & 1) + 1]);
             }
           }
         }
+#pragma unroll
+        for (int t = 0; t < kBK / 8; ++t)
+#pragma unroll
+          for (int e = 0; e < 4; e += 2) add2(s[t][e], s[t][e + 1], sl[t][e], sl[t][e + 1]);
         // cap, bias, mask; the block's maximum per row
         if (p.softcap > 0.f) {
 #pragma unroll
@@ -321,35 +353,37 @@ paged_attn_mma_kernel(const __grid_constant__ vila_paged_attn_params p, int tile
           for (int e = 0; e < 4; ++e) ps[e >> 1] += s[t][e];
 #pragma unroll
         for (int r = 0; r < 2; ++r) l[r] = l[r] * alpha[r] + quad_sum(ps[r]);
-        if (__any_sync(0xffffffffu, alpha[0] != 1.f || alpha[1] != 1.f)) {
-#pragma unroll
-          for (int t = 0; t < V / 8; ++t)
-#pragma unroll
-            for (int e = 0; e < 4; ++e) o[t][e] *= alpha[e >> 1];
-        }
         // weights (three parts) x values: 16 keys x 16 columns per ldmatrix
         const int vkey = (lane & 7) + (((lane >> 3) & 1) << 3), vc = lane >> 4;
+        uint32_t a[3][kBK / 16][4];
 #pragma unroll
-        for (int k = 0; k < kBK / 16; ++k) {
-          uint32_t a[3][4];
+        for (int k = 0; k < kBK / 16; ++k)
 #pragma unroll
           for (int e = 0; e < 4; ++e) {
             const float* w = &s[2 * k + (e >> 1)][2 * (e & 1)];
-            split3(w[0], w[1], a[0][e], a[1][e], a[2][e]);
+            split3(w[0], w[1], a[0][k][e], a[1][k][e], a[2][k][e]);
           }
 #pragma unroll
-          for (int t0 = 0; t0 < V / 16; t0 += 4) {
-            uint32_t vf[4][4];
+        for (int t0 = 0; t0 < V / 16; t0 += 2) {
+          uint32_t vf[kBK / 16][2][4];
 #pragma unroll
-            for (int t = 0; t < 4; ++t) ldsm4_t(vb + (16 * k + vkey) * VB + (((2 * (t0 + t) + vc) ^ (vkey & 7)) << 4), vf[t]);
+          for (int k = 0; k < kBK / 16; ++k)
 #pragma unroll
-            for (int part = 2; part >= 0; --part)
+            for (int t = 0; t < 2; ++t) ldsm4_t(vb + (16 * k + vkey) * VB + (((2 * (t0 + t) + vc) ^ (vkey & 7)) << 4), vf[k][t]);
+          float c[4][4];
+#pragma unroll
+          for (int part = 2; part >= 0; --part)
+#pragma unroll
+            for (int k = 0; k < kBK / 16; ++k)
 #pragma unroll
               for (int t = 0; t < 4; ++t) {
-                mma_bf16(o[2 * (t0 + t)], a[part], vf[t][0], vf[t][1]);
-                mma_bf16(o[2 * (t0 + t) + 1], a[part], vf[t][2], vf[t][3]);
+                if (part == 2 && k == 0) mma_bf16_first(c[t], a[part][k], vf[k][t / 2][2 * (t & 1)], vf[k][t / 2][2 * (t & 1) + 1]);
+                else mma_bf16(c[t], a[part][k], vf[k][t / 2][2 * (t & 1)], vf[k][t / 2][2 * (t & 1) + 1]);
               }
-          }
+#pragma unroll
+          for (int t = 0; t < 4; ++t)
+#pragma unroll
+            for (int e = 0; e < 4; e += 2) fma2(o[2 * t0 + t][e], o[2 * t0 + t][e + 1], alpha[e >> 1], c[t][e], c[t][e + 1]);
         }
       }
       set_sync();   // the set has read the buffer that its next block but one overwrites
