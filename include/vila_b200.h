@@ -361,9 +361,15 @@ typedef struct vila_glinear_params {
   int32_t M, N, K, groups, mode, a_row_div, act, flags;
 } vila_glinear_params;
 int vila_glinear(const vila_glinear_params* p, void* stream);
-/* Waits inside vila_glinear's tensor-core kernel that ran out of tries since the process started on the current
- * device (0 in a correct run; the launch's output is then incomplete).  Synchronises; -1: could not be read. */
+/* CTAs of vila_glinear's tensor-core kernel that gave up a wait since the process started on the current device (0 in a
+ * correct run; the launch's output is then incomplete).  Synchronises; -1: could not be read. */
 int vila_stalled_waits(void);
+/* 0, or 1 once after a launch of that kernel which had to give up (vila_last_error says so).  Reads a word of host memory
+ * and does not synchronise: after a synchronisation it speaks for everything launched before.  vila_glinear returns the
+ * same error before it launches anything. */
+int vila_wait_status(void);
+/* vila_glinear on its tensor-core kernel with waits that end after `tries` tries (test hook: 0 gives up at once). */
+int vila_glinear_tries(const vila_glinear_params* p, int tries, void* stream);
 
 /* vila_latent_attention — causal attention of H query heads over ONE shared latent per token
  * (keys and values are both the cached latent c_j of width R; the per-head key/value expansions

@@ -46,8 +46,8 @@ def test_glinear_plain(ops, M, N, K):
         z = ref / K ** 0.5
         want = torch.nn.functional.silu(z[:, 0::2]) * z[:, 1::2]
         assert rel(ops.glinear((a.float() / K ** 0.5).to(BF), w, swiglu=True, out_dtype=F32), want) < 2.0 ** -7   # a is rounded once more
-    from vila_b200 import _lib
-    assert _lib.load().vila_stalled_waits() == 0
+    torch.cuda.synchronize()
+    ops.check_waits()
 
 
 @pytest.mark.parametrize("T,E,top,W,ff", [(3, 8, 2, 128, 128), (8, 32, 4, 256, 192), (40, 5, 3, 136, 200), (200, 33, 2, 256, 264), (520, 4, 2, 320, 136)])
@@ -83,6 +83,48 @@ def test_glinear_batched(ops, M):
     a, w = randn(g, M, H * K), randn(g, H, N, K)
     ref = torch.einsum("mhk,hnk->mhn", a.double().view(M, H, K), w.double()).reshape(M, H * N)
     assert rel(ops.glinear(a, w, groups=H, a_group_off=K, o_group_off=N, out_dtype=F32), ref) < acc(K)
+
+
+@pytest.mark.parametrize("routed", [False, True])
+@pytest.mark.parametrize("rows", [40, 600])
+def test_glinear_waits_that_run_out_are_reported(ops, monkeypatch, rows, routed):
+    """waits of 0 tries give up at once, few tries somewhere under way: the launch ends, the next status says so once, and the
+    kernel works as before"""
+    from vila_b200 import _lib
+    g, K, N, E = gen(rows), 1024, 256, 4
+    a, w = randn(g, rows, K), randn(g, *((E, N, K) if routed else (N, K)))
+    kw = {}
+    if routed:
+        idx = torch.randint(0, E, (rows, 1), generator=g, device="cuda", dtype=torch.int32)
+        seg, srt = ops.moe_group(idx, E)
+        kw = dict(groups=E, seg=seg, a_rows=srt, a_row_div=1)
+    lib = _lib.load()
+    before = lib.vila_stalled_waits()
+
+    def limited(tries):
+        out = torch.full((rows, N), 7.0, device="cuda")
+        with monkeypatch.context() as m:
+            m.setattr(lib, "vila_glinear", lambda p, stream: lib.vila_glinear_tries(p, tries, stream))
+            ops.glinear(a, w, out=out, **kw)
+        torch.cuda.synchronize()
+        return out
+
+    want = limited(1 << 20)
+    ops.check_waits()
+    assert rel(want, ops.glinear(a, w, out_dtype=F32, **kw).double()) < acc(K)
+    for tries in (0, 1, 3, 30):
+        out = limited(tries)
+        if tries == 0 or not torch.equal(out, want):
+            with pytest.raises(RuntimeError, match="ran out"):
+                ops.check_waits()
+        else:
+            lib.vila_wait_status()
+        ops.check_waits()
+    assert lib.vila_stalled_waits() > before
+    limited(0)
+    with pytest.raises(RuntimeError, match="ran out"):
+        ops.glinear(a, w, out_dtype=F32, **kw)     # the next call says so as well
+    assert torch.equal(limited(1 << 20), want)
 
 
 @pytest.mark.parametrize("pairs,E", [(1, 1), (31, 5), (256, 32), (257, 7), (8192, 32), (8191, 300), (20000, 64), (600, 1500), (9000, 1100)])

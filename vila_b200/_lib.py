@@ -290,6 +290,8 @@ SIGNATURES = {
     "vila_gated_norm_residual": [c_void_p, c_void_p, c_int, c_i64, c_int, c_void_p, c_int, c_i64, c_void_p,
                                  c_int, c_void_p, c_int, c_float, c_float, c_int, c_int, c_void_p],
     "vila_stalled_waits": [],
+    "vila_wait_status": [],
+    "vila_glinear_tries": [C.POINTER(GLinearParams), c_int, c_void_p],
     "vila_glinear": [C.POINTER(GLinearParams), c_void_p],
     "vila_latent_attention": [C.POINTER(LatentAttnParams), c_void_p],
     "vila_latent_rope_append": [C.POINTER(LatentRopeParams), c_void_p],

@@ -369,6 +369,13 @@ int vila_gated_norm_residual(float* x, const void* part, int part_dtype, int64_t
 
 int vila_stalled_waits(void) { return static_cast<int>(vb::stalled_waits()); }
 
+int vila_wait_status(void) { return vb::wait_status(); }
+
+int vila_glinear_tries(const vila_glinear_params* p, int tries, void* stream) {
+  VB_REQUIRE_DEVICE();
+  return vb::glinear(*p, st(stream), nullptr, tries < 0 ? 0 : tries);
+}
+
 int vila_glinear(const vila_glinear_params* p, void* stream) {
   VB_REQUIRE_DEVICE();
   return vb::glinear(*p, st(stream));

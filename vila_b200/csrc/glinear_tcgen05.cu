@@ -27,6 +27,9 @@
 #include "dtype_any.cuh"
 #include "glinear_epi.cuh"
 
+#include <atomic>
+#include <mutex>
+
 namespace vb {
 namespace {
 
@@ -35,14 +38,25 @@ constexpr int kWBytes = kRowsW * kDepth * 2;
 constexpr int kGatherWarps = 4, kBox = 64;          // token rows of one TMA box
 constexpr int kMaxGroups = 1024;                    // groups whose tile offsets fit shared memory
 
-__device__ unsigned int g_gave_up;   // waits that ran out of tries (never in a correct run)
+constexpr int kTries = 1 << 20;                     // of a wait, then the launch gives up
+constexpr int kDrainTries = 1 << 14;                // of a wait for what is still in flight after that
 
-// An mbarrier wait that ends: a lost arrival must not leave the GPU spinning.
-__device__ __forceinline__ bool mbar_wait_limited(uint64_t* bar, uint32_t parity) {
-  for (int i = 0; i < (1 << 20); ++i)
+__device__ unsigned int g_gave_up;   // CTAs that gave up (none in a correct run)
+
+// An mbarrier wait that ends: a lost arrival must not leave the GPU spinning.  The first wait of a CTA that runs out of
+// tries sets `gave_up`, which ends the other warps' waits; a warp whose wait failed leaves its loop for the CTA's last
+// barrier.  No warp waits in any other way before that barrier.
+__device__ __forceinline__ bool mbar_wait_limited(uint64_t* bar, uint32_t parity, volatile int* gave_up, int tries) {
+  for (int i = 0; i < tries; ++i) {
     if (mbar_try_wait(bar, parity)) return true;
-  atomicAdd(&g_gave_up, 1u);
+    if (*gave_up) return false;
+  }
+  *gave_up = 1;
   return false;
+}
+__device__ __forceinline__ void mbar_drain(uint64_t* bar, uint32_t parity) {
+  for (int i = 0; i < kDrainTries; ++i)
+    if (mbar_try_wait(bar, parity)) return;
 }
 __device__ __forceinline__ void cp_async16(uint32_t dst, const void* src, bool ok) {
   const uint32_t n = ok ? 16u : 0u;   // 0: the 16 bytes are filled with zeros
@@ -111,7 +125,7 @@ constexpr int kGatedEpi = 64;
 template <int BT, int EPI>
 __global__ void __launch_bounds__(Shape<BT>::kThreads, Shape<BT>::kPerSm)
 glinear_tc_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_a,
-                  const vila_glinear_params p, const vila_glinear_ext x) {
+                  const vila_glinear_params p, const vila_glinear_ext x, int tries, volatile unsigned int* failed) {
   using S = Shape<BT>;
   constexpr int ST = S::kStages, kGather = S::kEpi, kTma = kGather + kGatherWarps, kMma = kTma + 1;
   extern __shared__ uint8_t smem_raw[];
@@ -120,7 +134,10 @@ glinear_tc_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
   uint64_t* empty_bar = full_bar + ST;
   uint64_t* acc_full = empty_bar + ST;   // [2]
   uint64_t* acc_free = acc_full + 2;     // [2]
-  uint32_t* tmem_ptr = reinterpret_cast<uint32_t*>(acc_free + 2);
+  uint64_t* meta_bar = acc_free + 2;     // a tile's output rows, weights and scales have been written
+  uint64_t* drain_bar = meta_bar + 1;
+  uint32_t* tmem_ptr = reinterpret_cast<uint32_t*>(drain_bar + 1);
+  volatile int* gave_up = reinterpret_cast<int*>(tmem_ptr + 1);
   int* orow_s = reinterpret_cast<int*>(smem + ST * S::kStage + 256);   // [2][BT] output row (-1: none)
   float* rs_s = reinterpret_cast<float*>(orow_s + 2 * BT);              // [2][BT] routing weight
   float* is_s = rs_s + 2 * BT;                                          // [2][BT] input scale
@@ -142,6 +159,9 @@ glinear_tc_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
       mbar_init(&acc_full[i], 1);
       mbar_init(&acc_free[i], S::kEpi);
     }
+    mbar_init(meta_bar, S::kEpi);
+    mbar_init(drain_bar, 1);
+    *gave_up = 0;
     fence_barrier_init();
   }
   if (warp == kMma) tmem_alloc<S::kCols>(tmem_ptr);
@@ -171,7 +191,7 @@ glinear_tc_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
 
   if (warp == kTma) {
     if (lane == 0) {
-      int s = 0;
+      int s = 0, rounds = 0;              // rounds: through all the stages
       uint32_t ph = 1;                    // parity to wait for on an empty barrier: the first round passes
       for (int it = blockIdx.x; it < total && ok; it += gridDim.x) {
         const Tile t = tile_at(p, BT, it, n_blocks, first);
@@ -180,7 +200,7 @@ glinear_tc_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
         const int col0 = p.mode == 0 ? t.g * static_cast<int>(p.a_group_off) : 0;
         const uint32_t bytes = kWBytes + boxes * box * kDepth * 2;
         for (int kb = 0; kb < nkb; ++kb) {
-          ok = mbar_wait_limited(&empty_bar[s], ph);
+          ok = mbar_wait_limited(&empty_bar[s], ph, gave_up, tries);
           if (!ok) break;
           uint8_t* st = smem + s * S::kStage;
           mbar_arrive_expect_tx(&full_bar[s], bytes);
@@ -190,10 +210,16 @@ glinear_tc_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
           if (++s == ST) {
             s = 0;
             ph ^= 1;
+            ++rounds;
           }
         }
       }
-      if (!ok) __nanosleep(1000000);   // requested tiles land before the CTA's memory is given back
+      // requested tiles land before the CTA's memory is given back: stages below s in this round, the others in the last
+      if (!ok)
+        for (int i = 0; i < ST; ++i) {
+          const int round = i < s ? rounds : rounds - 1;
+          if (round >= 0) mbar_drain(&full_bar[i], round & 1);
+        }
     }
   } else if (warp == kMma) {
     if (lane == 0) {
@@ -203,12 +229,12 @@ glinear_tc_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
         const Tile t = tile_at(p, BT, it, n_blocks, first);
         if (t.count <= 0) continue;
         const uint32_t idesc = make_idesc_bf16(kRowsW, (t.count + 15) & ~15, 0, 0), acc = tmem + (k & 1) * S::kAcc * BT;
-        ok = mbar_wait_limited(&acc_free[k & 1], ((k >> 1) & 1) ^ 1);
+        ok = mbar_wait_limited(&acc_free[k & 1], ((k >> 1) & 1) ^ 1, gave_up, tries);
         tc_fence_after();
         int part = 0, left = per_acc;
         uint32_t more = 0;                                // 0: first product of an accumulator
         for (int kb = 0; kb < nkb && ok; ++kb) {
-          ok = mbar_wait_limited(&full_bar[s], ph);
+          ok = mbar_wait_limited(&full_bar[s], ph, gave_up, tries);
           if (!ok) break;
           if (gathered) fence_proxy_async_smem();        // the copies that arrived here, before the products below
           tc_fence_after();
@@ -235,6 +261,10 @@ glinear_tc_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
         }
         if (ok) umma_commit(&acc_full[k & 1]);
         ++k;
+      }
+      if (!ok) {                          // products under way end before TMEM and the CTA's memory are given back
+        umma_commit(drain_bar);
+        mbar_drain(drain_bar, 0);
       }
     }
   } else if (warp >= kGather) {
@@ -264,7 +294,7 @@ glinear_tc_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
         look(it + gridDim.x);
         if (t.count <= 0) continue;
         for (int kb = 0; kb < nkb; ++kb) {
-          ok = mbar_wait_limited(&empty_bar[s], ph);
+          ok = mbar_wait_limited(&empty_bar[s], ph, gave_up, tries);
           if (!ok) break;
           const bool in_k = kb * kDepth + c * 8 < p.K;
 #pragma unroll
@@ -282,8 +312,7 @@ glinear_tc_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
     }
   } else {
     const int quad = warp & 3, half = warp >> 2;
-    constexpr int kEpiThreads = 32 * S::kEpi;
-    static_assert(BT <= kEpiThreads, "a thread looks up one token of a tile");
+    static_assert(BT <= 32 * S::kEpi, "a thread looks up one token of a tile");
     // what the epilogue of a tile needs to know of token tid is looked up while the tile before it is written out
     Tile t, next = {0, 0, 0, 0};
     int o_next;
@@ -315,8 +344,11 @@ glinear_tc_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
         is_s[buf + tid] = is_next;
       }
       look(it + gridDim.x);
-      asm volatile("bar.sync 1, %0;" ::"n"(kEpiThreads) : "memory");
-      ok = __all_sync(0xffffffffu, mbar_wait_limited(&acc_full[k & 1], (k >> 1) & 1));   // the TMEM loads need all lanes
+      __syncwarp();
+      if (lane == 0) mbar_arrive(meta_bar);
+      // all lanes or none: the TMEM loads need the whole warp
+      ok = __all_sync(0xffffffffu, mbar_wait_limited(meta_bar, k & 1, gave_up, tries) &&
+                                       mbar_wait_limited(&acc_full[k & 1], (k >> 1) & 1, gave_up, tries));
       if (!ok) break;
       tc_fence_after();
       const int n = t.n0 + quad * 32 + lane;             // this thread's weight row
@@ -374,10 +406,32 @@ glinear_tc_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
     tc_fence_after();
     tmem_dealloc<S::kCols>(tmem);
   }
+  if (tid == 0 && *gave_up) {
+    atomicAdd(&g_gave_up, 1u);
+    *failed = 1u;
+    __threadfence_system();
+  }
+}
+
+// A word of pinned host memory that a launch which gave up sets: the host reads it without waiting for the device.
+std::atomic<volatile unsigned int*> g_failed{nullptr};
+volatile unsigned int* failed_word() {
+  static std::once_flag once;
+  std::call_once(once, [] {
+    void* w = nullptr;
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;   // the first call may be under capture
+    cudaThreadExchangeStreamCaptureMode(&mode);
+    if (cudaHostAlloc(&w, sizeof(unsigned int), cudaHostAllocPortable | cudaHostAllocMapped) == cudaSuccess) {
+      *static_cast<volatile unsigned int*>(w) = 0u;
+      g_failed = static_cast<volatile unsigned int*>(w);
+    }
+    cudaThreadExchangeStreamCaptureMode(&mode);
+  });
+  return g_failed;
 }
 
 template <int BT, int EPI>
-int launch_epi(const CUtensorMap& tm, const CUtensorMap& ta, const vila_glinear_params& p, const vila_glinear_ext& x, cudaStream_t stream) {
+int launch_epi(const CUtensorMap& tm, const CUtensorMap& ta, const vila_glinear_params& p, const vila_glinear_ext& x, int tries, cudaStream_t stream) {
   using S = Shape<BT>;
   static PerDeviceOnce once;
   if (once.first())
@@ -386,22 +440,22 @@ int launch_epi(const CUtensorMap& tm, const CUtensorMap& ta, const vila_glinear_
   const long long tiles = tok * ((p.N + kRowsW - 1) / kRowsW) * (p.mode == 0 ? p.groups : 1);
   VB_CHECK(tiles < (1LL << 31), "glinear: too many tiles (M=%d N=%d groups=%d)", p.M, p.N, p.groups);
   const int grid = static_cast<int>(tiles < S::kPerSm * num_sms() ? tiles : S::kPerSm * num_sms());
-  VB_CUDA(launch_serial(glinear_tc_kernel<BT, EPI>, dim3(grid), dim3(S::kThreads), S::smem(p.mode == 1 ? p.groups : 0), stream, tm, ta, p, x));
+  VB_CUDA(launch_serial(glinear_tc_kernel<BT, EPI>, dim3(grid), dim3(S::kThreads), S::smem(p.mode == 1 ? p.groups : 0), stream, tm, ta, p, x, tries, failed_word()));
   return 0;
 }
 template <int BT>
-int launch(const CUtensorMap& tm, const CUtensorMap& ta, const vila_glinear_params& p, const vila_glinear_ext& x, cudaStream_t stream) {
-  if (p.flags & VILA_FLAG_GLU_CLAMP) return launch_epi<BT, kGatedEpi + VILA_FLAG_GLU_CLAMP>(tm, ta, p, x, stream);
-  if (p.flags & VILA_FLAG_GEGLU) return launch_epi<BT, kGatedEpi + VILA_FLAG_GEGLU>(tm, ta, p, x, stream);
-  if (p.flags & VILA_FLAG_SWIGLU) return launch_epi<BT, kGatedEpi + VILA_FLAG_SWIGLU>(tm, ta, p, x, stream);
+int launch(const CUtensorMap& tm, const CUtensorMap& ta, const vila_glinear_params& p, const vila_glinear_ext& x, int tries, cudaStream_t stream) {
+  if (p.flags & VILA_FLAG_GLU_CLAMP) return launch_epi<BT, kGatedEpi + VILA_FLAG_GLU_CLAMP>(tm, ta, p, x, tries, stream);
+  if (p.flags & VILA_FLAG_GEGLU) return launch_epi<BT, kGatedEpi + VILA_FLAG_GEGLU>(tm, ta, p, x, tries, stream);
+  if (p.flags & VILA_FLAG_SWIGLU) return launch_epi<BT, kGatedEpi + VILA_FLAG_SWIGLU>(tm, ta, p, x, tries, stream);
   switch (p.act) {
-    case VILA_ACT_SILU: return launch_epi<BT, VILA_ACT_SILU>(tm, ta, p, x, stream);
-    case VILA_ACT_RELU2: return launch_epi<BT, VILA_ACT_RELU2>(tm, ta, p, x, stream);
-    case VILA_ACT_GELU_TANH: return launch_epi<BT, VILA_ACT_GELU_TANH>(tm, ta, p, x, stream);
-    case VILA_ACT_GELU_ERF: return launch_epi<BT, VILA_ACT_GELU_ERF>(tm, ta, p, x, stream);
-    case VILA_ACT_XIELU: return launch_epi<BT, VILA_ACT_XIELU>(tm, ta, p, x, stream);
-    case VILA_ACT_SOFTCAP: return launch_epi<BT, VILA_ACT_SOFTCAP>(tm, ta, p, x, stream);
-    default: return launch_epi<BT, VILA_ACT_NONE>(tm, ta, p, x, stream);
+    case VILA_ACT_SILU: return launch_epi<BT, VILA_ACT_SILU>(tm, ta, p, x, tries, stream);
+    case VILA_ACT_RELU2: return launch_epi<BT, VILA_ACT_RELU2>(tm, ta, p, x, tries, stream);
+    case VILA_ACT_GELU_TANH: return launch_epi<BT, VILA_ACT_GELU_TANH>(tm, ta, p, x, tries, stream);
+    case VILA_ACT_GELU_ERF: return launch_epi<BT, VILA_ACT_GELU_ERF>(tm, ta, p, x, tries, stream);
+    case VILA_ACT_XIELU: return launch_epi<BT, VILA_ACT_XIELU>(tm, ta, p, x, tries, stream);
+    case VILA_ACT_SOFTCAP: return launch_epi<BT, VILA_ACT_SOFTCAP>(tm, ta, p, x, tries, stream);
+    default: return launch_epi<BT, VILA_ACT_NONE>(tm, ta, p, x, tries, stream);
   }
 }
 
@@ -421,7 +475,16 @@ unsigned int stalled_waits() {
   return cudaMemcpyFromSymbol(&n, g_gave_up, sizeof n) == cudaSuccess ? n : ~0u;
 }
 
-int glinear_tc(const vila_glinear_params& p, cudaStream_t stream, const vila_glinear_ext& x) {
+int wait_status() {
+  volatile unsigned int* w = g_failed;
+  if (w == nullptr || *w == 0u) return 0;
+  *w = 0u;
+  set_last_error("glinear: a wait of an earlier launch ran out of tries; that launch's output is incomplete");
+  return 1;
+}
+
+int glinear_tc(const vila_glinear_params& p, cudaStream_t stream, const vila_glinear_ext& x, int tries) {
+  VB_CHECK(failed_word() != nullptr, "glinear: no pinned host memory for the status word");
   CUtensorMap tm, ta;
   const uint64_t gs = p.groups == 1 ? static_cast<uint64_t>(p.N) * p.ldw : p.w_group_stride;
   if (int rc = make_tmap_3d_bf16(&tm, p.w, p.K, p.N, p.groups, p.ldw, gs, kDepth, kRowsW, 1, 128)) return rc;
@@ -433,9 +496,10 @@ int glinear_tc(const vila_glinear_params& p, cudaStream_t stream, const vila_gli
   const bool grouped = p.mode == 0 && p.groups > 1;
   const uint64_t a_cols = grouped ? (p.groups - 1) * static_cast<uint64_t>(p.a_group_off) + p.K : p.K;
   if (int rc = make_tmap_2d_bf16(&ta, p.a, p.M, a_cols, p.lda, bt < kBox ? bt : kBox, kDepth, 128)) return rc;
-  if (bt == 16) return launch<16>(tm, ta, p, x, stream);
-  if (bt == 64) return launch<64>(tm, ta, p, x, stream);
-  return launch<256>(tm, ta, p, x, stream);
+  if (tries < 0) tries = kTries;
+  if (bt == 16) return launch<16>(tm, ta, p, x, tries, stream);
+  if (bt == 64) return launch<64>(tm, ta, p, x, tries, stream);
+  return launch<256>(tm, ta, p, x, tries, stream);
 }
 
 }  // namespace vb

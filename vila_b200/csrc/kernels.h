@@ -310,8 +310,10 @@ int gather_rows(const void* src, const int32_t* rows, void* dst, int n_rows, int
 // bf16 operands on 16-byte boundaries with at least 128 weight rows: tcgen05 tiles (glinear_tcgen05.cu)
 bool glinear_tc_takes(const vila_glinear_params& p);
 unsigned int stalled_waits();
-int glinear_tc(const vila_glinear_params& p, cudaStream_t stream, const vila_glinear_ext& x);
-int glinear(const vila_glinear_params& p, cudaStream_t stream, const vila_glinear_ext* ext = nullptr);
+int wait_status();   // 1 (and the last error) once after a launch whose wait ran out of tries; does not synchronise
+int glinear_tc(const vila_glinear_params& p, cudaStream_t stream, const vila_glinear_ext& x, int tries);
+// tries >= 0: of every wait of the tcgen05 kernel (tests); otherwise its own limit
+int glinear(const vila_glinear_params& p, cudaStream_t stream, const vila_glinear_ext* ext = nullptr, int tries = -1);
 int latent_attention(const vila_latent_attn_params& p, cudaStream_t stream);
 int latent_rope_append(const vila_latent_rope_params& p, cudaStream_t stream);
 int hgrn2_scan(const vila_hgrn2_params& p, cudaStream_t stream);

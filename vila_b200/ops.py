@@ -495,6 +495,12 @@ def gated_norm_residual(x: torch.Tensor, part: torch.Tensor, *, n_partials: int 
         "vila_gated_norm_residual_scaled")
 
 
+def check_waits() -> None:
+    """Raise if a launch of glinear's tensor-core kernel gave up (a wait of its pipeline ran out of tries) since the last
+    check: its output is incomplete.  Costs a read of host memory; after a synchronisation it speaks for all launches so far."""
+    check(_lib.load().vila_wait_status(), "vila_glinear")
+
+
 def glinear(a: torch.Tensor, w: torch.Tensor, *, out: Optional[torch.Tensor] = None, out_dtype=None,
             bias: Optional[torch.Tensor] = None, act: int = ACT_NONE, swiglu: bool = False,
             groups: int = 1, a_group_off: int = 0, o_group_off: int = 0,

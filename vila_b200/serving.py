@@ -440,6 +440,7 @@ class TokenEngine:
         """entries: (sequence id, next token ids, indices among them whose logits are wanted).  All
         entries run as one batch on top of what earlier steps cached.  -> fp32 logits [wanted, vocab]
         in entry / index order (None if nothing is wanted)."""
+        ops.check_waits()   # of the steps so far
         entries = [e for e in entries if len(e[1])]
         if not entries:
             return None
@@ -519,4 +520,5 @@ def generate_tokens(model, prompts: Sequence[Sequence[int]], max_new_tokens: int
                 engine.release(("gen", r))
                 reserved -= pages_for(r)
                 del live[r]
+        ops.check_waits()       # the tokens above have been read from the device: they are of complete steps
     return out
