@@ -171,7 +171,10 @@ int vila_rope_kv_append_table(void* qkv, const void* rope_table, int S, int Hq, 
 /* Fused q/k/v projection for a short prefill chunk (M <= 384 tokens, head_dim 128):
  * qkv = x @ w^T + bias; RoPE on the q and k heads; q heads -> qkv_out[:, :Hq*128]; k / v heads ->
  * the paged pools (k_pool NULL: they stay in qkv_out) — vila_linear followed by vila_rope_kv_append
- * in ONE kernel, bit-identical to the two calls (rope_table: vila_rope_table of the chunk's positions).  Replaces Qwen2Attention's q_proj/k_proj/v_proj +
+ * in ONE kernel (rope_table: vila_rope_table of the chunk's positions).  Bit-identical to the two calls where vila_linear
+ * takes the swap-AB kernel as well.  Its sums over K run in another order, so that results may differ in the last place,
+ * for up to 4 rows of at most 20 M weights or 8 rows of 6 M, and for rows that fill 128-row tiles to nine tenths
+ * (116..128, 231..256, 346..384) of a layer of at most 74 128 x 128 tiles and K >= 512.  Replaces Qwen2Attention's q_proj/k_proj/v_proj +
  * apply_rotary_pos_emb + past_key_value.update (modeling_qwen2.py:223-226,99-160,262-266 of the
  * in-tree copy).  Returns 3 (and sets vila_last_error) when the shape is not covered: the caller
  * then issues the two separate calls. */

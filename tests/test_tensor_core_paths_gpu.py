@@ -390,3 +390,28 @@ def test_linear_few_rows(ops, M, N, K):
         assert rel(ops.linear(x, w, glu_clamp=(1.702, 0.5)), c * torch.sigmoid(1.702 * c) * (u.clamp(-0.5, 0.5) + 1)) < 2.0 ** -7
     many = ops.linear(torch.cat([x] * 3)[:8].contiguous(), w, static_w=True)
     assert torch.equal(many[:min(M, 8)], ops.linear(x, w, static_w=True))   # a row's result does not depend on how many there are
+
+
+@pytest.mark.parametrize("M", [1, 3, 4, 5, 8, 9, 100, 128, 200, 250, 300])
+@pytest.mark.parametrize("Hq,Hkv,K", [(6, 2, 512), (2, 1, 1288), (16, 2, 2048), (28, 4, 3584)])
+def test_linear_qkv_rope_equals_linear_and_rope(ops, M, Hq, Hkv, K):
+    """the fused projection against vila_linear + vila_rope_kv_append as they dispatch: the same bits where vila_linear takes
+    the swap-AB kernel too; few rows of few weights (another kernel) and rows that fill 128-row tiles (halves of K summed
+    apart) are another order of the sums: bf16 values that may be a last place apart"""
+    g, D, p0 = gen(M + K), 128, 77
+    few = (Hq + 2 * Hkv) * D * K <= (20000000 if M <= 4 else 6000000 if M <= 8 else 0)
+    halves = M in (128, 250) and (M + 127) // 128 * (Hq + 2 * Hkv) <= torch.cuda.get_device_properties(0).multi_processor_count // 2
+    same = (lambda a, b: rel(a, b.double()) < 2.0 ** -8) if few or halves else torch.equal
+    N = (Hq + 2 * Hkv) * D
+    x, w, b = randn(g, M, K), (randn(g, N, K).float() * K ** -0.5).to(BF), randn(g, N)
+    pos = torch.arange(p0, p0 + M, dtype=torch.int32, device="cuda") * 3 + 5
+    inv = (1.0 / (1e6 ** (torch.arange(0, D, 2, dtype=torch.float32) / D))).cuda()
+    table = torch.randperm(4, generator=torch.Generator().manual_seed(1)).to(torch.int32).cuda()
+    pools = [torch.zeros(4, 128, Hkv, D, dtype=BF, device="cuda") for _ in range(4)]
+    ref, tab = ops.linear(x, w, b), ops.rope_table(pos, D, inv)
+    plain = ref.clone()
+    ops.rope_kv_append(ref, pos, Hq, Hkv, D, inv, pools[0], pools[1], table, p0)
+    got = ops.linear_qkv_rope(x, w, b, tab, Hq, Hkv, D, pools[2], pools[3], table, p0)
+    assert same(got[:, :Hq * D], ref[:, :Hq * D]) and same(pools[2], pools[0]) and same(pools[3], pools[1])
+    ops.rope_kv_append(plain, pos, Hq, Hkv, D, inv)
+    assert same(ops.linear_qkv_rope(x, w, b, tab, Hq, Hkv, D), plain)
