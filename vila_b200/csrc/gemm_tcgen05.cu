@@ -691,9 +691,13 @@ int gemm_bf16(const __nv_bfloat16* A, int lda, const __nv_bfloat16* W, int ldw, 
   // down-proj 52 vs 90 us, gate/up 83 vs 86, qkv/o 21-23 vs 22 (profiles/r01_gemm_configs.md)
   const int sms = num_sms();
   const int mb = (M + BLOCK_M - 1) / BLOCK_M;
-  // Long-K GEMMs with at most one 128x128 tile per SM pair (ViT fc2: 72 tiles, K = 4304; projector):
-  // split K over a CTA pair with a DSMEM exchange -> all SMs stream operands (fc2 16.9 vs 24.7 us; 1024 x 1152 outputs:
-  // K = 1152 11.0 vs 13.9 us, K = 592 9.8 vs 11.7).
+  // At most one 128x128 tile per SM pair (ViT fc2: 72 tiles, K = 4304; projector): split K over a CTA pair with a DSMEM
+  // exchange -> all SMs stream operands (fc2 16.9 vs 24.7 us).  Down to K = 512 and to one row tile it is the faster form:
+  // 512 .. 4608 outputs, K = 512 | 1024 | 1984, against the swap-AB kernel that would take up to 384 rows
+  //   128 rows 6.0-6.7 | 7.1-8.0 | 9.1-10.7 us, there 6.7-6.9 | 8.3-9.8 | 10.2-12.1
+  //   256 rows 6.0-7.7 | 7.2-9.3 | 9.3-12.1 us, there 9.3-9.6 | 11.8-13.2 | 13.9-15.4
+  // and against 128x128 tiles of one CTA 512 rows 6.1-7.2 | 7.2-8.6 | 9.5-11.0 us, there 7.0-7.8 | 9.2-10.0 | 13.2-14.3;
+  // 1024 rows x 1152 outputs 7.7 | 9.0 | 11.5, there 7.9 | 10.3 | 14.7.  Below K = 512 a CTA would have four stages.
   const long tiles128 = static_cast<long>(mb) * ((N + 127) / 128);
   const bool split2 = tiles128 <= sms / 2 && K >= 512 && M * 10 >= mb * BLOCK_M * 9;
   if (split2) return launch_gemm<128, 6, kModeSplitK2>(A, lda, W, ldw, C, ldc, M, N, K, epi, -1, stream);
