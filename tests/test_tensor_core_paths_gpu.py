@@ -415,3 +415,44 @@ def test_linear_qkv_rope_equals_linear_and_rope(ops, M, Hq, Hkv, K):
     assert same(got[:, :Hq * D], ref[:, :Hq * D]) and same(pools[2], pools[0]) and same(pools[3], pools[1])
     ops.rope_kv_append(plain, pos, Hq, Hkv, D, inv)
     assert same(ops.linear_qkv_rope(x, w, b, tab, Hq, Hkv, D), plain)
+
+
+# ---- recurrences --------------------------------------------------------------------------------------------
+def hgrn2_inputs(g, T, H, dim, vdim, dtype=BF):
+    proj = randn(g, T, 2 * H * dim + H * vdim, dtype=dtype)
+    kw = dict(heads=H, dim=dim, vdim=vdim, q_off=0, f_off=H * dim, v_off=2 * H * dim, f_bias=torch.randn(H * dim, generator=g, device="cuda"),
+              lower=torch.rand(H * dim, generator=g, device="cuda") * 0.9)
+    q = torch.nn.functional.silu(proj[:, :H * dim].double()).view(T, H, dim)
+    low = kw["lower"].double()
+    f = (low + (1 - low) * torch.sigmoid(proj[:, H * dim:2 * H * dim].double() + kw["f_bias"].double())).view(T, H, dim)
+    return proj, kw, q, f, proj[:, 2 * H * dim:].double().view(T, H, vdim)
+
+
+def hgrn2_direct(q, f, v, S):
+    out = []
+    for t in range(q.shape[0]):
+        S = f[t][:, :, None] * S + (1 - f[t])[:, :, None] * v[t][:, None, :]
+        out.append(torch.einsum("hkv,hk->hv", S, q[t]))
+    return torch.stack(out), S
+
+
+@pytest.mark.parametrize("dim", [8, 20, 32, 40, 64, 100, 128, 250])
+@pytest.mark.parametrize("vdim", [24, 33, 64])
+@pytest.mark.parametrize("dtype", [BF, F32])
+def test_hgrn2_steps_and_portions_give_the_same_bits(ops, dim, vdim, dtype):
+    """a sequence token by token in steps of its own (one kernel), beside a prompt portion (another) and in one call"""
+    g, T, H = gen(dim + vdim), 19, 2
+    proj, kw, q, f, v = hgrn2_inputs(g, T, H, dim, vdim, dtype)
+    want, S = hgrn2_direct(q, f, v, torch.zeros(H, dim, vdim, device="cuda", dtype=torch.float64))
+    i32 = lambda r: torch.tensor(r, dtype=torch.int32, device="cuda")
+    whole = torch.full((4, H, dim, vdim), 9.0, device="cuda")
+    ref = ops.hgrn2_scan(proj, whole, i32([(0, T, 0, 1)]), **kw)
+    assert rel(ref.view(T, H, vdim), want) < 2e-6 and rel(whole[1], S) < 2e-6
+    state, got = torch.full_like(whole, -3.0), []
+    for t in range(T):
+        if t % 3 == 2:      # beside three rows of another sequence
+            got.append(ops.hgrn2_scan(torch.cat([proj[:3], proj[t:t + 1]]), state, i32([(0, 3, 0, 0), (3, 1, t, 2)]), **kw)[3:])
+        else:               # alone or with another single row
+            n = 1 + t % 2
+            got.append(ops.hgrn2_scan(proj[t:t + 1].repeat(n, 1), state, i32([(0, 1, t, 2), (1, 1, 0, 3)][:n]), **kw)[:1])
+    assert torch.equal(torch.cat(got), ref) and torch.equal(state[2], whole[1])

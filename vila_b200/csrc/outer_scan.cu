@@ -33,7 +33,7 @@
 // instruction issue (2.9 of 4 per clock).  2048 rows of one sequence, 16 heads of 128 x 128: decay 329 -> 238 us, gla 327 -> 243,
 // hgrn2 1208 -> 242 and ssd (64 heads of 64 x 128) 785 -> 304 from the forms that kept one column per thread group.
 // A column's sum runs in the same order whatever CPT and the batch are, and time runs in order: a row's result depends neither on
-// the batch nor on how its sequence was cut into steps.
+// the batch nor on how its sequence was cut into steps (single steps of hgrn2 run in hgrn2.cu, in the same order).
 #include <type_traits>
 #include "../../include/vila_b200.h"
 #include "common.cuh"
@@ -453,7 +453,7 @@ __global__ void __launch_bounds__(32 * (kOwnerWarps + kStageWarps)) outer_scan_k
     float* yy = y_s + bf * kChunk * COLS;
     const float4* sc = sc_s + bf * kChunk;
     if (!DELTA) {
-      // `count` tokens from t0 on: every token's sums over the state before its write, then its write
+      // `count` tokens from t0 on: every token's write, then its sums over the state
       auto tokens = [&](int t0, auto count) {
         constexpr int NT = decltype(count)::value, NS = NT * CPT, SPAN = R / NS;
         float d[NS];
