@@ -456,3 +456,43 @@ def test_hgrn2_steps_and_portions_give_the_same_bits(ops, dim, vdim, dtype):
             n = 1 + t % 2
             got.append(ops.hgrn2_scan(proj[t:t + 1].repeat(n, 1), state, i32([(0, 1, t, 2), (1, 1, 0, 3)][:n]), **kw)[:1])
     assert torch.equal(torch.cat(got), ref) and torch.equal(state[2], whole[1])
+
+
+@pytest.mark.parametrize("seqs,H,dim,vdim,off", [(24, 16, 128, 64, 0), (24, 16, 64, 33, 0), (30, 40, 20, 30, 0), (2, 3, 128, 64, 1), (24, 16, 128, 64, 1),
+                                                 (1, 2, 36, 34, 3)])
+def test_wide_scans(ops, seqs, H, dim, vdim, off):
+    """two and four columns per group of lanes (many sequences and heads), columns and channels that do not fill them, states
+    that do not start on 16 bytes (off numbers past one)"""
+    g, T = gen(dim + vdim), 18
+    lens = [(5 * s) % T + 1 for s in range(seqs)]
+    rows = [sum(lens[:s]) for s in range(seqs)]
+    R, spans = sum(lens), torch.tensor([(rows[s], lens[s], 3 if s % 2 else 0, seqs - 1 - s) for s in range(seqs)], dtype=torch.int32, device="cuda")
+
+    def state_of(*shape):
+        flat = torch.randn(int(torch.tensor(shape).prod()) + off, generator=g, device="cuda")
+        return flat[off:].view(*shape)
+
+    proj, kw, q, f, v = hgrn2_inputs(g, R, H, dim, vdim)
+    state = state_of(seqs, H, dim, vdim)
+    start = state.double()
+    got = ops.hgrn2_scan(proj, state, spans, **kw).view(R, H, vdim)
+    x, B, Cm = randn(g, R, H, vdim), randn(g, R, 1, dim), randn(g, R, 1, dim)
+    dt, z = randn(g, R, H), randn(g, R, H * vdim)
+    A_log, bias, D = (torch.randn(H, generator=g, device="cuda") * 0.5 for _ in range(3))
+    st2 = state_of(seqs, H, vdim, dim)
+    start2 = st2.double()
+    got2 = ops.ssd_scan(torch.cat([x.view(R, -1), B.view(R, -1), Cm.view(R, -1)], 1), dt, z, st2, spans, heads=H, vdim=vdim, nstate=dim, groups=1,
+                        dt_bias=bias, A_log=A_log, D=D).view(R, H, vdim)
+    step = torch.nn.functional.softplus(dt.double() + bias.double())
+    gate = torch.nn.functional.silu(z.double()).view(R, H, vdim)
+    for s in range(seqs):
+        r, n, slot = rows[s], lens[s], seqs - 1 - s
+        S = start[slot] if s % 2 else torch.zeros_like(start[slot])
+        want, S = hgrn2_direct(q[r:r + n], f[r:r + n], v[r:r + n], S)
+        assert rel(got[r:r + n], want) < 5e-6 and rel(state[slot], S) < 2e-6
+        S = start2[slot] if s % 2 else torch.zeros_like(start2[slot])
+        out = []
+        for t in range(r, r + n):
+            S = torch.exp(-torch.exp(A_log.double()) * step[t])[:, None, None] * S + (step[t][:, None] * x[t].double())[:, :, None] * B[t].double()
+            out.append((S @ Cm[t, 0].double() + D.double()[:, None] * x[t].double()) * gate[t])
+        assert rel(got2[r:r + n], torch.stack(out)) < 5e-6 and rel(st2[slot], S) < 2e-6

@@ -152,6 +152,7 @@ struct ScanArgs {
   const float* decay;           // decay: [H]
   int silu;                     // decay: q, k and v are pre-activations, SiLU is taken as they are read
   int vec_qk, vec_a;            // four-element loads of q | k and of z are aligned
+  int vec_s;                    // four-element accesses of the state are aligned
 };
 
 template <int MODE, int R, int KPT, int CPT, int kStageWarps>
@@ -386,7 +387,7 @@ __global__ void __launch_bounds__(32 * (kOwnerWarps + kStageWarps)) outer_scan_k
   // ---------------- owners of the state ----------------
   const int r = lane & (R - 1), cg = (warp * GPW + lane / R) * CPT;   // first column of this lane's group
   float* stp = p.state + ((static_cast<size_t>(slot) * p.H + h) * vdim + col0 + cg) * dim;
-  const bool vec_s4 = (dim & 3) == 0;
+  const bool vec_s4 = p.vec_s != 0;
   float4 S[CPT][NQ];
 #pragma unroll
   for (int c = 0; c < CPT; ++c)
@@ -417,7 +418,7 @@ __global__ void __launch_bounds__(32 * (kOwnerWarps + kStageWarps)) outer_scan_k
       }
   };
   auto entry = [&](int c, int j, int e) -> float& { return e == 0 ? S[c][j].x : e == 1 ? S[c][j].y : e == 2 ? S[c][j].z : S[c][j].w; };
-  const bool wide = vdim % CPT == 0 && col0 + cg < vdim;
+  const bool wide = p.vec_s && vdim % CPT == 0 && col0 + cg < vdim;
   if (HGRN && pos0 > 0)
     hgrn_rows([&](const float* s, int j, int e) {
       if (wide) {
@@ -630,7 +631,9 @@ int pick_columns(const ScanArgs& p, int nseq, cudaStream_t stream) {
 }
 
 template <int MODE>
-int scan_by_dim(const ScanArgs& p, int nseq, cudaStream_t stream) {
+int scan_by_dim(ScanArgs p, int nseq, cudaStream_t stream) {
+  // rows of the state: dim entries, hgrn2's vdim (the kernel checks that against its columns per lane)
+  p.vec_s = reinterpret_cast<uintptr_t>(p.state) % 16 == 0 && (MODE == kHgrn2 || p.dim % 4 == 0);
   if (p.dim <= 32) return pick_columns<MODE, 8, 4>(p, nseq, stream);
   if (p.dim <= 64) return pick_columns<MODE, 16, 4>(p, nseq, stream);
   if (p.dim <= 128) return pick_columns<MODE, 16, 8>(p, nseq, stream);
