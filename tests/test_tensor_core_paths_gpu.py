@@ -496,3 +496,18 @@ def test_wide_scans(ops, seqs, H, dim, vdim, off):
             S = torch.exp(-torch.exp(A_log.double()) * step[t])[:, None, None] * S + (step[t][:, None] * x[t].double())[:, :, None] * B[t].double()
             out.append((S @ Cm[t, 0].double() + D.double()[:, None] * x[t].double()) * gate[t])
         assert rel(got2[r:r + n], torch.stack(out)) < 5e-6 and rel(st2[slot], S) < 2e-6
+
+
+@pytest.mark.parametrize("dim", [20, 96, 126, 128])
+def test_hgrn2_infinite_value(ops, dim):
+    """channels past the head's do not turn an infinite value into NaN"""
+    g, T, H, vdim = gen(dim), 6, 2, 24
+    proj, kw, q, f, v = hgrn2_inputs(g, T, H, dim, vdim)
+    proj[:, :H * dim] = proj[:, :H * dim].abs() + 0.5               # positive queries
+    proj[2, 2 * H * dim + 7] = float("inf")
+    for n in (T, 1):
+        state, out = torch.zeros(1, H, dim, vdim, device="cuda"), []
+        for t in range(0, T, n):
+            out.append(ops.hgrn2_scan(proj[t:t + n], state, torch.tensor([(0, n, t, 0)], dtype=torch.int32, device="cuda"), **kw))
+        out = torch.cat(out).view(T, H, vdim)
+        assert torch.isinf(out[2:, 0, 7]).all() and torch.isfinite(out[:2]).all() and torch.isfinite(out[:, 0, :7]).all() and torch.isfinite(out[:, 1]).all()

@@ -441,6 +441,16 @@ __global__ void __launch_bounds__(32 * (kOwnerWarps + kStageWarps)) outer_scan_k
       P[c][j][0] = pair(S[c][j].x, S[c][j].y);
       P[c][j][1] = pair(S[c][j].z, S[c][j].w);
     }
+  // hgrn2: channels past the head's stay zero whatever the value is (their 1 - f is zero, but zero times infinity is not)
+  const bool padded = HGRN && dim < NP;
+  f2 live[HGRN ? NQ : 1][2];
+#pragma unroll
+  for (int j = 0; j < (HGRN ? NQ : 1); ++j)
+#pragma unroll
+    for (int e = 0; e < 2; ++e) {
+      const int left = dim - 4 * (r + R * j) - 2 * e;
+      live[j][e] = left >= 2 ? ~0ull : left == 1 ? 0xffffffffull : 0ull;
+    }
   constexpr int kSpan = R / NV;                    // neighbouring lanes that end up with the same sum
   const int mine = r / kSpan;                      // which of the NV sums this lane ends up with
   const int my_col = DELTA ? mine - CPT : mine;    // its column, if it is a read-out
@@ -485,6 +495,7 @@ __global__ void __launch_bounds__(32 * (kOwnerWarps + kStageWarps)) outer_scan_k
 #pragma unroll
               for (int e = 0; e < 2; ++e) {
                 P[c][j][e] = fma2(al[e], P[c][j][e], mul2(kp[e], w[c]));
+                if (HGRN && padded) P[c][j][e] &= live[j][e];
                 eq[c][e] = fma2(P[c][j][e], qp[e], eq[c][e]);
               }
           }
