@@ -37,13 +37,10 @@ PARITY_ROWS: List[dict] = []  # every check_close / report_rel call of this proc
 
 
 def _record(row: dict) -> None:
-    """Keep and print one parity measurement, and append it to $VILA_PARITY_REPORT (default:
-    gpurun_out/parity_report.jsonl when that directory exists) so the table can be committed."""
+    """Keep and print one parity measurement, and append it to the file that $VILA_PARITY_REPORT names, if it is set."""
     PARITY_ROWS.append(row)
     print("[parity] " + json.dumps(row))
     out = os.environ.get("VILA_PARITY_REPORT")
-    if out is None and os.path.isdir("gpurun_out"):
-        out = "gpurun_out/parity_report.jsonl"
     if out:
         try:
             with open(out, "a") as f:

@@ -1,6 +1,6 @@
 """CUDA-event timing (cold L2: 256 MB scratch write between launches, median of 20) of the data-movement kernels
 at their NVILA shapes: dynamic-S2 merge of 35 tiles, TSP pooling of 64 frames, chessboard merge, RoPE + KV append
-(table flavour), space-to-depth.  Writes gpurun_out/datamove.json."""
+(table flavour), space-to-depth.  Writes bench_out/datamove.json."""
 import json
 import statistics
 import sys
@@ -73,7 +73,7 @@ posv = torch.arange(Sv, dtype=torch.int32, device=dev)
 tbl = ops.rope_table(posv, D, inv)
 case("rope_kv_append_table S=16470", 2 * (2 * Sv * (Hq + Hkv) * D + 2 * Sv * Hkv * D),
      lambda: ops.rope_kv_append_table(qkv_big, tbl, Hq, Hkv, D, kpv, vpv, ptv, 0))
-out = Path("gpurun_out")
+out = Path("bench_out")
 if out.is_dir():
     (out / "datamove.json").write_text(json.dumps({"hbm_peak_gbs": PEAK, "note": "CUDA events, cold L2, median of 20",
                                                    "rows": rows}, indent=1))

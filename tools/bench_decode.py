@@ -35,5 +35,5 @@ for name, cls, kw in (("graph", GraphDecoder, {}), ("mega_s8", MegaDecoder, {"nu
         toks = dec.tokens(128)
     res[name] = {"ms_per_token": round(ms / 127, 4), "tok_s": round(127 / ms * 1e3, 1), "wall_s": round(wall, 3), "first_tokens": toks[:6]}
     print(name, res[name], flush=True)
-Path("gpurun_out").mkdir(exist_ok=True)
-Path("gpurun_out/bench_decode%s.json" % ("_tiny" if tiny else "")).write_text(json.dumps(res, indent=1))
+Path("bench_out").mkdir(exist_ok=True)
+Path("bench_out/bench_decode%s.json" % ("_tiny" if tiny else "")).write_text(json.dumps(res, indent=1))

@@ -62,5 +62,5 @@ for ctx in (279, 1000, 2000, 4000, 16448, 65814):
     res[str(ctx)] = row
     print(ctx, json.dumps(row), flush=True)
     del pools
-Path("gpurun_out").mkdir(exist_ok=True)
-Path("gpurun_out/bench_decode_attn.json").write_text(json.dumps(res, indent=1))
+Path("bench_out").mkdir(exist_ok=True)
+Path("bench_out/bench_decode_attn.json").write_text(json.dumps(res, indent=1))

@@ -28,5 +28,5 @@ for variant, tag in ((1, "v1"), (2, "v2"), (3, "v2_poly4")):
     flops = 4.0 * B * S * S * H * D * (0.5 if causal else 1.0)
     res[tag + ":" + name] = {"us": round(us, 1), "tflops": round(flops / us / 1e6, 1)}
     print(tag, name, res[tag + ":" + name], flush=True)
-Path("gpurun_out").mkdir(exist_ok=True)
-Path("gpurun_out/bench_fmha.json").write_text(json.dumps(res, indent=1))
+Path("bench_out").mkdir(exist_ok=True)
+Path("bench_out/bench_fmha.json").write_text(json.dumps(res, indent=1))

@@ -52,5 +52,5 @@ for name, (M, N, K) in shapes.items():
     print(name, (M, N, K), row, flush=True)
     del ws
     torch.cuda.empty_cache()
-Path("gpurun_out").mkdir(exist_ok=True)
-Path("gpurun_out/bench_gemm.json").write_text(json.dumps(res, indent=1))
+Path("bench_out").mkdir(exist_ok=True)
+Path("bench_out/bench_gemm.json").write_text(json.dumps(res, indent=1))

@@ -36,5 +36,5 @@ for name, (N, K, swiglu) in shapes.items():
         print(name, "variant", variant, f"{us:8.2f} us  {gbs:7.1f} GB/s  {gbs/peak:.3f}", flush=True)
     del ws
     torch.cuda.empty_cache()
-Path("gpurun_out").mkdir(exist_ok=True)
-Path("gpurun_out/bench_gemv.json").write_text(json.dumps(res, indent=1))
+Path("bench_out").mkdir(exist_ok=True)
+Path("bench_out/bench_gemv.json").write_text(json.dumps(res, indent=1))

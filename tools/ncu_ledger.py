@@ -1,7 +1,7 @@
 """One launch of every hot-path kernel at its NVILA-8B shape, bracketed by cudaProfilerStart/Stop, for
 
     ncu --set full --clock-control none --profile-from-start off \
-        -k regex:vb:: -f -o gpurun_out/ledger python tools/ncu_ledger.py
+        -k regex:vb:: -f -o bench_out/ledger python tools/ncu_ledger.py
 
 Each entry prints `LEDGER <index> <label> <algorithmic bytes> <algorithmic flops>` in launch order so
 tools/ncu_ledger_extract.py can put the algorithmic work beside ncu's dram bytes / durations.
@@ -245,7 +245,7 @@ def main():
         print("LEDGER %d | %s | %d | %d | %.2f us" % (i, label, nbytes, flops, us), flush=True)
         rows.append({"index": i, "label": label, "algorithmic_bytes": nbytes, "algorithmic_flops": flops,
                      "event_us_cold": round(us, 2)})
-    out = Path("gpurun_out")
+    out = Path("bench_out")
     if out.is_dir():
         (out / "ledger_labels.json").write_text(json.dumps(rows, indent=1))
 

@@ -1,4 +1,4 @@
-"""Read gpurun_out/ledger.ncu-rep (made by `tools/run_gpu_r2.sh ledger`) here — no GPU needed — and
+"""Read bench_out/ledger.ncu-rep here — no GPU needed — and
 write profiles/r02_ncu_ledger.json + a markdown table: per kernel launch the ncu duration (cold L2,
 serialised), DRAM bytes (dram__bytes_read.sum + dram__bytes_write.sum), DRAM / tensor-pipe
 utilisation, registers, shared memory, and beside them the ALGORITHMIC bytes / flops of the entry
@@ -12,7 +12,7 @@ import sys
 from pathlib import Path
 
 ROOT = Path(__file__).resolve().parent.parent
-rep = Path(sys.argv[1] if len(sys.argv) > 1 else ROOT / "gpurun_out/ledger_raw.csv")
+rep = Path(sys.argv[1] if len(sys.argv) > 1 else ROOT / "bench_out/ledger_raw.csv")
 labels = json.loads((rep.parent / "ledger_labels.json").read_text())
 peaks = {"hbm_gbs": 6574.5, "bf16_tflops": 1724.0}
 pk = ROOT / "MEASURED_PEAKS.json"

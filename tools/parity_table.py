@@ -1,11 +1,11 @@
-"""gpurun_out/parity_report.jsonl (every check_close / report_rel of a `pytest -m gpu` run) ->
+"""bench_out/parity_report.jsonl (every check_close / report_rel of a `pytest -m gpu` run) ->
 profiles/r02_parity.md + .jsonl.  Usage: python tools/parity_table.py [jsonl]"""
 import json
 import sys
 from pathlib import Path
 
 ROOT = Path(__file__).resolve().parent.parent
-src = Path(sys.argv[1] if len(sys.argv) > 1 else ROOT / "gpurun_out/parity_report.jsonl")
+src = Path(sys.argv[1] if len(sys.argv) > 1 else ROOT / "bench_out/parity_report.jsonl")
 rows = [json.loads(l) for l in src.read_text().splitlines() if l.strip()]
 seen, uniq = set(), []
 for r in rows:

@@ -1,5 +1,5 @@
 """One launch of the two-tile FMHA kernel at the 64-frame video shape (causal GQA, d=128, S=16470, paged)
-inside a cudaProfilerStart/Stop range — the target of `tools/run_gpu_r2.sh ncu_one`."""
+inside a cudaProfilerStart/Stop range."""
 import sys
 from pathlib import Path
 

@@ -1,7 +1,7 @@
-"""gpurun_out/bench_gemm.json -> profiles/r02_gemm_configs.md (markdown table)."""
+"""bench_out/bench_gemm.json -> profiles/r02_gemm_configs.md (markdown table)."""
 import json, sys
 from pathlib import Path
-d = json.loads(Path(sys.argv[1] if len(sys.argv) > 1 else "gpurun_out/bench_gemm.json").read_text())
+d = json.loads(Path(sys.argv[1] if len(sys.argv) > 1 else "bench_out/bench_gemm.json").read_text())
 cfgs = ["None", "2128", "2256", "4128", "4256", "5128", "3000", "3001"]
 names = {"None": "dispatch", "2128": "1-CTA 128x128", "2256": "1-CTA 128x256", "4128": "pair 256x128",
          "4256": "pair 256x256", "5128": "split-K pair", "3000": "skinny", "3001": "skinny pair"}

@@ -1,7 +1,6 @@
 """In-tree build of libvila_b200.so (sm_100a only) with nvcc.
 
-`python -m vila_b200.build` or `__graft_entry__.build()`.  The .so is git-ignored but travels with
-the gpurun snapshot; nothing is JIT-compiled at run time.
+`python -m vila_b200.build` or `__graft_entry__.build()`.  The .so is git-ignored; nothing is JIT-compiled at run time.
 """
 from __future__ import annotations
 

@@ -591,7 +591,7 @@ int launch_skinny(const __nv_bfloat16* A, int lda, const __nv_bfloat16* W, int l
   a.epi = epi;
   a.dbg = nullptr;
 #ifdef VILA_B200_DEBUG_HOOKS  // clock stamps, left out of the shipped library: no variable may name a pointer to write to
-  if (const char* e = getenv("VILA_B200_GEMM_DEBUG")) {  // hex device pointer (tools/skinny_phase_times.py)
+  if (const char* e = getenv("VILA_B200_GEMM_DEBUG")) {  // hex device pointer
     unsigned long long ptr = 0;
     if (sscanf(e, "%llx", &ptr) == 1) a.dbg = reinterpret_cast<long long*>(ptr);
   }
