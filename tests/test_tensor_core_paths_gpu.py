@@ -85,6 +85,42 @@ def test_glinear_batched(ops, M):
     assert rel(ops.glinear(a, w, groups=H, a_group_off=K, o_group_off=N, out_dtype=F32), ref) < acc(K)
 
 
+@pytest.mark.parametrize("K", [256, 2048, 8192])
+@pytest.mark.parametrize("positive", [False, True])
+def test_glinear_few_rows_sum_in_fp32(ops, K, positive):
+    """up to 16 rows, or 64 routed pairs: a lane's chain of K / 32 rounded multiply-adds (errors both ways) and five steps of
+    a tree, whatever the number of rows and outputs is"""
+    g = gen(K)
+    tol = (K / 32) ** 0.5 * 2.0 ** -25 + 5 * 2.0 ** -25
+    data = (lambda *s: randn(g, *s).abs()) if positive else (lambda *s: randn(g, *s))
+    for N in (130, 6002, 12004):
+        a, w = data(16, K), data(N, K)
+        ref, alone = a.double() @ w.double().T, ops.glinear(a[:1], w, out_dtype=F32)
+        for M in (1, 2, 3, 5, 8, 9, 16):
+            got = ops.glinear(a[:M], w, out_dtype=F32)
+            assert rel(got, ref[:M]) < tol and torch.equal(got[:1], alone)
+            z = torch.nn.functional.silu(ref[:M, 0::2]) * ref[:M, 1::2]
+            assert rel(ops.glinear(a[:M], w, swiglu=True, out_dtype=F32), z) < 3 * tol + 1e-6
+    for T, E, top in ((3, 8, 2), (16, 32, 4), (64, 4, 1), (32, 2, 2), (20, 1, 1)):
+        x, w = data(T, K), data(E, 256, K)
+        idx = torch.rand(T, E, generator=g, device="cuda").topk(top, 1).indices.to(torch.int32)
+        seg, srt = ops.moe_group(idx, E)
+        got = ops.glinear(x, w, groups=E, seg=seg, a_rows=srt, a_row_div=top, out_dtype=F32)
+        e, tok = idx.view(-1)[srt.long()].long(), srt.long() // top
+        assert rel(got, torch.einsum("rk,rnk->rn", x.double()[tok], w.double()[e])) < tol
+
+
+def test_glinear_one_row_at_every_tile_size(ops):
+    """the kernels of few, some and many rows cut K differently: a row's sums may differ by what each is off"""
+    g, K = gen(3), 2048
+    a, w = randn(g, 257, K), randn(g, 384, K)
+    ref = a.double() @ w.double().T
+    rows = [ops.glinear(a[:M], w, out_dtype=F32)[:1] for M in (1, 16, 17, 64, 65, 257)]
+    assert torch.equal(rows[0], rows[1]) and torch.equal(rows[2], rows[3]) and torch.equal(rows[4], rows[5])
+    for r in rows:
+        assert rel(r, ref[:1]) < acc(K) and rel(r, rows[0].double()) < 2 * acc(K)
+
+
 @pytest.mark.parametrize("routed", [False, True])
 @pytest.mark.parametrize("rows", [40, 600])
 def test_glinear_waits_that_run_out_are_reported(ops, monkeypatch, rows, routed):

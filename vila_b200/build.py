@@ -33,6 +33,7 @@ SOURCES = [
     "ragged_lm.cu",
     "glinear.cu",
     "glinear_tcgen05.cu",
+    "glinear_rows.cu",
     "latent_attn.cu",
     "hgrn2.cu",
     "short_conv.cu",

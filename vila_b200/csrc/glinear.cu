@@ -245,11 +245,6 @@ __device__ __forceinline__ void load8(const void* p, int dt, size_t i, float (&v
   }
 }
 
-__device__ __forceinline__ float finish(const vila_glinear_params& p, const vila_glinear_ext& x, float z, int g, int n) {
-  if (p.bias) z += ld_any(p.bias, p.w_dtype, static_cast<size_t>(g) * p.bias_group_stride + n);
-  return activate(z, p.act, x);
-}
-
 // vec: K % 8 == 0 and every row of A and W starts on an 8-element boundary (16 B bf16, 32 B fp32)
 __global__ void __launch_bounds__(kSmallWarps * 32) glinear_small_kernel(const vila_glinear_params p, const vila_glinear_ext x, int vec) {
   __shared__ int arow_s[kSmallRows], orow_s[kSmallRows];
@@ -350,6 +345,7 @@ int glinear(const vila_glinear_params& p, cudaStream_t stream, const vila_glinea
   VB_CHECK(p.act >= VILA_ACT_NONE && p.act <= VILA_ACT_SOFTCAP && (p.act != VILA_ACT_SOFTCAP || x.act_pos > 0.f),
            "glinear: act=%d (cap %f)", p.act, x.act_pos);
   VB_CHECK(p.a_rows == nullptr || p.a_row_div >= 1, "glinear: a_row_div=%d", p.a_row_div);
+  if (tries < 0 && glinear_rows_takes(p)) return glinear_rows(p, stream, x);
   if (glinear_tc_takes(p)) return glinear_tc(p, stream, x, tries);
   VB_CHECK(tries < 0, "glinear: the kernel with limited waits does not take this layer");
   const bool small = p.M <= 16;

@@ -33,6 +33,12 @@ __device__ __forceinline__ float glu(float g, float u, int flags, const vila_gli
   return (flags & VILA_FLAG_GEGLU ? gelu_tanh_exact_f(g) : silu_exact_f(g)) * u;
 }
 
+// bias and activation of one output
+__device__ __forceinline__ float finish(const vila_glinear_params& p, const vila_glinear_ext& x, float z, int g, int n) {
+  if (p.bias) z += ld_any(p.bias, p.w_dtype, static_cast<size_t>(g) * p.bias_group_stride + n);
+  return activate(z, p.act, x);
+}
+
 // scale of the INPUT row behind sorted position i (= output row: in_scale is only taken without o_rows)
 __device__ __forceinline__ float in_scale_of(const vila_glinear_params& p, const vila_glinear_ext& x, int i) {
   return x.in_scale ? x.in_scale[p.a_rows ? p.a_rows[i] : i] : 1.0f;

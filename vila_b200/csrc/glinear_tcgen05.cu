@@ -15,12 +15,14 @@
 //   MMA warp        TMEM allocation and tcgen05.mma into one of two accumulator sets: a tile's epilogue runs under
 //                   the next tile's products
 //
-// Tiles are dealt round-robin, token tiles fastest, so that the tiles that share weights run together.  Every output
-// is a sum over K in a fixed order, whatever tile, batch or group its row is in.
+// Tiles are dealt round-robin, token tiles fastest, so that the tiles that share weights run together.  A tile size sums K
+// in a fixed order, whatever tile or group a row is in, but the sizes cut K into different numbers of accumulators (kAcc):
+// the rounding of a row changes where the number of rows changes the tile size.  Few rows are served by glinear_rows.cu,
+// whose sums are rounded, not truncated.
 //
-// Measured against the CUDA-core and wmma forms it replaces for these operands: a head of 32768 x 2048 on 8 rows
-// 166 -> 33 us; the two projections of a routed block of 32 experts (1408 | 704 x 2048, 4 per token) on 2048 tokens
-// 720 -> 149 us (475 and 410 TFLOP/s, tiles of 128 - 256 tokens), on 8 tokens 145 -> 47 us.
+// Measured against the wmma form it replaces for these operands: the two projections of a routed block of 32 experts
+// (1408 | 704 x 2048, 4 per token) on 2048 tokens 720 -> 149 us (475 and 410 TFLOP/s, tiles of 128 - 256 tokens); the error
+// is the wmma form's (2.1e-6 at K = 2048, one accumulator) or less.
 #include "../../include/vila_b200.h"
 #include "common.cuh"
 #include "kernels.h"
@@ -75,7 +77,7 @@ template <int BT> struct Shape {   // BT: most tokens of a tile
   static constexpr int kPerSm = BT <= 64 ? 2 : 1;   // CTAs an SM holds
   static constexpr int kStage = kWBytes + BT * kDepth * 2;
   // K is summed in kAcc accumulators that the epilogue adds: the tensor core truncates as it accumulates, so the
-  // error of one long sum grows with its length (K = 2048: 2.1e-6 in one accumulator, 5e-7 in four)
+  // error of one long sum grows with its length (K = 2048: 2.1e-6 in one accumulator, 1.0e-6 in two, 4.7e-7 in four)
   static constexpr int kAcc = BT <= 16 ? 4 : (BT <= 64 ? 2 : 1);
   static constexpr int kCols = 2 * kAcc * BT;       // TMEM columns: the CTAs of an SM share 512
   static constexpr int kMeta = 2 * BT * 12;         // two tiles' output rows, routing weights, input scales
@@ -490,7 +492,7 @@ int glinear_tc(const vila_glinear_params& p, cudaStream_t stream, const vila_gli
   if (int rc = make_tmap_3d_bf16(&tm, p.w, p.K, p.N, p.groups, p.ldw, gs, kDepth, kRowsW, 1, 128)) return rc;
   // tokens of a tile: all of a plain layer's rows up to 256; of routed rows about twice the mean of a group.  Small
   // tiles leave room for two CTAs on an SM and more weight stages, which is what decoded tokens are bound by.
-  const int rows = p.mode == 0 ? p.M : 2 * ((p.M + p.groups - 1) / p.groups);
+  const int mean2 = 2 * ((p.M + p.groups - 1) / p.groups), rows = p.mode == 0 || p.M < mean2 ? p.M : mean2;
   const int bt = rows <= 16 ? 16 : (rows <= 64 ? 64 : 256);
   // A (consecutive rows): plain and routed layers end at column K, column groups at the row's end; rows past M read as zero
   const bool grouped = p.mode == 0 && p.groups > 1;

@@ -312,6 +312,9 @@ bool glinear_tc_takes(const vila_glinear_params& p);
 unsigned int stalled_waits();
 int wait_status();   // 1 (and the last error) once after a launch whose wait ran out of tries; does not synchronise
 int glinear_tc(const vila_glinear_params& p, cudaStream_t stream, const vila_glinear_ext& x, int tries);
+// few rows of bf16 operands: fp32 multiply-adds over the streamed weights (glinear_rows.cu)
+bool glinear_rows_takes(const vila_glinear_params& p);
+int glinear_rows(const vila_glinear_params& p, cudaStream_t stream, const vila_glinear_ext& x);
 // tries >= 0: of every wait of the tcgen05 kernel (tests); otherwise its own limit
 int glinear(const vila_glinear_params& p, cudaStream_t stream, const vila_glinear_ext* ext = nullptr, int tries = -1);
 int latent_attention(const vila_latent_attn_params& p, cudaStream_t stream);
