@@ -160,6 +160,10 @@ def test_glinear_waits_that_run_out_are_reported(ops, monkeypatch, rows, routed)
     limited(0)
     with pytest.raises(RuntimeError, match="ran out"):
         ops.glinear(a, w, out_dtype=F32, **kw)     # the next call says so as well
+    limited(0)
+    from vila_b200.serving import TokenEngine
+    with pytest.raises(RuntimeError, match="ran out"):
+        TokenEngine.step(object.__new__(TokenEngine), [])   # and the engine before it builds a step on that output
     assert torch.equal(limited(1 << 20), want)
 
 
