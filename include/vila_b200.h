@@ -736,6 +736,10 @@ typedef struct vila_ssd_scan_params {
   int32_t in_dtype, out_dtype, nseq, H, P, N, G;
 } vila_ssd_scan_params;
 int vila_ssd_scan(const vila_ssd_scan_params* p, void* stream);
+/* The same for sequences that have `rows` rows or fewer together, each row in one of them: portions of 48 rows or more run in
+ * chunks of 64 tokens where operands, sizes and alignment allow it, the others token by token.  Both have fp32 precision;
+ * the order of their sums differs. */
+int vila_ssd_scan_rows(const vila_ssd_scan_params* p, int rows, void* stream);
 
 /* vila_selective_scan — recurrence with a step size and decay per channel, fp32 state [slots, C, N]:
  *   dt_t,c = softplus(dt_raw_t,c + dt_bias_c),  S_t[c, n] = exp(-exp(A_log[c, n]) dt_t,c) S_{t-1}[c, n] + dt_t,c x_t,c B_t,n

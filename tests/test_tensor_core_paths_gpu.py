@@ -558,3 +558,96 @@ def test_hgrn2_infinite_value(ops, dim):
             out.append(ops.hgrn2_scan(proj[t:t + n], state, torch.tensor([(0, n, t, 0)], dtype=torch.int32, device="cuda"), **kw))
         out = torch.cat(out).view(T, H, vdim)
         assert torch.isinf(out[2:, 0, 7]).all() and torch.isfinite(out[:2]).all() and torch.isfinite(out[:, 0, :7]).all() and torch.isfinite(out[:, 1]).all()
+
+
+# ---- ssd scans in chunks of 64 tokens ---------------------------------------------------------------------------
+def ssd_inputs(lens, H, P, N, G, seed=3, gate=True, pad=8):
+    """x | B | C behind a SiLU, step sizes and gates as a projection leaves them; odd slots start in mid-sequence"""
+    g, T = gen(seed), sum(lens)
+    wide = torch.randn(T, H * P + 2 * G * N + pad, generator=g, device="cuda")
+    xbc = torch.nn.functional.silu(wide).to(BF)[:, :H * P + 2 * G * N]
+    z = torch.randn(T, H * P, generator=g, device="cuda").to(BF) if gate else None
+    dt = torch.randn(T, H + 1, generator=g, device="cuda").to(BF)[:, :H]
+    kw = dict(heads=H, vdim=P, nstate=N, groups=G, dt_bias=torch.rand(H, generator=g, device="cuda") * 2.3 - 4.6,
+              A_log=torch.log(1 + 15 * torch.rand(H, generator=g, device="cuda")), D=torch.randn(H, generator=g, device="cuda"))
+    state = torch.randn(len(lens) + 1, H, P, N, generator=g, device="cuda")
+    rows = [sum(lens[:s]) for s in range(len(lens))]
+    seqs = torch.tensor([(rows[s], n, 7 if s % 2 else 0, len(lens) - s) for s, n in enumerate(lens)], dtype=torch.int32, device="cuda")
+    return xbc, dt, z, state, seqs, kw
+
+
+def ssd_float64(xbc, dt, z, state, seqs, kw):
+    H, P, N, G = kw["heads"], kw["vdim"], kw["nstate"], kw["groups"]
+    u, S_all = xbc.double(), state.double()
+    out = torch.empty(u.shape[0], H, P, dtype=torch.float64, device="cuda")
+    step = torch.nn.functional.softplus(dt.double() + kw["dt_bias"].double())
+    A = torch.exp(kw["A_log"].double())
+    for r, n, pos, slot in seqs.tolist():
+        S = S_all[slot] if pos else torch.zeros_like(S_all[slot])
+        for t in range(r, r + n):
+            x = u[t, :H * P].view(H, P)
+            B, Cm = (u[t, H * P + i * G * N:H * P + (i + 1) * G * N].view(G, N).repeat_interleave(H // G, 0) for i in range(2))
+            S = torch.exp(-A * step[t])[:, None, None] * S + (step[t][:, None] * x)[:, :, None] * B[:, None]
+            out[t] = torch.einsum("hpn,hn->hp", S, Cm) + kw["D"].double()[:, None] * x
+        S_all[slot] = S
+    out = out.view(u.shape[0], -1)
+    return (out if z is None else out * torch.nn.functional.silu(z.double())), S_all
+
+
+@pytest.mark.parametrize("lens,H,P,N,G,gate", [([48], 2, 64, 128, 1, True), ([63, 64, 65], 4, 32, 128, 2, True), ([129, 47, 1, 192], 2, 48, 128, 2, False),
+                                               ([200], 3, 16, 128, 1, True), ([70, 48], 2, 96, 64, 1, True), ([66], 150, 32, 128, 5, True)])
+def test_ssd_chunks(ops, lens, H, P, N, G, gate):
+    """portions at the chunks' edges, beside shorter ones that go token by token; 16 and 32 columns per CTA"""
+    xbc, dt, z, state, seqs, kw = ssd_inputs(lens, H, P, N, G, gate=gate)
+    want, S = ssd_float64(xbc, dt, z, state, seqs, kw)
+    got_state = state.clone()
+    got = ops.ssd_scan(xbc, dt, z, got_state, seqs, **kw)
+    # fp32 roundings of a sum of decaying terms: a few units of 6e-8
+    assert rel(got, want) < 5e-7 and rel(got_state, S) < 5e-7 and torch.equal(got_state[0], state[0])
+    assert rel(ops.ssd_scan(xbc, dt, z, state.clone(), seqs, out_dtype=BF, **kw), want) < 4e-3
+    # a sequence's numbers depend neither on the batch nor on the others' lengths (columns per CTA differ)
+    for s, (r, n, pos, slot) in enumerate(seqs.tolist()):
+        one = state.clone()
+        alone = ops.ssd_scan(xbc[r:r + n], dt[r:r + n], None if z is None else z[r:r + n], one, torch.tensor([(0, n, pos, slot)], dtype=torch.int32, device="cuda"), **kw)
+        assert rel(alone, got[r:r + n]) < 5e-7 and rel(one[slot], got_state[slot]) < 5e-7
+
+
+def test_ssd_chunks_after_any_decay(ops):
+    """steps that forget the state at once and steps that keep it, in one chunk"""
+    xbc, dt, z, state, seqs, kw = ssd_inputs([100, 100], 2, 32, 128, 1)
+    dt = dt.float() * 1.0
+    dt[10::7], dt[13::11] = 60.0, -40.0
+    dt = dt.to(BF)
+    want, S = ssd_float64(xbc, dt, z, state, seqs, kw)
+    got = ops.ssd_scan(xbc, dt, z, state, seqs, **kw)
+    assert rel(got, want) < 5e-7 and rel(state[1:], S[1:]) < 5e-7
+
+
+@pytest.mark.parametrize("where", ["x", "B", "C", "dt", "z", "state", "nan"])
+def test_ssd_chunks_infinite_numbers(ops, where):
+    """rows before an infinite number stay as they are, the others are what the recurrence makes of it"""
+    H, P, N = 2, 32, 128
+    xbc, dt, z, state, seqs, kw = ssd_inputs([150, 70], H, P, N, 1)
+    inf, r = float("inf"), 80
+    if where == "x": xbc[r, 5] = inf
+    if where == "nan": xbc[r, 5] = float("nan")
+    if where == "B": xbc[r, H * P + 9] = -inf
+    if where == "C": xbc[r, H * P + N + 9] = inf
+    if where == "dt": dt[r, 1] = inf
+    if where == "z": z[r, 3], z[r + 1, 3] = inf, -inf
+    if where == "state": state[1, 0, 3, 4] = inf
+    from vila_b200 import _lib
+    lib, rows = _lib.load(), []
+    call = lib.vila_ssd_scan_rows
+    try:
+        for token_by_token in (False, True):
+            if token_by_token:
+                lib.vila_ssd_scan_rows = lambda p, n, stream: lib.vila_ssd_scan(p, stream)
+            st = state.clone()
+            rows.append((ops.ssd_scan(xbc, dt, z, st, seqs, **kw), st))
+    finally:
+        lib.vila_ssd_scan_rows = call
+    assert not torch.isfinite(rows[1][0]).all()
+    for a, b in zip(*rows):
+        ok = torch.isfinite(b)
+        assert torch.equal(torch.isnan(a), torch.isnan(b)) and torch.equal(torch.isfinite(a), ok) and rel(a[ok], b[ok].double()) < 5e-7

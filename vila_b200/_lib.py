@@ -332,6 +332,7 @@ SIGNATURES = {
     "vila_causal_conv_state": [C.POINTER(CausalConvParams), c_void_p],
     "vila_causal_conv_step": [C.POINTER(CausalConvParams), c_void_p],
     "vila_ssd_scan": [C.POINTER(SsdScanParams), c_void_p],
+    "vila_ssd_scan_rows": [C.POINTER(SsdScanParams), c_int, c_void_p],
     "vila_delta_scan": [C.POINTER(DeltaScanParams), c_void_p],
     "vila_gla_scan": [C.POINTER(GlaScanParams), c_void_p],
     "vila_decay_scan": [C.POINTER(DecayScanParams), c_void_p],

@@ -42,8 +42,9 @@ SOURCES = [
     "paged_attn_decode.cu",
     "ssm.cu",
     "outer_scan.cu",
+    "ssd_chunk.cu",
 ]
-HEADERS = ["common.cuh", "kernels.h", "dtype_any.cuh", "glinear_epi.cuh", "paged_attn_common.cuh", "../../include/vila_b200.h"]
+HEADERS = ["common.cuh", "kernels.h", "dtype_any.cuh", "glinear_epi.cuh", "paged_attn_common.cuh", "mma_bf16.cuh", "../../include/vila_b200.h"]
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",

@@ -601,7 +601,12 @@ int vila_gated_head_norm_act_rows(const float* o, const float* w, const void* ga
 
 int vila_ssd_scan(const vila_ssd_scan_params* p, void* stream) {
   VB_REQUIRE_DEVICE();
-  return vb::ssd_scan(*p, st(stream));
+  return vb::ssd_scan(*p, 0, st(stream));
+}
+
+int vila_ssd_scan_rows(const vila_ssd_scan_params* p, int rows, void* stream) {
+  VB_REQUIRE_DEVICE();
+  return vb::ssd_scan(*p, rows, st(stream));
 }
 
 int vila_selective_scan(const vila_selective_scan_params* p, void* stream) {

@@ -294,7 +294,11 @@ int gla_scan(const vila_gla_scan_params& p, cudaStream_t stream);
 int moe_route_scores(const vila_moe_route_params& p, cudaStream_t stream);
 int tanh_residual_rows(const vila_tanh_residual_params& p, cudaStream_t stream);
 int decay_scan(const vila_decay_scan_params& p, cudaStream_t stream);
-int ssd_scan(const vila_ssd_scan_params& p, cudaStream_t stream);
+// rows: of all sequences together; 0: not known
+int ssd_scan(const vila_ssd_scan_params& p, int rows, cudaStream_t stream);
+// portions of at least min_rows rows, nseq at most, in chunks on the tensor cores (ssd_chunk.cu)
+bool ssd_chunk_takes(const vila_ssd_scan_params& p);
+int ssd_chunk(const vila_ssd_scan_params& p, int nseq, int min_rows, cudaStream_t stream);
 int selective_scan(const vila_selective_scan_params& p, cudaStream_t stream);
 int norm_conv_rows(const vila_norm_conv_params& p, cudaStream_t stream);
 int rope_append(const vila_rope_append_params& p, cudaStream_t stream);

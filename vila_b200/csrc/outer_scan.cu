@@ -34,6 +34,7 @@
 // hgrn2 1208 -> 242 and ssd (64 heads of 64 x 128) 785 -> 304 from the forms that kept one column per thread group.
 // A column's sum runs in the same order whatever CPT and the batch are, and time runs in order: a row's result depends neither on
 // the batch nor on how its sequence was cut into steps (single steps of hgrn2 run in hgrn2.cu, in the same order).
+// Long portions of ssd run in ssd_chunk.cu, in another order of sums: there a row's last bits depend on the cut.
 #include <type_traits>
 #include "../../include/vila_b200.h"
 #include "common.cuh"
@@ -153,6 +154,7 @@ struct ScanArgs {
   int silu;                     // decay: q, k and v are pre-activations, SiLU is taken as they are read
   int vec_qk, vec_a;            // four-element loads of q | k and of z are aligned
   int vec_s;                    // four-element accesses of the state are aligned
+  int below;                    // > 0: only sequences of fewer rows (the others are another launch's)
 };
 
 template <int MODE, int R, int KPT, int CPT, int kStageWarps>
@@ -178,6 +180,10 @@ __global__ void __launch_bounds__(32 * (kOwnerWarps + kStageWarps)) outer_scan_k
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int* sq = p.seqs + 4 * blockIdx.x;
   const int row0 = sq[0], n = sq[1], pos0 = sq[2], slot = sq[3];
+  if (p.below > 0 && n >= p.below) {
+    griddep_wait();
+    return;
+  }
   const int h = blockIdx.y, dim = p.dim, vdim = p.vdim, kh = h / (p.H / p.G);
   const int col0 = blockIdx.z * COLS;
   const int nchunks = (n + kChunk - 1) / kChunk;
@@ -612,6 +618,7 @@ __global__ void __launch_bounds__(32 * (kOwnerWarps + kStageWarps)) outer_scan_k
       }
     });
   }
+  if (p.below > 0) griddep_wait();   // this launch ends after the one it may have started beside
 }
 
 template <int MODE, int R, int KPT, int CPT>
@@ -628,7 +635,9 @@ int launch_scan(const ScanArgs& p, int nseq, cudaStream_t stream) {
     VB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
   const dim3 grid(nseq, p.H, (p.vdim + COLS - 1) / COLS);
   VB_CHECK(grid.y <= 65535 && grid.z <= 65535, "outer_scan: H=%d vdim=%d", p.H, p.vdim);
-  VB_CUDA(launch_serial(kern, grid, dim3(32 * (kOwnerWarps + SW)), smem, stream, p));
+  // below: beside the launch that has the longer sequences (other rows and slots; that one started after all before it)
+  if (p.below > 0) VB_CUDA(launch_pdl(kern, grid, dim3(32 * (kOwnerWarps + SW)), smem, stream, p));
+  else VB_CUDA(launch_serial(kern, grid, dim3(32 * (kOwnerWarps + SW)), smem, stream, p));
   return 0;
 }
 
@@ -716,7 +725,7 @@ int decay_scan(const vila_decay_scan_params& p, cudaStream_t stream) {
   return scan_by_dim<kDecay>(a, p.nseq, stream);
 }
 
-int ssd_scan(const vila_ssd_scan_params& p, cudaStream_t stream) {
+int ssd_scan(const vila_ssd_scan_params& p, int rows, cudaStream_t stream) {
   if (p.nseq <= 0) return 0;
   VB_CHECK(p.H >= 1 && p.G >= 1 && p.H % p.G == 0 && p.P >= 1 && p.N >= 1 && p.N <= 256,
            "ssd_scan: H=%d G=%d P=%d N=%d (<= 256)", p.H, p.G, p.P, p.N);
@@ -735,6 +744,13 @@ int ssd_scan(const vila_ssd_scan_params& p, cudaStream_t stream) {
   a.H = p.H; a.G = p.G; a.dim = p.N; a.vdim = p.P;
   a.q_scale = 1.0f;
   a.vec_qk = p.N % 4 == 0 && rows_aligned4(a.q, p.ld_xbc, p.in_dtype) && rows_aligned4(a.k, p.ld_xbc, p.in_dtype);
+  // Chunks of 64 tokens from 48 rows on: 64 heads of 64 x 128 take 7.7 us for 32 rows one by one and 9.8 for 48, in chunks 8.3
+  // for both and 114 against 300 for 2048.  By each sequence's own rows, so that its numbers do not depend on the others.
+  constexpr int kChunkRows = 48;
+  if (rows - p.nseq + 1 >= kChunkRows && ssd_chunk_takes(p)) {
+    if (const int rc = ssd_chunk(p, min(p.nseq, rows / kChunkRows), kChunkRows, stream)) return rc;
+    a.below = kChunkRows;
+  }
   return scan_by_dim<kSsd>(a, p.nseq, stream);
 }
 

@@ -30,6 +30,7 @@
 #include "kernels.h"
 #include "dtype_any.cuh"
 #include "paged_attn_common.cuh"
+#include "mma_bf16.cuh"
 
 namespace vb {
 namespace {
@@ -38,25 +39,6 @@ constexpr int kBK = 64;      // keys of a block
 constexpr int kMaxWarps = 8;
 constexpr float kLog2e = 1.44269504f;   // 1 / ln 2
 
-__device__ __forceinline__ void ldsm4(uint32_t addr, uint32_t (&r)[4]) {
-  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
-               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr));
-}
-__device__ __forceinline__ void ldsm4_t(uint32_t addr, uint32_t (&r)[4]) {
-  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
-               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr));
-}
-__device__ __forceinline__ void mma_bf16(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
-  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-               : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
-               : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
-}
-// the same into fresh sums
-__device__ __forceinline__ void mma_bf16_first(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
-  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};"
-               : "=f"(c[0]), "=f"(c[1]), "=f"(c[2]), "=f"(c[3])
-               : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1), "f"(0.f));
-}
 // two of a fragment's sums at a time: c0, c1 (or c2, c3) belong to one row
 using f2 = unsigned long long;
 __device__ __forceinline__ f2 pair(float x, float y) {
@@ -74,17 +56,6 @@ __device__ __forceinline__ void add2(float& ax, float& ay, float cx, float cy) {
   f2 r;
   asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(pair(ax, ay)), "l"(pair(cx, cy)));
   unpair(r, ax, ay);
-}
-// two fp32 numbers -> three packed pairs of bf16 that add up to them (the last part takes what 16 bits leave)
-__device__ __forceinline__ void split3(float x, float y, uint32_t& hi, uint32_t& mid, uint32_t& lo) {
-  hi = pack_bf16(x, y);
-  const float x1 = x - bf_lo(hi), y1 = y - bf_hi(hi);
-  mid = pack_bf16(x1, y1);
-  lo = pack_bf16(x1 - bf_lo(mid), y1 - bf_hi(mid));
-}
-__device__ __forceinline__ void cp16(uint32_t dst, const void* src, bool ok) {
-  const uint32_t n = ok ? 16u : 0u;   // 0: zeros
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(n) : "memory");
 }
 __device__ __forceinline__ float ex2(float x) {
   float y;

@@ -1072,7 +1072,7 @@ def ssd_scan(xbc: torch.Tensor, dt: torch.Tensor, z: Optional[torch.Tensor], sta
     p.state, p.seqs, p.out, p.ld_out = _p(state), _i32(seqs, "seqs"), _p(out), out.stride(0)
     p.in_dtype, p.out_dtype = _dt(xbc, "xbc"), _dt(out, "out")
     p.nseq, p.H, p.P, p.N, p.G = seqs.shape[0], heads, vdim, nstate, groups
-    check(_lib.load().vila_ssd_scan(C.byref(p), _stream()), "vila_ssd_scan")
+    check(_lib.load().vila_ssd_scan_rows(C.byref(p), T, _stream()), "vila_ssd_scan_rows")
     return out
 
 
