@@ -651,3 +651,45 @@ def test_ssd_chunks_infinite_numbers(ops, where):
     for a, b in zip(*rows):
         ok = torch.isfinite(b)
         assert torch.equal(torch.isnan(a), torch.isnan(b)) and torch.equal(torch.isfinite(a), ok) and rel(a[ok], b[ok].double()) < 5e-7
+
+
+@pytest.mark.parametrize("M,N,K", [(1, 128, 2048), (8, 130, 2056), (9, 129, 4096), (16, 4097, 4104), (16, 200, 8192), (3, 17000, 1032), (5, 33000, 512), (16, 333, 264),
+                                   (2, 144, 8)])
+def test_few_rows_stream(ops, M, N, K):
+    """CTAs that stay and those that don't: ragged columns, a last tile of one weight row, token rows that do not fit in shared memory"""
+    g = gen(M + N + K)
+    a, w, b = randn(g, M, K + 8)[:, :K], randn(g, N, K), randn(g, N)
+    ref = a.double() @ w.double().T
+    got = ops.glinear(a, w, out_dtype=F32)
+    # about 32 roundings of at most 2^-24 each, taken as independent
+    assert rel(got, ref) < 32 ** 0.5 * 2.0 ** -24
+    assert rel(ops.glinear(a, w, bias=b, act=ops.ACT_RELU2, out_dtype=F32), torch.relu(ref + b.double()) ** 2) < 3 * 32 ** 0.5 * 2.0 ** -24
+    # a row's sums do not depend on the other rows
+    assert torch.equal(ops.glinear(a[:1], w, out_dtype=F32), got[:1])
+    if N % 2 == 0:
+        z = ref / K ** 0.5
+        want = torch.nn.functional.silu(z[:, 0::2]) * z[:, 1::2]
+        assert rel(ops.glinear((a.float() / K ** 0.5).to(BF), w, swiglu=True, out_dtype=F32), want) < 2.0 ** -7   # a is rounded once more
+
+
+@pytest.mark.parametrize("T,E,top,N,K,shared", [(16, 40, 4, 256, 1024, True), (16, 3, 2, 1000, 2048, True), (12, 70, 5, 130, 4096, False), (21, 33, 3, 144, 1040, False),
+                                                (1, 9, 4, 1040, 1024, True), (16, 4, 4, 200, 704, True)])
+def test_few_pairs_stream(ops, T, E, top, N, K, shared):
+    """groups without rows and with more than a pass of eight, rows that several pairs share or do not"""
+    g = gen(T + E + N)
+    idx = torch.rand(T, E, generator=g, device="cuda").topk(min(top, E)).indices.to(torch.int32)
+    top = idx.shape[1]
+    idx[:, 0] = 1                                                     # group 1 has T pairs, group 0 none but by chance
+    seg, srt = ops.moe_group(idx, E)
+    w = randn(g, E, N, K)
+    a = randn(g, T if shared else T * top, K)
+    wt, scale = torch.rand(T * top, generator=g, device="cuda"), torch.rand(a.shape[0], generator=g, device="cuda")
+    rows = a.double().repeat_interleave(top, 0) if shared else a.double()
+    ref = torch.einsum("rk,rnk->rn", rows, w[idx.view(-1).long()].double())
+    kw = dict(groups=E, seg=seg, a_rows=srt, a_row_div=top if shared else 1, out_dtype=F32)
+    got = ops.glinear(a, w, o_rows=srt, row_scale=wt, out_rows_total=T * top, **kw)
+    assert rel(got, ref * wt.double()[:, None]) < 2 * 32 ** 0.5 * 2.0 ** -24
+    glu = ops.glinear(a, w, glu_clamp=(1.702, 7.0), **kw)              # sorted order
+    z = ref[srt.long()]
+    gt, u = torch.clamp_max(z[:, 0::2], 7.0), torch.clamp(z[:, 1::2], -7.0, 7.0)
+    assert rel(glu, gt * torch.sigmoid(1.702 * gt) * (u + 1)) < 1e-6
