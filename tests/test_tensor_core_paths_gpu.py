@@ -307,6 +307,19 @@ def test_paged_attention_prompt_extremes(ops):
     assert torch.isnan(ops.paged_attention(q, pool, tables, tiles, **kw)[3, :128]).all()
 
 
+@pytest.mark.parametrize("cap", [0.01, 1.0, 11.3, 1e9])
+@pytest.mark.parametrize("max_rows,talk", [(16, False), (1, False), (16, True)])
+def test_paged_attention_scores_around_the_cap(ops, cap, max_rows, talk):
+    """scores far below the cap, next to it (where tanh changes its form) and above it; the same bits wherever a tile begins"""
+    form = dict(softcap=cap, **(dict(talk=True) if talk else {}))
+    got, want, (q, pool, tables, tiles, o) = attention_case(ops, form, 8, 2, 128, 128, 64, [(70, 30)], seed=3, scale=0.3, max_rows=max_rows)
+    assert rel(got, want) < 3e-6
+    if max_rows == 16 and not talk:
+        kw = dict(heads=8, kv_heads=2, dim=128, vdim=128, page=64, scale=0.3, out_dtype=F32, max_rows=16, **o)
+        other = torch.tensor([(r, min(16, 70 - r), 30 + r, 0) for r in range(5, 70, 16)], dtype=torch.int32, device="cuda")
+        assert torch.equal(ops.paged_attention(q, pool, tables, other, **kw)[5:], got[5:])
+
+
 @pytest.mark.parametrize("max_rows,nsplit", [(16, 1), (1, 1), (1, 8)])
 def test_paged_attention_sink_switched_off(ops, max_rows, nsplit):
     """a sink of -inf (or below every score) adds nothing to a head's sum; the other heads keep theirs"""

@@ -17,8 +17,8 @@
 //
 // Bound by the tensor pipe (mma.sync: 1024 multiply-adds per clock and SM measured), six products where bf16 attention
 // issues two.  Tiled on the CUDA cores the same attention ran at 10 TFLOP/s (two shared-memory reads per 16
-// multiply-adds).  2048 causal rows, 16 heads over 4, 128 columns: 1560 us there with capped scores, 247 here (174 without the
-// cap's tanh).
+// multiply-adds).  2048 causal rows, 16 heads over 4, 128 columns: 1560 us there with capped scores, 193 here (186 without the
+// cap; 251 with tanhf for every score).
 //
 // The tensor core truncates as it accumulates, and the truncations of a sum all go one way: with running sums over all keys
 // the rows were 2.8e-6 off at 2048 keys and 2.6e-5 at 16384, where fp32 multiply-adds are 8e-7 and 2.3e-6 off.  So a block's
@@ -56,6 +56,29 @@ __device__ __forceinline__ void add2(float& ax, float& ay, float cx, float cy) {
   f2 r;
   asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(pair(ax, ay)), "l"(pair(cx, cy)));
   unpair(r, ax, ay);
+}
+__device__ __forceinline__ f2 mul2(f2 a, f2 b) {
+  f2 r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ f2 fma2(f2 a, f2 b, f2 c) {
+  f2 r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+// capped() of two scores up to the cap, the same operations
+__device__ __forceinline__ void cap2(float& a, float& b, float inv) {
+  const f2 s = pair(a, b), x = mul2(s, pair(inv, inv)), u = mul2(x, x);
+  f2 r = pair(cap_poly(7), cap_poly(7));
+#pragma unroll
+  for (int k = 6; k >= 0; --k) r = fma2(r, u, pair(cap_poly(k), cap_poly(k)));
+  unpair(mul2(s, r), a, b);
+}
+__device__ __noinline__ float capped_apart(float cap, float s) {   // any score
+  vila_paged_attn_params p;
+  p.softcap = cap;
+  return capped(p, s);
 }
 __device__ __forceinline__ float ex2(float x) {
   float y;
@@ -180,6 +203,7 @@ paged_attn_mma_kernel(const __grid_constant__ vila_paged_attn_params p, int tile
     wlo[r] = p.window > 0 ? pos[r] - p.window + 1 : 0;
   }
   const int keep = p.window > 0 ? p.keep_first : 0;
+  const float cap_inv = cap_inverse(p);
   const int row_max = pos0 + n - 1, lo_min = first_key(p, pos0), lo_max = first_key(p, max(row_max, 0));
   const size_t prow = static_cast<size_t>(p.G) * (MAPS * D + V);   // elements of a pool row
   const __nv_bfloat16* pool = static_cast<const __nv_bfloat16*>(p.pool);
@@ -273,10 +297,22 @@ paged_attn_mma_kernel(const __grid_constant__ vila_paged_attn_params p, int tile
           for (int e = 0; e < 4; e += 2) add2(s[t][e], s[t][e + 1], sl[t][e], sl[t][e + 1]);
         // cap, bias, mask; the block's maximum per row
         if (p.softcap > 0.f) {
+          bool over = false;
 #pragma unroll
           for (int t = 0; t < kBK / 8; ++t)
 #pragma unroll
-            for (int e = 0; e < 4; ++e) s[t][e] = capped(p, s[t][e]);
+            for (int e = 0; e < 4; ++e) over |= over_cap(p, s[t][e]);
+          if (over) {
+#pragma unroll
+            for (int t = 0; t < kBK / 8; ++t)
+#pragma unroll
+              for (int e = 0; e < 4; ++e) s[t][e] = capped_apart(p.softcap, s[t][e]);
+          } else {
+#pragma unroll
+            for (int t = 0; t < kBK / 8; ++t)
+#pragma unroll
+              for (int e = 0; e < 4; e += 2) cap2(s[t][e], s[t][e + 1], cap_inv);
+          }
         }
         if (p.dist_bias) {
 #pragma unroll
