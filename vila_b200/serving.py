@@ -356,43 +356,65 @@ class TokenEngine:
         return True
 
     # ---- one step -----------------------------------------------------------------------------------
+    def _stage(self, parts) -> torch.Tensor:
+        """int32 arrays one after another in pinned host memory: copies from it run in the stream, without a wait of the host
+        (the allocator hands a block out again only after the copies from it)"""
+        flat = torch.empty(sum(len(p) for p in parts), dtype=torch.int32, pin_memory=torch.device(self.model.device).type == "cuda")
+        host, at = flat.numpy(), 0
+        for p in parts:
+            host[at:at + len(p)] = p
+            at += len(p)
+        return flat
+
     def _build(self, entries):
-        c, dev = self.cache, self.model.device
+        """-> index arrays of the step (pinned; the wanted rows are the last of them), their sizes"""
+        c = self.cache
         ids, rows, seqs, tiles, dec, want_rows = [], [], [], [], [], []
         poss, prevs, rseq = [], [], []
         ctx, kv_tiles, ctx_at = [], [], 0
         dirty, at = False, 0
+        singles = all(len(tokens) == 1 for _, tokens, _ in entries)   # decoded tokens: plain lists
         for seq_id, tokens, want in entries:
             n = len(tokens)
             if n == 0:
                 continue
             s = self.admit(seq_id)
             dirty |= self._reserve(s, s.length + n)
-            pos = np.arange(s.length, s.length + n)
-            pages = np.asarray(s.pages, dtype=np.int64)
-            rows.append(pages[pos // c.page] * c.page + pos % c.page)
-            ids.append(np.asarray(tokens, dtype=np.int64))
-            poss.append(pos)
-            prevs.append(np.concatenate(([s.last_token], ids[-1][:-1])))
-            rseq.append(np.full(n, len(seqs)))
-            s.last_token = int(tokens[-1])
-            seqs.append((at, n, s.length, s.slot))
-            if n == 1:
-                dec.append((at, 1, s.length, s.slot))
+            last = int(tokens[-1])
+            if singles:
+                pos = s.length
+                rows.append(s.pages[pos // c.page] * c.page + pos % c.page)
+                ids.append(last)
+                poss.append(pos)
+                prevs.append(s.last_token)
+                rseq.append(len(dec) // 4)
+                dec.extend((at, 1, pos, s.slot))
             else:
-                for o in range(0, n, TILE_ROWS):
-                    tiles.append((at + o, min(TILE_ROWS, n - o), s.length + o, s.slot))
+                pos = np.arange(s.length, s.length + n)
+                pages = np.asarray(s.pages, dtype=np.int64)
+                rows.append(pages[pos // c.page] * c.page + pos % c.page)
+                ids.append(np.asarray(tokens, dtype=np.int64))
+                poss.append(pos)
+                prevs.append(np.concatenate(([s.last_token], ids[-1][:-1])))
+                rseq.append(np.full(n, len(seqs)))
+                seqs.append((at, n, s.length, s.slot))
+                if n == 1:
+                    dec.append((at, 1, s.length, s.slot))
+                else:
+                    for o in range(0, n, TILE_ROWS):
+                        tiles.append((at + o, min(TILE_ROWS, n - o), s.length + o, s.slot))
+                        if self.unfold_ratio > 0:
+                            kv_tiles.append((at + o, min(TILE_ROWS, n - o), s.length + o, ctx_at))
                     if self.unfold_ratio > 0:
-                        kv_tiles.append((at + o, min(TILE_ROWS, n - o), s.length + o, ctx_at))
-                if self.unfold_ratio > 0:
-                    allpos = np.arange(0, s.length + n)
-                    ctx.append(pages[allpos // c.page] * c.page + allpos % c.page)
-                    ctx_at += s.length + n
+                        allpos = np.arange(0, s.length + n)
+                        ctx.append(pages[allpos // c.page] * c.page + allpos % c.page)
+                        ctx_at += s.length + n
+            s.last_token = last
             want_rows.extend(at + int(k) for k in want)
             s.length += n
             at += n
         if dirty:
-            c.page_tables.copy_(torch.from_numpy(c.page_tables_host))
+            c.page_tables.copy_(self._stage([c.page_tables_host.reshape(-1)]).view_as(c.page_tables), non_blocking=True)
         tile_rows = sum(t[1] for t in tiles)
         unfold = bool(tiles) and self.unfold_ratio > 0 and tile_rows * self.unfold_ratio >= ctx_at
         if unfold:
@@ -400,12 +422,14 @@ class TokenEngine:
         else:
             ctx, kv_tiles = [], []
         # one host->device copy for all index arrays of the step
-        parts = [np.concatenate(ids), np.concatenate(rows), np.asarray(seqs).reshape(-1),
-                 np.asarray(tiles).reshape(-1), np.asarray(dec).reshape(-1),
-                 np.concatenate(ctx) if ctx else np.zeros(0), np.asarray(kv_tiles).reshape(-1),
-                 np.concatenate(poss), np.concatenate(prevs), np.concatenate(rseq)]
-        flat = torch.from_numpy(np.concatenate(parts).astype(np.int32))
-        return flat, [p.size for p in parts], want_rows
+        if singles:
+            parts = [ids, rows, dec, [], dec, [], [], poss, prevs, rseq, want_rows]
+        else:
+            parts = [np.concatenate(ids), np.concatenate(rows), np.asarray(seqs).reshape(-1),
+                     np.asarray(tiles).reshape(-1), np.asarray(dec).reshape(-1),
+                     np.concatenate(ctx) if ctx else [], np.asarray(kv_tiles).reshape(-1),
+                     np.concatenate(poss), np.concatenate(prevs), np.concatenate(rseq), want_rows]
+        return self._stage(parts), [len(p) for p in parts]
 
     @staticmethod
     def _views(flat: torch.Tensor, sizes) -> RaggedBatch:
@@ -431,7 +455,7 @@ class TokenEngine:
                 lg = self.model.logits(x)
             ent = self._decode_graphs[T] = (g, static, x, lg)
         g, static, x, lg = ent
-        static.copy_(flat)
+        static.copy_(flat, non_blocking=True)
         g.replay()
         return x, lg
 
@@ -439,27 +463,30 @@ class TokenEngine:
     def step(self, entries, layer_outputs: Optional[list] = None) -> Optional[torch.Tensor]:
         """entries: (sequence id, next token ids, indices among them whose logits are wanted).  All
         entries run as one batch on top of what earlier steps cached.  -> fp32 logits [wanted, vocab]
-        in entry / index order (None if nothing is wanted)."""
+        in entry / index order (None if nothing is wanted).  The host does not wait for the device: reading the logits does."""
         ops.check_waits()   # of the steps so far
         entries = [e for e in entries if len(e[1])]
         if not entries:
             return None
-        flat, sizes, want_rows = self._build(entries)
-        T = sizes[0]
+        flat, sizes = self._build(entries)
+        T, n_want = sizes[0], sizes.pop()
+        arrays = flat[:flat.numel() - n_want]
         decode_only = sizes[3] == 0 and sizes[6] == 0 and layer_outputs is None
         if self.graphs and decode_only and self._decode_seen.get(T, 0) >= 1:
-            x, all_logits = self._decode_step_graphed(flat, sizes)
-            if not want_rows:
+            x, all_logits = self._decode_step_graphed(arrays, sizes)
+            if not n_want:
                 return None
-            sel = torch.tensor(want_rows, dtype=torch.long, device=x.device)
-            return all_logits.index_select(0, sel)
+            want = flat[arrays.numel():]
+            if want.tolist() == list(range(T)):   # the usual case; the graph's output is overwritten by the next replay
+                return all_logits.clone()
+            return all_logits.index_select(0, want.to(x.device, non_blocking=True))
         if decode_only:
             self._decode_seen[T] = self._decode_seen.get(T, 0) + 1
-        x = self.model.forward_step(self._views(flat.to(self.model.device), sizes), self.cache, layer_outputs)
-        if not want_rows:
+        dev = flat.to(self.model.device, non_blocking=True)
+        x = self.model.forward_step(self._views(dev[:arrays.numel()], sizes), self.cache, layer_outputs)
+        if not n_want:
             return None
-        sel = torch.tensor(want_rows, dtype=torch.long, device=x.device)
-        return self.model.logits(x.index_select(0, sel))
+        return self.model.logits(x.index_select(0, dev[arrays.numel():]))
 
 
 @torch.inference_mode()
