@@ -655,6 +655,25 @@ def test_checkpoint_round_trip_and_registry(cuda, tmp_path):
     assert torch.equal(a, b)
 
 
+def test_steps_run_ahead_of_the_device(cuda):
+    """steps whose logits nobody reads yet, more of them than the device has finished, against steps with a wait in between"""
+    from vila_b200.serving import TokenEngine
+    cfg, model = build("aligned", BF, seed=9)
+    toks = [tokens_for(cfg, 60, s) for s in (1, 2)]
+
+    def run(wait):
+        eng, out = TokenEngine(model, 192, 2), []
+        entries = [[(i, toks[i][:20 + i], [0, 19]) for i in range(2)]]
+        entries += [[(i, toks[i][20 + i + k:21 + i + k], [0] if k % 3 else []) for i in range(2)] for k in range(30)]
+        entries += [[(1, toks[1][51:52], [0]), (0, toks[0][50:58], [7, 3])]]
+        for e in entries:
+            out.append(eng.step(e))
+            if wait:
+                torch.cuda.synchronize()
+        return torch.cat([o for o in out if o is not None])
+    assert torch.equal(run(False), run(True))
+
+
 def test_command_line_generates_ids(cuda, tmp_path, capsys):
     from llava.cli import infer
     cfg, model = build("ones", F32, seed=8)
