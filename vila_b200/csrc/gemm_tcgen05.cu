@@ -5,7 +5,12 @@
 //   * fp32 accumulators live in TMEM, double-buffered so the epilogue of one work segment overlaps
 //     the main loop of the next
 //   * epilogue warps read TMEM with tcgen05.ld (lane == output row) and fuse
-//     bias / GELU / SwiGLU / residual (+ broadcast "row modulo" residual for position embeddings)
+//     bias / GELU / SwiGLU / residual (+ broadcast "row modulo" residual for position embeddings).
+//     For short K the epilogue is what a tile takes (K = 1152: 5 us of products in a 256 x 256 tile), and it was bound by
+//     latency and by half-sector accesses: eight warps (four before), residual rows requested a chunk ahead and while the
+//     products run, 32 bytes per lane and access.  13312 rows: 1152 x 592 with residual 61 -> 34 us, 1152 x 1152 70 -> 39,
+//     3456 x 1152 92 -> 77, 4304 x 1152 with GELU 149 -> 113, 1152 x 4304 116 -> 109; 1024 rows 11.1 -> 9.4, 15.4 -> 12.7,
+//     19.5 -> 16.6; 16470 x 37888 x 3584 2905 -> 2785
 //   * scheduling: data-parallel over output tiles, or STREAM-K when the tile count does not fill the
 //     148 SMs evenly (skinny prefill GEMMs, M = 280): the (tile, k-block) iteration space is cut
 //     into equal contiguous ranges, each partial tile is parked in its own fp32 workspace slot and
@@ -28,7 +33,8 @@ namespace {
 constexpr int BLOCK_M = 128;
 constexpr int BLOCK_K = 64;  // 64 bf16 = 128 bytes = one 128B-swizzle row
 constexpr int UMMA_K = 16;
-constexpr int kNumThreads = 192;  // warp0: TMA, warp1: MMA + TMEM alloc, warps 2..5: epilogue
+constexpr int kEpiWarps = 8;      // two per TMEM lane quadrant, each with half of the 32-column chunks
+constexpr int kNumThreads = 64 + 32 * kEpiWarps;  // warp0: TMA, warp1: MMA + TMEM alloc, warps 2..9: epilogue
 
 // kPair: a 2-CTA cluster computes one (2*BLOCK_M) x BLOCK_N tile with tcgen05.mma.cta_group::2 —
 // each CTA stages its own 128 rows of A and HALF of the W tile (BLOCK_N/2 rows); the tensor cores of
@@ -52,6 +58,16 @@ struct GemmSmem {
   static constexpr int kTotal = kStages * kStageBytes + kBarrierBytes + 1024;  // + align slack
 };
 
+
+// 32 bytes (a whole sector of a row) per lane
+__device__ __forceinline__ void ldg_v8(const void* p, uint4& a, uint4& b) {
+  asm volatile("ld.global.v8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+               : "=r"(a.x), "=r"(a.y), "=r"(a.z), "=r"(a.w), "=r"(b.x), "=r"(b.y), "=r"(b.z), "=r"(b.w) : "l"(p) : "memory");
+}
+__device__ __forceinline__ void stg_v8(void* p, const uint4& a, const uint4& b) {
+  asm volatile("st.global.v8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};"
+               ::"l"(p), "r"(a.x), "r"(a.y), "r"(a.z), "r"(a.w), "r"(b.x), "r"(b.y), "r"(b.z), "r"(b.w) : "memory");
+}
 
 __device__ __forceinline__ float4 ld_cg_v4(const float* p) {
   float4 r;
@@ -168,8 +184,8 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a,
     mbar_init(&tmem_full[0], 1);
     mbar_init(&tmem_full[1], 1);
     // pair: one arrival per epilogue warp of BOTH CTAs, on the leader's barrier
-    mbar_init(&tmem_empty[0], kPair ? 8 : 128);
-    mbar_init(&tmem_empty[1], kPair ? 8 : 128);
+    mbar_init(&tmem_empty[0], kPair ? 2 * kEpiWarps : 32 * kEpiWarps);
+    mbar_init(&tmem_empty[1], kPair ? 2 * kEpiWarps : 32 * kEpiWarps);
     fence_barrier_init();
   }
   if (warp == 1) {
@@ -297,6 +313,9 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a,
   } else {
     // ===================== epilogue warps (TMEM -> regs -> global) =====================
     const int quad = warp & 3;  // TMEM lane quadrant this warp may access
+    const int upper = (warp - 2) >> 2;  // which half of the quadrant's chunks this warp takes
+    const bool wide_c = ldc % 16 == 0 && reinterpret_cast<uintptr_t>(C) % 32 == 0;
+    const bool wide_res = epi.ld_res % 16 == 0 && reinterpret_cast<uintptr_t>(epi.residual) % 32 == 0;
     const int epi_tid = threadIdx.x - 64;
     Sched sch(M, N, K, BLOCK_N, stream_k, TILE_M, worker, n_workers);
     int as = 0;
@@ -306,20 +325,45 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a,
     while (sch.next(t, kb0, kb1)) {
       int m_blk, n_blk;
       tile_coords(t, num_m_blocks, num_n_blocks, m_blk, n_blk);
-      mbar_wait(&tmem_full[as], aphase);
-      tc_fence_after();
       const int row = m_blk * TILE_M + static_cast<int>(mrank) * BLOCK_M + quad * 32 + lane;
       const bool row_ok = row < M;
+      constexpr int kHalfChunks = BLOCK_N / 64;  // 32-column chunks per half
+      constexpr int kMine = (kSplit2 ? kHalfChunks : BLOCK_N / 32) / 2;
+      static_assert(kMine >= 1, "gemm: a chunk for every epilogue warp");
+      const int c_lo = (kSplit2 ? static_cast<int>(rank) * kHalfChunks : 0) + upper * kMine, c_hi = c_lo + kMine;
+      // this row's residual, a chunk ahead: the first one while the accumulator is still being computed
+      const __nv_bfloat16* res_row = nullptr;
+      if (epi.residual != nullptr && row_ok) {
+        const int rr = epi.res_row_mod > 0 ? (row % epi.res_row_mod) : row;
+        res_row = epi.residual + static_cast<size_t>(rr) * epi.ld_res;
+      }
+      uint4 res_next[4];
+      auto fetch_residual = [&](int c) {
+        const int n0 = n_blk * BLOCK_N + c * 32;
+#pragma unroll
+        for (int g = 0; g < 4; g += 2) {
+          if (res_row == nullptr || c >= c_hi) continue;
+          const __nv_bfloat16* src = res_row + n0 + g * 8;
+          if (wide_res && n0 + g * 8 + 16 <= N) {
+            ldg_v8(src, res_next[g], res_next[g + 1]);
+          } else {
+            if (n0 + g * 8 < N) res_next[g] = ldg_v4(src);
+            if (n0 + g * 8 + 8 < N) res_next[g + 1] = ldg_v4(src + 8);
+          }
+        }
+      };
+      fetch_residual(c_lo);
+      mbar_wait(&tmem_full[as], aphase);
+      tc_fence_after();
       const uint32_t t_row = tmem_base + (static_cast<uint32_t>(quad * 32) << 16) + as * BLOCK_N;
       const bool partial = !kSplit2 && ((kb0 != 0) || (kb1 != sch.nkb));
       // split-K pair: park the column half the PEER finalises ([col/4][row] float4 -> conflict-free
       // for the writer here and for the peer's DSMEM reads), then meet the peer at the cluster barrier
-      constexpr int kHalfChunks = BLOCK_N / 64;  // 32-column chunks per half
       float4* xchg = reinterpret_cast<float4*>(smem_a);  // the pipeline stages are dead by now
       if (kSplit2) {
         const int c_peer = static_cast<int>(1u - rank) * kHalfChunks;
 #pragma unroll 1
-        for (int c = 0; c < kHalfChunks; ++c) {
+        for (int c = upper * kMine; c < (upper + 1) * kMine; ++c) {
           uint32_t r[32];
           tmem_ld_32x32b_x32(t_row + (c_peer + c) * 32, r);
           tmem_ld_wait();
@@ -354,7 +398,7 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a,
         slot0 = epi.splitk_ws + tile_base + row_off;
         float* mine = epi.splitk_ws + tile_base + static_cast<size_t>(my_slot) * (BLOCK_M * BLOCK_N) + row_off;
 #pragma unroll 1
-        for (int c = 0; c < BLOCK_N / 32; ++c) {
+        for (int c = c_lo; c < c_hi; ++c) {
           uint32_t r[32];
           tmem_ld_32x32b_x32(t_row + c * 32, r);
           tmem_ld_wait();
@@ -368,7 +412,7 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a,
         tc_fence_before();
         mbar_arrive(&tmem_empty[as]);  // TMEM stage is free again
         __threadfence();
-        asm volatile("bar.sync 1, 128;" ::: "memory");
+        asm volatile("bar.sync 1, %0;" ::"n"(32 * kEpiWarps) : "memory");
         if (epi_tid == 0) {
           const int add = kb1 - kb0;
           const int prev = atomicAdd(&epi.splitk_counters[t], add);
@@ -376,23 +420,20 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a,
           if (last) epi.splitk_counters[t] = 0;  // self-cleaning
           *last_flag = last;
         }
-        asm volatile("bar.sync 1, 128;" ::: "memory");
+        asm volatile("bar.sync 1, %0;" ::"n"(32 * kEpiWarps) : "memory");
         finalize = (*last_flag != 0);
         from_ws = true;
         if (finalize) __threadfence();
-        asm volatile("bar.sync 1, 128;" ::: "memory");  // everyone has read last_flag
+        asm volatile("bar.sync 1, %0;" ::"n"(32 * kEpiWarps) : "memory");  // everyone has read last_flag
       }
       if (finalize) {
-        const __nv_bfloat16* res_row = nullptr;
-        if (epi.residual != nullptr && row_ok) {
-          const int rr = epi.res_row_mod > 0 ? (row % epi.res_row_mod) : row;
-          res_row = epi.residual + static_cast<size_t>(rr) * epi.ld_res;
-        }
-        const int c_lo = kSplit2 ? static_cast<int>(rank) * kHalfChunks : 0;
-        const int c_hi = kSplit2 ? c_lo + kHalfChunks : BLOCK_N / 32;
 #pragma unroll 1
         for (int c = c_lo; c < c_hi; ++c) {
           float v[32];
+          uint4 res[4];
+#pragma unroll
+          for (int g = 0; g < 4; ++g) res[g] = res_next[g];
+          fetch_residual(c + 1);
           const int n0 = n_blk * BLOCK_N + c * 32;
           if (!from_ws) {
             uint32_t r[32];
@@ -405,7 +446,7 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a,
 #pragma unroll
               for (int g = 0; g < 8; ++g) {
                 const float4 q = ld_dsmem_v4f(
-                    xchg_peer + static_cast<uint32_t>(((c - c_lo) * 8 + g) * BLOCK_M + quad * 32 + lane) * 16u);
+                    xchg_peer + static_cast<uint32_t>(((c - static_cast<int>(rank) * kHalfChunks) * 8 + g) * BLOCK_M + quad * 32 + lane) * 16u);
                 v[4 * g + 0] += q.x; v[4 * g + 1] += q.y; v[4 * g + 2] += q.z; v[4 * g + 3] += q.w;
               }
             }
@@ -486,39 +527,46 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a,
             }
             continue;
           }
-          if (epi.act != ACT_NONE) {
+          // one loop per activation: its instructions lie together (chosen inside one loop, 32 bodies of all activations
+          // did not fit the instruction cache: 13312 x 4304 x 1152 with GELU 317 us)
+          auto activate = [&](auto f) {
 #pragma unroll
-            for (int j = 0; j < 32; ++j) {
-              float x = bf16_round(v[j]);
-              v[j] = epi.act == ACT_GELU_TANH
-                         ? gelu_tanh_f(x)
-                         : (epi.act == ACT_GELU_ERF ? gelu_erf_f(x)
-                                                    : (epi.act == ACT_RELU2 ? fmaxf(x, 0.f) * fmaxf(x, 0.f)
-                                                       : (epi.act == ACT_XIELU ? xielu_fast_f(x, epi.act_pos, epi.act_neg) : silu_f(x))));
-            }
+            for (int j = 0; j < 32; ++j) v[j] = f(bf16_round(v[j]));
+          };
+          switch (epi.act) {
+            case ACT_NONE: break;
+            case ACT_GELU_TANH: activate([](float x) { return gelu_tanh_f(x); }); break;
+            case ACT_GELU_ERF: activate([](float x) { return gelu_erf_f(x); }); break;
+            case ACT_RELU2: activate([](float x) { return fmaxf(x, 0.f) * fmaxf(x, 0.f); }); break;
+            case ACT_XIELU: activate([&](float x) { return xielu_fast_f(x, epi.act_pos, epi.act_neg); }); break;
+            default: activate([](float x) { return silu_f(x); });
           }
           if (row_ok) {
+            uint4 o[4];
 #pragma unroll
             for (int g = 0; g < 4; ++g) {
-              if (n0 + g * 8 < N) {
-                float* w = v + g * 8;
-                if (res_row != nullptr) {
-                  const uint4 b = ldg_v4(res_row + n0 + g * 8);
-                  w[0] = bf16_round(w[0]) + bf_lo(b.x);
-                  w[1] = bf16_round(w[1]) + bf_hi(b.x);
-                  w[2] = bf16_round(w[2]) + bf_lo(b.y);
-                  w[3] = bf16_round(w[3]) + bf_hi(b.y);
-                  w[4] = bf16_round(w[4]) + bf_lo(b.z);
-                  w[5] = bf16_round(w[5]) + bf_hi(b.z);
-                  w[6] = bf16_round(w[6]) + bf_lo(b.w);
-                  w[7] = bf16_round(w[7]) + bf_hi(b.w);
-                }
-                uint4 o;
-                o.x = pack_bf16(w[0], w[1]);
-                o.y = pack_bf16(w[2], w[3]);
-                o.z = pack_bf16(w[4], w[5]);
-                o.w = pack_bf16(w[6], w[7]);
-                stg_v4(C + static_cast<size_t>(row) * ldc + n0 + g * 8, o);
+              float* w = v + g * 8;
+              if (res_row != nullptr) {
+                const uint4 b = res[g];
+                w[0] = bf16_round(w[0]) + bf_lo(b.x);
+                w[1] = bf16_round(w[1]) + bf_hi(b.x);
+                w[2] = bf16_round(w[2]) + bf_lo(b.y);
+                w[3] = bf16_round(w[3]) + bf_hi(b.y);
+                w[4] = bf16_round(w[4]) + bf_lo(b.z);
+                w[5] = bf16_round(w[5]) + bf_hi(b.z);
+                w[6] = bf16_round(w[6]) + bf_lo(b.w);
+                w[7] = bf16_round(w[7]) + bf_hi(b.w);
+              }
+              o[g] = make_uint4(pack_bf16(w[0], w[1]), pack_bf16(w[2], w[3]), pack_bf16(w[4], w[5]), pack_bf16(w[6], w[7]));
+            }
+            __nv_bfloat16* dst = C + static_cast<size_t>(row) * ldc + n0;
+#pragma unroll
+            for (int g = 0; g < 4; g += 2) {
+              if (wide_c && n0 + g * 8 + 16 <= N) {
+                stg_v8(dst + g * 8, o[g], o[g + 1]);
+              } else {
+                if (n0 + g * 8 < N) stg_v4(dst + g * 8, o[g]);
+                if (n0 + g * 8 + 8 < N) stg_v4(dst + g * 8 + 8, o[g + 1]);
               }
             }
           }
