@@ -23,6 +23,8 @@
 //   mm_projector Linear layers          (base_projector.py:145-162)
 //   Qwen2 q/k/v/o, gate/up/down, lm_head (modeling_qwen2.py:164-176,223-226)
 //   patch-embed conv as im2col GEMM     (modeling_siglip.py:269-275,322-328)
+#include <math.h>
+
 #include "common.cuh"
 #include "kernels.h"
 
@@ -729,40 +731,48 @@ int gemm_bf16(const __nv_bfloat16* A, int lda, const __nv_bfloat16* W, int ldw, 
   VB_CHECK(epi.rope_table == nullptr, "gemm: the fused RoPE epilogue is only available through gemm_qkv_rope_bf16");
   // decoded tokens: the weight stream alone
   if (gemm_rows_takes(A, lda, W, ldw, M, N, K, epi)) return gemm_rows(A, lda, W, ldw, C, ldc, M, N, K, epi, stream);
-  // Tile-shape heuristic. N=256 tiles keep the MMA (not shared-memory bandwidth) the limiter when
-  // there is enough work; N=128 otherwise; stream-K (inside launch_gemm) fixes SM under-fill.
-  // Measured on B200 (tools/bench_gemm.py): 128x256 tiles win as soon as they fill ~70 % of the
-  // SMs (the 256-wide tile keeps the MMA, not shared-memory bandwidth, the limiter); otherwise
-  // 128x128; 64-wide tiles only for narrow outputs.
-  // Few tokens (short-prompt prefill, projector): the weights dominate the traffic -> swap-AB kernel
-  // (every weight byte enters an SM once; cluster split-K fills the machine).  B200, M = 279:
-  // down-proj 52 vs 90 us, gate/up 83 vs 86, qkv/o 21-23 vs 22 (profiles/r01_gemm_configs.md)
-  const int sms = num_sms();
-  const int mb = (M + BLOCK_M - 1) / BLOCK_M;
-  // At most one 128x128 tile per SM pair (ViT fc2: 72 tiles, K = 4304; projector): split K over a CTA pair with a DSMEM
-  // exchange -> all SMs stream operands (fc2 16.9 vs 24.7 us).  Down to K = 512 and to one row tile it is the faster form:
-  // 512 .. 4608 outputs, K = 512 | 1024 | 1984, against the swap-AB kernel that would take up to 384 rows
-  //   128 rows 6.0-6.7 | 7.1-8.0 | 9.1-10.7 us, there 6.7-6.9 | 8.3-9.8 | 10.2-12.1
-  //   256 rows 6.0-7.7 | 7.2-9.3 | 9.3-12.1 us, there 9.3-9.6 | 11.8-13.2 | 13.9-15.4
-  // and against 128x128 tiles of one CTA 512 rows 6.1-7.2 | 7.2-8.6 | 9.5-11.0 us, there 7.0-7.8 | 9.2-10.0 | 13.2-14.3;
-  // 1024 rows x 1152 outputs 7.7 | 9.0 | 11.5, there 7.9 | 10.3 | 14.7.  Below K = 512 a CTA would have four stages.
-  const long tiles128 = static_cast<long>(mb) * ((N + 127) / 128);
-  const bool split2 = tiles128 <= sms / 2 && K >= 512 && M * 10 >= mb * BLOCK_M * 9;
-  if (split2) return launch_gemm<128, 6, kModeSplitK2>(A, lda, W, ldw, C, ldc, M, N, K, epi, -1, stream);
+  // The forms of the kernel by what they would take: a start and so much per round of tiles and element of K.  Fitted to one
+  // to sixteen rounds of K = 592 .. 18944 (rows 17 .. 2000, outputs 1024 .. 37888).
+  //   128 x 128 tiles, K halved over a CTA pair (one round of up to 74)  4.6 + 2.45e-3 K     K = 1024: 7.1   3584: 15
+  //   128 x 128 tiles of one CTA                                         3.6 + 4.55e-3 K               8.5         20.5
+  //   128 x 256 tiles of one CTA                                         3.4 + 5.80e-3 K               9.4         25
+  //   256 x 256 tiles of a CTA pair                                      4.4 + 5.00e-3 K               9.6         22
+  // e.g. (us; before: 256-wide tiles from 70 % of the SMs on, pairs from 85 %, halves only for rows that fill their tiles)
+  //   800 x 3088 x 1024 11.2 (14.0), 800 x 1024 x 2688 12 (17), 1000 x 2560 x 2048 16 (23), 400 x 2048 x 11008 32 (53)
+  const long sms = num_sms(), mb = (M + 127) / 128, mb2 = (M + 255) / 256, nb = (N + 127) / 128, nb2 = (N + 255) / 256;
+  const auto rounds = [](long tiles, long at_once) { return static_cast<double>((tiles + at_once - 1) / at_once); };
+  const double mbytes = 2e-6 * N * K;
+  const double t_half = mb * nb <= sms / 2 && K >= 512 ? 4.6 + 2.45e-3 * K : 1e30;
+  const double t_128 = 3.6 + 4.55e-3 * K * rounds(mb * nb, sms);
+  const double t_256 = 3.4 + 5.80e-3 * K * rounds(mb * nb2, sms);
+  const double t_pair = 4.4 + 5.00e-3 * K * rounds(mb2 * nb2, sms / 2);
+  const double t_tiles = fmin(fmin(t_half, t_128), fmin(t_256, t_pair));
   if (M <= 384) {
-    const int rc = gemm_skinny_bf16(A, lda, W, ldw, C, ldc, M, N, K, epi, 0, stream);
-    if (rc >= 0) return rc;
+    // Few tokens: the swap-AB kernel (every weight byte enters an SM once, K split over a cluster) where the weight stream is
+    // what counts: 6 us + 0.027 a row + 0.20 a MB, 0.0003 more per row.  With an activation its epilogue counts as well and
+    // tiles are ahead (22016 gated outputs x 2048 on 40 | 140 | 279 rows 25 | 31 | 35 us, there 33 | 38 | 51; 4304 x 1152 with
+    // GELU on 100 rows 9, there 15) unless they nearly fill one round too many (37888 x 3584 on 279 rows 83 and 81, and
+    // behind other kernels 90).  Without one, where they fill one round (no faster than the weights at 4.8 TB/s): 279 rows x
+    // 3088 x 1024 8.8 and 14.5, 200 x 2048 x 2048 9.7 and 13.8, but 3584 x 18944 91 and 54; up to 32 rows and for more than
+    // 8192 outputs never.
+    // A projection with no more than a bias onto whole 128-column heads may be the other half of vila_linear_qkv_rope: it
+    // stays where that has the same bits (rows that fill their tiles: K halved, as ever).
+    const bool plain = epi.act == ACT_NONE && epi.swiglu == 0;
+    const bool heads = plain && epi.residual == nullptr && epi.bias != nullptr && N % 128 == 0;
+    const bool one_round = mb * nb <= sms || mb2 * nb2 <= sms / 2;
+    const double t_swap = 6.0 + 0.027 * M + (0.20 + 0.0003 * M) * mbytes;
+    const bool ahead = M > 32 && N <= 8192 && (t_half < 1.05 * t_swap || (one_round && fmax(t_tiles, 4.0 + 0.21 * mbytes) < 0.95 * t_swap));
+    const bool tiles = M <= 16 ? false : heads ? t_half < 1e30 && M * 10 >= mb * 128 * 9 : plain ? ahead : mbytes < 16 || t_tiles < 0.7 * t_swap;
+    if (!tiles) {
+      const int rc = gemm_skinny_bf16(A, lda, W, ldw, C, ldc, M, N, K, epi, 0, stream);
+      if (rc >= 0) return rc;
+    }
+    if (heads && t_half < 1e30) return launch_gemm<128, 6, kModeSplitK2>(A, lda, W, ldw, C, ldc, M, N, K, epi, -1, stream);
   }
-  // CTA pairs (256 x 256 tiles, cta_group::2) once they fill ~85 % of the SM pairs: fewer bytes per
-  // MAC through each SM's L2 port and shared memory (8192^3: 752 vs 859 us; 2048x37888x3584: 355 vs 396)
-  const long pair_tiles = static_cast<long>((M + 2 * BLOCK_M - 1) / (2 * BLOCK_M)) * ((N + 255) / 256);
-  const long m_pad_pair = (M + 2 * BLOCK_M - 1) / (2 * BLOCK_M) * (2L * BLOCK_M), m_pad_single = static_cast<long>(mb) * BLOCK_M;
-  if (pair_tiles * 20 >= 17L * (sms / 2) && m_pad_pair * 8 <= m_pad_single * 9)  // no extra row padding
-    return launch_gemm<256, 6, kModePair>(A, lda, W, ldw, C, ldc, M, N, K, epi, -1, stream);
-  const long tiles256 = static_cast<long>(mb) * ((N + 255) / 256);
-  if (tiles256 * 10 >= 7L * sms)
-    return launch_gemm<256, 4>(A, lda, W, ldw, C, ldc, M, N, K, epi, -1, stream);
+  if (t_half <= t_tiles) return launch_gemm<128, 6, kModeSplitK2>(A, lda, W, ldw, C, ldc, M, N, K, epi, -1, stream);
   if (N < 128) return launch_gemm<64, 8>(A, lda, W, ldw, C, ldc, M, N, K, epi, -1, stream);
+  if (t_pair <= t_tiles) return launch_gemm<256, 6, kModePair>(A, lda, W, ldw, C, ldc, M, N, K, epi, -1, stream);
+  if (t_256 <= t_tiles) return launch_gemm<256, 4>(A, lda, W, ldw, C, ldc, M, N, K, epi, -1, stream);
   return launch_gemm<128, 6>(A, lda, W, ldw, C, ldc, M, N, K, epi, -1, stream);
 }
 

@@ -136,7 +136,8 @@ __device__ __noinline__ void row_again(const vila_paged_attn_params& p, int row,
 // in shared memory has MAPS * D columns.
 // exp(s - m) is taken as 2^(s log2 e - m log2 e) with one fused multiply-add: the rounded m log2 e is common to a row's
 // weights and cancels in their quotient, which leaves the rounding of the difference, as in exp(s - m).
-template <int D, int MAPS, int V, int SETS>
+// CAP: with capped scores (a kernel of its own: the others were 4 % slower for its instructions).
+template <int D, int MAPS, int V, int SETS, bool CAP>
 __global__ void __launch_bounds__(32 * (SETS == 2 ? 8 : kMaxWarps), 1)
 paged_attn_mma_kernel(const __grid_constant__ vila_paged_attn_params p, int tiles_per_cta) {
   constexpr int KB = MAPS * D * 2, VB = V * 2;             // bytes of a key's / value's row
@@ -296,7 +297,7 @@ paged_attn_mma_kernel(const __grid_constant__ vila_paged_attn_params p, int tile
 #pragma unroll
           for (int e = 0; e < 4; e += 2) add2(s[t][e], s[t][e + 1], sl[t][e], sl[t][e + 1]);
         // cap, bias, mask; the block's maximum per row
-        if (p.softcap > 0.f) {
+        if (CAP) {
           bool over = false;
 #pragma unroll
           for (int t = 0; t < kBK / 8; ++t)
@@ -505,14 +506,18 @@ paged_attn_mma_kernel(const __grid_constant__ vila_paged_attn_params p, int tile
   }
 }
 
-template <int D, int MAPS, int V, int SETS>
-int launch_sets(const vila_paged_attn_params& p, int warps, int tpc, cudaStream_t stream) {
-  auto kernel = paged_attn_mma_kernel<D, MAPS, V, SETS>;
+template <int D, int MAPS, int V, int SETS, bool CAP>
+int launch_kernel(const vila_paged_attn_params& p, int warps, int tpc, cudaStream_t stream) {
+  auto kernel = paged_attn_mma_kernel<D, MAPS, V, SETS, CAP>;
   const int smem = warps * 3 * (D / 16) * 512 + SETS * 2 * kBK * (MAPS * D + V) * 2;
   static PerDeviceOnce once;
   if (once.first()) VB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 224 * 1024));
   VB_CUDA(launch_serial(kernel, dim3((p.ntiles + tpc - 1) / tpc, p.G), dim3(32 * warps * SETS), smem, stream, p, tpc));
   return 0;
+}
+template <int D, int MAPS, int V, int SETS>
+int launch_sets(const vila_paged_attn_params& p, int warps, int tpc, cudaStream_t stream) {
+  return p.softcap > 0.f ? launch_kernel<D, MAPS, V, SETS, true>(p, warps, tpc, stream) : launch_kernel<D, MAPS, V, SETS, false>(p, warps, tpc, stream);
 }
 template <int D, int MAPS, int V>
 int launch(const vila_paged_attn_params& p, cudaStream_t stream) {
