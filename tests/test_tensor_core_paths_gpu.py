@@ -706,3 +706,35 @@ def test_few_pairs_stream(ops, T, E, top, N, K, shared):
     z = ref[srt.long()]
     gt, u = torch.clamp_max(z[:, 0::2], 7.0), torch.clamp(z[:, 1::2], -7.0, 7.0)
     assert rel(glu, gt * torch.sigmoid(1.702 * gt) * (u + 1)) < 1e-6
+
+
+@pytest.mark.parametrize("T,width,identity", [(1, 2048, "some"), (8, 2048, "some"), (16, 2048, "some"), (16, 1024, "some"), (16, 2048, "all"), (8, 1024, "all")])
+def test_few_pairs_without_a_group(ops, T, width, identity):
+    """choices of identity outputs are in no segment: 28 experts + 4 such outputs, the sorted list ends before its storage does.
+    The positions behind it name another pair here, whose weight is infinite and whose row is NaN: nothing of them may count."""
+    E, top, ff = 28, 4, 1024
+    g = gen(T + width)
+    idx = torch.rand(T, E + 4, generator=g, device="cuda").topk(top).indices.to(torch.int32)
+    idx[:, -1] = E + 1                                                # a pair without a group in every row
+    if identity == "all":
+        idx[:] = E
+    seg, srt = ops.moe_group(idx, E)
+    live = int((idx < E).sum())
+    assert int(seg[-1]) == live < T * top
+    srt[live:] = top - 1                                              # pair of row 0 that is in no segment
+    up, down, h = randn(g, E, ff, width), randn(g, E, width, ff) * 0.05, randn(g, T, width)
+    wt = torch.rand(T * top, generator=g, device="cuda")
+    wt[top - 1] = float("inf")
+    pairs, expert = srt[:live].long(), idx.view(-1)[srt[:live].long()].long()
+    act = ops.glinear(h, up, groups=E, seg=seg, a_rows=srt, a_row_div=top, act=ops.ACT_GELU_ERF)
+    want = torch.nn.functional.gelu(torch.einsum("rk,rnk->rn", h.double()[pairs // top], up[expert].double()))
+    if live:
+        assert rel(act[:live], want) < 2.0 ** -8
+    act[live:] = float("nan")
+    rows = torch.zeros(T * top, width, device="cuda")
+    ops.glinear(act, down, groups=E, seg=seg, o_rows=srt, row_scale=wt, out=rows)
+    want = torch.zeros(T * top, width, dtype=torch.float64, device="cuda")
+    want[pairs] = torch.einsum("rk,rnk->rn", act[:live].double(), down[expert].double()) * wt.double()[pairs, None]
+    assert torch.equal(rows[want.abs().sum(1) == 0], torch.zeros_like(rows[want.abs().sum(1) == 0]))
+    if live:
+        assert rel(rows, want) < 2 * 32 ** 0.5 * 2.0 ** -24

@@ -77,6 +77,9 @@ __global__ void __launch_bounds__(32 * kStay, 1) glinear_stream_kernel(const vil
   const int kw = warp % KW, rw = warp / KW;
   const int tiles = (p.N + 15) / 16, per_warp = ((p.K + 31) / 32 + KW - 1) / KW, pitch = (2 * p.K + 127) / 128 * 128 + 64;
   const int step = gridDim.x * RW, first = blockIdx.x * RW + rw;
+  // Pairs outside [seg[0], seg[groups]) belong to no group (M only bounds them, identity choices lie there): nobody has written
+  // their rows, nothing of them is read.
+  const int live0 = ROUTED ? max(p.seg[0], 0) : 0, live1 = ROUTED ? min(p.M, p.seg[p.groups]) : p.M;
   if (ROUTED && warp == 0) {
     int count = 0;
     for (int g0 = 0; g0 < p.groups; g0 += 32) {
@@ -101,26 +104,31 @@ __global__ void __launch_bounds__(32 * kStay, 1) glinear_stream_kernel(const vil
     int before = 0;
 #pragma unroll
     for (int hf = 0; hf < 2; ++hf) {
-      const int i = 32 * hf + lane, row = i < p.M ? (p.a_rows ? p.a_rows[i] / p.a_row_div : i) : -1;
+      const int i = 32 * hf + lane;
+      const bool live = i >= live0 && i < live1;
+      const int row = live ? (p.a_rows ? p.a_rows[i] / p.a_row_div : i) : -1;
       row_s[i] = row;
       __syncwarp();
       int same = i;
       for (int j = 32 * hf + 31; j >= 0; --j)
         if (row_s[j] == row && j <= i) same = j;
-      const unsigned fresh = __ballot_sync(0xffffffffu, same == i && i < p.M);
-      if (same == i && i < p.M) {
+      const unsigned fresh = __ballot_sync(0xffffffffu, same == i && live);
+      if (same == i && live) {
         at_s[i] = before + __popc(fresh & ((1u << lane) - 1u));
         uniq_s[at_s[i]] = row;
       }
       __syncwarp();
-      if (same != i) at_s[i] = at_s[same];
+      if (same != i && live) at_s[i] = at_s[same];
       before += __popc(fresh);
     }
     if (lane == 0) counts_s[1] = before;
-  } else if (warp < 4 && threadIdx.x - 64 < p.M) {
-    const int i = threadIdx.x - 64, orow = p.o_rows ? p.o_rows[i] : i;
-    orow_s[i] = orow;
-    scale_s[i] = make_float2(in_scale_of(p, x, orow), p.row_scale ? p.row_scale[orow] : 1.0f);
+  } else if (warp == 2 || warp == 3) {
+    const int i = threadIdx.x - 64;
+    if (i >= live0 && i < live1) {
+      const int orow = p.o_rows ? p.o_rows[i] : i;
+      orow_s[i] = orow;
+      scale_s[i] = make_float2(in_scale_of(p, x, orow), p.row_scale ? p.row_scale[orow] : 1.0f);
+    }
   }
   __syncthreads();
   const bool staged = counts_s[1] * pitch <= token_bytes;
