@@ -112,6 +112,25 @@ def test_linear_streamk_epilogues_and_workspace_is_clean(cuda):
     assert rel_err(out, ref) < 1e-2
 
 
+@pytest.mark.parametrize("block_n", [64, 128, 256, 1128, 4128, 4256, 5128])
+def test_linear_tiles_gated_unit_takes_no_residual(cuda, block_n):
+    """the tiled kernels' gated units add no residual and read none: one of N / 2 columns is as good as no residual"""
+    import ctypes
+    from vila_b200 import _lib
+    ops = _ops()
+    ops.ensure_workspace("cuda")
+    M, N, K = 200, 544, 256
+    g = torch.Generator(device="cuda").manual_seed(block_n)
+    x = bf(torch.randn(M, K, device=cuda, generator=g))
+    w = bf(torch.randn(N, K, device=cuda, generator=g) / math.sqrt(K))
+    res = torch.full((2 * M, N // 2), float("nan"), dtype=torch.bfloat16, device=cuda)[:M]
+    out, want = torch.empty(M, N // 2, dtype=torch.bfloat16, device=cuda), ops.linear(x, w, swiglu=True, block_n=block_n)
+    p = lambda t: ctypes.c_void_p(t.data_ptr())
+    ops.check(_lib.load().vila_linear_cfg(block_n, p(x), K, p(w), K, None, p(res), N // 2, 0, p(out), N // 2, M, N, K, 0, 1,
+                                          ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)), "vila_linear_cfg")
+    assert torch.equal(out, want) and torch.isfinite(out).all()
+
+
 @pytest.mark.parametrize("M", [1, 33, 279, 384])
 def test_linear_qkv_rope_fused_equals_two_kernels(cuda, M):
     """q/k/v projection with RoPE + paged KV append fused into the GEMM epilogue must be bit-identical

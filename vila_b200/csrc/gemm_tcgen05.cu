@@ -333,9 +333,10 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a,
       constexpr int kMine = (kSplit2 ? kHalfChunks : BLOCK_N / 32) / 2;
       static_assert(kMine >= 1, "gemm: a chunk for every epilogue warp");
       const int c_lo = (kSplit2 ? static_cast<int>(rank) * kHalfChunks : 0) + upper * kMine, c_hi = c_lo + kMine;
-      // this row's residual, a chunk ahead: the first one while the accumulator is still being computed
+      // this row's residual, a chunk ahead: the first one while the accumulator is still being computed.  A gated unit adds
+      // none here (its rows would have N / 2 columns, not the N that are read).
       const __nv_bfloat16* res_row = nullptr;
-      if (epi.residual != nullptr && row_ok) {
+      if (epi.residual != nullptr && epi.swiglu == 0 && row_ok) {
         const int rr = epi.res_row_mod > 0 ? (row % epi.res_row_mod) : row;
         res_row = epi.residual + static_cast<size_t>(rr) * epi.ld_res;
       }
