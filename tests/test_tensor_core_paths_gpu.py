@@ -618,11 +618,30 @@ def test_ssd_chunks(ops, lens, H, P, N, G, gate):
     # fp32 roundings of a sum of decaying terms: a few units of 6e-8
     assert rel(got, want) < 5e-7 and rel(got_state, S) < 5e-7 and torch.equal(got_state[0], state[0])
     assert rel(ops.ssd_scan(xbc, dt, z, state.clone(), seqs, out_dtype=BF, **kw), want) < 4e-3
-    # a sequence's numbers depend neither on the batch nor on the others' lengths (columns per CTA differ)
+    # a sequence's numbers depend neither on the batch nor on the others' lengths
     for s, (r, n, pos, slot) in enumerate(seqs.tolist()):
         one = state.clone()
         alone = ops.ssd_scan(xbc[r:r + n], dt[r:r + n], None if z is None else z[r:r + n], one, torch.tensor([(0, n, pos, slot)], dtype=torch.int32, device="cuda"), **kw)
-        assert rel(alone, got[r:r + n]) < 5e-7 and rel(one[slot], got_state[slot]) < 5e-7
+        assert torch.equal(alone, got[r:r + n]) and torch.equal(one[slot], got_state[slot])
+
+
+@pytest.mark.parametrize("odd", [False, True])
+def test_ssd_chunks_same_bits_in_either_width(ops, odd):
+    """one sequence of 32 heads x 64 takes CTAs of 16 columns, three take CTAs of 32: the same bits, also beside an infinite
+    value, whose 16 columns alone are walked token by token"""
+    H, P, N = 32, 64, 128
+    xbc, dt, z, state, seqs, kw = ssd_inputs([200, 150, 100], H, P, N, 1)
+    if odd:
+        xbc[70, 3 * P + 18] = float("inf")
+        state[2, 5, 40, 7] = float("nan")                             # of the second sequence, which starts in mid-sequence
+    batch = state.clone()
+    got = ops.ssd_scan(xbc, dt, z, batch, seqs, **kw)
+    assert torch.isfinite(got).all() != odd
+    for r, n, pos, slot in seqs.tolist():
+        one = state.clone()
+        alone = ops.ssd_scan(xbc[r:r + n], dt[r:r + n], z[r:r + n], one, torch.tensor([(0, n, pos, slot)], dtype=torch.int32, device="cuda"), **kw)
+        for a, b in ((alone, got[r:r + n]), (one[slot], batch[slot])):
+            assert torch.equal(torch.nan_to_num(a, 1.5, 2.5, 3.5), torch.nan_to_num(b, 1.5, 2.5, 3.5))
 
 
 def test_ssd_chunks_after_any_decay(ops):

@@ -19,8 +19,11 @@
 //   warps 8 - 15   cp.async of chunk c + 2; rows of chunk c: read-out, weights x x and D x summed, gated, stored
 // with one barrier per chunk for all, and one for the rows.
 //
-// A chunk that holds an infinite or NaN number, or meets one in the state, is walked token by token by the same fragments:
+// Columns of a chunk that meet an infinite or NaN number are walked token by token by the same fragments, 16 of them at a time:
 // zero weights and zero parts would meet the infinite number, which they do not in the recurrence.
+//
+// PT = 1 and 2 give the same bits (channels are summed by sixteens, then pairwise), so a sequence's numbers do not depend on
+// how many others the launch has.
 //
 // 2048 rows of one sequence: 64 heads of 64 x 128 in 114 us (token by token, bound by instruction issue: 300), 32 heads 98
 // (212), 128 heads 235 (593).  A chunk takes 5700 clocks: read-out 2400, update 1600, beside them scores and weights 4500,
@@ -62,7 +65,7 @@ struct Shape {
   static constexpr int kCB = 2 * kL * kRow, kX = kL * kXRow;   // C | B and x of a chunk: three buffers each
   static constexpr int kXW = PT * 4 * 3 * 512;            // weighted x: two buffers
   static constexpr int kYO = NQ * kL * kYRow * 4, kYH = kL * 3 / 2 * kYRow * 4;   // partial rows: one and two buffers
-  static constexpr int kSmem = 3 * (kCB + kX) + 2 * (kXW + kYH) + kYO + 4 * static_cast<int>(sizeof(Scalars)) + 16;
+  static constexpr int kSmem = 3 * (kCB + kX) + 2 * (kXW + kYH) + kYO + 4 * static_cast<int>(sizeof(Scalars)) + 16 * PT;
   static_assert(NS >= 16 && kSmem <= 227 * 1024, "ssd_chunk: shape");
 };
 
@@ -96,7 +99,7 @@ __global__ void __launch_bounds__(kThreads, 1) ssd_chunk_kernel(const __grid_con
   uint8_t* yo_s = xw_s + 2 * T::kXW;                      // read-outs of the state's warps
   uint8_t* yh_s = yo_s + T::kYO;                      // weights x x: rows 0 - 63, then rows 32 - 63 of a second warp
   Scalars* sc_s = reinterpret_cast<Scalars*>(yh_s + 2 * T::kYH);
-  volatile int* odd_s = reinterpret_cast<int*>(sc_s + 4); // chunk c goes token by token
+  volatile int* odd_s = reinterpret_cast<int*>(sc_s + 4); // [chunk & 3][16-column tile]: goes token by token
 
   // this CTA's sequence: the blockIdx.x-th of those that are not outer_scan's
   const int* sq = p.seqs;
@@ -125,7 +128,7 @@ __global__ void __launch_bounds__(kThreads, 1) ssd_chunk_kernel(const __grid_con
   // ldmatrix addresses: rows lane & 15 with 8-column halves by lane >> 4, or rows by (lane & 7, lane >> 4) with halves by bit 3
   const int ra = lane & 15, ca = (lane >> 4) * 16;
   const int rt = (lane & 7) + ((lane >> 4) << 3), ct = ((lane >> 3) & 1) * 16;
-  if (tid < 4) odd_s[tid] = 0;
+  if (tid < 4 * PT) odd_s[tid] = 0;
 
   // Rows of a chunk: this thread's are columns ocol .. of row tid / 8.
   constexpr int OC = T::PC / 8;                           // 4 or 2
@@ -152,7 +155,7 @@ __global__ void __launch_bounds__(kThreads, 1) ssd_chunk_kernel(const __grid_con
   auto rows_out = [&](int ch) {
     const int tok = ch * kL + orow;
     if (tok >= n) return;
-    const bool walked = odd_s[ch & 3] != 0;               // the read-outs are whole rows then
+    const bool walked = odd_s[(ch & 3) * PT + ocol / 16] != 0;   // the read-outs are whole rows then
     const float* yo = reinterpret_cast<const float*>(yo_s) + orow * T::kYRow + ocol;
     const float* yh = reinterpret_cast<const float*>(yh_s + (ch & 1) * T::kYH) + orow * T::kYRow + ocol;
     const uint8_t* xr = x_s + (ch % 3) * T::kX + orow * T::kXRow + 2 * ocol;
@@ -280,7 +283,7 @@ __global__ void __launch_bounds__(kThreads, 1) ssd_chunk_kernel(const __grid_con
     __syncthreads();
     for (int it = -1; it < nchunks; ++it) {
       load();
-      if (ht == 0) odd_s[(it + 2) & 3] = 0;
+      if (ht < PT) odd_s[((it + 2) & 3) * PT + ht] = 0;
       if (it >= 0) fetch_z(it);
       const int ch = it + 1;
       if (ch < nchunks) {
@@ -378,15 +381,18 @@ __global__ void __launch_bounds__(kThreads, 1) ssd_chunk_kernel(const __grid_con
           else blocks(std::integral_constant<int, 1>());
           // rows 32 - 63 have a second warp, whose rows stand behind the others
           float* y = reinterpret_cast<float*>(yh_s + (ch & 1) * T::kYH) + (ri + (j0 ? 32 : 0)) * T::kYRow + 2 * tig;
-          float odd = 0.f;
 #pragma unroll
-          for (int u = 0; u < 2 * PT; ++u)
+          for (int q = 0; q < PT; ++q) {
+            float odd = 0.f;
 #pragma unroll
-            for (int r = 0; r < 2; ++r) {
-              odd = fmaf(Y[u][2 * r], 0.f, fmaf(Y[u][2 * r + 1], 0.f, odd));
-              *reinterpret_cast<float2*>(y + 8 * r * T::kYRow + 8 * u) = make_float2(Y[u][2 * r], Y[u][2 * r + 1]);
-            }
-          if (!(odd == 0.f)) odd_s[ch & 3] = 1;
+            for (int u = 2 * q; u < 2 * q + 2; ++u)
+#pragma unroll
+              for (int r = 0; r < 2; ++r) {
+                odd = fmaf(Y[u][2 * r], 0.f, fmaf(Y[u][2 * r + 1], 0.f, odd));
+                *reinterpret_cast<float2*>(y + 8 * r * T::kYRow + 8 * u) = make_float2(Y[u][2 * r], Y[u][2 * r + 1]);
+              }
+            if (!(odd == 0.f)) odd_s[(ch & 3) * PT + q] = 1;
+          }
         }
       }
       if (it >= 0) {
@@ -402,6 +408,7 @@ __global__ void __launch_bounds__(kThreads, 1) ssd_chunk_kernel(const __grid_con
 
   // ---------------- the state's warps ----------------
   constexpr int NT = T::NS / 8, KS = T::NS / 16;          // 8- and 16-channel tiles of a warp
+  static_assert(KS <= 2, "ssd_chunk: two partial rows at most");
   const int pt = warp % PT, nq = warp / PT, n0 = nq * T::NS;
   // S[t][e]: columns gid (e < 2) and gid + 8 of the warp's 16, channels n0 + 8 t + 2 tig + (e & 1)
   float S[NT][4];
@@ -421,7 +428,7 @@ __global__ void __launch_bounds__(kThreads, 1) ssd_chunk_kernel(const __grid_con
     for (int t = 0; t < NT; ++t)
 #pragma unroll
       for (int e = 0; e < 4; ++e) odd = fmaf(S[t][e], 0.f, odd);
-    if (!(odd == 0.f)) odd_s[ch & 3] = 1;
+    if (!(odd == 0.f)) odd_s[(ch & 3) * PT + pt] = 1;
   };
   __syncthreads();
   check(0);
@@ -431,8 +438,8 @@ __global__ void __launch_bounds__(kThreads, 1) ssd_chunk_kernel(const __grid_con
     const uint32_t cb = sm0 + (ch % 3) * T::kCB, bb = cb + kL * T::kRow;
     fetch_z(ch);
     float* yw = reinterpret_cast<float*>(yo_s) + (nq * kL + gid) * T::kYRow + 16 * pt + 2 * tig;
-    if (odd_s[ch & 3] == 0) {
-      // ---- read-out: the state in three parts against C; the first parts of every 16 channels in sums of their own
+    if (odd_s[(ch & 3) * PT + pt] == 0) {
+      // ---- read-out: the state in three parts against C, every 16 channels in sums of their own (the same in both widths)
       uint32_t sp[KS][2][3][2];
 #pragma unroll
       for (int k = 0; k < KS; ++k)
@@ -446,28 +453,34 @@ __global__ void __launch_bounds__(kThreads, 1) ssd_chunk_kernel(const __grid_con
         uint32_t cf[KS][4];
 #pragma unroll
         for (int k = 0; k < KS; ++k) ldsm4(cb + (16 * i + ra) * T::kRow + 2 * n0 + 32 * k + ca, cf[k]);
-        float Y[KS][2][4], Yl[2][4];
+        float Y[KS][2][4], Yl[KS][2][4];
 #pragma unroll
         for (int k = 0; k < KS; ++k)
 #pragma unroll
           for (int u = 0; u < 2; ++u) {
             mma_bf16_first(Y[k][u], cf[k], sp[k][u][0][0], sp[k][u][0][1]);
-            if (k == 0) mma_bf16_first(Yl[u], cf[k], sp[k][u][2][0], sp[k][u][2][1]);
-            else mma_bf16(Yl[u], cf[k], sp[k][u][2][0], sp[k][u][2][1]);
+            mma_bf16_first(Yl[k][u], cf[k], sp[k][u][2][0], sp[k][u][2][1]);
           }
 #pragma unroll
         for (int k = 0; k < KS; ++k)
 #pragma unroll
-          for (int u = 0; u < 2; ++u) mma_bf16(Yl[u], cf[k], sp[k][u][1][0], sp[k][u][1][1]);
+          for (int u = 0; u < 2; ++u) mma_bf16(Yl[k][u], cf[k], sp[k][u][1][0], sp[k][u][1][1]);
 #pragma unroll
         for (int u = 0; u < 2; ++u)
 #pragma unroll
           for (int r = 0; r < 2; ++r) {
             const float e = sc.ec[16 * i + gid + 8 * r];
-            float a = Yl[u][2 * r], b = Yl[u][2 * r + 1];
+            float a[KS], b[KS];
 #pragma unroll
-            for (int k = 0; k < KS; ++k) add2(a, b, Y[k][u][2 * r], Y[k][u][2 * r + 1]);
-            *reinterpret_cast<float2*>(yw + (16 * i + 8 * r) * T::kYRow + 8 * u) = make_float2(a * e, b * e);
+            for (int k = 0; k < KS; ++k) {
+              a[k] = Yl[k][u][2 * r];
+              b[k] = Yl[k][u][2 * r + 1];
+              add2(a[k], b[k], Y[k][u][2 * r], Y[k][u][2 * r + 1]);
+              a[k] *= e;
+              b[k] *= e;
+              if (k) add2(a[0], b[0], a[k], b[k]);        // two of rows_out's partial rows
+            }
+            *reinterpret_cast<float2*>(yw + (16 * i + 8 * r) * T::kYRow + 8 * u) = make_float2(a[0], b[0]);
           }
       }
       // ---- the state's update
@@ -514,7 +527,7 @@ __global__ void __launch_bounds__(kThreads, 1) ssd_chunk_kernel(const __grid_con
 #pragma unroll
         for (int r = 0; r < 2; ++r) {
           const float w = step * __bfloat162float(xs[t * (T::PC + 8) + 16 * pt + gid + 8 * r]);
-          float y = 0.f;
+          float y[KS];
 #pragma unroll
           for (int k = 0; k < NT; ++k)
 #pragma unroll
@@ -522,10 +535,11 @@ __global__ void __launch_bounds__(kThreads, 1) ssd_chunk_kernel(const __grid_con
               const int at = t * (N + 8) + n0 + 8 * k + 2 * tig + e;
               float& s = S[k][2 * r + e];
               s = fmaf(gt, s, __bfloat162float(bs[at]) * w);
-              y = fmaf(s, __bfloat162float(cs[at]), y);
+              y[k / 2] = fmaf(s, __bfloat162float(cs[at]), k % 2 || e ? y[k / 2] : 0.f);
             }
-          y = quad_sum(y);
-          if (tig == 0) yw[(t - gid) * T::kYRow + gid + 8 * r] = y;
+#pragma unroll
+          for (int k = 0; k < KS; ++k) y[k] = quad_sum(y[k]);
+          if (tig == 0) yw[(t - gid) * T::kYRow + gid + 8 * r] = KS == 2 ? y[0] + y[KS - 1] : y[0];
         }
       }
     }
