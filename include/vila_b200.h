@@ -738,7 +738,8 @@ typedef struct vila_ssd_scan_params {
 int vila_ssd_scan(const vila_ssd_scan_params* p, void* stream);
 /* The same for sequences that have `rows` rows or fewer together, each row in one of them: portions of 48 rows or more run in
  * chunks of 64 tokens where operands, sizes and alignment allow it, the others token by token.  Both have fp32 precision;
- * the order of their sums differs. */
+ * the order of their sums differs.  Sequences that share rows are more than `rows` allows for: those past the first
+ * rows / 48 long ones go token by token. */
 int vila_ssd_scan_rows(const vila_ssd_scan_params* p, int rows, void* stream);
 
 /* vila_selective_scan — recurrence with a step size and decay per channel, fp32 state [slots, C, N]:

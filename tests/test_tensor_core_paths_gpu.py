@@ -655,6 +655,21 @@ def test_ssd_chunks_after_any_decay(ops):
     assert rel(got, want) < 5e-7 and rel(state[1:], S[1:]) < 5e-7
 
 
+@pytest.mark.parametrize("rows,copies", [(60, 2), (100, 5), (48, 40)])
+def test_ssd_chunks_of_sequences_that_share_their_rows(ops, rows, copies):
+    """several states advanced over the same rows: more long sequences than rows of their own would allow"""
+    H, P, N = 2, 32, 128
+    xbc, dt, z, state, _, kw = ssd_inputs([rows], H, P, N, 1)
+    state = torch.randn(1, H, P, N, device="cuda", generator=gen(2)).repeat(copies + 1, 1, 1, 1)
+    seqs = torch.tensor([(0, rows, 5, copies - s) for s in range(copies)], dtype=torch.int32, device="cuda")
+    want, S = ssd_float64(xbc, dt, z, state, seqs[:1], kw)
+    untouched = state[0].clone()
+    got = ops.ssd_scan(xbc, dt, z, state, seqs, **kw)
+    assert rel(got, want) < 5e-7 and torch.equal(state[0], untouched)
+    for slot in range(1, copies + 1):
+        assert rel(state[slot], S[copies]) < 5e-7
+
+
 @pytest.mark.parametrize("where", ["x", "B", "C", "dt", "z", "state", "nan"])
 def test_ssd_chunks_infinite_numbers(ops, where):
     """rows before an infinite number stay as they are, the others are what the recurrence makes of it"""

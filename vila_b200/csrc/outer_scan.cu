@@ -154,7 +154,7 @@ struct ScanArgs {
   int silu;                     // decay: q, k and v are pre-activations, SiLU is taken as they are read
   int vec_qk, vec_a;            // four-element loads of q | k and of z are aligned
   int vec_s;                    // four-element accesses of the state are aligned
-  int below;                    // > 0: only sequences of fewer rows (the others are another launch's)
+  int below, chunked;           // > 0: the first `chunked` sequences of `below` rows or more are another launch's
 };
 
 template <int MODE, int R, int KPT, int CPT, int kStageWarps>
@@ -181,8 +181,16 @@ __global__ void __launch_bounds__(32 * (kOwnerWarps + kStageWarps)) outer_scan_k
   const int* sq = p.seqs + 4 * blockIdx.x;
   const int row0 = sq[0], n = sq[1], pos0 = sq[2], slot = sq[3];
   if (p.below > 0 && n >= p.below) {
-    griddep_wait();
-    return;
+    // Which of the long ones this is.  The other launch has a grid for as many as the rows hold; sequences that read the same
+    // rows (into states of their own) can be more.
+    int before = 0;
+    if (blockIdx.x >= static_cast<unsigned>(p.chunked))
+      for (unsigned s0 = 0; s0 < blockIdx.x; s0 += 32)
+        before += __popc(__ballot_sync(0xffffffffu, s0 + lane < blockIdx.x && p.seqs[4 * (s0 + lane) + 1] >= p.below));
+    if (before < p.chunked) {
+      griddep_wait();
+      return;
+    }
   }
   const int h = blockIdx.y, dim = p.dim, vdim = p.vdim, kh = h / (p.H / p.G);
   const int col0 = blockIdx.z * COLS;
@@ -748,8 +756,9 @@ int ssd_scan(const vila_ssd_scan_params& p, int rows, cudaStream_t stream) {
   // for both and 114 against 300 for 2048.  By each sequence's own rows, so that its numbers do not depend on the others.
   constexpr int kChunkRows = 48;
   if (rows - p.nseq + 1 >= kChunkRows && ssd_chunk_takes(p)) {
-    if (const int rc = ssd_chunk(p, min(p.nseq, rows / kChunkRows), kChunkRows, stream)) return rc;
     a.below = kChunkRows;
+    a.chunked = min(p.nseq, rows / kChunkRows);
+    if (const int rc = ssd_chunk(p, a.chunked, kChunkRows, stream)) return rc;
   }
   return scan_by_dim<kSsd>(a, p.nseq, stream);
 }
