@@ -339,7 +339,9 @@ __device__ __forceinline__ void combine_maps(const vila_paged_attn_params& p, co
 //   Ss [BQ * H][BK] raw scores | Ps [BQ * H][BK] weights | talk [H * H] | m, l, alpha [BQ * H]
 // H and G count score heads (a head's maps singly), the value heads are GV = G / maps.
 // DS = D4 + 4: consecutive keys start 4 banks apart, so the float4 reads of 8 keys do not collide.
-template <int NACC>   // few accumulators: registers for four CTAs on an SM, whose loads and barriers then overlap
+// CAP: with capped scores, whose instructions are not in the other form (uncapped prompts of mixed heads ran 3 % slower for
+// them in tiles of 4 rows).
+template <int NACC, bool CAP>   // few accumulators: registers for four CTAs on an SM, whose loads and barriers then overlap
 __global__ void __launch_bounds__(kThreads, NACC <= 2 ? 4 : (NACC <= 8 ? 2 : 1)) paged_attn_kernel(const vila_paged_attn_params p, const AttnShape sh) {
   extern __shared__ __align__(16) float sm[];
   // H, G: the heads this CTA serves (all of them, or one value head with its key and query heads: h0 + h, g0 + g)
@@ -422,7 +424,7 @@ __global__ void __launch_bounds__(kThreads, NACC <= 2 ? 4 : (NACC <= 8 ? 2 : 1))
         const float4 a = qr[k], c = kr[k];
         s = fmaf(a.x, c.x, s); s = fmaf(a.y, c.y, s); s = fmaf(a.z, c.z, s); s = fmaf(a.w, c.w, s);
       }
-      Ss[idx] = capped(p, s);
+      Ss[idx] = CAP ? capped(p, s) : s;
     }
     __syncthreads();
     if (after) {
@@ -570,7 +572,7 @@ __global__ void __launch_bounds__(kThreads, NACC <= 2 ? 4 : (NACC <= 8 ? 2 : 1))
 //                  (Ps is [row block][key][4]): 2 shared loads per 16 multiply-adds
 // Shared memory (floats): Qs [R][D4] | Ks [BK][G][DS] | Vs [BK][G][V4] | Ss [R][BK] | Ps [R / 4][BK][4] |
 //   m, l, alpha [R] | talk [H * H]
-template <int NACC, int NT, int TR>
+template <int NACC, int NT, int TR, bool CAP>
 __global__ void __launch_bounds__(NT) paged_attn_tile4_kernel(const vila_paged_attn_params p, const AttnShape sh) {
   extern __shared__ __align__(16) float sm[];
   // H, G: the heads this CTA serves (all of them, or one K/V head with its query heads: global heads h0 + h, g0 + g)
@@ -651,8 +653,8 @@ __global__ void __launch_bounds__(NT) paged_attn_tile4_kernel(const vila_paged_a
       }
 #pragma unroll
       for (int a = 0; a < TR; ++a) {
-        Ss[(r0 + a) * BK + jp] = capped(p, s[a][0]);
-        Ss[(r0 + a) * BK + jp + HK] = capped(p, s[a][1]);
+        Ss[(r0 + a) * BK + jp] = CAP ? capped(p, s[a][0]) : s[a][0];
+        Ss[(r0 + a) * BK + jp + HK] = CAP ? capped(p, s[a][1]) : s[a][1];
       }
     }
     __syncthreads();
@@ -981,10 +983,10 @@ int paged_attention(const vila_paged_attn_params& p, cudaStream_t stream) {
       const dim3 grid4(p.ntiles, sh.sub, sh.hsplit);
 #define VB_PAGED4(N, NT, TR)                                                                                     \
   do {                                                                                                           \
+    const auto kernel = p.softcap > 0.f ? paged_attn_tile4_kernel<N, NT, TR, true> : paged_attn_tile4_kernel<N, NT, TR, false>; \
     if (smem4 > 48 * 1024)                                                                                       \
-      VB_CUDA(cudaFuncSetAttribute(paged_attn_tile4_kernel<N, NT, TR>,                                           \
-                                   cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem4)));       \
-    VB_CUDA(launch_serial(paged_attn_tile4_kernel<N, NT, TR>, grid4, dim3(NT), smem4, stream, p, sh));           \
+      VB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem4))); \
+    VB_CUDA(launch_serial(kernel, grid4, dim3(NT), smem4, stream, p, sh));                                       \
   } while (0)
       if (nt == 512) {
         if (nacc4 <= 1) VB_PAGED4(1, 512, 2);
@@ -1012,10 +1014,10 @@ int paged_attention(const vila_paged_attn_params& p, cudaStream_t stream) {
   const dim3 grid(p.ntiles, sh.sub * sh.hsplit, p.nsplit);
 #define VB_PAGED(N)                                                                                              \
   do {                                                                                                           \
+    const auto kernel = p.softcap > 0.f ? paged_attn_kernel<N, true> : paged_attn_kernel<N, false>;              \
     if (smem > 48 * 1024)                                                                                        \
-      VB_CUDA(cudaFuncSetAttribute(paged_attn_kernel<N>, cudaFuncAttributeMaxDynamicSharedMemorySize,            \
-                                   static_cast<int>(smem)));                                                     \
-    VB_CUDA(launch_serial(paged_attn_kernel<N>, grid, dim3(kThreads), smem, stream, p, sh));                     \
+      VB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem))); \
+    VB_CUDA(launch_serial(kernel, grid, dim3(kThreads), smem, stream, p, sh));                                   \
   } while (0)
   // weights mixed after the softmax + split keys: the (max, sum) launch, then the launch that adds the values
   const int launches = (p.talk_after != 0 && p.nsplit > 1) ? 2 : 1;
