@@ -46,8 +46,10 @@ __device__ __forceinline__ float head_scale(const vila_paged_attn_params& p, int
 // A head's own scaled score, bounded to (-softcap, softcap) when a cap is set: cap tanh(s / cap).  Scores up to the cap itself
 // take s R((s / cap)^2) with R(u) = tanh(sqrt u) / sqrt u, an entire quotient on [0, 1] whose nearest pole (-pi^2 / 4) lets
 // Chebyshev interpolation of degree 7 be 4e-9 close: 3.3e-8 off in fp32 (rms; a correctly rounded quotient, tanh and product
-// 4.2e-8) at 10 multiply-adds where the quotient and tanhf took 50 instructions.  By the score alone, so that it does not
-// depend on its neighbours.
+// 4.2e-8) at 10 multiply-adds where the quotient and tanhf took 50 instructions.  Scores above the cap take
+// cap (1 - 2 / (e^(2 s / cap) + 1)), whose quotient is below 0.24 there, so that the approximate exponential and reciprocal cost
+// less than a rounding of the result: 1.8e-8 - 4.0e-8 off (rms; at most 1.4e-7) over 1 < s / cap < 9 for caps of 0.01 - 50, where
+// cap tanhf(s / cap) is 1.8e-8 - 4.4e-8 (1.7e-7).  By the score alone, so that it does not depend on its neighbours.
 __device__ __forceinline__ constexpr float cap_poly(int k) {
   constexpr float c[8] = {1.0f, -0.33333277702331543f, 0.1333213895559311f, -0.05386970564723015f,
                           0.02146141044795513f, -0.007912484928965569f, 0.002278647618368268f, -0.000352328090230003f};
@@ -55,11 +57,18 @@ __device__ __forceinline__ constexpr float cap_poly(int k) {
 }
 __device__ __forceinline__ float cap_inverse(const vila_paged_attn_params& p) { return p.softcap > 1e-30f ? 1.0f / p.softcap : 0.f; }
 __device__ __forceinline__ bool over_cap(const vila_paged_attn_params& p, float s) { return !(fabsf(s) <= p.softcap); }
-__device__ __forceinline__ float capped_over(const vila_paged_attn_params& p, float s) { return p.softcap * tanhf(s / p.softcap); }
+__device__ __forceinline__ float cap_inverse_over(float inverse) { return inverse > 0.f ? 2.8853900817779268f * inverse : INFINITY; }   // 2 log2 e / cap
+__device__ __forceinline__ float capped_over(float cap, float inverse_over, float s) {
+  float e, q;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e) : "f"(fabsf(s) * inverse_over));
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(q) : "f"(e + 1.0f));
+  return copysignf(fmaf(-2.0f * cap, q, cap), s);
+}
 __device__ __forceinline__ float capped(const vila_paged_attn_params& p, float s) {
   if (!(p.softcap > 0.f)) return s;
-  if (over_cap(p, s)) return capped_over(p, s);
-  const float x = s * cap_inverse(p), u = __fmul_rn(x, x);
+  const float inv = cap_inverse(p);
+  if (over_cap(p, s)) return capped_over(p.softcap, cap_inverse_over(inv), s);
+  const float x = s * inv, u = __fmul_rn(x, x);
   float r = cap_poly(7);
 #pragma unroll
   for (int k = 6; k >= 0; --k) r = fmaf(r, u, cap_poly(k));

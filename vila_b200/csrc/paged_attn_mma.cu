@@ -75,11 +75,6 @@ __device__ __forceinline__ void cap2(float& a, float& b, float inv) {
   for (int k = 6; k >= 0; --k) r = fma2(r, u, pair(cap_poly(k), cap_poly(k)));
   unpair(mul2(s, r), a, b);
 }
-__device__ __noinline__ float capped_apart(float cap, float s) {   // any score
-  vila_paged_attn_params p;
-  p.softcap = cap;
-  return capped(p, s);
-}
 __device__ __forceinline__ float ex2(float x) {
   float y;
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
@@ -303,11 +298,17 @@ paged_attn_mma_kernel(const __grid_constant__ vila_paged_attn_params p, int tile
           for (int t = 0; t < kBK / 8; ++t)
 #pragma unroll
             for (int e = 0; e < 4; ++e) over |= over_cap(p, s[t][e]);
-          if (over) {
+          if (__any_sync(0xffffffffu, over)) {
+            const float cap_inv_over = cap_inverse_over(cap_inv);
 #pragma unroll
             for (int t = 0; t < kBK / 8; ++t)
 #pragma unroll
-              for (int e = 0; e < 4; ++e) s[t][e] = capped_apart(p.softcap, s[t][e]);
+              for (int e = 0; e < 4; e += 2) {
+                const float a = s[t][e], b = s[t][e + 1];
+                cap2(s[t][e], s[t][e + 1], cap_inv);
+                if (over_cap(p, a)) s[t][e] = capped_over(p.softcap, cap_inv_over, a);
+                if (over_cap(p, b)) s[t][e + 1] = capped_over(p.softcap, cap_inv_over, b);
+              }
           } else {
 #pragma unroll
             for (int t = 0; t < kBK / 8; ++t)
