@@ -167,6 +167,44 @@ def test_glinear_waits_that_run_out_are_reported(ops, monkeypatch, rows, routed)
     assert torch.equal(limited(1 << 20), want)
 
 
+def test_engine_reports_a_step_that_gave_up_before_a_second_one_builds_on_it(ops):
+    """a step whose logits nobody reads gives up behind a second of other work: the step after next raises"""
+    from vila_b200 import _lib
+    from vila_b200.serving import TokenEngine
+    lib, g = _lib.load(), gen(1)
+    a, w = randn(g, 64, 256), randn(g, 256, 256)
+
+    class Model:
+        device, dtype, tries = torch.device("cuda", torch.cuda.current_device()), BF, 1 << 20
+        latent_widths = state_shapes = staticmethod(dict)
+
+        def forward_step(self, batch, cache, layer_outputs=None):
+            if self.tries == 0:
+                torch.cuda._sleep(2_000_000_000)
+                with pytest.MonkeyPatch.context() as m:
+                    m.setattr(lib, "vila_glinear", lambda p, stream: lib.vila_glinear_tries(p, 0, stream))
+                    ops.glinear(a, w)
+            return a
+
+    ops.check_waits()
+    model = Model()
+    engine = TokenEngine(model, 256, 1, graphs=False)
+    engine.step([(0, [1, 2, 3], [])])
+    model.tries = 0
+    engine.step([(0, [4], [])])
+    model.tries = 1 << 20
+    engine.step([(0, [5], [])])
+    try:
+        with pytest.raises(RuntimeError, match="ran out"):
+            engine.step([(0, [6], [])])
+    finally:
+        torch.cuda.synchronize()
+        lib.vila_wait_status()
+    assert engine.length(0) == 5
+    engine.step([(0, [6], [])])
+    ops.check_waits()
+
+
 @pytest.mark.parametrize("pairs,E", [(1, 1), (31, 5), (256, 32), (257, 7), (8192, 32), (8191, 300), (20000, 64), (600, 1500), (9000, 1100)])
 def test_moe_group_is_a_stable_sort(ops, pairs, E):
     """expert segments in pair order; indices of no expert (identity choices) belong to no segment"""

@@ -312,6 +312,8 @@ class TokenEngine:
     model.logits).  `max_tokens` bounds the tokens live sequences hold together (each rounded up to a
     page), `slots` the number of live sequences."""
 
+    _unread = ()   # (number, event behind it) of the last steps whose logits nobody wanted
+
     def __init__(self, model, max_tokens: int, slots: int = 4, page: int = LATENT_PAGE, graphs: bool = True):
         self.model = model
         self.cache = HybridCache(model, max_tokens, slots, page)
@@ -325,6 +327,8 @@ class TokenEngine:
         self.graphs = graphs
         self._decode_graphs: Dict[int, tuple] = {}
         self._decode_seen: Dict[int, int] = {}
+        self._unread = deque()
+        self._steps = 0
 
     # ---- sequences --------------------------------------------------------------------------------
     def admit(self, seq_id) -> _Sequence:
@@ -463,11 +467,23 @@ class TokenEngine:
     def step(self, entries, layer_outputs: Optional[list] = None) -> Optional[torch.Tensor]:
         """entries: (sequence id, next token ids, indices among them whose logits are wanted).  All
         entries run as one batch on top of what earlier steps cached.  -> fp32 logits [wanted, vocab]
-        in entry / index order (None if nothing is wanted).  The host does not wait for the device: reading the logits does."""
+        in entry / index order (None if nothing is wanted).  The host does not wait for the device: reading the logits does.
+        A step without any is waited for by the step after next, so that no second one builds on a step that gave up a wait
+        of its kernels (raised here)."""
+        while self._unread and self._unread[0][0] < self._steps:
+            self._unread.popleft()[1].synchronize()
         ops.check_waits()   # of the steps so far
         entries = [e for e in entries if len(e[1])]
         if not entries:
             return None
+        logits = self._step(entries, layer_outputs)
+        self._steps += 1
+        if logits is None and torch.device(self.model.device).type == "cuda":
+            self._unread.append((self._steps, torch.cuda.Event()))
+            self._unread[-1][1].record(torch.cuda.current_stream(self.model.device))
+        return logits
+
+    def _step(self, entries, layer_outputs: Optional[list]) -> Optional[torch.Tensor]:
         flat, sizes = self._build(entries)
         T, n_want = sizes[0], sizes.pop()
         arrays = flat[:flat.numel() - n_want]
