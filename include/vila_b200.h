@@ -174,7 +174,8 @@ int vila_rope_kv_append_table(void* qkv, const void* rope_table, int S, int Hq, 
  * in ONE kernel (rope_table: vila_rope_table of the chunk's positions).  Bit-identical to the two calls where vila_linear
  * takes the swap-AB kernel as well.  Its sums over K run in another order, so that results may differ in the last place,
  * for up to 4 rows of at most 20 M weights or 8 rows of 6 M, and for rows that fill 128-row tiles to nine tenths
- * (116..128, 231..256, 346..384) of a layer of at most 74 128 x 128 tiles and K >= 512.  Replaces Qwen2Attention's q_proj/k_proj/v_proj +
+ * (116..128, 231..256, 346..384) of a layer of at most 74 128 x 128 tiles and K >= 512; without a bias also for 33..384 rows
+ * of any layer of up to 8192 outputs (vila_linear may take tiles there).  Replaces Qwen2Attention's q_proj/k_proj/v_proj +
  * apply_rotary_pos_emb + past_key_value.update (modeling_qwen2.py:223-226,99-160,262-266 of the
  * in-tree copy).  Returns 3 (and sets vila_last_error) when the shape is not covered: the caller
  * then issues the two separate calls. */

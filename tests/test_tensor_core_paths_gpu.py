@@ -515,6 +515,32 @@ def test_linear_qkv_rope_equals_linear_and_rope(ops, M, Hq, Hkv, K):
     assert same(ops.linear_qkv_rope(x, w, b, tab, Hq, Hkv, D), plain)
 
 
+@pytest.mark.parametrize("M", [16, 32, 33, 100, 200, 300, 384])
+@pytest.mark.parametrize("Hq,Hkv,K", [(2, 1, 1288), (16, 2, 2048), (28, 4, 3584)])
+def test_linear_qkv_rope_without_a_bias(ops, M, Hq, Hkv, K):
+    """the same bits up to 32 rows; from 33 on vila_linear may take tiles, which sum K in another order"""
+    g, D = gen(M + K), 128
+    N = (Hq + 2 * Hkv) * D
+    x, w = randn(g, M, K), (randn(g, N, K).float() * K ** -0.5).to(BF)
+    pos = torch.arange(M, dtype=torch.int32, device="cuda")
+    inv = (1.0 / (1e6 ** (torch.arange(0, D, 2, dtype=torch.float32) / D))).cuda()
+    ref, tab = ops.linear(x, w), ops.rope_table(pos, D, inv)
+    ops.rope_kv_append(ref, pos, Hq, Hkv, D, inv)
+    got = ops.linear_qkv_rope(x, w, None, tab, Hq, Hkv, D)
+    assert torch.equal(got, ref) if M <= 32 else rel(got, ref.double()) < 2.0 ** -8
+
+
+@pytest.mark.parametrize("M,N,K,act,form", [(256, 3584, 4608, 1, 5128), (256, 2048, 4608, 1, 5128), (100, 3584, 4608, 2, 5128), (17, 3584, 4608, 2, 3000), (279, 3584, 18944, 0, 3000),
+                                            (64, 2048, 2048, 0, 5128), (32, 2048, 2048, 0, 3000), (384, 1024, 1024, 0, 5128)])
+def test_linear_few_tokens_take_the_form_that_is_ahead(ops, M, N, K, act, form):
+    """which form vila_linear takes up to 384 rows, by its bits: K summed in order, in the halves of a CTA pair or by a cluster"""
+    g = gen(M + N)
+    x, w = randn(g, M, K), (randn(g, N, K).float() * K ** -0.5).to(BF)
+    got = ops.linear(x, w, act=act)
+    others = [f for f in (128, 3000, 5128) if f != form and (f != 5128 or (M + 127) // 128 * ((N + 127) // 128) <= 74)]
+    assert torch.equal(got, ops.linear(x, w, act=act, block_n=form)) and not any(torch.equal(got, ops.linear(x, w, act=act, block_n=f)) for f in others)
+
+
 # ---- recurrences --------------------------------------------------------------------------------------------
 def hgrn2_inputs(g, T, H, dim, vdim, dtype=BF):
     proj = randn(g, T, 2 * H * dim + H * vdim, dtype=dtype)

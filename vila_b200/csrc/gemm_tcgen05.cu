@@ -751,19 +751,23 @@ int gemm_bf16(const __nv_bfloat16* A, int lda, const __nv_bfloat16* W, int ldw, 
   if (M <= 384) {
     // Few tokens: the swap-AB kernel (every weight byte enters an SM once, K split over a cluster) where the weight stream is
     // what counts: 6 us + 0.027 a row + 0.20 a MB, 0.0003 more per row.  With an activation its epilogue counts as well and
-    // tiles are ahead (22016 gated outputs x 2048 on 40 | 140 | 279 rows 25 | 31 | 35 us, there 33 | 38 | 51; 4304 x 1152 with
-    // GELU on 100 rows 9, there 15) unless they nearly fill one round too many (37888 x 3584 on 279 rows 83 and 81, and
-    // behind other kernels 90).  Without one, where they fill one round (no faster than the weights at 4.8 TB/s): 279 rows x
-    // 3088 x 1024 8.8 and 14.5, 200 x 2048 x 2048 9.7 and 13.8, but 3584 x 18944 91 and 54; up to 32 rows and for more than
+    // tiles are ahead: any form up to 16 MB of weights (4304 x 1152 with GELU on 100 rows 8.1, there 14.0), the halves of K
+    // always where they are by the two estimates (3584 x 4608 with GELU on 100 | 256 rows 16.4 | 17.5, there
+    // 19.8 | 23.2), the others from 0.7 of that estimate on (22016 gated outputs x 2048 on 40 | 279 rows 24 | 34,
+    // there 33 | 50).  Theirs is too low for large weights on partly filled row blocks: 37888 x 3584 on 279 rows, the third
+    // block with 23 of 128, should be 66 and is 81, there 82 (behind other kernels 90 and 82).
+    // Without an activation, where they fill one round (no faster than the weights at 4.8 TB/s): 279 rows x
+    // 3088 x 1024 7.9 and 14.2, 200 x 2048 x 2048 9.3 and 14.0, but 3584 x 18944 90 and 55; up to 32 rows and for more than
     // 8192 outputs never.
-    // A projection with no more than a bias onto whole 128-column heads may be the other half of vila_linear_qkv_rope: it
-    // stays where that has the same bits (rows that fill their tiles: K halved, as ever).
+    // A projection with a bias and no more onto whole 128-column heads may be the other half of vila_linear_qkv_rope: it
+    // stays where that has the same bits (rows that fill their tiles: K halved, as ever).  Without a bias it goes by the
+    // time, and the header says so (1024 x 1024 on 279 rows 6.4, there 13.0).
     const bool plain = epi.act == ACT_NONE && epi.swiglu == 0;
     const bool heads = plain && epi.residual == nullptr && epi.bias != nullptr && N % 128 == 0;
     const bool one_round = mb * nb <= sms || mb2 * nb2 <= sms / 2;
     const double t_swap = 6.0 + 0.027 * M + (0.20 + 0.0003 * M) * mbytes;
     const bool ahead = M > 32 && N <= 8192 && (t_half < 1.05 * t_swap || (one_round && fmax(t_tiles, 4.0 + 0.21 * mbytes) < 0.95 * t_swap));
-    const bool tiles = M <= 16 ? false : heads ? t_half < 1e30 && M * 10 >= mb * 128 * 9 : plain ? ahead : mbytes < 16 || t_tiles < 0.7 * t_swap;
+    const bool tiles = M <= 16 ? false : heads ? t_half < 1e30 && M * 10 >= mb * 128 * 9 : plain ? ahead : mbytes < 16 || t_half < t_swap || t_tiles < 0.7 * t_swap;
     if (!tiles) {
       const int rc = gemm_skinny_bf16(A, lda, W, ldw, C, ldc, M, N, K, epi, 0, stream);
       if (rc >= 0) return rc;
