@@ -10,7 +10,7 @@
 //     latency and by half-sector accesses: eight warps (four before), residual rows requested a chunk ahead and while the
 //     products run, 32 bytes per lane and access.  13312 rows: 1152 x 592 with residual 61 -> 34 us, 1152 x 1152 70 -> 39,
 //     3456 x 1152 92 -> 77, 4304 x 1152 with GELU 149 -> 113, 1152 x 4304 116 -> 109; 1024 rows 11.1 -> 9.4, 15.4 -> 12.7,
-//     19.5 -> 16.6; 16470 x 37888 x 3584 2905 -> 2785
+//     19.5 -> 16.6.  K of 3584 and more on 16470 rows: no change beyond what the power cap makes two runs differ by
 //   * scheduling: data-parallel over output tiles, or STREAM-K when the tile count does not fill the
 //     148 SMs evenly (skinny prefill GEMMs, M = 280): the (tile, k-block) iteration space is cut
 //     into equal contiguous ranges, each partial tile is parked in its own fp32 workspace slot and
