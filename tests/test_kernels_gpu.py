@@ -131,6 +131,33 @@ def test_linear_tiles_gated_unit_takes_no_residual(cuda, block_n):
     assert torch.equal(out, want) and torch.isfinite(out).all()
 
 
+@pytest.mark.parametrize("block_n", [None, 64, 128, 256, 1128, 4128, 4256, 5128])
+@pytest.mark.parametrize("N", [136, 264, 520])
+@pytest.mark.parametrize("shift_out,shift_res", [(0, 0), (8, 0), (0, 8), (8, 8)])
+def test_linear_wide_accesses_at_row_ends(cuda, block_n, N, shift_out, shift_res):
+    """rows of 16-column strides that end on half of a 32-byte access, out and residual on 32 bytes or on 16 only: values,
+    the columns beside them, and the residual in place"""
+    ops = _ops()
+    ops.ensure_workspace("cuda")
+    M, K, wide = 200, 256, N + 24
+    assert wide % 16 == 0 and N % 16 == 8
+    g = torch.Generator(device="cuda").manual_seed(N + shift_out + 2 * shift_res)
+    x = bf(torch.randn(M, K, device=cuda, generator=g))
+    w = bf(torch.randn(N, K, device=cuda, generator=g) / math.sqrt(K))
+    b = bf(torch.randn(N, device=cuda, generator=g))
+    res = bf(torch.randn(M, wide, device=cuda, generator=g))[:, shift_res:shift_res + N]
+    base = torch.full((M, wide), 7.0, dtype=torch.bfloat16, device=cuda)
+    out = base[:, shift_out:shift_out + N]
+    ops.linear(x, w, b, residual=res, out=out, block_n=block_n)
+    ref = rb(rb(x.float() @ w.float().t() + b.float()) + res.float())
+    assert rel_err(out, ref) < 8e-3
+    assert bool((base[:, :shift_out] == 7.0).all()) and bool((base[:, shift_out + N:] == 7.0).all())
+    inplace = res.clone()
+    want = out.clone()
+    ops.linear(x, w, b, residual=inplace, out=inplace, block_n=block_n)
+    assert torch.equal(inplace, want)
+
+
 @pytest.mark.parametrize("M", [1, 33, 279, 384])
 def test_linear_qkv_rope_fused_equals_two_kernels(cuda, M):
     """q/k/v projection with RoPE + paged KV append fused into the GEMM epilogue must be bit-identical
