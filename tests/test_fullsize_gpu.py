@@ -212,9 +212,9 @@ def test_cfg4_dynamic_s2_full_size(cuda):
 
 
 def test_cfg4_matches_oracle_full_depth(cuda):
-    """BASELINE configs[3] (producible layout): 1 + 4 + 5x6 = 35 tiles -> tower -> S2
+    """the multi-scale layout of a wide 4K frame: 1 + 4 + 5x6 = 35 tiles -> tower -> S2
     merge to the largest scale -> C = 3456 projector -> re-stitch, against the oracle; plus the
-    fp32 / fp16 pixel inputs the reference feeds (ADVICE r1)."""
+    fp32 / fp16 pixel inputs the reference feeds."""
     model = get_model("s2")
     cfg = model.config
     bs = (5, 6)
