@@ -64,9 +64,7 @@ __device__ __forceinline__ float capped_over(float cap, float inverse_over, floa
   asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(q) : "f"(e + 1.0f));
   return copysignf(fmaf(-2.0f * cap, q, cap), s);
 }
-__device__ __forceinline__ float capped(const vila_paged_attn_params& p, float s) {
-  if (!(p.softcap > 0.f)) return s;
-  const float inv = cap_inverse(p);
+__device__ __forceinline__ float capped(const vila_paged_attn_params& p, float s, float inv) {   // inv: cap_inverse
   if (over_cap(p, s)) return capped_over(p.softcap, cap_inverse_over(inv), s);
   const float x = s * inv, u = __fmul_rn(x, x);
   float r = cap_poly(7);
@@ -74,6 +72,7 @@ __device__ __forceinline__ float capped(const vila_paged_attn_params& p, float s
   for (int k = 6; k >= 0; --k) r = fmaf(r, u, cap_poly(k));
   return s * r;
 }
+__device__ __forceinline__ float capped(const vila_paged_attn_params& p, float s) { return p.softcap > 0.f ? capped(p, s, cap_inverse(p)) : s; }
 __device__ __forceinline__ float dist_bias(const vila_paged_attn_params& p, int dist, int h) {
   return __ldg(p.dist_bias + static_cast<size_t>(min(dist, p.dist_rows - 1)) * p.H + h);
 }
