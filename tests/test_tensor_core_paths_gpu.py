@@ -765,7 +765,7 @@ def test_ssd_chunks_infinite_numbers(ops, where):
 
 
 @pytest.mark.parametrize("M,N,K", [(1, 128, 2048), (8, 130, 2056), (9, 129, 4096), (16, 4097, 4104), (16, 200, 8192), (3, 17000, 1032), (5, 33000, 512), (16, 333, 264),
-                                   (2, 144, 8)])
+                                   (2, 144, 8), (3, 1024, 1024), (8, 7104, 256), (4, 7120, 1024), (9, 4096, 256), (7, 4112, 248), (16, 2048, 128)])
 def test_few_rows_stream(ops, M, N, K):
     """CTAs that stay and those that don't: ragged columns, a last tile of one weight row, token rows that do not fit in shared memory"""
     g = gen(M + N + K)
@@ -777,6 +777,11 @@ def test_few_rows_stream(ops, M, N, K):
     assert rel(ops.glinear(a, w, bias=b, act=ops.ACT_RELU2, out_dtype=F32), torch.relu(ref + b.double()) ** 2) < 3 * 32 ** 0.5 * 2.0 ** -24
     # a row's sums do not depend on the other rows
     assert torch.equal(ops.glinear(a[:1], w, out_dtype=F32), got[:1])
+    # products of one sign: truncations of 16 terms at 2^-24 of their sum (a bias), the additions after them rounded at no more
+    # than 2^-24 of the whole in each of four levels, and the last bit
+    pos = ops.glinear(a.abs(), w.abs(), out_dtype=F32)
+    want = a.double().abs() @ w.double().abs().T
+    assert rel(pos, want) < (1 + 5 ** 0.5) * 2.0 ** -24 and float(((pos.double() - want) / want).mean().abs()) < 2.0 ** -24
     if N % 2 == 0:
         z = ref / K ** 0.5
         want = torch.nn.functional.silu(z[:, 0::2]) * z[:, 1::2]

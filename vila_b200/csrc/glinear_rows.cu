@@ -5,9 +5,11 @@
 // of 32768 x 2048: 40 us, 16 rows 72), and a running tensor-core sum over K is truncated at every step (K = 2048 in one
 // accumulator: 2.1e-6 off).  Sums of 16 products lose 1 - 2e-8, and their rounded additions in chains of 8 - 16 and a tree
 // over the warps no more than the multiply-adds did: 7.8e-8 off at K = 2048 (7.9e-8), 8.3e-8 at 4096 (9.5e-8), 6.6e-8 at 704
-// (6.5e-8).  A tile is 16 weight rows x 8 or 16 token rows.  A lane's 16 bytes of a weight row are its share of two products'
-// fragments, with the token rows' columns dealt alike, so both are loaded as they lie.  A sum's order depends on K, N and the
-// number of groups, not on how many rows there are (pairs: from 4 M weights on they take the other form).
+// (6.5e-8).  Where all products have one sign the truncation is a bias, 1.3e-8 whatever K is: 4.0 - 4.6e-8 off at K = 512, 4.2 -
+// 4.6e-8 at 2048, 4.5e-8 at 8192 (multiply-adds 3.9 - 4.3e-8, 3.9 - 4.5e-8, 4.5 - 4.8e-8).
+// A tile is 16 weight rows x 8 or 16 token rows.  A lane's 16 bytes of a weight row are its share of two products' fragments,
+// with the token rows' columns dealt alike, so both are loaded as they lie.  A sum's order depends on K, N and the number of
+// groups, not on how many rows there are (pairs: from 4 M weights on they take the other form, see the rule).
 //
 // Measured, in brackets the multiply-adds: 32768 x 2048 on 1 | 8 | 16 rows 24.2 | 25.9 | 29.1 us (28 | 41 | 72), 65536 x 4096 on
 // 8 rows 86 = 6.2 TB/s (132), 128 x 8192 on one row 6.1 (8.9), 1024 x 2048 on 8 rows 4.8 (5.8), routed 1408 x 2048 on 32
@@ -110,7 +112,7 @@ __global__ void __launch_bounds__(32 * kStay, 1) glinear_stream_kernel(const vil
       row_s[i] = row;
       __syncwarp();
       int same = i;
-      for (int j = 32 * hf + 31; j >= 0; --j)
+      for (int j = min(32 * hf + 31, live1 - 1); j >= live0; --j)
         if (row_s[j] == row && j <= i) same = j;
       const unsigned fresh = __ballot_sync(0xffffffffu, same == i && live);
       if (same == i && live) {
@@ -252,7 +254,7 @@ constexpr int kRowsOf(int kw) { return kWarps / kw * 16; }   // weight rows of a
 
 // NT * 8 token rows from m0 on (the first nr of them exist) times the CTA's weight rows from n_cta on.  KW warps share 16 weight
 // rows, each with every KW-th piece of 32 columns.
-template <int KW, int NT>
+template <int KW, int NT, bool AHEAD>
 __device__ __forceinline__ void rows_pass(const vila_glinear_params& p, const vila_glinear_ext& x, int g, int n_cta, int m0, int nr, float* red) {
   constexpr int NP = kInFlight / 2, kRows = kRowsOf(KW), kPitch = kRows + 4;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, gid = lane >> 2, tig = lane & 3;
@@ -287,15 +289,23 @@ __device__ __forceinline__ void rows_pass(const vila_glinear_params& p, const vi
     for (int t = 0; t < NT; ++t)
 #pragma unroll
       for (int e = 0; e < 8; ++e) acc[t][e >> 2][e & 3] = 0.f;
+    uint4 xv[NP][NT];
+    const auto fetch = [&](int q) {
+      const int k = k0 + 32 * KW * q;
+#pragma unroll
+      for (int t = 0; t < NT; ++t) xv[q][t] = k < p.K ? __ldg(reinterpret_cast<const uint4*>(xr[t] + k)) : zero;
+    };
+    if (AHEAD) {
+#pragma unroll
+      for (int q = 0; q < NP; ++q) fetch(q);
+    }
 #pragma unroll
     for (int q = 0; q < NP; ++q) {
       const int k = k0 + 32 * KW * q;
       if (k - 8 * tig >= p.K) break;                      // uniform over the warp
-      uint4 xv[NT];
+      if (!AHEAD) fetch(q);
 #pragma unroll
-      for (int t = 0; t < NT; ++t) xv[t] = k < p.K ? __ldg(reinterpret_cast<const uint4*>(xr[t] + k)) : zero;
-#pragma unroll
-      for (int t = 0; t < NT; ++t) piece(acc[t], w[q][0], w[q][1], xv[t]);
+      for (int t = 0; t < NT; ++t) piece(acc[t], w[q][0], w[q][1], xv[q][t]);
       const int kn = k + 32 * KW * NP;
       w[q][0] = kn < p.K ? ld_once(w0 + kn, policy) : zero;
       w[q][1] = kn < p.K ? ld_once(w1 + kn, policy) : zero;
@@ -337,14 +347,18 @@ __device__ __forceinline__ void rows_pass(const vila_glinear_params& p, const vi
   }
 }
 
-template <int KW, int NT>
-__global__ void __launch_bounds__(32 * kWarps, NT == 1 ? 4 : 2) glinear_rows_kernel(const vila_glinear_params p, const vila_glinear_ext x) {
+// AHEAD: a pass's token rows are requested before its first weights are waited for.  For grids that the SMs hold at once and
+// more than two pieces a warp, where a piece's way to L2 would otherwise follow the one before it (1024 x 1024 on one row 3.7 -> 3.3 us, a routed 512 x 2048
+// on one pair 7.0 -> 4.9); larger ones hide it behind a fourth CTA on the SM, which the registers would cost them (2048 x 704
+// on 32 pairs of 32 experts 19.0, 21.0 with it).
+template <int KW, int NT, bool AHEAD>
+__global__ void __launch_bounds__(32 * kWarps, NT == 1 ? (AHEAD ? 3 : 4) : 2) glinear_rows_kernel(const vila_glinear_params p, const vila_glinear_ext x) {
   __shared__ float red[KW * 8 * NT * (kRowsOf(KW) + 4)];
   const int g = blockIdx.y, n0 = blockIdx.x * kRowsOf(KW);
   const int begin = p.mode == 0 ? 0 : p.seg[g], end = p.mode == 0 ? p.M : p.seg[g + 1];
   for (int m0 = begin; m0 < end; m0 += 8 * NT) {
     if (m0 > begin) __syncthreads();                      // the pass before has been read
-    rows_pass<KW, NT>(p, x, g, n0, m0, min(8 * NT, end - m0), red);
+    rows_pass<KW, NT, AHEAD>(p, x, g, n0, m0, min(8 * NT, end - m0), red);
   }
 }
 
@@ -368,7 +382,9 @@ int launch_stream(const vila_glinear_params& p, const vila_glinear_ext& x, cudaS
 template <int KW, int NT>
 int launch_rows(const vila_glinear_params& p, const vila_glinear_ext& x, cudaStream_t stream) {
   const dim3 grid((p.N + kRowsOf(KW) - 1) / kRowsOf(KW), p.groups);
-  VB_CUDA(launch_serial(glinear_rows_kernel<KW, NT>, grid, dim3(32 * kWarps), 0, stream, p, x));
+  constexpr bool kAhead = NT == 1;
+  if (kAhead && p.K > 64 * KW && static_cast<long>(grid.x) * grid.y <= 3L * num_sms()) VB_CUDA(launch_serial(glinear_rows_kernel<KW, NT, kAhead>, grid, dim3(32 * kWarps), 0, stream, p, x));
+  else VB_CUDA(launch_serial(glinear_rows_kernel<KW, NT, false>, grid, dim3(32 * kWarps), 0, stream, p, x));
   return 0;
 }
 template <int KW>
@@ -388,13 +404,18 @@ bool glinear_rows_takes(const vila_glinear_params& p) {
 // CTAs that stay take what streams long enough to pay for their start (token rows, pass list: 1 - 2 us): one layer of 2048
 // columns and more (8 rows x 2048 x 4096: 7.2 us, 13 in the other form; 1024 x 1024: 4.1, 3.6) or of 16 M weights (4 x 32768 x
 // 1024: 14.6, 19.5), routed passes of 1024 columns and 4 M weights (8 x 4 pairs x 1408 x 2048: 23.7, 28; one token's two
-// pairs x 1024 x 1024: 5.7, 5.2; 704 columns: 21, 19.5).  16 warps a tile where rows are long or tiles few, else 8 (16 x 32768
-// x 2048: 34 and 29; 8 x 65536 x 4096: 86 and 89).
+// pairs x 1024 x 1024: 5.7, 5.2; 704 columns: 21, 19.5) unless the SMs hold all tiles of all groups at once and a group has four
+// pairs on average or fewer (1 - 16 pairs of 4 experts x 512 x 2048: 5.0 - 5.5 there, 5.8 - 7.5).  16 warps a tile where rows are long or tiles few, else 8 (16 x 32768
+// x 2048: 34 and 29; 8 x 65536 x 4096: 86 and 89).  The other form: 8 warps a tile, 4 for rows of up to 128 columns,
+// and of up to 256 where outputs are many (512 | 8192 outputs on one row 2.4 | 3.5 us with 8, 2.5 | 3.3 with 4, on 16 rows
+// 2.4 | 5.1 and 2.9 | 3.9; 2048 x 128 on 4 rows 2.4 and 2.3).
 int glinear_rows(const vila_glinear_params& p, cudaStream_t stream, const vila_glinear_ext& x) {
   const long weights = static_cast<long>(p.N) * p.K;
-  const bool stay = p.mode != 0 ? p.K >= 1024 && weights * min(p.M, p.groups) >= 4L << 20 : p.groups == 1 && (p.K >= 2048 || weights >= 16L << 20);
+  const long tiles = static_cast<long>((p.N + 15) / 16) * p.groups;
+  const bool few = tiles <= 3L * num_sms() && p.M <= 4 * p.groups;
+  const bool stay = p.mode != 0 ? p.K >= 1024 && weights * min(p.M, p.groups) >= 4L << 20 && !few : p.groups == 1 && (p.K >= 2048 || weights >= 16L << 20);
   if (stay) return p.K >= 4096 || (p.mode == 0 && p.N <= 16 * num_sms()) ? launch_stream<16>(p, x, stream) : launch_stream<8>(p, x, stream);
-  return p.K <= 256 ? launch<4>(p, x, stream) : launch<8>(p, x, stream);
+  return p.K <= 128 || (p.K <= 256 && static_cast<long>(p.N) * p.groups >= 4096) ? launch<4>(p, x, stream) : launch<8>(p, x, stream);
 }
 
 }  // namespace vb
