@@ -338,8 +338,9 @@ int vila_gated_norm_residual(float* x, const void* part, int part_dtype, int64_t
                              int bias_dtype, const void* w, int w_dtype, float w_offset, float eps,
                              int rows, int cols, void* stream);
 
-/* vila_glinear — any-shape (grouped) linear layer with fp32 accumulation (bf16 operands on 16-byte boundaries, N >= 128 and
- * more than 16 rows or 64 routed pairs: tcgen05, otherwise CUDA cores):
+/* vila_glinear — any-shape (grouped) linear layer with fp32 accumulation (bf16 operands on 16-byte boundaries and N >= 128:
+ * tcgen05 for more than 16 rows or 64 routed pairs, mma.sync with every 16 products in a fresh sum for fewer; otherwise
+ * CUDA cores):
  *   out = act(a · w[g]^T + bias[g]) (* row_scale)
  * mode 0 (batched): every group g sees all M rows; its A columns start at g * a_group_off and its
  *   output columns at g * o_group_off (per-head projections); groups == 1 is a plain linear layer.

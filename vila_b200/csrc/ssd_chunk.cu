@@ -8,7 +8,8 @@
 // cut into three bf16 parts (8 + 8 + 8 bits) whose products with a bf16 number are exact.  The tensor core truncates as it
 // accumulates: products of full size go into fresh sums of 16 terms (64 for the update), which join by rounded additions.
 // c is summed in 64 bits and kept in two fp32 numbers, so that exp(c_i - c_j) has the rounding of the difference only.
-// Relative error against float64, 2048 rows, 64 heads of 64 x 128: rows 8.3e-8, state 6.8e-8 (token by token 8.6e-8, 8.5e-8).
+// Relative error against float64, 2048 rows, 64 heads of 64 x 128: rows 8.3e-8, state 6.8e-8 (token by token 8.6e-8, 8.5e-8);
+// where x, B, C and the state have one sign, so that truncations add up: 8.7e-8, 7.9e-8 (8.7e-8, 9.5e-8).
 //
 // Grid (sequence, head, 16 PT columns of P): a CTA walks the chunks of its sequence in order.
 //   warps 0 - 7    hold the state in mma fragments (16 columns x N PT / 8 channels a warp: the accumulator layout of the update
@@ -26,7 +27,7 @@
 // how many others the launch has.
 //
 // 2048 rows of one sequence: 64 heads of 64 x 128 in 114 us (token by token, bound by instruction issue: 300), 32 heads 98
-// (212), 128 heads 235 (593).  A chunk takes 5700 clocks: read-out 2400, update 1600, beside them scores and weights 4500,
+// (212), 128 heads 234 (593).  A chunk takes 5700 clocks: read-out 2400, update 1600, beside them scores and weights 4500,
 // rows out 800.  The tensor pipe is busy for 2100 of them and shared memory's for 2700; what is left is latency of the
 // chains load -> products -> parts -> products.  One set of eight warps that did all in turn took 8000 clocks.
 #include <type_traits>

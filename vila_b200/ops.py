@@ -509,7 +509,7 @@ def glinear(a: torch.Tensor, w: torch.Tensor, *, out: Optional[torch.Tensor] = N
             out_rows_total: Optional[int] = None, glu_clamp: Optional[Tuple[float, float]] = None,
             act_params: Optional[Tuple[float, float]] = None, in_scale: Optional[torch.Tensor] = None,
             geglu: bool = False) -> torch.Tensor:
-    """Any-shape (grouped) linear layer, fp32 accumulation on the CUDA cores (vila_glinear).
+    """Any-shape (grouped) linear layer, fp32 accumulation (vila_glinear; the header says on which cores).
     w [N, K] (groups == 1) or [groups, N, K].  Batched groups (seg None): group g reads the A columns
     [g * a_group_off, + K) and writes the output columns [g * o_group_off, + N).  Segmented (seg int32
     [groups + 1]): the rows of group g are the sorted positions seg[g]..seg[g+1]; see the header.
