@@ -358,6 +358,14 @@ def test_paged_attention_scores_around_the_cap(ops, cap, max_rows, talk):
         assert torch.equal(ops.paged_attention(q, pool, tables, other, **kw)[5:], got[5:])
 
 
+@pytest.mark.parametrize("max_rows,talk", [(16, False), (1, False), (16, True)])
+def test_paged_attention_scores_far_above_the_cap(ops, max_rows, talk):
+    """scores whose exponential is infinite are the cap itself"""
+    form = dict(softcap=5.0, **(dict(talk=True) if talk else {}))
+    got, want, _ = attention_case(ops, form, 8, 2, 128, 128, 64, [(40, 30)], seed=4, scale=1e25, max_rows=max_rows)
+    assert torch.isfinite(got).all() and rel(got, want) < 3e-6
+
+
 @pytest.mark.parametrize("max_rows,nsplit", [(16, 1), (1, 1), (1, 8)])
 def test_paged_attention_sink_switched_off(ops, max_rows, nsplit):
     """a sink of -inf (or below every score) adds nothing to a head's sum; the other heads keep theirs"""
