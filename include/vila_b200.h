@@ -116,11 +116,12 @@ typedef struct vila_fmha_params {
   float scale;
 } vila_fmha_params;
 int vila_fmha(const vila_fmha_params* p, void* stream);
-/* test hook (like vila_linear_cfg): same, forcing the kernel flavour instead of the size heuristic:
- *   0 heuristic; 1 one query tile per CTA (fmha_fwd_kernel); 2 two query tiles per CTA with ping-pong
- *   softmax warpgroups and the O accumulator in TMEM (fmha2_fwd_kernel; needs Sq > 128, D in 72..96 or 128);
- *   3 / 4: as 2 with every 4th / every 2nd exponential as an FMA-pipe polynomial (measured slower) */
+/* test hook (like vila_linear_cfg): same, forcing the form instead of the size heuristic (D 64, 65 .. 96 or 128):
+ *   0 heuristic; 1 one query tile at a time; 2 two query tiles, whose softmax and products alternate (one where Sq <= 128);
+ *   3 / 4: as 2 */
 int vila_fmha_cfg(int variant, const vila_fmha_params* p, void* stream);
+/* the same with waits that end after `tries` tries (test hook: 0 gives up at once, see vila_wait_status). */
+int vila_fmha_tries(int variant, const vila_fmha_params* p, int tries, void* stream);
 
 /* im2col for Conv2d(3,1152,k=14,s=14) (modeling_siglip.py:269-275): pixels [B,C,H,W] ->
  * out [B*(H/P)*(W/P), k_pad], column = (c, ky, kx); columns >= C*P*P are zero. */
@@ -369,9 +370,9 @@ int vila_glinear(const vila_glinear_params* p, void* stream);
 /* CTAs of vila_glinear's tensor-core kernel that gave up a wait since the process started on the current device (0 in a
  * correct run; the launch's output is then incomplete).  Synchronises; -1: could not be read. */
 int vila_stalled_waits(void);
-/* 0, or 1 once after a launch of that kernel which had to give up (vila_last_error says so).  Reads a word of host memory
- * and does not synchronise: after a synchronisation it speaks for everything launched before.  vila_glinear returns the
- * same error before it launches anything. */
+/* 0, or 1 once after a launch of that kernel or of vila_fmha which had to give up (vila_last_error says so).  Reads a word
+ * of host memory and does not synchronise: after a synchronisation it speaks for everything launched before.  vila_glinear
+ * and vila_fmha return the same error before they launch anything. */
 int vila_wait_status(void);
 /* vila_glinear on its tensor-core kernel with waits that end after `tries` tries (test hook: 0 gives up at once). */
 int vila_glinear_tries(const vila_glinear_params* p, int tries, void* stream);

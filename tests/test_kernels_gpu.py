@@ -357,7 +357,7 @@ def test_fmha_paged(cuda):
     assert rel_err(out, ref) < 1.5e-2
 
 
-# ---- the two-tile kernel (fmha2_fwd_kernel: ping-pong softmax warpgroups, O in TMEM with lazy rescale)
+# ---- one and two query tiles at a time (fmha_pipe_kernel: O in TMEM with lazy rescale)
 # forced through vila_fmha_cfg(variant=2); the heuristic only picks it once 256-row CTAs fill 148 SMs --
 @pytest.mark.parametrize("B", [1, 8, 64])
 def test_fmha2_noncausal_siglip(cuda, B):
@@ -419,10 +419,61 @@ def test_fmha2_lazy_rescale_growing_maxima(cuda):
         k = bf(torch.randn(S, Hkv, D, device=cuda, generator=g) * ramp)
         v = bf(torch.randn(S, Hkv, D, device=cuda, generator=g))
         ref = ref_attention(q[None], k[None], v[None], causal, D ** -0.5)[0]
-        for variant in (1, 2, 3, 4):  # 3 / 4: two-tile kernel with every 4th / 2nd exp2 as a polynomial
+        for variant in (1, 2, 3, 4):  # 3 / 4: as 2
             out = ops.fmha(q, k, v, B=1, Sq=S, Sk=S, causal=causal, scale=D ** -0.5, variant=variant)
             assert torch.isfinite(out.float()).all()
             report_rel(f"fmha{variant} growing maxima d={D}", out, ref, 1.5e-2)
+
+
+@pytest.mark.parametrize("D", [64, 72, 80, 88, 96, 128])
+@pytest.mark.parametrize("variant", [1, 2])
+def test_fmha_edges_of_tiles(cuda, D, variant):
+    """rows, keys and heads where the tiles, the halves of a key block and the rounds of the persistent CTAs end"""
+    from tests.helpers import report_rel
+    ops = _ops()
+    for (B, Sq, Sk, Hq, Hkv, causal) in [(1, 1, 1, 1, 1, False), (2, 128, 128, 4, 2, True), (1, 129, 193, 4, 1, True),
+                                         (2, 40, 65, 4, 4, False), (1, 257, 257, 2, 1, True), (2, 130, 64, 4, 2, False),
+                                         (5, 385, 385, 40, 8, True), (3, 513, 200, 32, 32, False),
+                                         (9, 513, 100, 32, 32, False)]:
+        if D == 64 and variant == 2 and Sq == 1:
+            continue
+        g = torch.Generator(device="cuda").manual_seed(D + Sq)
+        q, k, v = (bf(torch.randn(B * S, H, D, device=cuda, generator=g)) for S, H in ((Sq, Hq), (Sk, Hkv), (Sk, Hkv)))
+        ref = ref_attention(q.view(B, Sq, Hq, D), k.view(B, Sk, Hkv, D), v.view(B, Sk, Hkv, D), causal, D ** -0.5)
+        out = ops.fmha(q, k, v, B=B, Sq=Sq, Sk=Sk, causal=causal, scale=D ** -0.5, variant=variant)
+        report_rel(f"fmha{variant} d={D} B={B} {Sq}x{Sk}", out.view(B, Sq, Hq, D), ref, 1.5e-2)
+        assert torch.equal(out, ops.fmha(q, k, v, B=B, Sq=Sq, Sk=Sk, causal=causal, scale=D ** -0.5, variant=variant))
+
+
+@pytest.mark.parametrize("variant", [1, 2])
+def test_fmha_waits_that_run_out_are_reported(cuda, monkeypatch, variant):
+    """waits of 0 tries give up at once, few tries somewhere under way: the launch ends, the next status says so once"""
+    from vila_b200 import _lib
+    ops, lib = _ops(), _lib.load()
+    g = torch.Generator(device="cuda").manual_seed(3)
+    q, k, v = (bf(torch.randn(600, 16, 128, device=cuda, generator=g)) for _ in range(3))
+
+    def limited(tries):
+        with monkeypatch.context() as m:
+            m.setattr(lib, "vila_fmha_cfg", lambda n, p, stream: lib.vila_fmha_tries(n, p, tries, stream))
+            out = ops.fmha(q, k, v, B=1, Sq=600, Sk=600, causal=True, scale=0.1, variant=variant)
+        torch.cuda.synchronize()
+        return out
+
+    want = limited(1 << 20)
+    ops.check_waits()
+    for tries in (0, 1, 3, 30):
+        out = limited(tries)
+        if tries == 0 or not torch.equal(out, want):
+            with pytest.raises(RuntimeError, match="ran out"):
+                ops.check_waits()
+        else:
+            lib.vila_wait_status()
+        ops.check_waits()
+    limited(0)
+    with pytest.raises(RuntimeError, match="ran out"):
+        ops.fmha(q, k, v, B=1, Sq=600, Sk=600, causal=True, scale=0.1)   # the next call says so as well
+    assert torch.equal(limited(1 << 20), want)
 
 
 # ------------------------------------------------------------------------------------------------

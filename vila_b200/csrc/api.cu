@@ -146,6 +146,11 @@ int vila_fmha_cfg(int variant, const vila_fmha_params* p, void* stream) {
   return vb::fmha_prefill_cfg(variant, to_fmha(p), st(stream));
 }
 
+int vila_fmha_tries(int variant, const vila_fmha_params* p, int tries, void* stream) {
+  VB_REQUIRE_DEVICE();
+  return vb::fmha_prefill_cfg(variant, to_fmha(p), st(stream), tries);
+}
+
 int vila_patch_im2col(const void* pixels, void* out, int B, int C, int H, int W, int patch,
                       int k_pad, void* stream) {
   VB_REQUIRE_DEVICE();

@@ -171,6 +171,24 @@ __device__ __forceinline__ void mbar_wait(uint64_t* bar, uint32_t parity) {
   }
 }
 
+// An mbarrier wait that ends: a lost arrival must not leave the GPU spinning.  The first wait of a CTA that runs out of
+// tries sets `gave_up`, which ends the other warps' waits; a warp whose wait failed leaves its loop for the CTA's last
+// barrier (or, where warps meet at other barriers on the way, runs it to its end without waiting).
+constexpr int kTries = 1 << 20;        // of a wait, then the launch gives up
+constexpr int kDrainTries = 1 << 14;   // of a wait for what is still in flight after that
+__device__ __forceinline__ bool mbar_wait_limited(uint64_t* bar, uint32_t parity, volatile int* gave_up, int tries) {
+  for (int i = 0; i < tries; ++i) {
+    if (mbar_try_wait(bar, parity)) return true;
+    if (*gave_up) return false;
+  }
+  *gave_up = 1;
+  return false;
+}
+__device__ __forceinline__ void mbar_drain(uint64_t* bar, uint32_t parity) {
+  for (int i = 0; i < kDrainTries; ++i)
+    if (mbar_try_wait(bar, parity)) return;
+}
+
 // ----------------------------------------------------------------------------------------------
 // TMA (cp.async.bulk.tensor) — loads arrive on an mbarrier with complete_tx::bytes
 // ----------------------------------------------------------------------------------------------
@@ -248,6 +266,20 @@ __device__ __forceinline__ void umma_f16(uint32_t d_tmem, uint64_t a_desc, uint6
       "}\n"
       :
       : "r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
+
+// the same with A in TMEM: 128 lanes x 16 bf16 in 8 columns from a_tmem on
+__device__ __forceinline__ void umma_f16_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc,
+                                            uint32_t accumulate) {
+  asm volatile(
+      "{\n\t"
+      ".reg .pred p;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t"
+      "}\n"
+      :
+      : "r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate)
       : "memory");
 }
 

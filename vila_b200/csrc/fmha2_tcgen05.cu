@@ -1,18 +1,31 @@
-// Flash-attention forward v2 for sm_100a: TWO 128-row query tiles per CTA with ping-pong softmax
-// warpgroups, so the tensor core works on one tile while the other tile's softmax runs.
+// Flash-attention forward for sm_100a: one persistent CTA per SM walks units of one or two 128-row query tiles.
 //
-//   warps 0-3  (WG0): softmax + O accumulation of query tile 0   (thread == query row == TMEM lane)
-//   warps 4-7  (WG1): the same for query tile 1
-//   warp  8        : TMA producer — Q0,Q1 once, then ONE ring over the sequence K0,V0,K1,V1,...
-//   warp  9        : tcgen05.mma issuer + TMEM allocator
-//   TMEM: S0 @0, S1 @128 (fp32 128x128 each), O0 @256, O1 @384
-//   MMA issue order per KV block j:  PV0(j) S0(j+1) PV1(j) S1(j+1)  — each softmax warpgroup always
-//   has its next S tile being computed while it accumulates O, and the tensor pipe alternates tiles.
+//   warps 0 - 7 (and 8 - 15)  softmax of query tile 0 (and 1): eight warps a tile, two threads a row (keys 0 - 63 and 64 - 127
+//                             of a block), so that four warps per scheduler hide the latency of the loads, the row maxima and
+//                             the exponentials; with one thread a row the exponential unit was busy for 40 % of the time
+//   next two warps            TMA: Q tiles, and ONE ring over the sequence K0, V0, K1, V1, ...; rows of O
+//   last one or two warps     a tile's tcgen05.mma issuer (one issuer for both tiles was what the kernel waited for)
+//   TMEM: scores at 0 and 128 (fp32 128 x 128 each), O of tile 0 / 1 at 256 / 384
 //
-// Same math / rounding as v1 (fmha_tcgen05.cu): S = QK^T in fp32, online softmax in fp32 with exp2,
-// P cast to bf16 for the PV MMA, O accumulated in TMEM by the PV MMA itself with a lazy (exact)
-// rescale when a row maximum moves by more than 2^8, d=72 zero-padded to 96
-// by TMA OOB fill (SW64 chunks), d=128 as two SW128 chunks, V consumed as the MN-major B operand.
+// The weights go back to TMEM as bf16 over the scores that they come from and are the A operand of the PV product from
+// there: in shared memory they cost its port 48 KB a block beside the 64 KB of the operands and the 32 KB that arrive.
+//   two tiles: each PV(j) S(j+1) in turn: the tensor pipe works on one tile under the other's softmax
+//   one tile:  S(j+1) PV(j): two score buffers, taken in turn
+// The products of one thread execute in order, so scores may follow the weights that a product issued before still reads.
+// Descriptors are a base plus constants: made anew for every instruction, the issue alone took 85 clocks of the 64 that a
+// product of 128 x 128 x 16 needs.
+//
+// Bound by the chain of a tile (two tiles: scores 500 clocks at 128 columns, maxima and exponentials 1500, product 500) and by
+// the exponential unit (1024 a tile and block).  Before (four softmax warps a tile, weights through shared memory, one CTA a
+// pair of tiles): 16 heads of 72 columns, 1024 x 1024, 1 / 4 / 13 images 20.4 / 46.8 / 136.8 us, now 16.8 / 44.0 / 114.1; causal,
+// 28 heads of 128 over 4, 279 / 1024 / 2500 / 8000 / 16470 rows 9.8 / 33 / 91 / 550 / 1955, now 7.5 / 14.2 / 49.7 / 384 / 1545 (1260 TFLOP/s).
+//
+// S = QK^T in fp32, online softmax in fp32 with exp2, P rounded to bf16 for PV, O accumulated in TMEM by the PV product
+// itself with a lazy (exact) rescale when a row maximum moves by more than 2^8.  D = 65 .. 96 zero-padded by TMA fill (SW64
+// chunks of 32 columns; up to 80 columns products stop there), D = 64 and 128 as SW128 chunks, V the MN-major B operand.
+//
+// Replaces flash_attn_func in SiglipFlashAttention2 (modeling_siglip.py:583-585, non-causal, scale 72^-0.5) and HF
+// _flash_attention_forward for Qwen2 (modeling_qwen2.py:191-310; causal GQA).
 #include <math.h>
 
 #include "common.cuh"
@@ -23,20 +36,23 @@ namespace {
 
 constexpr int BQ = 128;
 constexpr int BKV = 128;
-constexpr int kThreads2 = 320;
 
-template <int DP, int CW>
-struct Cfg2 {
-  static constexpr int kChunks = DP / CW;
+template <int DP, int CW, int TILES>
+struct Shape {
+  static constexpr int kChunks = (DP + CW - 1) / CW;
   static constexpr int kChunkBytes = 128 * CW * 2;
   static constexpr int kTileBytes = kChunks * kChunkBytes;  // one 128-row Q / K / V tile
   static constexpr uint32_t kLayout = CW == 64 ? kLayoutSW128 : kLayoutSW64;
   static constexpr int kSwizzleBytes = CW * 2;
   static constexpr int kSBO = 8 * CW * 2;
-  static constexpr int kPBytes = BQ * BKV * 2;
-  static constexpr int kRing = DP == 128 ? 3 : 4;  // K/V ring slots
-  static constexpr int kNumBars = 2 + 2 * kRing + 12;
-  static constexpr int kSmem = 2 * kTileBytes + kRing * kTileBytes + 2 * kPBytes + kNumBars * 8 + 16 + 1024;
+  static constexpr int kQ = TILES == 2 && DP == 128 ? 1 : 2;   // Q buffers of a tile: the next unit's arrives under this one's products
+  static constexpr int kRing = DP == 128 ? 4 : 5;           // K / V slots
+  static constexpr int kSoftmaxWarps = 8 * TILES;
+  static constexpr int kProducer = kSoftmaxWarps, kStore = kProducer + 1, kMma = kStore + 1;   // warps
+  static constexpr int kThreads = 32 * (kMma + TILES);
+  static constexpr int kHalf = DP / 2;                      // O columns of a thread
+  static constexpr int kNumBars = 2 * kRing + 6 * kQ + 10;
+  static constexpr int kSmem = (TILES * kQ + kRing) * kTileBytes + TILES * 2 * 2 * BQ * 4 + kNumBars * 8 + 16 + 1024;
 };
 
 __device__ __forceinline__ float ex2f(float x) {
@@ -44,28 +60,7 @@ __device__ __forceinline__ float ex2f(float x) {
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
   return y;
 }
-
-// exp2 on the FMA pipe (Cody-Waite split + degree-3 minimax polynomial, max relative error 7.5e-5,
-// far below the bf16 rounding P gets anyway).  On B200 MUFU.EX2 runs at 16 lanes/clk/SM: the 2 x 16K
-// exponentials of one KV block (two query tiles) take as long as its four 128x128x128 MMAs, so the
-// softmax warpgroups and the tensor pipe are co-limiting; moving every 4th exponential to the FMA
-// pipe takes the MUFU below the MMA time.
-__device__ __forceinline__ float ex2_poly(float x) {
-  x = fmaxf(x, -125.f);
-  const float xf = x + 12582912.f;          // 1.5 * 2^23: rounds x to an integer in the low mantissa bits
-  const float fr = x - (xf - 12582912.f);   // fractional part in [-0.5, 0.5]
-  float p = fmaf(fr, 0.0551716685f, 0.2426111251f);
-  p = fmaf(fr, p, 0.6932609677f);
-  p = fmaf(fr, p, 0.9999280572f);
-  return __int_as_float(__float_as_int(p) + (__float_as_int(xf) << 23));
-}
-// kPolyEvery (template parameter): every n-th exponential of a row uses ex2_poly (0: none).  MEASURED
-// (tools/bench_fmha.py, S = 65.8K causal): 0 -> 963 TF/s, 4 -> 884, 2 -> 830: the softmax warps are
-// issue-slot bound as much as MUFU bound, the ~10-instruction polynomial costs more than it frees.
-// It stays as a selectable flavour (vila_fmha_cfg 3 / 4); the default is 0.
-
-// Blackwell packed fp32 (two lanes per instruction: FFMA2 / FADD2) and 3-input max (FMNMX3): the
-// softmax loop is issue-slot bound, these halve its arithmetic instruction count.
+// packed fp32 and 3-input maximum: half the instructions of the softmax
 __device__ __forceinline__ void ffma2(float& d0, float& d1, float a0, float a1, float b, float c) {
   asm("{.reg .b64 ra, rb, rc, rd; mov.b64 ra, {%2,%3}; mov.b64 rb, {%4,%4}; mov.b64 rc, {%5,%5}; "
       "fma.rn.f32x2 rd, ra, rb, rc; mov.b64 {%0,%1}, rd;}"
@@ -83,85 +78,87 @@ __device__ __forceinline__ float fmax3(float a, float b, float c) {
   asm("max.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
   return d;
 }
+// the two warps that share 32 rows meet at barrier id; true if any of their threads says so
+__device__ __forceinline__ bool pair_any(int id, bool v) {
+  uint32_t r;
+  asm volatile(
+      "{.reg .pred p, q; setp.ne.b32 p, %1, 0; bar.red.or.pred q, %2, 64, p; selp.u32 %0, 1, 0, q;}"
+      : "=r"(r)
+      : "r"(v ? 1u : 0u), "r"(id)
+      : "memory");
+  return r != 0;
+}
+// a chunk of O from shared memory; the tensor's ends are not written past
+__device__ __forceinline__ void store_chunk(const CUtensorMap* m, uint32_t src, int c0, int h, int row, int b) {
+  asm volatile("cp.async.bulk.tensor.4d.global.shared::cta.bulk_group [%0, {%2, %3, %4, %5}], [%1];" ::"l"(
+                   reinterpret_cast<uint64_t>(m)),
+               "r"(src), "r"(c0), "r"(h), "r"(row), "r"(b)
+               : "memory");
+}
+__device__ __forceinline__ void pair_sync(int id) { asm volatile("bar.sync %0, 64;" ::"r"(id) : "memory"); }
 
-struct Args2 {
-  __nv_bfloat16* o;
-  int64_t o_tok_stride, o_head_stride;
+struct Args {
   const int32_t* page_table;
   int page_table_stride;
-  int Sq, Sk, Hq, Hkv, D, causal, paged;
+  int Sq, Sk, Hq, Hkv, D, causal, paged, B;
+  int units;                  // query units (of TILES tiles) of a sequence and head
   float scale_log2;
 };
 
-template <int DP, int CW, int kPolyEvery>
-__global__ void __launch_bounds__(kThreads2, 1)
-fmha2_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
-                 const __grid_constant__ CUtensorMap tm_v, Args2 a) {
-  using C = Cfg2<DP, CW>;
+template <int DP, int CW, int TILES>
+__global__ void __launch_bounds__(Shape<DP, CW, TILES>::kThreads, 1)
+fmha_pipe_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
+                 const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_o, const Args a, int tries, volatile unsigned int* failed) {
+  using C = Shape<DP, CW, TILES>;
   constexpr int R = C::kRing;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
                                              ~static_cast<uintptr_t>(1023));
-  uint8_t* q_s = smem;                              // 2 tiles
-  uint8_t* ring_s = q_s + 2 * C::kTileBytes;        // R tiles
-  uint8_t* p_s = ring_s + R * C::kTileBytes;        // 2 x [128][128] bf16
-  uint64_t* bars = reinterpret_cast<uint64_t*>(p_s + 2 * C::kPBytes);
-  uint64_t* q_full = bars;                 // [2]
-  uint64_t* r_full = bars + 2;             // [R]
-  uint64_t* r_empty = bars + 2 + R;        // [R]
-  uint64_t* s_full = bars + 2 + 2 * R;     // [2]
-  uint64_t* s_free = s_full + 2;           // [2]
-  uint64_t* p_full = s_full + 4;           // [2]
-  uint64_t* p_free = s_full + 6;           // [2]
-  uint64_t* o_full = s_full + 8;           // [2]
-  uint64_t* o_free = s_full + 10;          // [2]
-  uint32_t* tmem_ptr = reinterpret_cast<uint32_t*>(s_full + 12);
+  uint8_t* q_s = smem;                                  // [tile][buffer]
+  uint8_t* ring_s = q_s + TILES * C::kQ * C::kTileBytes;
+  float* xm = reinterpret_cast<float*>(ring_s + R * C::kTileBytes);   // [tile][half][row] maxima, then sums
+  float* xl = xm + TILES * 2 * BQ;
+  uint64_t* r_full = reinterpret_cast<uint64_t*>(xl + TILES * 2 * BQ);   // [R]
+  uint64_t* r_empty = r_full + R;                       // [R]
+  uint64_t* q_full = r_empty + R;                       // [tile][buffer]
+  uint64_t* q_empty = q_full + 2 * C::kQ;               // [tile][buffer]
+  uint64_t* s_full = q_empty + 2 * C::kQ;               // [2]: by score buffer
+  uint64_t* p_full = s_full + 2;                        // [2]
+  uint64_t* o_full = p_full + 2;                        // [2]: by tile
+  uint64_t* o_free = o_full + 2;                        // [2]
+  uint64_t* o_ready = o_free + 2;                       // [tile][buffer]: rows stand in the Q buffer
+  uint64_t* fin = o_ready + 2 * C::kQ;                  // [2]
+  uint32_t* tmem_ptr = reinterpret_cast<uint32_t*>(fin + 2);
+  volatile int* gave_up = reinterpret_cast<int*>(tmem_ptr + 1);
 
-  const int warp = threadIdx.x >> 5;
+  const int warp = __shfl_sync(0xffffffffu, static_cast<int>(threadIdx.x) >> 5, 0);   // known to be the same for a warp
   const int lane = threadIdx.x & 31;
-  const int h = blockIdx.y;
-  const int b = blockIdx.z;
-  const int hk = h / (a.Hq / a.Hkv);
   const int off = a.Sk - a.Sq;
-  // causal: CTAs are dispatched in blockIdx order, so map the FIRST CTAs to the LAST (longest-KV)
-  // query tiles — the tail of the grid is then made of the cheapest tiles
-  const int qpair = a.causal ? static_cast<int>(gridDim.x) - 1 - static_cast<int>(blockIdx.x)
-                             : static_cast<int>(blockIdx.x);
-
-  int nblk[2];
-#pragma unroll
-  for (int t = 0; t < 2; ++t) {
-    const int qt = qpair * 2 + t;
-    int n = 0;
-    if (qt * BQ < a.Sq) {
-      int kv_end = a.Sk;
-      if (a.causal) {
-        const int q_last = min((qt + 1) * BQ, a.Sq) - 1;
-        kv_end = min(a.Sk, q_last + off + 1);
-      }
-      n = (kv_end + BKV - 1) / BKV;
-    }
-    nblk[t] = n;
-  }
-  const int nmax = max(nblk[0], nblk[1]);
+  const int heads = a.Hq * a.B;
+  const int total = a.units * heads;
 
   if (threadIdx.x == 0) {
-    for (int i = 0; i < 2; ++i) {
-      mbar_init(&q_full[i], 1);
-      mbar_init(&s_full[i], 1);
-      mbar_init(&s_free[i], 128);
-      mbar_init(&p_full[i], 128);
-      mbar_init(&p_free[i], 1);
-      mbar_init(&o_full[i], 1);
-      mbar_init(&o_free[i], 128);
-    }
     for (int i = 0; i < R; ++i) {
       mbar_init(&r_full[i], 1);
-      mbar_init(&r_empty[i], 1);
+      mbar_init(&r_empty[i], TILES);
     }
+    for (int i = 0; i < 2; ++i) {
+      mbar_init(&s_full[i], 1);
+      mbar_init(&p_full[i], 8);
+      mbar_init(&o_full[i], 1);
+      mbar_init(&o_free[i], 8);
+    }
+    for (int i = 0; i < 2 * C::kQ; ++i) {
+      mbar_init(&q_full[i], 1);
+      mbar_init(&q_empty[i], 1);
+      mbar_init(&o_ready[i], 8);
+    }
+    mbar_init(&fin[0], 1);
+    mbar_init(&fin[1], 1);
+    *gave_up = 0;
     fence_barrier_init();
   }
-  if (warp == 9) tmem_alloc<512>(tmem_ptr);
+  if (warp == C::kMma) tmem_alloc<512>(tmem_ptr);
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
@@ -169,268 +166,372 @@ fmha2_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
   griddep_launch_dependents();
   griddep_wait();
 
-  if (warp == 8) {
+  // The CTA's units in turn.  Causal: the longest first, and back and forth over the CTAs from round to round, so that each
+  // gets about the same; otherwise the units of a head next to each other.
+  struct Unit {
+    int u, h, b, n[2], nmax;
+  };
+  auto unit = [&](int round, Unit& w) {
+    const int g = static_cast<int>(gridDim.x), c = static_cast<int>(blockIdx.x);
+    const int i = round * g + ((round & 1) ? g - 1 - c : c);
+    if (i >= total) return false;
+    int hb;
+    if (a.causal) {
+      w.u = a.units - 1 - i / heads;
+      hb = i % heads;
+    } else {
+      w.u = i % a.units;
+      hb = i / a.units;
+    }
+    w.b = hb / a.Hq;
+    w.h = hb - w.b * a.Hq;
+    w.nmax = 0;
+#pragma unroll
+    for (int t = 0; t < 2; ++t) {
+      const int q0 = (w.u * TILES + t) * BQ;
+      int n = 0;
+      if (t < TILES && q0 < a.Sq) {
+        int kv_end = a.Sk;
+        if (a.causal) kv_end = min(a.Sk, min(q0 + BQ, a.Sq) + off);
+        n = (kv_end + BKV - 1) / BKV;
+      }
+      w.n[t] = n;
+      w.nmax = max(w.nmax, n);
+    }
+    return true;
+  };
+  const int rounds = (total + static_cast<int>(gridDim.x) - 1) / static_cast<int>(gridDim.x);
+
+  // The producer and the issuers run as whole warps whose values are the same in all lanes (they stay in uniform registers) and
+  // elect a lane for what is issued.
+  auto wait = [&](uint64_t* bar, int phase) { return __all_sync(0xffffffffu, mbar_wait_limited(bar, phase & 1, gave_up, tries)); };
+  if (warp == C::kProducer) {
     // ===================== TMA producer =====================
-    if (lane == 0 && nmax > 0) {
+    if (elect_one()) {
       tma_prefetch_desc(&tm_q);
       tma_prefetch_desc(&tm_k);
       tma_prefetch_desc(&tm_v);
-      for (int t = 0; t < 2; ++t) {
-        if (nblk[t] == 0) continue;
-        mbar_arrive_expect_tx(&q_full[t], C::kTileBytes);
-#pragma unroll
-        for (int c = 0; c < C::kChunks; ++c)
-          tma_load_4d(q_s + t * C::kTileBytes + c * C::kChunkBytes, &tm_q, &q_full[t], c * CW, h,
-                      b * a.Sq + (qpair * 2 + t) * BQ, 0);
-      }
-      for (int i = 0; i < 2 * nmax; ++i) {  // item 2j = K(j), 2j+1 = V(j)
-        const int j = i >> 1;
-        const int slot = i % R;
-        int tok, page;
-        if (a.paged) {
-          tok = 0;
-          page = a.page_table ? a.page_table[b * a.page_table_stride + j] : j;
-        } else {
-          tok = b * a.Sk + j * BKV;
-          page = 0;
-        }
-        mbar_wait(&r_empty[slot], ((i / R) & 1) ^ 1);
-        mbar_arrive_expect_tx(&r_full[slot], C::kTileBytes);
-        const CUtensorMap* tm = (i & 1) ? &tm_v : &tm_k;
-#pragma unroll
-        for (int c = 0; c < C::kChunks; ++c)
-          tma_load_4d(ring_s + slot * C::kTileBytes + c * C::kChunkBytes, tm, &r_full[slot], c * CW,
-                      hk, tok, page);
-      }
     }
-  } else if (warp == 9) {
-    // ===================== MMA issuer =====================
-    if (lane == 0 && nmax > 0) {
-      constexpr uint32_t idesc_s = make_idesc_bf16(BQ, BKV, 0, 0);
-      constexpr uint32_t idesc_o = make_idesc_bf16(BQ, DP, 0, 1);
-      auto ring_wait = [&](int i) { mbar_wait(&r_full[i % R], (i / R) & 1); };
-      auto ring_release = [&](int i) { umma_commit(&r_empty[i % R]); };
-      auto issue_s = [&](int t, int j) {  // S_t(j) = Q_t K(j)^T
-        mbar_wait(&s_free[t], (j & 1) ^ 1);
-        tc_fence_after();
-        const uint8_t* ks = ring_s + ((2 * j) % R) * C::kTileBytes;
+    int slot = 0, ph = 1, items = 0, qn[2] = {0, 0};
+    bool ok = true;
+    Unit w;
+    for (int r = 0; ok && r < rounds; ++r) {
+      if (!unit(r, w)) continue;
+      const int hk = w.h / (a.Hq / a.Hkv);
+      auto load = [&](const CUtensorMap* tm, int tok, int page) {
+        ok = wait(&r_empty[slot], ph);
+        if (!ok) return;
+        if (elect_one()) {
+          mbar_arrive_expect_tx(&r_full[slot], C::kTileBytes);
 #pragma unroll
-        for (int c = 0; c < C::kChunks; ++c) {
+          for (int c = 0; c < C::kChunks; ++c)
+            tma_load_4d(ring_s + slot * C::kTileBytes + c * C::kChunkBytes, tm, &r_full[slot], c * CW, hk, tok, page);
+        }
+        ++items;
+        if (++slot == R) {
+          slot = 0;
+          ph ^= 1;
+        }
+      };
+      for (int j = 0; ok && j < w.nmax; ++j) {
+        int tok = 0, page = 0;
+        if (a.paged) page = a.page_table ? a.page_table[w.b * a.page_table_stride + j] : j;
+        else tok = w.b * a.Sk + j * BKV;
+        load(&tm_k, tok, page);
+        if (j == 0) {   // behind the first keys: those wait for a slot only, the queries for the last unit's scores
 #pragma unroll
-          for (int k = 0; k < CW / 16; ++k) {
-            const uint64_t ad = make_smem_desc(
-                smem_u32(q_s + t * C::kTileBytes + c * C::kChunkBytes) + k * 32, 16, C::kSBO, C::kLayout);
-            const uint64_t bd =
-                make_smem_desc(smem_u32(ks + c * C::kChunkBytes) + k * 32, 16, C::kSBO, C::kLayout);
-            umma_f16(tmem_base + t * BKV, ad, bd, idesc_s, (c | k) != 0 ? 1u : 0u);
+          for (int t = 0; t < TILES; ++t) {
+            if (w.n[t] == 0 || !ok) continue;
+            const int qb = qn[t] % C::kQ, at = t * C::kQ + qb;
+            ok = wait(&q_empty[at], qn[t] / C::kQ + 1);
+            if (!ok) continue;
+            if (elect_one()) {
+              mbar_arrive_expect_tx(&q_full[at], C::kTileBytes);
+#pragma unroll
+              for (int c = 0; c < C::kChunks; ++c)
+                tma_load_4d(q_s + at * C::kTileBytes + c * C::kChunkBytes, &tm_q, &q_full[at], c * CW, w.h,
+                            w.b * a.Sq + (w.u * TILES + t) * BQ, 0);
+            }
+            ++qn[t];
           }
         }
-        umma_commit(&s_full[t]);
-      };
-      auto issue_pv = [&](int t, int j) {  // O_t(j) = P_t(j) V(j)
-        mbar_wait(&p_full[t], j & 1);  // also orders this PV after any O rescale of block j
-        tc_fence_after();
-        const uint8_t* vs = ring_s + ((2 * j + 1) % R) * C::kTileBytes;
+        if (ok) load(&tm_v, tok, page);
+      }
+    }
+    if (!ok) {   // copies in flight land before the CTA ends
+      for (int k = max(0, items - R); k < items; ++k) mbar_drain(&r_full[k % R], (k / R) & 1);
+      for (int t = 0; t < TILES; ++t)
+        for (int k = max(0, qn[t] - C::kQ); k < qn[t]; ++k) mbar_drain(&q_full[t * C::kQ + k % C::kQ], (k / C::kQ) & 1);
+    }
+  } else if (warp == C::kStore) {
+    // ===================== rows of O =====================
+    int un[2] = {0, 0};
+    bool ok = true;
+    Unit w;
+    for (int r = 0; ok && r < rounds; ++r) {
+      if (!unit(r, w)) continue;
 #pragma unroll
-        for (int k = 0; k < BKV / 16; ++k) {
-          const uint64_t ad = make_smem_desc(
-              smem_u32(p_s + t * C::kPBytes + (k >> 2) * (BQ * 128)) + (k & 3) * 32, 16, 1024, kLayoutSW128);
-          const uint64_t bd = make_smem_desc(smem_u32(vs) + k * 16 * (CW * 2), C::kChunkBytes, C::kSBO,
-                                             C::kLayout);
-          umma_f16(tmem_base + 256 + t * 128, ad, bd, idesc_o, (j | k) != 0 ? 1u : 0u);
+      for (int t = 0; t < TILES; ++t) {
+        if (w.n[t] == 0 || !ok) continue;
+        const int at = t * C::kQ + un[t] % C::kQ;
+        ok = wait(&o_ready[at], un[t] / C::kQ);
+        if (!ok) continue;
+        if (elect_one()) {
+#pragma unroll
+          for (int c = 0; c < C::kChunks; ++c)
+            if (c * CW < a.D) store_chunk(&tm_o, smem_u32(q_s) + at * C::kTileBytes + c * C::kChunkBytes, c * CW, w.h, (w.u * TILES + t) * BQ, w.b);
+          asm volatile("cp.async.bulk.commit_group;\ncp.async.bulk.wait_group.read 0;" ::: "memory");
+          mbar_arrive(&q_empty[at]);
         }
-        umma_commit(&p_free[t]);
+        __syncwarp();
+        ++un[t];
+      }
+    }
+  } else if (warp >= C::kMma) {
+    // ===================== MMA issuer of tile t =====================
+    const int t = TILES == 2 ? warp - C::kMma : 0;
+    constexpr uint32_t idesc_s = make_idesc_bf16(BQ, BKV, 0, 0);
+    constexpr uint32_t idesc_o = make_idesc_bf16(BQ, DP, 0, 1);
+    constexpr int kSteps = CW / 16, kTile16 = C::kTileBytes >> 4;
+    const uint64_t qd0 = make_smem_desc(smem_u32(q_s) + t * C::kQ * C::kTileBytes, 16, C::kSBO, C::kLayout);
+    const uint64_t kd0 = make_smem_desc(smem_u32(ring_s), 16, C::kSBO, C::kLayout);
+    const uint64_t vd0 = make_smem_desc(smem_u32(ring_s), C::kChunkBytes, C::kSBO, C::kLayout);
+    const uint32_t o_tmem = tmem_base + 256 + t * 128;
+    bool ok = true;
+    int slot = 0, ph = 0, g = 0, units = 0;   // ring; blocks and units of the tile so far
+    auto advance = [&]() {
+      if (++slot == R) {
+        slot = 0;
+        ph ^= 1;
+      }
+    };
+    // scores of block n against the K in `slot`
+    auto issue_s = [&](int n, int slot_k) {
+      tc_fence_after();
+      const int sb = TILES == 2 ? t : n & 1, qb = units % C::kQ;
+      if (elect_one()) {
+        const uint64_t qd = qd0 + static_cast<uint32_t>(qb * kTile16), kd = kd0 + static_cast<uint32_t>(slot_k * kTile16);
+        const uint32_t d = tmem_base + sb * BKV;
+#pragma unroll
+        for (int k = 0; k < DP / 16; ++k) {
+          const int o = (k / kSteps) * (C::kChunkBytes >> 4) + (k % kSteps) * 2;
+          umma_f16(d, qd + o, kd + o, idesc_s, k != 0 ? 1u : 0u);
+        }
+        umma_commit(&s_full[sb]);
+        umma_commit(&r_empty[slot_k]);
+      }
+      __syncwarp();
+    };
+    auto issue_pv = [&](int n, int slot_v, bool first) {
+      tc_fence_after();
+      const int sb = TILES == 2 ? t : n & 1;
+      if (elect_one()) {
+        const uint64_t vd = vd0 + static_cast<uint32_t>(slot_v * kTile16);
+        const uint32_t p = tmem_base + sb * BKV;
+#pragma unroll
+        for (int k = 0; k < BKV / 16; ++k)   // weights of keys 16 k ..: 8 columns, each half's from its own scores' first on
+          umma_f16_ts(o_tmem, p + (k >> 2) * 64 + (k & 3) * 8, vd + k * (16 * CW * 2 >> 4), idesc_o, k != 0 || !first ? 1u : 0u);
         umma_commit(&o_full[t]);
-      };
-      // prologue: S_t(0)
-      ring_wait(0);
-      for (int t = 0; t < 2; ++t) {
-        if (nblk[t] == 0) continue;
-        mbar_wait(&q_full[t], 0);
-        issue_s(t, 0);
+        umma_commit(&r_empty[slot_v]);
       }
-      ring_release(0);
-      for (int j = 0; j < nmax; ++j) {
-        // S(j+1) BEFORE PV(j): the softmax warpgroups release the S buffer as soon as they hold block
-        // j's scores in registers, so the tensor pipe computes Q K(j+1)^T while they exponentiate
-        if (j + 1 < nmax) {
-          ring_wait(2 * (j + 1));                   // K(j+1)
-          for (int t = 0; t < 2; ++t)
-            if (j + 1 < nblk[t]) issue_s(t, j + 1);
-          ring_release(2 * (j + 1));
+      __syncwarp();
+    };
+    Unit w;
+    for (int r = 0; ok && r < rounds; ++r) {
+      if (!unit(r, w)) continue;
+      const int n = TILES == 2 && t == 1 ? w.n[1] : w.n[0];
+      ok = wait(&r_full[slot], ph);
+      if (ok && n > 0) {
+        ok = wait(&q_full[t * C::kQ + units % C::kQ], units / C::kQ);
+        if (ok) issue_s(g, slot);
+      }
+      if (!ok) break;
+      if (n == 0 && elect_one()) mbar_arrive(&r_empty[slot]);
+      advance();
+      for (int j = 0; j < n; ++j, ++g) {
+        const int slot_v = slot, ph_v = ph;
+        advance();
+        const int slot_k = slot, ph_k = ph;
+        const bool more = j + 1 < n;
+        if (TILES == 1 && more) {
+          ok = wait(&r_full[slot_k], ph_k);
+          if (!ok) break;
+          issue_s(g + 1, slot_k);
         }
-        ring_wait(2 * j + 1);                       // V(j)
-        for (int t = 0; t < 2; ++t)
-          if (j < nblk[t]) issue_pv(t, j);
-        ring_release(2 * j + 1);
+        ok = wait(&r_full[slot_v], ph_v) && (TILES == 1 || !more || wait(&r_full[slot_k], ph_k)) && (j > 0 || wait(&o_free[t], units + 1)) &&
+             wait(&p_full[TILES == 2 ? t : g & 1], TILES == 2 ? g : g >> 1);   // also orders this PV after any rescale of block j
+        if (!ok) break;
+        issue_pv(g, slot_v, j == 0);
+        if (TILES == 2 && more) issue_s(g + 1, slot_k);
+        if (more) advance();
       }
+      // blocks that only the other tile sees: K and V from block n on (the first K is counted above)
+      for (int i = n == 0 ? 1 : 2 * n; ok && i < 2 * w.nmax; ++i) {
+        ok = wait(&r_full[slot], ph);
+        if (ok && elect_one()) mbar_arrive(&r_empty[slot]);
+        advance();
+      }
+      if (!ok) break;
+      units += n > 0;
+    }
+    if (!ok) {   // products in flight end before their operands and TMEM go
+      if (elect_one()) umma_commit(&fin[t]);
+      mbar_drain(&fin[t], 0);
     }
   } else {
-    // ===================== softmax warpgroups =====================
-    const int t = warp >> 2;                 // query tile of this warpgroup
-    const int row = threadIdx.x & 127;
-    const int qt = qpair * 2 + t;
-    const int q_idx = qt * BQ + row;
-    const uint32_t lane_addr = static_cast<uint32_t>((warp & 3) * 32) << 16;
-    const int n = nblk[t];
-    uint8_t* my_p = p_s + t * C::kPBytes;
-    // O accumulates in TMEM across KV blocks (the PV MMA runs with accumulate=1).  Each row keeps a
-    // reference maximum m_ref; the accumulator is rescaled (tcgen05.ld -> scale -> tcgen05.st) only
-    // when a row's running maximum exceeds m_ref by more than 2^8 (exact: P, l and O all use the same
-    // m_ref, the final division by l cancels it).  The decision is per warp (TMEM ld/st are
-    // warp-collective on the warp's own 32 lanes).
-    float m_ref = -INFINITY, l = 0.f;
-    const uint32_t o_addr = tmem_base + lane_addr + 256 + t * 128;
-
-    for (int j = 0; j < n; ++j) {
-      mbar_wait(&s_full[t], j & 1);
-      tc_fence_after();
-      const uint32_t s_addr = tmem_base + lane_addr + t * BKV;
-      const int kv0 = j * BKV;
-      const bool need_mask = (kv0 + BKV > a.Sk) || (a.causal && (kv0 + BKV - 1 > qt * BQ + off));
-      const int kv_lim = a.causal ? min(a.Sk - 1, q_idx + off) : a.Sk - 1;
-
-      // the whole 128-column score row of this thread in registers with ONE TMEM round trip, then the
-      // S buffer goes back to the tensor pipe (was: two passes of four dependent 32-column loads)
-      uint32_t r[BKV];
-#pragma unroll
-      for (int c = 0; c < BKV / 32; ++c) tmem_ld_32x32b_x32(s_addr + c * 32, r + c * 32);
-      tmem_ld_wait();
-      tc_fence_before();
-      mbar_arrive(&s_free[t]);
-      float mx = -INFINITY;
-      if (need_mask) {
-#pragma unroll
-        for (int i = 0; i < BKV; ++i) mx = fmaxf(mx, (kv0 + i <= kv_lim) ? __uint_as_float(r[i]) : -INFINITY);
-      } else {
-        // four independent max chains (two warps per scheduler: little latency hiding, so the
-        // dependent chains of the row reductions are kept short)
-        float m4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
-#pragma unroll
-        for (int i = 0; i < BKV; i += 8) {
-#pragma unroll
-          for (int q = 0; q < 4; ++q)
-            m4[q] = fmax3(m4[q], __uint_as_float(r[i + 2 * q]), __uint_as_float(r[i + 2 * q + 1]));
-        }
-        mx = fmaxf(fmaxf(m4[0], m4[1]), fmaxf(m4[2], m4[3]));
-      }
-      const float m_blk = mx * a.scale_log2;
-      if (j == 0) {
-        m_ref = (m_blk == -INFINITY) ? 0.f : m_blk;
-      } else {
-        const bool need = m_blk > m_ref + 8.0f;
-        if (__any_sync(0xffffffffu, need)) {
-          const float m_new = need ? m_blk : m_ref;
-          const float alpha = ex2f(m_ref - m_new);  // 1 for rows that keep their reference
-          mbar_wait(&o_full[t], (j - 1) & 1);       // PV(j-1) has landed in TMEM
-          tc_fence_after();
-          // rare path (a row maximum moved by more than 2^8): 8 columns at a time so that it adds no
-          // register pressure to the hot loop, which holds the whole score row
-#pragma unroll 1
-          for (int c = 0; c < DP / 8; ++c) {
-            uint32_t o8[8];
-            tmem_ld_32x32b_x8(o_addr + c * 8, o8);
-            tmem_ld_wait();
-#pragma unroll
-            for (int i = 0; i < 8; ++i) o8[i] = __float_as_uint(__uint_as_float(o8[i]) * alpha);
-            tmem_st_32x32b_x8(o_addr + c * 8, o8);
-          }
-          tmem_st_wait();
-          l *= alpha;
-          m_ref = m_new;
-        }
-      }
-
-      mbar_wait(&p_free[t], (j & 1) ^ 1);
-      float rowsum = 0.f, rowsum1 = 0.f, rs2 = 0.f, rs3 = 0.f;  // 4 independent accumulation chains
-      const float neg_m = -m_ref;
-      // 8 columns at a time: exponentials -> bf16 -> one 16-byte store (keeps the live set small: the
-      // 128 score registers + 8 temporaries; a 32-wide temporary array spilled to local memory)
-#pragma unroll
-      for (int g8 = 0; g8 < BKV / 8; ++g8) {
-        float p[8];
+    // ===================== softmax =====================
+    const int t = TILES == 2 ? warp >> 3 : 0, half = (warp >> 2) & 1, quad = warp & 3;
+    const int row = quad * 32 + lane, id = 1 + t * 4 + quad;
+    const uint32_t lane_addr = tmem_base + (static_cast<uint32_t>(quad * 32) << 16);
+    const uint32_t o_addr = lane_addr + 256 + t * 128 + half * C::kHalf;
+    float *xm_t = xm + t * 2 * BQ + row, *xl_t = xl + t * 2 * BQ + row;
+    int g = 0, units = 0;   // blocks and units of the tile so far
+    Unit w;
+    for (int r = 0; r < rounds; ++r) {
+      if (!unit(r, w) || w.n[t] == 0) continue;
+      const int n = w.n[t], q0 = (w.u * TILES + t) * BQ;
+      const int kv_lim = a.causal ? min(a.Sk - 1, q0 + row + off) : a.Sk - 1;
+      // O accumulates in TMEM across KV blocks.  Each row keeps a reference maximum m_ref; the accumulator is rescaled only
+      // when a row's maximum exceeds m_ref by more than 2^8 (exact: P, l and O all use the same m_ref, the final division
+      // by l cancels it).  The two warps of a row decide together.
+      float m_ref = 0.f, l = 0.f;
+      for (int j = 0; j < n; ++j, ++g) {
+        const int sb = TILES == 2 ? t : g & 1;
+        const uint32_t s_addr = lane_addr + sb * BKV + half * 64;
+        wait(&s_full[sb], TILES == 2 ? g : g >> 1);
+        tc_fence_after();
+        const int kv0 = j * BKV + half * 64;
+        const bool need_mask = (kv0 + 64 > a.Sk) || (a.causal && (kv0 + 63 > q0 + off));
+        uint32_t s[64];
+        tmem_ld_32x32b_x32(s_addr, s);
+        tmem_ld_32x32b_x32(s_addr + 32, s + 32);
+        tmem_ld_wait();
         if (need_mask) {
 #pragma unroll
-          for (int i = 0; i < 8; ++i) {
-            const float arg = __uint_as_float(r[g8 * 8 + i]) * a.scale_log2 - m_ref;
-            const float e = (kv0 + g8 * 8 + i <= kv_lim) ? ex2f(arg) : 0.f;
-            p[i] = e;
-            rowsum += e;
-          }
-        } else {
-#pragma unroll
-          for (int i = 0; i < 8; i += 2) {
-            float a0, a1;
-            ffma2(a0, a1, __uint_as_float(r[g8 * 8 + i]), __uint_as_float(r[g8 * 8 + i + 1]), a.scale_log2, neg_m);
-            constexpr int kP = kPolyEvery > 0 ? kPolyEvery : 1;
-            p[i] = (kPolyEvery > 0 && (i % kP) == kP - 1) ? ex2_poly(a0) : ex2f(a0);
-            p[i + 1] = (kPolyEvery > 0 && ((i + 1) % kP) == kP - 1) ? ex2_poly(a1) : ex2f(a1);
-            if ((i & 2) == 0) fadd2(rowsum, rowsum1, p[i], p[i + 1]);
-            else fadd2(rs2, rs3, p[i], p[i + 1]);
-          }
+          for (int i = 0; i < 64; ++i)
+            if (kv0 + i > kv_lim) s[i] = 0xff800000u;
         }
-        // P layout: two [128 rows][64 cols] SW128 chunks; 16-byte piece (g8 & 7) of chunk (g8 >> 3)
-        uint8_t* prow = my_p + (g8 >> 3) * (BQ * 128) + row * 128;
-        uint4 v4;
-        v4.x = pack_bf16(p[0], p[1]);
-        v4.y = pack_bf16(p[2], p[3]);
-        v4.z = pack_bf16(p[4], p[5]);
-        v4.w = pack_bf16(p[6], p[7]);
-        *reinterpret_cast<uint4*>(prow + (((g8 & 7) ^ (row & 7)) << 4)) = v4;
-      }
-      rowsum += rowsum1 + (rs2 + rs3);
-      l += rowsum;
-      fence_proxy_async_smem();
-      tc_fence_before();
-      mbar_arrive(&p_full[t]);
-    }
-
-    if (n > 0) {
-      mbar_wait(&o_full[t], (n - 1) & 1);
-      tc_fence_after();
-      const float inv = l > 0.f ? 1.f / l : 0.f;
-      __nv_bfloat16* dst = a.o + static_cast<int64_t>(b * a.Sq + q_idx) * a.o_tok_stride +
-                           static_cast<int64_t>(h) * a.o_head_stride;
+        float m4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};   // short chains
+#pragma unroll
+        for (int i = 0; i < 64; i += 8)
+#pragma unroll
+          for (int q = 0; q < 4; ++q) m4[q] = fmax3(m4[q], __uint_as_float(s[i + 2 * q]), __uint_as_float(s[i + 2 * q + 1]));
+        float mx = fmaxf(fmaxf(m4[0], m4[1]), fmaxf(m4[2], m4[3])) * a.scale_log2;
+        if (pair_any(id, j == 0 || mx > m_ref + 8.0f)) {
+          xm_t[half * BQ] = mx;
+          pair_sync(id);
+          mx = fmaxf(mx, xm_t[(half ^ 1) * BQ]);
+          if (j == 0) {
+            m_ref = mx == -INFINITY ? 0.f : mx;
+          } else {
+            const float m_new = mx > m_ref + 8.0f ? mx : m_ref;
+            const float alpha = ex2f(m_ref - m_new);                      // 1 for rows that keep their reference
+            wait(&o_full[t], g - 1);   // PV(j - 1) has landed
+            tc_fence_after();
 #pragma unroll 1
-      for (int c = 0; c < DP / 32; ++c) {
-        uint32_t r[32];
-        tmem_ld_32x32b_x32(o_addr + c * 32, r);
-        tmem_ld_wait();
-        if (q_idx < a.Sq) {
+            for (int c = 0; c < C::kHalf / 8; ++c) {   // rare: few registers rather than few round trips
+              uint32_t o8[8];
+              tmem_ld_32x32b_x8(o_addr + c * 8, o8);
+              tmem_ld_wait();
 #pragma unroll
-          for (int g = 0; g < 4; ++g) {
-            if (c * 32 + g * 8 < a.D) {
-              uint4 v4;
-              v4.x = pack_bf16(__uint_as_float(r[g * 8 + 0]) * inv, __uint_as_float(r[g * 8 + 1]) * inv);
-              v4.y = pack_bf16(__uint_as_float(r[g * 8 + 2]) * inv, __uint_as_float(r[g * 8 + 3]) * inv);
-              v4.z = pack_bf16(__uint_as_float(r[g * 8 + 4]) * inv, __uint_as_float(r[g * 8 + 5]) * inv);
-              v4.w = pack_bf16(__uint_as_float(r[g * 8 + 6]) * inv, __uint_as_float(r[g * 8 + 7]) * inv);
-              stg_v4(dst + c * 32 + g * 8, v4);
+              for (int i = 0; i < 8; ++i) o8[i] = __float_as_uint(__uint_as_float(o8[i]) * alpha);
+              tmem_st_32x32b_x8(o_addr + c * 8, o8);
             }
+            l *= alpha;
+            m_ref = m_new;
           }
         }
+        float l4[4] = {0.f, 0.f, 0.f, 0.f};
+        const float neg_m = -m_ref;
+#pragma unroll
+        for (int i = 0; i < 64; i += 4) {
+          float e[4];
+          ffma2(e[0], e[1], __uint_as_float(s[i]), __uint_as_float(s[i + 1]), a.scale_log2, neg_m);
+          ffma2(e[2], e[3], __uint_as_float(s[i + 2]), __uint_as_float(s[i + 3]), a.scale_log2, neg_m);
+#pragma unroll
+          for (int q = 0; q < 4; ++q) e[q] = ex2f(e[q]);
+          fadd2(l4[0], l4[1], e[0], e[1]);
+          fadd2(l4[2], l4[3], e[2], e[3]);
+          s[i / 2] = pack_bf16(e[0], e[1]);
+          s[i / 2 + 1] = pack_bf16(e[2], e[3]);
+        }
+        tmem_st_32x32b_x32(s_addr, s);
+        l += (l4[0] + l4[1]) + (l4[2] + l4[3]);
+        tmem_st_wait();
+        // One tile: the last product but one may be under way still (with two, these scores came behind it).  The wait below
+        // tells the last two apart only if the first of them has landed when the second can begin.
+        if (TILES == 1 && j == n - 1 && j > 0) wait(&o_full[t], g - 1);
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&p_full[sb]);
       }
+      // ---- O / l
+      xl_t[half * BQ] = l;
+      pair_sync(id);
+      l += xl_t[(half ^ 1) * BQ];
+      wait(&o_full[t], g - 1);
+      tc_fence_after();
+      uint32_t o[C::kHalf];
+#pragma unroll
+      for (int c = 0; c < C::kHalf / 8; ++c) tmem_ld_32x32b_x8(o_addr + c * 8, o + c * 8);
+      tmem_ld_wait();
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&o_free[t]);
+      // Rows go out by TMA from the unit's Q tile, which its last scores have left: 16-byte stores of a row per lane held the
+      // load / store unit for 2500 clocks a unit, and the softmax warps that issued the copies waited as long for TMA's queue.
+      const float inv = l > 0.f ? 1.f / l : 0.f;
+      const int qb = t * C::kQ + units % C::kQ;
+      const uint32_t out = smem_u32(q_s) + qb * C::kTileBytes + row * (CW * 2);
+      const int swz = CW == 64 ? row & 7 : (row >> 1) & 3;
+#pragma unroll
+      for (int c = 0; c < C::kHalf / 8; ++c) {
+        const int col = half * C::kHalf + c * 8, piece = (col % CW) / 8;
+        asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(out + (col / CW) * C::kChunkBytes + ((piece ^ swz) << 4)),
+                     "r"(pack_bf16(__uint_as_float(o[c * 8 + 0]) * inv, __uint_as_float(o[c * 8 + 1]) * inv)),
+                     "r"(pack_bf16(__uint_as_float(o[c * 8 + 2]) * inv, __uint_as_float(o[c * 8 + 3]) * inv)),
+                     "r"(pack_bf16(__uint_as_float(o[c * 8 + 4]) * inv, __uint_as_float(o[c * 8 + 5]) * inv)),
+                     "r"(pack_bf16(__uint_as_float(o[c * 8 + 6]) * inv, __uint_as_float(o[c * 8 + 7]) * inv))
+                     : "memory");
+      }
+      fence_proxy_async_smem();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&o_ready[qb]);
+      ++units;
     }
   }
 
   tc_fence_before();
   __syncthreads();
-  if (warp == 9) {
+  if (warp == C::kMma) {
     tc_fence_after();
     tmem_dealloc<512>(tmem_base);
   }
+  if (threadIdx.x == 0 && *gave_up) {
+    *failed = 1u;
+    __threadfence_system();
+  }
 }
 
-template <int DP, int CW, int kPolyEvery>
-int launch_fmha2(const FmhaParams& p, cudaStream_t stream) {
-  using C = Cfg2<DP, CW>;
-  CUtensorMap tq, tk, tv;
+template <int DP, int CW, int TILES>
+int launch(const FmhaParams& p, cudaStream_t stream, int tries) {
+  using C = Shape<DP, CW, TILES>;
+  static_assert(C::kSmem <= 227 * 1024, "fmha: shared memory");
+  volatile unsigned int* failed = failed_word();
+  VB_CHECK(failed != nullptr, "fmha: no pinned host memory for the status word");
+  CUtensorMap tq, tk, tv, to;
   {
     uint64_t dims[4] = {(uint64_t)p.D, (uint64_t)p.Hq, (uint64_t)p.B * p.Sq, 1};
     uint64_t str[3] = {(uint64_t)p.q_head_stride, (uint64_t)p.q_tok_stride,
                        (uint64_t)p.q_tok_stride * p.B * p.Sq};
     uint32_t box[4] = {CW, 1, BQ, 1};
     if (make_tmap_nd_bf16(&tq, p.q, 4, dims, str, box, C::kSwizzleBytes)) return 1;
+  }
+  {
+    uint64_t dims[4] = {(uint64_t)p.D, (uint64_t)p.Hq, (uint64_t)p.Sq, (uint64_t)p.B};
+    uint64_t str[3] = {(uint64_t)p.o_head_stride, (uint64_t)p.o_tok_stride, (uint64_t)p.o_tok_stride * p.Sq};
+    uint32_t box[4] = {CW, 1, BQ, 1};
+    if (make_tmap_nd_bf16(&to, p.o, 4, dims, str, box, C::kSwizzleBytes)) return 1;
   }
   const bool paged = p.kv_page_stride != 0;
   {
@@ -447,42 +548,71 @@ int launch_fmha2(const FmhaParams& p, cudaStream_t stream) {
     if (make_tmap_nd_bf16(&tk, p.k, 4, dims, str, box, C::kSwizzleBytes)) return 1;
     if (make_tmap_nd_bf16(&tv, p.v, 4, dims, str, box, C::kSwizzleBytes)) return 1;
   }
-  Args2 a;
-  a.o = p.o;
-  a.o_tok_stride = p.o_tok_stride;
-  a.o_head_stride = p.o_head_stride;
+  Args a;
   a.page_table = p.page_table;
   a.page_table_stride = p.page_table_stride;
-  a.Sq = p.Sq; a.Sk = p.Sk; a.Hq = p.Hq; a.Hkv = p.Hkv; a.D = p.D;
+  a.Sq = p.Sq; a.Sk = p.Sk; a.Hq = p.Hq; a.Hkv = p.Hkv; a.D = p.D; a.B = p.B;
   a.causal = p.causal;
   a.paged = paged ? 1 : 0;
+  a.units = (p.Sq + TILES * BQ - 1) / (TILES * BQ);
   a.scale_log2 = p.scale * 1.4426950408889634f;
-  auto kern = fmha2_fwd_kernel<DP, CW, kPolyEvery>;
+  auto kern = fmha_pipe_kernel<DP, CW, TILES>;
   static PerDeviceOnce attr_once;
   if (attr_once.first()) {
     VB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kSmem));
   }
-  const int q_tiles = (p.Sq + BQ - 1) / BQ;
-  dim3 grid((q_tiles + 1) / 2, p.Hq, p.B);
-  VB_CUDA(launch_pdl(kern, grid, dim3(kThreads2), C::kSmem, stream, tq, tk, tv, a));
+  const long total = static_cast<long>(a.units) * p.Hq * p.B;
+  VB_CHECK(total < (1L << 30), "fmha: too many query tiles");
+  const int grid = static_cast<int>(total < num_sms() ? total : num_sms());
+  VB_CUDA(launch_pdl(kern, dim3(grid), dim3(C::kThreads), C::kSmem, stream, tq, tk, tv, to, a, tries, failed));
   return 0;
+}
+
+template <int DP, int CW>
+int launch_tiles(const FmhaParams& p, int tiles, cudaStream_t stream, int tries) {
+  return tiles == 2 ? launch<DP, CW, 2>(p, stream, tries) : launch<DP, CW, 1>(p, stream, tries);
 }
 
 }  // namespace
 
-// returns -1 when the shape is not handled by v2 (caller uses v1)
-int fmha_prefill_v2(const FmhaParams& p, cudaStream_t stream, int poly_every) {  // default 0, see kPolyEvery
-  if (p.D == 128) {
-    if (poly_every == 4) return launch_fmha2<128, 64, 4>(p, stream);
-    if (poly_every == 2) return launch_fmha2<128, 64, 2>(p, stream);
-    return launch_fmha2<128, 64, 0>(p, stream);
-  }
-  if (p.D <= 96 && p.D > 64) {
-    if (poly_every == 4) return launch_fmha2<96, 32, 4>(p, stream);
-    if (poly_every == 2) return launch_fmha2<96, 32, 2>(p, stream);
-    return launch_fmha2<96, 32, 0>(p, stream);
-  }
-  return -1;
+int fmha_prefill(const FmhaParams& p, cudaStream_t stream) { return fmha_prefill_cfg(0, p, stream); }
+
+// variant: 0 by size, 1 one query tile at a time, 2 (3, 4) two; tries >= 0: of every wait (tests)
+int fmha_prefill_cfg(int variant, const FmhaParams& p, cudaStream_t stream, int tries) {
+  VB_CHECK(variant >= 0 && variant <= 4, "fmha: unknown variant %d", variant);
+  VB_CHECK(p.B > 0 && p.Sq > 0 && p.Sk > 0, "fmha: empty problem");
+  VB_CHECK(p.Hq % p.Hkv == 0, "fmha: Hq (%d) must be a multiple of Hkv (%d)", p.Hq, p.Hkv);
+  VB_CHECK(p.D % 8 == 0, "fmha: head dim must be a multiple of 8 (got %d)", p.D);
+  VB_CHECK(p.q_tok_stride % 8 == 0 && p.q_head_stride % 8 == 0 && p.kv_tok_stride % 8 == 0 &&
+               p.kv_head_stride % 8 == 0 && p.o_tok_stride % 8 == 0 && p.o_head_stride % 8 == 0,
+           "fmha: strides must be multiples of 8 elements (16 bytes)");
+  VB_CHECK(!p.causal || p.Sk >= p.Sq, "fmha: causal needs Sk >= Sq");
+  if (wait_status()) return 1;   // an earlier launch gave up: nothing is built on its output
+  if (tries < 0) tries = kTries;
+  // Two tiles at a time take 1.6 times as long per key block as one (13 x 16 heads of 1024 keys, head size 72: 23.5 and 14.5
+  // us a round of units).  Key blocks per CTA: whole rounds of equal units, or (causal, dealt evenly) the mean, but no less
+  // than the longest unit.  1 / 2 / 3 / 4 / 7 / 13 images: one 17, 31, 39, 56, 84, 167 us, two 25, 26, 46, 46, 76, 121; causal,
+  // 28 heads of 128, 600 / 1024 / 1500 / 2500 / 8000 rows: 10, 14.4, 25, 52, 414 and 15, 22, 31, 51, 389.
+  const int q_tiles = (p.Sq + BQ - 1) / BQ;
+  auto blocks = [&](int per) {
+    const int units = (q_tiles + per - 1) / per;
+    const long heads = static_cast<long>(p.Hq) * p.B, sms = num_sms();
+    if (!p.causal) return (units * heads + sms - 1) / sms * ((p.Sk + BKV - 1) / BKV);
+    long sum = 0, most = 0;
+    for (int u = 1; u <= units; ++u) {
+      most = (min(p.Sk, min(u * per * BQ, p.Sq) + p.Sk - p.Sq) + BKV - 1) / BKV;
+      sum += most;
+    }
+    return max(most, (sum * heads + sms - 1) / sms);
+  };
+  const int tiles = variant == 0 ? (8 * blocks(2) < 5 * blocks(1) ? 2 : 1) : variant == 1 || q_tiles == 1 ? 1 : 2;
+  if (p.D == 128) return launch_tiles<128, 64>(p, tiles, stream, tries);
+  if (p.D > 80 && p.D <= 96) return launch_tiles<96, 32>(p, tiles, stream, tries);
+  if (p.D > 64 && p.D <= 80) return launch_tiles<80, 32>(p, tiles, stream, tries);
+  VB_CHECK(variant < 2 || p.D == 64, "fmha: the two-tile kernel does not cover head dim %d", p.D);
+  if (p.D == 64) return launch_tiles<64, 64>(p, tiles, stream, tries);
+  set_last_error("fmha: unsupported head dim %d (supported: 64, 65..96, 128)", p.D);
+  return 1;
 }
 
 }  // namespace vb

@@ -33,6 +33,25 @@
 #include <mutex>
 
 namespace vb {
+// A word of pinned host memory that a launch which gave up sets: the host reads it without waiting for the device.
+namespace {
+std::atomic<volatile unsigned int*> g_failed{nullptr};
+}
+volatile unsigned int* failed_word() {
+  static std::once_flag once;
+  std::call_once(once, [] {
+    void* w = nullptr;
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;   // the first call may be under capture
+    cudaThreadExchangeStreamCaptureMode(&mode);
+    if (cudaHostAlloc(&w, sizeof(unsigned int), cudaHostAllocPortable | cudaHostAllocMapped) == cudaSuccess) {
+      *static_cast<volatile unsigned int*>(w) = 0u;
+      g_failed = static_cast<volatile unsigned int*>(w);
+    }
+    cudaThreadExchangeStreamCaptureMode(&mode);
+  });
+  return g_failed;
+}
+
 namespace {
 
 constexpr int kRowsW = 128, kDepth = 64;            // weight rows and K columns of a stage
@@ -40,26 +59,7 @@ constexpr int kWBytes = kRowsW * kDepth * 2;
 constexpr int kGatherWarps = 4, kBox = 64;          // token rows of one TMA box
 constexpr int kMaxGroups = 1024;                    // groups whose tile offsets fit shared memory
 
-constexpr int kTries = 1 << 20;                     // of a wait, then the launch gives up
-constexpr int kDrainTries = 1 << 14;                // of a wait for what is still in flight after that
-
 __device__ unsigned int g_gave_up;   // CTAs that gave up (none in a correct run)
-
-// An mbarrier wait that ends: a lost arrival must not leave the GPU spinning.  The first wait of a CTA that runs out of
-// tries sets `gave_up`, which ends the other warps' waits; a warp whose wait failed leaves its loop for the CTA's last
-// barrier.  No warp waits in any other way before that barrier.
-__device__ __forceinline__ bool mbar_wait_limited(uint64_t* bar, uint32_t parity, volatile int* gave_up, int tries) {
-  for (int i = 0; i < tries; ++i) {
-    if (mbar_try_wait(bar, parity)) return true;
-    if (*gave_up) return false;
-  }
-  *gave_up = 1;
-  return false;
-}
-__device__ __forceinline__ void mbar_drain(uint64_t* bar, uint32_t parity) {
-  for (int i = 0; i < kDrainTries; ++i)
-    if (mbar_try_wait(bar, parity)) return;
-}
 __device__ __forceinline__ void cp_async16(uint32_t dst, const void* src, bool ok) {
   const uint32_t n = ok ? 16u : 0u;   // 0: the 16 bytes are filled with zeros
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(n) : "memory");
@@ -415,23 +415,6 @@ glinear_tc_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
   }
 }
 
-// A word of pinned host memory that a launch which gave up sets: the host reads it without waiting for the device.
-std::atomic<volatile unsigned int*> g_failed{nullptr};
-volatile unsigned int* failed_word() {
-  static std::once_flag once;
-  std::call_once(once, [] {
-    void* w = nullptr;
-    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;   // the first call may be under capture
-    cudaThreadExchangeStreamCaptureMode(&mode);
-    if (cudaHostAlloc(&w, sizeof(unsigned int), cudaHostAllocPortable | cudaHostAllocMapped) == cudaSuccess) {
-      *static_cast<volatile unsigned int*>(w) = 0u;
-      g_failed = static_cast<volatile unsigned int*>(w);
-    }
-    cudaThreadExchangeStreamCaptureMode(&mode);
-  });
-  return g_failed;
-}
-
 template <int BT, int EPI>
 int launch_epi(const CUtensorMap& tm, const CUtensorMap& ta, const vila_glinear_params& p, const vila_glinear_ext& x, int tries, cudaStream_t stream) {
   using S = Shape<BT>;
@@ -481,7 +464,7 @@ int wait_status() {
   volatile unsigned int* w = g_failed;
   if (w == nullptr || *w == 0u) return 0;
   *w = 0u;
-  set_last_error("glinear: a wait of an earlier launch ran out of tries; that launch's output is incomplete");
+  set_last_error("a wait of an earlier launch (linear layer or attention) ran out of tries; that launch's output is incomplete");
   return 1;
 }
 

@@ -71,10 +71,9 @@ struct FmhaParams {
   float scale;      // softmax scale (1/sqrt(D))
 };
 int fmha_prefill(const FmhaParams& p, cudaStream_t stream);
-int fmha_prefill_cfg(int variant, const FmhaParams& p, cudaStream_t stream);  // 0 auto, 1 one-tile, 2 two-tile
-// poly_every: every n-th exponential on the FMA pipe (0 = none, the default; 4; 2) — test/bench hook
-int fmha_prefill_v2(const FmhaParams& p, cudaStream_t stream, int poly_every = 0);  // -1: shape not handled
-// split-KV mode of the one-tile kernel for decode at long context (see fmha_tcgen05.cu)
+// variant: 0 by size, 1 one query tile at a time, 2 .. 4 two; tries >= 0: of every wait (tests), otherwise the kernel's limit
+int fmha_prefill_cfg(int variant, const FmhaParams& p, cudaStream_t stream, int tries = -1);
+// split-KV attention for decode at long context (see fmha_tcgen05.cu)
 // counters != nullptr ([Hq] ints, zero-initialised once): the last split CTA of a head combines into p.o
 int fmha_decode_split(const FmhaParams& p, const int32_t* n_tok_minus_1, int split_tokens,
                       float* o_partial, float* lse, int* counters, cudaStream_t stream);
@@ -314,6 +313,7 @@ int gather_rows(const void* src, const int32_t* rows, void* dst, int n_rows, int
 // bf16 operands on 16-byte boundaries with at least 128 weight rows: tcgen05 tiles (glinear_tcgen05.cu)
 bool glinear_tc_takes(const vila_glinear_params& p);
 unsigned int stalled_waits();
+volatile unsigned int* failed_word();   // pinned host memory that a launch which gave up sets; nullptr: there is none
 int wait_status();   // 1 (and the last error) once after a launch whose wait ran out of tries; does not synchronise
 int glinear_tc(const vila_glinear_params& p, cudaStream_t stream, const vila_glinear_ext& x, int tries);
 // few rows of bf16 operands: fp32 multiply-adds over the streamed weights (glinear_rows.cu)
