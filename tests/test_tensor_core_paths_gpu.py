@@ -418,6 +418,41 @@ def test_paged_attention_prompt_infinite_entries(ops, form, rep):
             assert int(seen.sum()) > T - 3 and rel(got[seen], ref[seen]) < 3e-6
 
 
+MIX_FORMS = {"talk": dict(talk=True), "sink": dict(talk=True, sink=True, softcap=5.0, gate=True), "chunk": dict(talk=True, chunk=24, dist_bias=30),
+             "after": dict(talk=True, talk_after=True), "after_window": dict(talk=True, talk_after=True, window=21, keep_first=3, head_scale=True, gate=True)}
+
+
+@pytest.mark.parametrize("form", list(MIX_FORMS))
+@pytest.mark.parametrize("H,G", [(2, 1), (7, 7), (8, 2), (16, 4), (17, 17), (32, 32), (32, 8)])
+@pytest.mark.parametrize("seqs", [[(2, 0)], [(16, 0), (17, 63), (3, 128)], [(33, 300), (64, 1)]])
+def test_paged_attention_prompt_mixed_heads(ops, form, H, G, seqs):
+    """a mixed score (weight) is a sum over H heads of mean square 1 + 0.09 H: the 3e-6 of one head times its root, at most 6e-6;
+    tiles of 1 to 16 rows, one and two heads a warp, warps without a head, rows alone"""
+    for D in (64, 128):
+        got, want, (q, pool, tables, tiles, o) = attention_case(ops, MIX_FORMS[form], H, G, D, D, 48 if H == 8 else 64, seqs, seed=H)
+        assert rel(got, want) < 6e-6
+        one = torch.stack([tiles[-1, 0] + tiles[-1, 1] - 1, torch.ones_like(tiles[-1, 0]), tiles[-1, 2] + tiles[-1, 1] - 1, tiles[-1, 3]])[None].contiguous()
+        alone = ops.paged_attention(q, pool, tables, one, heads=H, kv_heads=G, dim=D, vdim=D, page=48 if H == 8 else 64, scale=0.1, out_dtype=F32,
+                                    max_rows=16, **o)
+        assert torch.equal(alone[-1], got[-1])
+
+
+@pytest.mark.parametrize("form", list(MIX_FORMS))
+@pytest.mark.parametrize("H", [4, 20])
+def test_paged_attention_prompt_mixed_heads_infinite_value(ops, form, H):
+    """an infinite value reaches the rows that see it (all heads of its value head) and nothing else"""
+    T, j, D, o = 70, 37, 128, MIX_FORMS[form]
+    got, want, (q, pool, tables, tiles, o) = attention_case(ops, o, H, H // 2, D, D, 64, [(T, 0)], seed=H)
+    bad = pool.clone()
+    bad[int(tables[0, j // 64]) * 64 + j % 64, H // 2 * D + 5] = float("inf")
+    inf = ops.paged_attention(q, bad, tables, tiles, heads=H, kv_heads=H // 2, dim=D, vdim=D, page=64, scale=0.1, out_dtype=F32, max_rows=16, **o).view(T, H, D)
+    want, reach = want.view(T, H, D), min(T, j + o.get("window", T), (j // o["chunk"] + 1) * o["chunk"] if "chunk" in o else T)
+    assert torch.isinf(inf[j:reach, :2, 5]).all()
+    keep = torch.ones_like(want, dtype=torch.bool)
+    keep[j:reach, :2, 5] = False
+    assert torch.isfinite(inf[keep]).all() and rel(inf[keep], want[keep]) < 6e-6
+
+
 def test_paged_attention_decode_skips_empty_tiles(ops):
     """a tile of no rows names an output row but has nothing to write"""
     for nsplit in (1, 4):

@@ -39,6 +39,7 @@ SOURCES = [
     "short_conv.cu",
     "paged_attn.cu",
     "paged_attn_mma.cu",
+    "paged_attn_mix.cu",
     "paged_attn_decode.cu",
     "ssm.cu",
     "outer_scan.cu",

@@ -563,7 +563,7 @@ __global__ void __launch_bounds__(kThreads, NACC <= 2 ? 4 : (NACC <= 8 ? 2 : 1))
   }
 }
 
-// Prompt portions: BQ (a multiple of 4) rows x all heads per CTA, register-tiled.  Score rows are ordered
+// Prompt portions that neither tensor-core kernel takes: BQ (a multiple of 4) rows x all heads per CTA, register-tiled.  Score rows are ordered
 // head-major (r = h * BQ + i) so that 4 consecutive score rows are 4 query rows of ONE head: they share
 // the key / value head, and a thread that owns such a block of 4 keeps
 //   scores:        TR (4, or 2 with 512 threads) rows x 2 keys (jp and jp + BK / 2) per thread, q and k as float4
@@ -960,6 +960,7 @@ int paged_attention(const vila_paged_attn_params& p, cudaStream_t stream) {
   VB_CHECK(p.max_rows >= 1 && p.max_rows <= 16 && (p.nsplit == 1 || p.max_rows == 1),
            "paged_attention: max_rows=%d nsplit=%d (key splitting serves one-row tiles)", p.max_rows, p.nsplit);
   if (paged_attention_mma_takes(p)) return paged_attention_mma(p, stream);
+  if (paged_attention_mix_takes(p)) return paged_attention_mix(p, stream);
   if (paged_attention_decode_takes(p)) return paged_attention_decode(p, stream);
   AttnShape sh;
   sh.phase = -1;
