@@ -40,6 +40,7 @@ SOURCES = [
     "paged_attn.cu",
     "paged_attn_mma.cu",
     "paged_attn_mix.cu",
+    "paged_attn_tc.cu",
     "paged_attn_decode.cu",
     "ssm.cu",
     "outer_scan.cu",

@@ -304,6 +304,8 @@ int rope_append(const vila_rope_append_params& p, cudaStream_t stream);
 // prompt portions over a bf16 pool, head sizes 64 / 128, heads not mixed: tensor cores (paged_attn_mma.cu)
 bool paged_attention_mix_takes(const vila_paged_attn_params& p);   // prompt portions of mixed heads
 int paged_attention_mix(const vila_paged_attn_params& p, cudaStream_t stream);
+bool paged_attention_tc_takes(const vila_paged_attn_params& p);    // prompt portions, 128 columns
+int paged_attention_tc(const vila_paged_attn_params& p, cudaStream_t stream);
 bool paged_attention_mma_takes(const vila_paged_attn_params& p);
 int paged_attention_mma(const vila_paged_attn_params& p, cudaStream_t stream);
 // decoded tokens over a bf16 pool, 128 key and value columns, heads not mixed (paged_attn_decode.cu)

@@ -959,6 +959,7 @@ int paged_attention(const vila_paged_attn_params& p, cudaStream_t stream) {
            "paged_attention: maps=%d (two maps per head take no head mixing, sink, distance bias or head scale)", p.maps);
   VB_CHECK(p.max_rows >= 1 && p.max_rows <= 16 && (p.nsplit == 1 || p.max_rows == 1),
            "paged_attention: max_rows=%d nsplit=%d (key splitting serves one-row tiles)", p.max_rows, p.nsplit);
+  if (paged_attention_tc_takes(p)) return paged_attention_tc(p, stream);
   if (paged_attention_mma_takes(p)) return paged_attention_mma(p, stream);
   if (paged_attention_mix_takes(p)) return paged_attention_mix(p, stream);
   if (paged_attention_decode_takes(p)) return paged_attention_decode(p, stream);

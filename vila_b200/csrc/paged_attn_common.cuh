@@ -84,4 +84,86 @@ __device__ __forceinline__ float out_gate(const vila_paged_attn_params& p, int r
   return p.gate ? sigmoid_f(ld_any(p.gate, p.gate_dtype, static_cast<size_t>(row) * p.ldg + h)) : 1.0f;
 }
 
+constexpr float kLog2e = 1.44269504f;   // 1 / ln 2
+
+// two fp32 numbers at a time
+using f2 = unsigned long long;
+__device__ __forceinline__ f2 pair(float x, float y) {
+  f2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(x), "f"(y));
+  return r;
+}
+__device__ __forceinline__ void unpair(f2 v, float& x, float& y) { asm("mov.b64 {%0, %1}, %2;" : "=f"(x), "=f"(y) : "l"(v)); }
+__device__ __forceinline__ void fma2(float& ax, float& ay, float m, float cx, float cy) {   // a = a m + c
+  f2 r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(pair(ax, ay)), "l"(pair(m, m)), "l"(pair(cx, cy)));
+  unpair(r, ax, ay);
+}
+__device__ __forceinline__ void add2(float& ax, float& ay, float cx, float cy) {
+  f2 r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(pair(ax, ay)), "l"(pair(cx, cy)));
+  unpair(r, ax, ay);
+}
+__device__ __forceinline__ f2 mul2(f2 a, f2 b) {
+  f2 r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ f2 fma2(f2 a, f2 b, f2 c) {
+  f2 r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+// capped() of two scores up to the cap, the same operations
+__device__ __forceinline__ void cap2(float& a, float& b, float inv) {
+  const f2 s = pair(a, b), x = mul2(s, pair(inv, inv)), u = mul2(x, x);
+  f2 r = pair(cap_poly(7), cap_poly(7));
+#pragma unroll
+  for (int k = 6; k >= 0; --k) r = fma2(r, u, pair(cap_poly(k), cap_poly(k)));
+  unpair(mul2(s, r), a, b);
+}
+__device__ __forceinline__ float ex2(float x) {
+  float y;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+// log2(e) x, rounded (never fused into what follows: a maximum's value has to be the same wherever it is used)
+__device__ __forceinline__ float log2_units(float x) { return __fmul_rn(x, kLog2e); }
+
+// A row of one score head again, key by key in fp32 multiply-adds, into dst (V numbers, divided by their weights' sum): what
+// the CUDA-core kernels compute.  Rows that met an infinite or NaN number come here, because the parts of a finite number
+// hold zeros and zero times infinity is NaN where the whole number times infinity is not.  A warp per row.
+template <int D, int MAPS, int V>
+__device__ __noinline__ void row_again(const vila_paged_attn_params& p, int row, int pos, int slot, int h, int map, float* dst) {
+  constexpr int DL = D / 32, VL = V / 32;                 // columns of a lane
+  const int lane = threadIdx.x & 31, g = h / (p.H / p.G);
+  const int32_t* pt = p.page_tables + static_cast<size_t>(slot) * p.pt_stride;
+  const size_t prow = static_cast<size_t>(p.G) * (MAPS * D + V);
+  const __nv_bfloat16* pool = static_cast<const __nv_bfloat16*>(p.pool);
+  const size_t koff = static_cast<size_t>(g * MAPS + map) * D + DL * lane, voff = static_cast<size_t>(p.G) * MAPS * D + static_cast<size_t>(g) * V + VL * lane;
+  const float sc = head_scale(p, h);
+  float q[DL], acc[VL];
+#pragma unroll
+  for (int e = 0; e < DL; ++e) q[e] = p.q[((static_cast<size_t>(row) * p.H + h) * MAPS + map) * D + DL * lane + e] * sc;
+#pragma unroll
+  for (int e = 0; e < VL; ++e) acc[e] = 0.f;
+  float m = p.sink ? p.sink[h] : kNegBig, l = p.sink ? 1.0f : 0.0f;
+  for (int j = 0; j <= pos; ++j) {
+    if (!sees(p, pos, j)) continue;
+    const __nv_bfloat16* at = pool + pool_row(pt, p.page, j) * prow;
+    float s = 0.f;
+#pragma unroll
+    for (int e = 0; e < DL; ++e) s = fmaf(q[e], __bfloat162float(at[koff + e]), s);
+    s = capped(p, warp_sum(s));
+    if (p.dist_bias) s += dist_bias(p, pos - j, h);
+    const float mn = fmaxf(m, s), w = expf(s - mn), alpha = expf(m - mn);
+    l = fmaf(l, alpha, w);
+    m = mn;
+#pragma unroll
+    for (int e = 0; e < VL; ++e) acc[e] = fmaf(w, __bfloat162float(at[voff + e]), acc[e] * alpha);
+  }
+#pragma unroll
+  for (int e = 0; e < VL; ++e) dst[VL * lane + e] = acc[e] * (1.0f / l);
+}
+
 }  // namespace vb

@@ -33,14 +33,7 @@ namespace {
 
 constexpr int kBK = 16;       // keys of a block
 constexpr int kRows = 8;
-constexpr float kLog2e = 1.44269504f;
 
-__device__ __forceinline__ float ex2(float x) {
-  float y;
-  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-  return y;
-}
-__device__ __forceinline__ float log2_units(float x) { return __fmul_rn(x, kLog2e); }   // never fused into what follows
 __device__ __forceinline__ uint4 ld_pool(const __nv_bfloat16* p) {   // stays where it is written, a stage ahead of its use
   uint4 v;
   asm volatile("ld.global.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p) : "memory");
@@ -136,8 +129,9 @@ __global__ void __launch_bounds__(512, 1) paged_attn_mix_kernel(const __grid_con
   float* X = Qs + H * kRows * QS;                            // two buffers [H][8 rows][4 lanes: keys 2 t, 2 t + 1, 2 t + 8, 2 t + 9]
   float* talk = X + 2 * H * kRows * kBK;                     // [H][TS]
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, gid = lane >> 2, tig = lane & 3;
-  const int* tile = p.tiles + 4 * (static_cast<int>(gridDim.x) - 1 - blockIdx.x);   // late rows, which see most keys, first
-  const int i0 = (static_cast<int>(gridDim.y) - 1 - blockIdx.y) * kRows;
+  const int at = static_cast<int>(gridDim.x) - 1 - blockIdx.x, parts = (p.max_rows + kRows - 1) / kRows;   // late rows, which see most keys, first
+  const int* tile = p.tiles + 4 * (at / parts);
+  const int i0 = at % parts * kRows;
   if (i0 >= tile[1]) return;
   const int row0 = tile[0] + i0, n = min(kRows, tile[1] - i0), pos0 = tile[2] + i0;
   const int32_t* pt = p.page_tables + static_cast<size_t>(tile[3]) * p.pt_stride;
@@ -441,7 +435,9 @@ int launch(const vila_paged_attn_params& p, cudaStream_t stream) {
   auto kernel = paged_attn_mix_kernel<D, HW, AFTER>;
   static PerDeviceOnce once;
   if (once.first()) VB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem_bytes<D>(16 * HW))));
-  VB_CUDA(launch_serial(kernel, dim3(p.ntiles, (p.max_rows + kRows - 1) / kRows), dim3(32 * ((p.H + HW - 1) / HW)), smem_bytes<D>(p.H), stream, p));
+  const long ctas = static_cast<long>(p.ntiles) * ((p.max_rows + kRows - 1) / kRows);
+  VB_CHECK(ctas < (1L << 31), "paged_attention: too many tiles");
+  VB_CUDA(launch_serial(kernel, dim3(static_cast<unsigned>(ctas)), dim3(32 * ((p.H + HW - 1) / HW)), smem_bytes<D>(p.H), stream, p));
   return 0;
 }
 template <int D>

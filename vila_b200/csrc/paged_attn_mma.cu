@@ -1,4 +1,5 @@
-// vila_paged_attention for prompt portions over a bf16 pool on the tensor cores, in fp32 precision.
+// vila_paged_attention for prompt portions over a bf16 pool on the tensor cores, in fp32 precision: two maps, 64 columns, and 128
+// columns off the 16-byte boundaries of paged_attn_tc.cu.
 //
 // The keys and values are bf16 numbers; the queries and the softmax weights are fp32 and stay so: each is cut into
 // three bf16 parts (8 + 8 + 8 bits) whose products with a bf16 number are exact, and the three products are summed
@@ -13,7 +14,7 @@
 // on its tile), and the two are merged at the end.  The sets run freely against each other, one's softmax under the
 // other's products, and the longest chain of blocks is half as long.  Blocks come by cp.async into double buffers of
 // 16-byte pieces swizzled over 8 rows (the ldmatrix reads of 8 keys fall into different banks).  CTAs of late
-// positions, which see most keys, start first.
+// positions, which see most keys, start first, those of all key heads.
 //
 // Bound by the tensor pipe (mma.sync: 1024 multiply-adds per clock and SM measured), six products where bf16 attention
 // issues two.  Tiled on the CUDA cores the same attention ran at 10 TFLOP/s (two shared-memory reads per 16
@@ -37,51 +38,7 @@ namespace {
 
 constexpr int kBK = 64;      // keys of a block
 constexpr int kMaxWarps = 8;
-constexpr float kLog2e = 1.44269504f;   // 1 / ln 2
 
-// two of a fragment's sums at a time: c0, c1 (or c2, c3) belong to one row
-using f2 = unsigned long long;
-__device__ __forceinline__ f2 pair(float x, float y) {
-  f2 r;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(x), "f"(y));
-  return r;
-}
-__device__ __forceinline__ void unpair(f2 v, float& x, float& y) { asm("mov.b64 {%0, %1}, %2;" : "=f"(x), "=f"(y) : "l"(v)); }
-__device__ __forceinline__ void fma2(float& ax, float& ay, float m, float cx, float cy) {   // a = a m + c
-  f2 r;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(pair(ax, ay)), "l"(pair(m, m)), "l"(pair(cx, cy)));
-  unpair(r, ax, ay);
-}
-__device__ __forceinline__ void add2(float& ax, float& ay, float cx, float cy) {
-  f2 r;
-  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(pair(ax, ay)), "l"(pair(cx, cy)));
-  unpair(r, ax, ay);
-}
-__device__ __forceinline__ f2 mul2(f2 a, f2 b) {
-  f2 r;
-  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-  return r;
-}
-__device__ __forceinline__ f2 fma2(f2 a, f2 b, f2 c) {
-  f2 r;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-  return r;
-}
-// capped() of two scores up to the cap, the same operations
-__device__ __forceinline__ void cap2(float& a, float& b, float inv) {
-  const f2 s = pair(a, b), x = mul2(s, pair(inv, inv)), u = mul2(x, x);
-  f2 r = pair(cap_poly(7), cap_poly(7));
-#pragma unroll
-  for (int k = 6; k >= 0; --k) r = fma2(r, u, pair(cap_poly(k), cap_poly(k)));
-  unpair(mul2(s, r), a, b);
-}
-__device__ __forceinline__ float ex2(float x) {
-  float y;
-  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-  return y;
-}
-// log2(e) x, rounded (never fused into what follows: a maximum's value has to be the same wherever it is used)
-__device__ __forceinline__ float log2_units(float x) { return __fmul_rn(x, kLog2e); }
 __device__ __forceinline__ float quad_max(float v) {
   v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, 1));
   return fmaxf(v, __shfl_xor_sync(0xffffffffu, v, 2));
@@ -89,42 +46,6 @@ __device__ __forceinline__ float quad_max(float v) {
 __device__ __forceinline__ float quad_sum(float v) {
   v += __shfl_xor_sync(0xffffffffu, v, 1);
   return v + __shfl_xor_sync(0xffffffffu, v, 2);
-}
-
-// A row of one score head again, key by key in fp32 multiply-adds, into dst (V numbers, divided by their weights' sum): what
-// the CUDA-core kernels compute.  Rows that met an infinite or NaN number come here, because the parts of a finite number
-// hold zeros and zero times infinity is NaN where the whole number times infinity is not.  A warp per row.
-template <int D, int MAPS, int V>
-__device__ __noinline__ void row_again(const vila_paged_attn_params& p, int row, int pos, int slot, int h, int map, float* dst) {
-  constexpr int DL = D / 32, VL = V / 32;                 // columns of a lane
-  const int lane = threadIdx.x & 31, g = h / (p.H / p.G);
-  const int32_t* pt = p.page_tables + static_cast<size_t>(slot) * p.pt_stride;
-  const size_t prow = static_cast<size_t>(p.G) * (MAPS * D + V);
-  const __nv_bfloat16* pool = static_cast<const __nv_bfloat16*>(p.pool);
-  const size_t koff = static_cast<size_t>(g * MAPS + map) * D + DL * lane, voff = static_cast<size_t>(p.G) * MAPS * D + static_cast<size_t>(g) * V + VL * lane;
-  const float sc = head_scale(p, h);
-  float q[DL], acc[VL];
-#pragma unroll
-  for (int e = 0; e < DL; ++e) q[e] = p.q[((static_cast<size_t>(row) * p.H + h) * MAPS + map) * D + DL * lane + e] * sc;
-#pragma unroll
-  for (int e = 0; e < VL; ++e) acc[e] = 0.f;
-  float m = p.sink ? p.sink[h] : kNegBig, l = p.sink ? 1.0f : 0.0f;
-  for (int j = 0; j <= pos; ++j) {
-    if (!sees(p, pos, j)) continue;
-    const __nv_bfloat16* at = pool + pool_row(pt, p.page, j) * prow;
-    float s = 0.f;
-#pragma unroll
-    for (int e = 0; e < DL; ++e) s = fmaf(q[e], __bfloat162float(at[koff + e]), s);
-    s = capped(p, warp_sum(s));
-    if (p.dist_bias) s += dist_bias(p, pos - j, h);
-    const float mn = fmaxf(m, s), w = expf(s - mn), alpha = expf(m - mn);
-    l = fmaf(l, alpha, w);
-    m = mn;
-#pragma unroll
-    for (int e = 0; e < VL; ++e) acc[e] = fmaf(w, __bfloat162float(at[voff + e]), acc[e] * alpha);
-  }
-#pragma unroll
-  for (int e = 0; e < VL; ++e) dst[VL * lane + e] = acc[e] * (1.0f / l);
 }
 
 // D: columns of a map, MAPS: maps of a head, V: value columns, SETS: sets of warps that share the key blocks.  A key's row
@@ -141,8 +62,8 @@ paged_attn_mma_kernel(const __grid_constant__ vila_paged_attn_params p, int tile
   extern __shared__ __align__(128) uint8_t sm[];
   const int lane = threadIdx.x & 31, W = (blockDim.x >> 5) / SETS;   // warps of a set
   const int set = (threadIdx.x >> 5) / W, warp = (threadIdx.x >> 5) - set * W;
-  const int rep = p.H / p.G, SH = rep * MAPS, g = blockIdx.y;
-  const int tile0 = (gridDim.x - 1 - blockIdx.x) * tiles_per_cta, ntile = min(tiles_per_cta, p.ntiles - tile0);
+  const int rep = p.H / p.G, SH = rep * MAPS, g = blockIdx.x % p.G;
+  const int tile0 = (gridDim.x / p.G - 1 - blockIdx.x / p.G) * tiles_per_cta, ntile = min(tiles_per_cta, p.ntiles - tile0);
   const int my_tile = warp / SH, sh = warp - my_tile * SH;  // this warp's tile and score head
   const int h = g * rep + sh / MAPS, map = sh % MAPS;
   const bool active = my_tile < ntile;
@@ -513,7 +434,9 @@ int launch_kernel(const vila_paged_attn_params& p, int warps, int tpc, cudaStrea
   const int smem = warps * 3 * (D / 16) * 512 + SETS * 2 * kBK * (MAPS * D + V) * 2;
   static PerDeviceOnce once;
   if (once.first()) VB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 224 * 1024));
-  VB_CUDA(launch_serial(kernel, dim3((p.ntiles + tpc - 1) / tpc, p.G), dim3(32 * warps * SETS), smem, stream, p, tpc));
+  const long ctas = static_cast<long>((p.ntiles + tpc - 1) / tpc) * p.G;
+  VB_CHECK(ctas < (1L << 31), "paged_attention: too many tiles");
+  VB_CUDA(launch_serial(kernel, dim3(static_cast<unsigned>(ctas)), dim3(32 * warps * SETS), smem, stream, p, tpc));
   return 0;
 }
 template <int D, int MAPS, int V, int SETS>
