@@ -6,15 +6,19 @@
 // are swapped: the UMMA M dimension (TMEM lanes) carries WEIGHT rows and the UMMA N dimension carries
 // ALL tokens (padded only to a multiple of 32, issued as one or two equal UMMA N chunks), so every
 // weight byte enters an SM exactly once, and the K dimension is split across CTAs so that the machine
-// is filled.  Partial sums of the splits are parked in fp32 workspace slots and added in a fixed
-// order by the last-arriving CTA (deterministic).
+// is filled.  The splits of a weight block are a cluster: each parks its partial in its own shared memory and finishes
+// a share of the tokens from all of them, in rank order (where no such cluster fits, the partials go to fp32 workspace
+// slots that the last-arriving CTA adds in a fixed order).
+// Weights of a round and more are not split: a CTA (pair) per SM takes the weight blocks in turn, and one's epilogue
+// (11000 clocks of 279 tokens) is under the next one's products; their accumulators share what 512 columns do not hold twice.
 //
 // Two flavours of the same kernel:
 //   kPair = false : one CTA = 128 weight rows, tcgen05.mma.cta_group::1, loads the whole token tile
 //   kPair = true  : a 2-CTA cluster = 256 weight rows, ONE tcgen05.mma.cta_group::2 (M = 256) issued
 //                   by the leader CTA; each CTA stages its own 128 weight rows plus HALF of the token
 //                   tile (the tensor cores of both SMs read both halves), which halves the token
-//                   bytes per SM — the term that bounds the single-CTA flavour.  Both CTAs' TMA loads
+//                   bytes per SM — the term that bounds the single-CTA flavour (shared memory's port: 53 KB in and 70 KB out
+//                   per 64 columns of K at 279 tokens, 960 clocks; a pair's CTA 690).  Both CTAs' TMA loads
 //                   signal the leader's "full" barrier; the leader's tcgen05.commit multicasts the
 //                   "stage free" / "accumulator ready" arrivals to both CTAs.
 //
@@ -25,6 +29,8 @@
 //              feature n, column == token m.  Each chunk is transposed through a shared-memory
 //              staging tile so that C[m, n0..] leaves the SM as 16-byte vectors in 256-byte rows;
 //              bias / GELU / residual / SwiGLU with the rounding points of gemm_tcgen05.cu.
+// us, before and now (one lane's branch as issuer, a CTA per weight block, partials 4 bytes at a time): 279 rows x 37888 x
+// 3584 gated 80 -> 64, 3584 x 18944 52 -> 46, 4608 x 3584 21 -> 18, 2048 x 11008 29 -> 25; 40 rows 51 -> 43, 34 -> 27, 13.4 -> 10.2, 18 -> 13.
 #include <cstdio>
 #include <cstdlib>
 
@@ -40,13 +46,15 @@ constexpr int kThreads = 320;  // warp 0 TMA, warp 1 MMA, warps 2..9 two epilogu
 constexpr size_t kCounterBytes = 64 * 1024;
 constexpr int kStgPitch = BW * 2 + 16;           // staging row (one token, 128 features) + pad
 constexpr int kStgBytes = 2 * 32 * kStgPitch;    // double buffer of 32 tokens
+constexpr int kBarBytes = 256;
 
 
 struct SkinnyArgs {
   __nv_bfloat16* C;
   int ldc, M, N, K;
-  int m_pad;        // tokens padded to a multiple of 32 (<= 512)
-  int chunk;        // tokens per UMMA instruction: m_pad (<= 256) or m_pad / 2
+  int m_pad;        // tokens padded to whole chunks (<= 512)
+  int chunk;        // tokens per UMMA instruction
+  int units;        // weight blocks (pairs of them) x splits
   int stages;
   int splits;       // k-splits per weight block (pair mode: per pair of weight blocks)
   int kb_per_split;
@@ -176,6 +184,105 @@ __device__ __forceinline__ void readout_rope(const uint8_t* buf, int epi_tid, in
   }
 }
 
+// Sum of the cluster's parked partials (K splits, rank order), bias, activation, rotation, residual, store: tokens
+// 8 split + warp, 8 splits further on, ..., four at a time; lane = features 4 lane .. of the block's 128.
+__device__ __forceinline__ void finish_cluster(const float* dump, int warp, int lane, int split, int n_blk, const SkinnyArgs& a) {
+  constexpr int U = 4;
+  const GemmEpilogue& e = a.epi;
+  const int n = n_blk * BW + 4 * lane;
+  const bool n_ok = n < a.N;
+  const int step = 8 * a.splits;
+  float bias[4] = {0.f, 0.f, 0.f, 0.f};
+  if (e.bias != nullptr) {
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+      if (n + k < a.N) bias[k] = __bfloat162float(e.bias[n + k]);
+  }
+  const bool is_q = n_blk < e.rope_hq, is_v = n_blk >= e.rope_hq + e.rope_hkv;   // with a rope_table: this block's head
+  const uint32_t at = smem_u32(dump) + 16u * lane;
+  for (int m0 = split * 8 + warp; m0 < a.M; m0 += U * step) {
+    float v[U][4];
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+#pragma unroll
+      for (int k = 0; k < 4; ++k) v[u][k] = 0.f;
+#pragma unroll 4
+    for (int s = 0; s < a.splits; ++s) {
+      const uint32_t base = mapa_u32(at, static_cast<uint32_t>(s));
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        if (m0 + u * step >= a.M) continue;
+        const float4 x = ld_dsmem_v4f(base + static_cast<uint32_t>(m0 + u * step) * (BW * 4));
+        v[u][0] += x.x;
+        v[u][1] += x.y;
+        v[u][2] += x.z;
+        v[u][3] += x.w;
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int m = m0 + u * step;
+      if (m >= a.M) break;   // the same for the warp
+#pragma unroll
+      for (int k = 0; k < 4; ++k) v[u][k] += bias[k];
+      if (e.swiglu) {
+        float y[2];
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+          const float zg = v[u][2 * k], zu = v[u][2 * k + 1];
+          y[k] = e.swiglu == 1   ? bf16_round(silu_f(bf16_round(zg))) * bf16_round(zu)
+                 : e.swiglu == 2 ? glu_clamp_fast_f(zg, zu, e.act_pos, e.act_neg)
+                                 : gelu_tanh_f(zg) * zu;
+        }
+        uint32_t o = pack_bf16(y[0], y[1]);
+        if (n_ok && e.residual != nullptr) {
+          const int rr = e.res_row_mod > 0 ? m % e.res_row_mod : m;
+          const uint32_t b = *reinterpret_cast<const uint32_t*>(e.residual + static_cast<size_t>(rr) * e.ld_res + n / 2);
+          o = pack_bf16(bf_lo(o) + bf_lo(b), bf_hi(o) + bf_hi(b));
+        }
+        if (n_ok) *reinterpret_cast<uint32_t*>(a.C + static_cast<size_t>(m) * a.ldc + n / 2) = o;
+        continue;
+      }
+      if (e.act != ACT_NONE) {
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          const float xb = bf16_round(v[u][k]);
+          v[u][k] = e.act == ACT_GELU_TANH  ? gelu_tanh_f(xb)
+                    : e.act == ACT_GELU_ERF ? gelu_erf_f(xb)
+                    : e.act == ACT_RELU2    ? fmaxf(xb, 0.f) * fmaxf(xb, 0.f)
+                    : e.act == ACT_XIELU    ? xielu_fast_f(xb, e.act_pos, e.act_neg)
+                                            : silu_f(xb);
+        }
+      }
+      uint2 o = make_uint2(pack_bf16(v[u][0], v[u][1]), pack_bf16(v[u][2], v[u][3]));
+      __nv_bfloat16* dst = a.C + static_cast<size_t>(m) * a.ldc + n;
+      if (e.rope_table != nullptr) {   // as readout_rope: lanes 0 - 15 hold the pairs' first halves, 16 - 31 their second
+        const uint32_t p0 = __shfl_xor_sync(0xffffffffu, o.x, 16), p1 = __shfl_xor_sync(0xffffffffu, o.y, 16);
+        if (!is_v) {
+          const __nv_bfloat16* t = e.rope_table + static_cast<size_t>(m) * 128 + 4 * (lane & 15);
+          const uint2 cv = *reinterpret_cast<const uint2*>(t), sv = *reinterpret_cast<const uint2*>(t + 64);
+          const float sign = lane < 16 ? -1.f : 1.f;
+          auto turn = [&](uint32_t x, uint32_t y, uint32_t c, uint32_t sn) {
+            return pack_bf16(bf16_round(bf_lo(x) * bf_lo(c)) + bf16_round(sign * bf_lo(y) * bf_lo(sn)),
+                             bf16_round(bf_hi(x) * bf_hi(c)) + bf16_round(sign * bf_hi(y) * bf_hi(sn)));
+          };
+          o = make_uint2(turn(o.x, p0, cv.x, sv.x), turn(o.y, p1, cv.y, sv.y));
+        }
+        if (!is_q && e.k_pool != nullptr) {
+          const int cpos = e.cache_pos0 + m;
+          const int page = e.page_table[cpos >> 7], hk = (n_blk - e.rope_hq) % e.rope_hkv;
+          dst = (is_v ? e.v_pool : e.k_pool) + ((static_cast<size_t>(page) * 128 + (cpos & 127)) * e.rope_hkv + hk) * 128 + 4 * lane;
+        }
+      } else if (n_ok && e.residual != nullptr) {
+        const int rr = e.res_row_mod > 0 ? m % e.res_row_mod : m;
+        const uint2 b = *reinterpret_cast<const uint2*>(e.residual + static_cast<size_t>(rr) * e.ld_res + n);
+        o = make_uint2(pack_bf16(bf_lo(o.x) + bf_lo(b.x), bf_hi(o.x) + bf_hi(b.x)), pack_bf16(bf_lo(o.y) + bf_lo(b.y), bf_hi(o.y) + bf_hi(b.y)));
+      }
+      if (n_ok) *reinterpret_cast<uint2*>(dst) = o;
+    }
+  }
+}
+
 template <bool kPair>
 __global__ void __launch_bounds__(kThreads, 1)
 gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_x,
@@ -189,15 +296,16 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
   uint8_t* bar_base = stg + kStgBytes;
   uint64_t* full_bar = reinterpret_cast<uint64_t*>(bar_base);
   uint64_t* empty_bar = full_bar + 8;
-  uint64_t* acc_full = empty_bar + 8;
-  uint32_t* tmem_ptr = reinterpret_cast<uint32_t*>(acc_full + 1);
+  uint64_t* acc_full = empty_bar + 8;     // [2]: of even and odd weight blocks
+  uint64_t* acc_free = acc_full + 2;      // [2]: the block after this one may be accumulated (the leader's, in a pair)
+  uint32_t* tmem_ptr = reinterpret_cast<uint32_t*>(acc_free + 2);
   uint32_t* last_flag = tmem_ptr + 1;
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, static_cast<int>(threadIdx.x) >> 5, 0), lane = threadIdx.x & 31;
   const uint32_t rank = kPair ? cluster_ctarank() : 0u;
-  const int unit = kPair ? static_cast<int>(blockIdx.x >> 1) : static_cast<int>(blockIdx.x);
-  const int nb = unit / a.splits, split = unit - nb * a.splits;
-  const int n_blk = kPair ? nb * 2 + static_cast<int>(rank) : nb;
+  const int unit0 = kPair ? static_cast<int>(blockIdx.x >> 1) : static_cast<int>(blockIdx.x);
+  const int unit_step = kPair ? static_cast<int>(gridDim.x >> 1) : static_cast<int>(gridDim.x);
+  const int split = unit0 % a.splits;   // more than one: a single unit
   const int nkb = (a.K + BK - 1) / BK;
   const int kb0 = split * a.kb_per_split;
   const int kb1 = min(nkb, kb0 + a.kb_per_split);
@@ -209,7 +317,10 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
       mbar_init(&full_bar[i], 1);
       mbar_init(&empty_bar[i], 1);
     }
-    mbar_init(acc_full, 1);
+    mbar_init(&acc_full[0], 1);
+    mbar_init(&acc_full[1], 1);
+    mbar_init(&acc_free[0], kPair ? 16 : 8);
+    mbar_init(&acc_free[1], kPair ? 16 : 8);
     fence_barrier_init();
   }
   if (warp == 1) {
@@ -231,83 +342,109 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
     asm volatile("mov.u32 %0, %%smid;" : "=r"(smid));
     dbg[6] = smid;
   }
+  // Whole warps whose values are the same in all lanes (they stay in uniform registers); a lane is elected for what is issued.
+  // As a branch of one lane the issue of a product of 144 tokens took 105 clocks of the 79 that the product takes, and the
+  // loads waited for it.
   if (warp == 0) {
-    if (lane == 0) {
-      long long w_empty = 0;
-      // every load of the pair reports to the LEADER's full barrier
-      auto full_addr = [&](int i) {
-        const uint32_t own = smem_u32(&full_bar[i]);
-        return kPair ? mapa_u32(own, 0) : own;
-      };
-      auto load = [&](void* dst, const CUtensorMap* tm, int i, int c0, int c1) {
-        if (kPair) tma_load_2d_pair(dst, tm, full_addr(i), c0, c1);
-        else tma_load_2d(dst, tm, &full_bar[i], c0, c1);
-      };
-      const uint32_t tx_bytes = static_cast<uint32_t>(stage_bytes) * (kPair ? 2u : 1u);
-      // weights are parameters: their first stages are requested before the dependency wait
-      const int pre = a.epi.static_w ? min(a.stages, kb1 - kb0) : 0;
+    long long w_empty = 0;
+    // every load of the pair reports to the LEADER's full barrier
+    auto load = [&](void* dst, const CUtensorMap* tm, int i, int c0, int c1) {
+      if (kPair) tma_load_2d_pair(dst, tm, mapa_u32(smem_u32(&full_bar[i]), 0), c0, c1);
+      else tma_load_2d(dst, tm, &full_bar[i], c0, c1);
+    };
+    const uint32_t tx_bytes = static_cast<uint32_t>(stage_bytes) * (kPair ? 2u : 1u);
+    // weights are parameters: their first stages are requested before the dependency wait
+    int pre = a.epi.static_w ? min(a.stages, kb1 - kb0) : 0;
+    auto w_row = [&](int unit) { return (kPair ? unit / a.splits * 2 + static_cast<int>(rank) : unit / a.splits) * BW; };
+    const bool lead = elect_one();
+    if (lead) {
       for (int i = 0; i < pre; ++i) {
         if (rank == 0) mbar_arrive_expect_tx(&full_bar[i], tx_bytes);
-        load(smem + i * stage_bytes, &tmap_w, i, (kb0 + i) * BK, n_blk * BW);
+        load(smem + i * stage_bytes, &tmap_w, i, (kb0 + i) * BK, w_row(unit0));
       }
-      griddep_wait();
-      int stage = 0;
-      uint32_t phase = 0;
+    }
+    __syncwarp();
+    griddep_wait();
+    int stage = 0;
+    uint32_t phase = 0;
+    for (int unit = unit0; unit < a.units; unit += unit_step) {
+      const int row = w_row(unit);
       for (int kb = kb0; kb < kb1; ++kb) {
         uint8_t* st = smem + stage * stage_bytes;
-        if (kb - kb0 >= pre) {
+        const bool fresh = pre <= 0;
+        if (fresh) {
           const long long c0 = dbg ? clock64() : 0;
           mbar_wait(&empty_bar[stage], phase ^ 1);
           if (dbg) w_empty += clock64() - c0;
-          if (rank == 0) mbar_arrive_expect_tx(&full_bar[stage], tx_bytes);
-          load(st, &tmap_w, stage, kb * BK, n_blk * BW);
+        } else {
+          --pre;
         }
-        uint8_t* xs = st + BW * BK * 2;
-        // one box per UMMA token chunk (rows >= M are zero-filled); a pair CTA stages its half
-        const int box = kPair ? a.chunk / 2 : a.chunk;
-        for (int n0 = 0, o = 0; n0 < a.m_pad; n0 += a.chunk, o += box)
-          load(xs + o * 128, &tmap_x, stage, kb * BK, n0 + static_cast<int>(rank) * box);
+        __syncwarp();
+        if (lead) {
+          if (fresh) {
+            if (rank == 0) mbar_arrive_expect_tx(&full_bar[stage], tx_bytes);
+            load(st, &tmap_w, stage, kb * BK, row);
+          }
+          uint8_t* xs = st + BW * BK * 2;
+          // one box per UMMA token chunk (rows >= M are zero-filled); a pair CTA stages its half
+          const int box = kPair ? a.chunk / 2 : a.chunk;
+          for (int n0 = 0, o = 0; n0 < a.m_pad; n0 += a.chunk, o += box)
+            load(xs + o * 128, &tmap_x, stage, kb * BK, n0 + static_cast<int>(rank) * box);
+        }
+        __syncwarp();
         if (++stage == a.stages) {
           stage = 0;
           phase ^= 1;
         }
       }
-      if (dbg) dbg[4] = w_empty;
     }
+    if (dbg && lane == 0) dbg[4] = w_empty;
   } else if (warp == 1) {
-    if (lane == 0 && kb1 > kb0 && rank == 0) {
-      int stage = 0;
+    if (kb1 > kb0 && rank == 0) {
+      const bool lead = elect_one();   // one thread issues all products: commits speak for its own
+      int stage = 0, tile = 0;
       uint32_t phase = 0;
       long long w_full = 0;
       const long long m0 = dbg ? clock64() : 0;
-      for (int kb = kb0; kb < kb1; ++kb) {
-        const long long c0 = dbg ? clock64() : 0;
-        mbar_wait(&full_bar[stage], phase);
-        if (dbg) w_full += clock64() - c0;
-        tc_fence_after();
-        const uint32_t wa = smem_u32(smem + stage * stage_bytes);
-        const uint32_t xa = wa + BW * BK * 2;
-        const uint32_t idesc = make_idesc_bf16(kPair ? 256 : 128, a.chunk, 0, 0);
-        for (int n0 = 0; n0 < a.m_pad; n0 += a.chunk) {
-          const uint64_t ad = make_smem_desc(wa, 16, 1024, kLayoutSW128);
-          const uint64_t bd = make_smem_desc(xa + (kPair ? n0 / 2 : n0) * 128, 16, 1024, kLayoutSW128);
+      const uint32_t idesc = make_idesc_bf16(kPair ? 256 : 128, a.chunk, 0, 0);
+      const uint64_t wd0 = make_smem_desc(smem_u32(smem), 16, 1024, kLayoutSW128);
+      const uint32_t stage16 = static_cast<uint32_t>(stage_bytes) >> 4, x16 = BW * BK * 2 >> 4;
+      const uint32_t chunk16 = static_cast<uint32_t>(kPair ? a.chunk / 2 : a.chunk) * 128 >> 4;
+      for (int unit = unit0; unit < a.units; unit += unit_step, ++tile) {
+        if (tile > 0) mbar_wait(&acc_free[(tile - 1) & 1], ((tile - 1) >> 1) & 1);
+        for (int kb = kb0; kb < kb1; ++kb) {
+          const long long c0 = dbg ? clock64() : 0;
+          mbar_wait(&full_bar[stage], phase);
+          if (dbg) w_full += clock64() - c0;
+          __syncwarp();
+          const uint64_t ad = wd0 + stage * stage16;
+          tc_fence_after();
+          if (lead) {
+            uint32_t d = tmem_base + ((tile & 1) ? 512 - a.m_pad : 0);
+            uint64_t bd = ad + x16;
+            for (int n0 = 0; n0 < a.m_pad; n0 += a.chunk, d += a.chunk, bd += chunk16) {
 #pragma unroll
-          for (int k = 0; k < BK / 16; ++k) {
-            const uint32_t acc = (kb != kb0 || k != 0) ? 1u : 0u;
-            if (kPair) umma_f16_pair(tmem_base + n0, ad + 2 * k, bd + 2 * k, idesc, acc);
-            else umma_f16(tmem_base + n0, ad + 2 * k, bd + 2 * k, idesc, acc);
+              for (int k = 0; k < BK / 16; ++k) {
+                const uint32_t acc = (kb != kb0 || k != 0) ? 1u : 0u;
+                if (kPair) umma_f16_pair(d, ad + 2 * k, bd + 2 * k, idesc, acc);
+                else umma_f16(d, ad + 2 * k, bd + 2 * k, idesc, acc);
+              }
+            }
+            if (kPair) umma_commit_pair(&empty_bar[stage]);
+            else umma_commit(&empty_bar[stage]);
+            if (kb == kb1 - 1) {
+              if (kPair) umma_commit_pair(&acc_full[tile & 1]);
+              else umma_commit(&acc_full[tile & 1]);
+            }
+          }
+          __syncwarp();
+          if (++stage == a.stages) {
+            stage = 0;
+            phase ^= 1;
           }
         }
-        if (kPair) umma_commit_pair(&empty_bar[stage]);
-        else umma_commit(&empty_bar[stage]);
-        if (++stage == a.stages) {
-          stage = 0;
-          phase ^= 1;
-        }
       }
-      if (kPair) umma_commit_pair(acc_full);
-      else umma_commit(acc_full);
-      if (dbg) {
+      if (dbg && lane == 0) {
         dbg[2] = w_full;
         dbg[3] = clock64() - m0;
       }
@@ -321,8 +458,7 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
   const int wg = warp >= 6 ? 1 : 0;
   const int epi_tid = static_cast<int>(threadIdx.x) - 64 - wg * 128;
   const int n_local = quad * 32 + lane;
-  const int n = n_blk * BW + n_local;
-  const bool n_ok = n < a.N;
+  int n_blk = kPair ? unit0 / a.splits * 2 + static_cast<int>(rank) : unit0 / a.splits;
   const uint32_t t_row = tmem_base + (static_cast<uint32_t>(quad * 32) << 16);
   const int n_chunks = a.m_pad / 32;
   bool finalize = true;
@@ -332,8 +468,8 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
     // ---- phase 1: wait for the accumulator; split-K partials leave TMEM ----
     griddep_wait();
     e0 = dbg ? clock64() : 0;
-    if (kb1 > kb0) {
-      mbar_wait(acc_full, 0);
+    if (kb1 > kb0 && a.splits > 1) {
+      mbar_wait(&acc_full[0], 0);
       tc_fence_after();
     }
     e1 = dbg ? clock64() : 0;
@@ -385,38 +521,62 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
   const long long p1 = dbg ? clock64() : 0;
   if (a.cluster_k) cluster_sync_all();
   const long long p2 = dbg ? clock64() : 0;
-  if (warp >= 2 && finalize) {
+  if (warp >= 2 && a.cluster_k) {
+    // ---- phase 2 of a cluster: a warp per token, four features a lane, 16 bytes of every partial at a time (a feature per lane
+    // and 4 bytes at a time, staged and transposed: 3000 clocks more for 279 tokens); the partials in rank order
+    finish_cluster(dump, warp - 2, lane, split, n_blk, a);
+  } else if (warp >= 2 && finalize) {
     // ---- phase 2: bias / activation / transposition / store ----
     const bool swiglu = a.epi.swiglu != 0;
     const int act = a.epi.act;
-    const bool dsmem = a.cluster_k && a.splits > 1;
-    const float bias = (a.epi.bias != nullptr && n_ok) ? __bfloat162float(a.epi.bias[n]) : 0.f;
-    // output row geometry of this CTA: features [nc0, nc0 + 128 or 64)
-    const int nc0 = swiglu ? (n_blk * BW) >> 1 : n_blk * BW;
     const int n_out = swiglu ? a.N >> 1 : a.N;
-    const int c_first = dsmem ? split : 0, c_step = dsmem ? a.splits : 1;
     uint8_t* buf = stg + wg * (32 * kStgPitch);
+    int tile = 0;
 #pragma unroll 1
-    for (int c = c_first + wg * c_step; c < n_chunks; c += 2 * c_step) {
-      if (c * 32 >= a.M) break;
+    for (int unit = unit0; unit < a.units; unit += unit_step, ++tile) {
+    n_blk = kPair ? unit / a.splits * 2 + static_cast<int>(rank) : unit / a.splits;
+    const int n = n_blk * BW + n_local;
+    const float bias = (a.epi.bias != nullptr && n < a.N) ? __bfloat162float(a.epi.bias[n]) : 0.f;
+    // output row geometry of this weight block: features [nc0, nc0 + 128 or 64)
+    const int nc0 = swiglu ? (n_blk * BW) >> 1 : n_blk * BW;
+    // Weight blocks accumulate in the first and in the last columns in turn.  What both use is read first (of the first ones the
+    // last tokens), then the next block may start; with nothing in common it may as soon as the block before this one is done.
+    const int common = max(0, 2 * a.m_pad - 512) / 32;
+    auto next_may_start = [&]() {
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) {
+        if (kPair) mbar_arrive_cluster(mapa_u32(smem_u32(&acc_free[tile & 1]), 0));
+        else mbar_arrive(&acc_free[tile & 1]);
+      }
+    };
+    if (a.splits == 1) {
+      if (common == 0) next_may_start();
+      mbar_wait(&acc_full[tile & 1], (tile >> 1) & 1);
+      tc_fence_after();
+    }
+    const uint32_t t_tile = t_row + ((tile & 1) ? 512 - a.m_pad : 0);
+    bool told = common == 0;
+#pragma unroll 1
+    for (int i = wg; i < n_chunks; i += 2) {
+      const int c = (tile & 1) ? i : n_chunks - 1 - i;
+      const bool in = c * 32 < a.M;
       float v[32];
-      if (dsmem) {
-        // rank order 0..splits-1 (lowest k first); this CTA's own partial comes from local smem
+      if (a.splits == 1) {
+        if (in) {
+          uint32_t r[32];
+          tmem_ld_32x32b_x32(t_tile + c * 32, r);
+          tmem_ld_wait();
 #pragma unroll
-        for (int j = 0; j < 32; ++j) v[j] = 0.f;
-        const uint32_t off = smem_u32(dump) + static_cast<uint32_t>((c * 32) * BW + n_local) * 4u;
-#pragma unroll 1
-        for (int s = 0; s < a.splits; ++s) {
-          if (s == split) {
-#pragma unroll
-            for (int j = 0; j < 32; ++j) v[j] += dump[(c * 32 + j) * BW + n_local];
-          } else {
-            const uint32_t base = mapa_u32(off, static_cast<uint32_t>(s));
-#pragma unroll
-            for (int j = 0; j < 32; ++j) v[j] += ld_dsmem_f32(base + j * (BW * 4));
-          }
+          for (int j = 0; j < 32; ++j) v[j] = __uint_as_float(r[j]);
         }
-      } else if (a.splits > 1) {
+        if (!told && i + 2 >= common) {
+          next_may_start();
+          told = true;
+        }
+      }
+      if (!in) continue;
+      if (a.splits > 1) {
 #pragma unroll
         for (int j = 0; j < 32; ++j) v[j] = 0.f;
 #pragma unroll 1
@@ -425,12 +585,6 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
 #pragma unroll
           for (int j = 0; j < 32; ++j) v[j] += __ldcg(sp + static_cast<size_t>(j) * BW);
         }
-      } else {
-        uint32_t r[32];
-        tmem_ld_32x32b_x32(t_row + c * 32, r);
-        tmem_ld_wait();
-#pragma unroll
-        for (int j = 0; j < 32; ++j) v[j] = __uint_as_float(r[j]);
       }
       if (swiglu) {
         // lanes (2i, 2i+1) hold (gate_i, up_i) of the interleaved weight rows.  The pair splits the
@@ -483,6 +637,7 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
       else readout<16>(buf, epi_tid, c, nc0, n_out, a);
       epi_group_sync(wg);  // the staging tile may be overwritten
     }
+    }
   }
 
   if (dbg && threadIdx.x == 64) {
@@ -533,11 +688,11 @@ int launch_skinny(const __nv_bfloat16* A, int lda, const __nv_bfloat16* W, int l
   }
   const int x_rows = kPair ? m_pad / 2 : m_pad;
   const int stage_bytes = BW * BK * 2 + x_rows * BK * 2;
-  const int budget = 227 * 1024 - 1024 - kStgBytes - 256;
+  const int budget = 227 * 1024 - 1024 - kStgBytes - kBarBytes;
   int stages = budget / stage_bytes;
   if (stages > 8) stages = 8;
   if (stages < 2) return -1;
-  const size_t smem = static_cast<size_t>(stages) * stage_bytes + kStgBytes + 256 + 1024;
+  const size_t smem = static_cast<size_t>(stages) * stage_bytes + kStgBytes + kBarBytes + 1024;
   auto kern = gemm_skinny_kernel<kPair>;
   static PerDeviceOnce attr_once;
   if (attr_once.first()) {
@@ -584,6 +739,7 @@ int launch_skinny(const __nv_bfloat16* A, int lda, const __nv_bfloat16* W, int l
   a.cluster_k = cluster_k;
   a.m_pad = m_pad;
   a.chunk = m_pad > 256 ? m_pad / 2 : m_pad;  // multiple of 16; pair halves are multiples of 8 rows
+  a.units = nb_units * splits;
   a.splits = splits;
   a.kb_per_split = kb_per_split;
   a.counters = static_cast<int*>(ws_ptr);
@@ -600,7 +756,8 @@ int launch_skinny(const __nv_bfloat16* A, int lda, const __nv_bfloat16* W, int l
   CUtensorMap tw, tx;
   if (make_tmap_2d_bf16(&tw, W, N, K, ldw, BW, BK, 128)) return 1;
   if (make_tmap_2d_bf16(&tx, A, M, K, lda, kPair ? a.chunk / 2 : a.chunk, BK, 128)) return 1;
-  const int grid = nb_units * splits * (kPair ? 2 : 1);
+  // whole weight blocks: a CTA per SM takes them in turn, one's epilogue under the next one's products
+  const int grid = (splits == 1 && a.units > slots ? slots : a.units) * (kPair ? 2 : 1);
   VB_CUDA(launch_pdl_cluster(kern, dim3(grid), dim3(kThreads), smem, stream,
                              dim3(kPair ? 2 : (cluster_k ? splits : 1), 1, 1), tw, tx, a));
   return 0;

@@ -757,8 +757,11 @@ int gemm_bf16(const __nv_bfloat16* A, int lda, const __nv_bfloat16* W, int ldw, 
     // there 33 | 50).  Theirs is too low for large weights on partly filled row blocks: 37888 x 3584 on 279 rows, the third
     // block with 23 of 128, should be 66 and is 81, there 82 (behind other kernels 90 and 82).
     // Without an activation, where they fill one round (no faster than the weights at 4.8 TB/s): 279 rows x
-    // 3088 x 1024 7.9 and 14.2, 200 x 2048 x 2048 9.3 and 14.0, but 3584 x 18944 90 and 55; up to 32 rows and for more than
-    // 8192 outputs never.
+    // 3088 x 1024 7.9 and 14.2, 200 x 2048 x 2048 9.3 and 14.0, but 3584 x 18944 90 and 46; up to 56 rows (40 rows x 4608 x 3584
+    // 12.9 and 10.2, 2560 x 2048 8.7 and 6.8) and for more than 8192 outputs never.
+    // Weights of a round of CTA pairs and more (18944 outputs) go to the swap-AB kernel's pairs, whole blocks of 256 in turn: 6 us +
+    // 0.04 a row + 0.118 a MB, 0.0002 more per row.  40 / 100 / 279 / 384 rows x 37888 x 3584 gated 43 / 46 / 64 / 81 (one CTA a
+    // block 43 / 47 / 71 / 92, tiles 46 / 48 / 82 / 92), 22016 x 2048 20.5 / 21 / 32 / 45 (22 / 24 / 35 / 47 and 22 / 23 / 33 / 34).
     // A projection with a bias and no more onto whole 128-column heads may be the other half of vila_linear_qkv_rope: it
     // stays where that has the same bits (rows that fill their tiles: K halved, as ever).  Without a bias it goes by the
     // time, and the header says so (1024 x 1024 on 279 rows 6.4, there 13.0).
@@ -766,10 +769,12 @@ int gemm_bf16(const __nv_bfloat16* A, int lda, const __nv_bfloat16* W, int ldw, 
     const bool heads = plain && epi.residual == nullptr && epi.bias != nullptr && N % 128 == 0;
     const bool one_round = mb * nb <= sms || mb2 * nb2 <= sms / 2;
     const double t_swap = 6.0 + 0.027 * M + (0.20 + 0.0003 * M) * mbytes;
-    const bool ahead = M > 32 && N <= 8192 && (t_half < 1.05 * t_swap || (one_round && fmax(t_tiles, 4.0 + 0.21 * mbytes) < 0.95 * t_swap));
-    const bool tiles = M <= 16 ? false : heads ? t_half < 1e30 && M * 10 >= mb * 128 * 9 : plain ? ahead : mbytes < 16 || t_half < t_swap || t_tiles < 0.7 * t_swap;
+    const bool whole = (nb + 1) / 2 >= sms / 2;
+    const double t_whole = 6.0 + 0.04 * M + (0.118 + 0.0002 * M) * mbytes;
+    const bool ahead = M > 56 && N <= 8192 && (t_half < 1.05 * t_swap || (one_round && fmax(t_tiles, 4.0 + 0.21 * mbytes) < 0.95 * t_swap));
+    const bool tiles = M <= 16 ? false : heads ? t_half < 1e30 && M * 10 >= mb * 128 * 9 : plain ? ahead : whole ? fmax(1.25 * t_tiles, 4.0 + 0.18 * mbytes) < t_whole : mbytes < 16 || t_half < t_swap || t_tiles < 0.7 * t_swap;
     if (!tiles) {
-      const int rc = gemm_skinny_bf16(A, lda, W, ldw, C, ldc, M, N, K, epi, 0, stream);
+      const int rc = gemm_skinny_bf16(A, lda, W, ldw, C, ldc, M, N, K, epi, whole && M > 16 ? 1 : 0, stream);
       if (rc >= 0) return rc;
     }
     if (heads && t_half < 1e30) return launch_gemm<128, 6, kModeSplitK2>(A, lda, W, ldw, C, ldc, M, N, K, epi, -1, stream);
