@@ -229,6 +229,18 @@ def test_moe_route_forms_agree(ops, rows, cols):
         assert torch.equal(one[0][0], idx[r]) and torch.equal(one[1][0], wt[r]) and torch.equal(one[2][0], gate[r])
 
 
+@pytest.mark.parametrize("rows,cols,pad", [(1184, 4, 4), (1200, 132, 4), (1185, 1028, 12), (1191, 2048, 0)])
+@pytest.mark.parametrize("E,groups", [(8, 2), (32, 4), (33, 3), (100, 5)])
+def test_moe_route_tiles_give_the_bits_of_one_token(ops, rows, cols, pad, E, groups):
+    """tiles of 16 tokens x 32 experts x 128 columns, the last ones in part: choice and weights of a token alone"""
+    g = gen(rows + E)
+    x, w, c = randn(g, rows, cols + pad)[:, :cols], randn(g, E, cols, dtype=F32) * cols ** -0.5, randn(g, E, dtype=F32) * 0.05
+    idx, wt = ops.moe_route_sigmoid(x, w, c, 3, groups, 2)
+    for r in sorted({0, 15, 16, rows // 2, rows - 2, rows - 1}):
+        one = ops.moe_route_sigmoid(x[r:r + 1].contiguous(), w, c, 3, groups, 2)
+        assert torch.equal(one[0][0], idx[r]) and torch.equal(one[1][0], wt[r])
+
+
 @pytest.mark.parametrize("rows,cols,np_", [(1, 4, 1), (3, 1028, 2), (300, 2048, 4), (5, 136, 7)])
 @pytest.mark.parametrize("a_dt", [None, BF, F32])
 def test_residual_add_vec_equals_the_general_form(ops, rows, cols, np_, a_dt):

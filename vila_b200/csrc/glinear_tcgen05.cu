@@ -21,7 +21,7 @@
 // whose sums are rounded, not truncated.
 //
 // Measured against the wmma form it replaces for these operands: the two projections of a routed block of 32 experts
-// (1408 | 704 x 2048, 4 per token) on 2048 tokens 720 -> 149 us (475 and 410 TFLOP/s, tiles of 128 - 256 tokens); the error
+// (1408 | 704 x 2048, 4 per token) on 2048 tokens 720 -> 139 us (94 and 45: tiles of 128 - 256 tokens); the error
 // is the wmma form's (2.1e-6 at K = 2048, one accumulator) or less.
 #include "../../include/vila_b200.h"
 #include "common.cuh"
@@ -31,6 +31,7 @@
 
 #include <atomic>
 #include <mutex>
+#include <type_traits>
 
 namespace vb {
 // A word of pinned host memory that a launch which gave up sets: the host reads it without waiting for the device.
@@ -80,7 +81,7 @@ template <int BT> struct Shape {   // BT: most tokens of a tile
   // error of one long sum grows with its length (K = 2048: 2.1e-6 in one accumulator, 1.0e-6 in two, 4.7e-7 in four)
   static constexpr int kAcc = BT <= 16 ? 4 : (BT <= 64 ? 2 : 1);
   static constexpr int kCols = 2 * kAcc * BT;       // TMEM columns: the CTAs of an SM share 512
-  static constexpr int kMeta = 2 * BT * 12;         // two tiles' output rows, routing weights, input scales
+  static constexpr int kMeta = 2 * BT * 16;         // two tiles' output rows, routing weights, input scales
   static constexpr size_t smem(int groups) { return 1024 + static_cast<size_t>(kStages) * kStage + 256 + kMeta + 8 * (groups + 1); }
 };
 
@@ -140,7 +141,7 @@ glinear_tc_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
   uint64_t* drain_bar = meta_bar + 1;
   uint32_t* tmem_ptr = reinterpret_cast<uint32_t*>(drain_bar + 1);
   volatile int* gave_up = reinterpret_cast<int*>(tmem_ptr + 1);
-  int* orow_s = reinterpret_cast<int*>(smem + ST * S::kStage + 256);   // [2][BT] output row (-1: none)
+  long long* orow_s = reinterpret_cast<long long*>(smem + ST * S::kStage + 256);   // [2][BT] where the output row starts (-1: none)
   float* rs_s = reinterpret_cast<float*>(orow_s + 2 * BT);              // [2][BT] routing weight
   float* is_s = rs_s + 2 * BT;                                          // [2][BT] input scale
   int* first = reinterpret_cast<int*>(is_s + 2 * BT);                   // [2][groups + 1], see tile_at
@@ -341,7 +342,7 @@ glinear_tc_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
       }
       const int cols = (t.count + 15) & ~15, buf = (k & 1) * BT;
       if (tid < cols) {
-        orow_s[buf + tid] = o_next;
+        orow_s[buf + tid] = o_next < 0 ? -1ll : static_cast<long long>(o_next) * p.ldo;
         rs_s[buf + tid] = rs_next;
         is_s[buf + tid] = is_next;
       }
@@ -358,44 +359,54 @@ glinear_tc_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
       const float bias = p.bias && n_ok ? ld_any(p.bias, p.w_dtype, static_cast<size_t>(t.g) * p.bias_group_stride + n) : 0.f;
       const size_t o_col0 = p.mode == 0 ? static_cast<size_t>(t.g) * p.o_group_off : 0;
       const uint32_t acc = tmem + (static_cast<uint32_t>(quad * 32) << 16) + (k & 1) * S::kAcc * BT;
-      for (int t0 = 16 * half; t0 < cols; t0 += 4 * S::kEpi) {
-        float r[16];
-        tmem_ld_32x32b_x16(acc + t0, reinterpret_cast<uint32_t*>(r));
-        tmem_ld_wait();
-        for (int q = 1; q < parts; ++q) {
-          float more[16];
-          tmem_ld_32x32b_x16(acc + t0 + q * BT, reinterpret_cast<uint32_t*>(more));
+      // The output's type is asked once a tile, a row's offset (which the thread that looked the row up multiplied) is added: with both per
+      // output a tile of 128 x 256 took 10400 clocks, twice its products at K = 704.
+      auto write = [&](auto* out) {
+        using T = std::remove_pointer_t<decltype(out)>;
+        auto store = [&](long long off, float v) {
+          if (off >= 0 && n_ok) {
+            if constexpr (sizeof(T) == 4) out[off] = v;
+            else out[off] = __float2bfloat16_rn(v);
+          }
+        };
+        out += EPI >= kGatedEpi ? o_col0 + (n >> 1) : o_col0 + n;
+        for (int t0 = 16 * half; t0 < cols; t0 += 4 * S::kEpi) {
+          float r[16];
+          tmem_ld_32x32b_x16(acc + t0, reinterpret_cast<uint32_t*>(r));
           tmem_ld_wait();
+          for (int q = 1; q < parts; ++q) {
+            float more[16];
+            tmem_ld_32x32b_x16(acc + t0 + q * BT, reinterpret_cast<uint32_t*>(more));
+            tmem_ld_wait();
 #pragma unroll
-          for (int e = 0; e < 16; ++e) r[e] += more[e];
-        }
-        int orow[16];
-        float rs[16], is[16];
-#pragma unroll
-        for (int e = 0; e < 16; e += 4) {
-          *reinterpret_cast<int4*>(orow + e) = *reinterpret_cast<const int4*>(orow_s + buf + t0 + e);
-          *reinterpret_cast<float4*>(rs + e) = *reinterpret_cast<const float4*>(rs_s + buf + t0 + e);
-          *reinterpret_cast<float4*>(is + e) = *reinterpret_cast<const float4*>(is_s + buf + t0 + e);
-        }
-        if (EPI >= kGatedEpi) {
-          // the lanes of a column pair hold gate and up: of two tokens each lane finishes one
-#pragma unroll
-          for (int e = 0; e < 16; e += 2) {
-            const float za = fmaf(r[e], is[e], bias), zb = fmaf(r[e + 1], is[e + 1], bias);
-            const float other = __shfl_xor_sync(0xffffffffu, odd ? za : zb, 1);
-            const int o = odd ? orow[e + 1] : orow[e];
-            const float v = glu(odd ? other : za, odd ? zb : other, EPI - kGatedEpi, x) * (odd ? rs[e + 1] : rs[e]);
-            if (o >= 0 && n_ok) st_any(p.out, p.out_dtype, static_cast<size_t>(o) * p.ldo + o_col0 + (n >> 1), v);
+            for (int e = 0; e < 16; ++e) r[e] += more[e];
           }
-        } else {
 #pragma unroll
-          for (int e = 0; e < 16; ++e) {
-            const float z = fmaf(r[e], is[e], bias);
-            if (orow[e] >= 0 && n_ok)
-              st_any(p.out, p.out_dtype, static_cast<size_t>(orow[e]) * p.ldo + o_col0 + n, activate(z, EPI, x) * rs[e]);
+          for (int e0 = 0; e0 < 16; e0 += 4) {
+            longlong2 off[2];
+            off[0] = *reinterpret_cast<const longlong2*>(orow_s + buf + t0 + e0);
+            off[1] = *reinterpret_cast<const longlong2*>(orow_s + buf + t0 + e0 + 2);
+            const float4 rs4 = *reinterpret_cast<const float4*>(rs_s + buf + t0 + e0), is4 = *reinterpret_cast<const float4*>(is_s + buf + t0 + e0);
+            const float rs[4] = {rs4.x, rs4.y, rs4.z, rs4.w}, is[4] = {is4.x, is4.y, is4.z, is4.w};
+            if (EPI >= kGatedEpi) {
+              // the lanes of a column pair hold gate and up: of two tokens each lane finishes one
+#pragma unroll
+              for (int e = 0; e < 4; e += 2) {
+                const float za = fmaf(r[e0 + e], is[e], bias), zb = fmaf(r[e0 + e + 1], is[e + 1], bias);
+                const float other = __shfl_xor_sync(0xffffffffu, odd ? za : zb, 1);
+                store(odd ? off[e / 2].y : off[e / 2].x,
+                      glu(odd ? other : za, odd ? zb : other, EPI - kGatedEpi, x) * (odd ? rs[e + 1] : rs[e]));
+              }
+            } else {
+#pragma unroll
+              for (int e = 0; e < 4; ++e)
+                store(e & 1 ? off[e / 2].y : off[e / 2].x, activate(fmaf(r[e0 + e], is[e], bias), EPI, x) * rs[e]);
+            }
           }
         }
-      }
+      };
+      if (p.out_dtype == VILA_DT_F32) write(static_cast<float*>(p.out));
+      else write(static_cast<__nv_bfloat16*>(p.out));
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(&acc_free[k & 1]);
