@@ -18,7 +18,8 @@ FLAG_GEGLU = 8
 
 
 def _stream() -> int:
-    return torch.cuda.current_stream().cuda_stream
+    """The current device's current stream.  (torch.cuda.current_stream builds an object for it: 1.5 us of every call.)"""
+    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
 
 
 def _p(t: Optional[torch.Tensor]) -> Optional[int]:
