@@ -476,6 +476,32 @@ def test_paged_attention_decode_skips_empty_tiles(ops):
         assert bool((out[1] == 7.0).all()) and torch.equal(out[0], got[0]) and torch.equal(out[2], got[2])
 
 
+@pytest.mark.parametrize("dim,rot,halves,H,dtype,pool_dtype", [(64, 64, True, 5, BF, BF), (128, 40, False, 3, F32, BF), (128, 56, True, 4, BF, F32),
+                                                               (256, 256, False, 2, BF, BF)])
+@pytest.mark.parametrize("k_values", [False, True])
+def test_rope_append_tokens_of_a_cta(ops, dim, rot, halves, H, dtype, pool_dtype, k_values):
+    """two tokens per CTA and a last one with one: the bits of one per CTA, and within rounding of rows that start off 8 bytes"""
+    T = 4 * torch.cuda.get_device_properties(0).multi_processor_count + 3
+    g, G = gen(dim), 2
+    V = dim if k_values else 20
+    n = (H + G) * dim + (0 if k_values else G * V)
+    qkv = randn(g, T, n, dtype=dtype)
+    off = torch.cat([qkv.new_zeros(1), qkv.flatten()])[1:].view(T, n)
+    pos, rows = (torch.randperm(T, generator=g, device="cuda").int() for _ in range(2))
+    inv = 10000.0 ** (-2.0 * torch.arange(rot // 2, device="cuda", dtype=torch.float64) / rot)
+    out = []
+    for x, step in ((qkv, T), (qkv, 100), (off, T)):
+        pool, q = torch.zeros(T, G * (dim + V), device="cuda", dtype=pool_dtype), []
+        for t in range(0, T, step):
+            s = slice(t, t + step)
+            q.append(ops.rope_append(x[s], pos[s].contiguous(), rows[s].contiguous(), pool, heads=H, kv_heads=G, dim=dim, vdim=V, inv_freq=inv,
+                                     unit_norm=True, eps=1e-5, halves=halves, v_from_k=k_values))
+        out.append((torch.cat(q), pool))
+    assert torch.equal(out[0][0], out[1][0]) and torch.equal(out[0][1], out[1][1])
+    # fp32: the norm's sum of dim squares in another order; bf16: one step of rounding
+    assert rel(out[0][0], out[2][0].double()) < 5e-7 and rel(out[0][1], out[2][1].double()) < (5e-7 if pool_dtype == F32 else 2 ** -7)
+
+
 @pytest.mark.parametrize("dim,rot,halves", [(2, 2, False), (64, 64, True), (96, 32, False), (128, 64, True), (130, 128, False), (256, 256, True)])
 @pytest.mark.parametrize("dtype", [BF, F32])
 def test_rope_append_pairs(ops, dim, rot, halves, dtype):

@@ -207,6 +207,158 @@ __global__ void __launch_bounds__(kThreads) rope_append_pairs_kernel(const vila_
   }
 }
 
+// Head sizes of 64, 128 and 256.  The form above is bound by its instructions (220 a head: 2-byte accesses, a whole warp and
+// 64-bit addresses for one head), not by its bytes, so here a lane has eight columns, two runs of four that are rotated with
+// each other, and a warp 4, 2 or 1 heads at a time; from more than four CTAs an SM on, two tokens share a CTA and the latency
+// of their angles (double sincos).  bf16 in and out, us, before and now: 16 heads of 128 over 4 on 8 / 592 / 800 / 2048 / 4096
+// tokens 3.9 / 6.2 / 7.8 / 15.0 / 27.5, now 3.0 / 4.2 / 4.9 / 9.0 / 15.0; 32 of 64 over 32 6.6 / 9.7 / 12.8 / 24.2 / 51.5, now
+// 3.4 / 5.1 / 6.8 / 12.4 / 29.3 (4.0 TB/s).  One token a CTA: 592 and 800 tokens 4.2 and 6.4, two 4.6 and 4.9; four tokens a CTA
+// are 0.2 - 0.9 ahead of two where there are few heads and 1 - 3 behind where there are 64.
+template <bool BF16>
+struct Four {
+  uint4 raw;
+  __device__ __forceinline__ void load(const void* p, size_t at) {
+    if (BF16) {
+      const uint2 v = *reinterpret_cast<const uint2*>(static_cast<const __nv_bfloat16*>(p) + at);
+      raw.x = v.x;
+      raw.y = v.y;
+    } else {
+      raw = *reinterpret_cast<const uint4*>(static_cast<const float*>(p) + at);
+    }
+  }
+  __device__ __forceinline__ void get(float (&v)[4]) const {
+    if (BF16) {
+      v[0] = bf_lo(raw.x), v[1] = bf_hi(raw.x), v[2] = bf_lo(raw.y), v[3] = bf_hi(raw.y);
+    } else {
+      v[0] = __uint_as_float(raw.x), v[1] = __uint_as_float(raw.y), v[2] = __uint_as_float(raw.z), v[3] = __uint_as_float(raw.w);
+    }
+  }
+};
+__device__ __forceinline__ void store_four(void* p, int dt, size_t at, const float (&v)[4]) {
+  if (dt) *reinterpret_cast<float4*>(static_cast<float*>(p) + at) = make_float4(v[0], v[1], v[2], v[3]);
+  else *reinterpret_cast<uint2*>(static_cast<__nv_bfloat16*>(p) + at) = make_uint2(pack_bf16(v[0], v[1]), pack_bf16(v[2], v[3]));
+}
+
+template <bool BF16, int LPH, int TOK>   // LPH: lanes of a head
+__global__ void __launch_bounds__(kThreads) rope_append_vec_kernel(const vila_rope_append_params p) {
+  extern __shared__ __align__(16) float cs[];   // of each token: cos [rot/2] | sin [rot/2]
+  constexpr int kDim = LPH * 8, kHeads = 32 / LPH;
+  const int t0 = blockIdx.x * TOK, nt = min(TOK, p.T - t0), half = p.rot_dims >> 1;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, sub = lane / LPH, j = lane % LPH;
+  const int maps = maps_of(p.maps), HQ = p.H * maps, GK = p.G * maps, heads = HQ + GK, V = p.G * p.vdim;
+  const int groups = (heads + kHeads - 1) / kHeads;
+  const int koff = GK * kDim, width = koff + V;
+  const bool halves = p.rot_layout == 1, turned = (halves ? 4 * j < half : 8 * j < p.rot_dims);
+  const int c0 = !halves ? 8 * j : turned ? 4 * j : p.rot_dims + 8 * j - 2 * half;
+  const int c1 = halves && turned ? c0 + half : c0 + 4;
+  // this warp's groups of heads, of all tokens one after the other
+  int tok = 0, gr = warp - kWarps;
+  auto step = [&]() {
+    gr += kWarps;
+    while (gr >= groups && tok < nt) {
+      gr -= groups;
+      ++tok;
+    }
+  };
+  Four<BF16> x, y;
+  auto fetch = [&]() {
+    const int hh = gr * kHeads + sub;
+    if (hh >= heads) return;
+    const size_t src = static_cast<size_t>(t0 + tok) * p.ldq + hh * kDim;
+    x.load(p.qkv, src + c0);
+    y.load(p.qkv, src + c1);
+  };
+  step();
+  if (tok < nt) fetch();
+  const float mag = p.rot_mscale != 0.f ? p.rot_mscale : 1.0f;
+  for (int c = tid; c < nt * half; c += kThreads) {
+    const int at = TOK == 1 ? 0 : c / half, i = c - at * half;
+    double s, co;
+    sincos(static_cast<double>(p.positions[t0 + at]) * p.inv_freq[i], &s, &co);
+    cs[at * p.rot_dims + i] = static_cast<float>(co) * mag;
+    cs[at * p.rot_dims + half + i] = static_cast<float>(s) * mag;
+  }
+  __syncthreads();
+  while (tok < nt) {
+    const int t = t0 + tok, hh = gr * kHeads + sub;
+    const bool live = hh < heads, is_q = hh < HQ;
+    float u[4] = {}, v[4] = {}, ru[4], rv[4];
+    if (live) {
+      x.get(u);
+      y.get(v);
+    }
+#pragma unroll
+    for (int k = 0; k < 4; ++k) ru[k] = u[k], rv[k] = v[k];
+    if (turned) {
+      const float* angle = cs + tok * p.rot_dims;
+      if (halves) {
+        const float4 c = *reinterpret_cast<const float4*>(angle + 4 * j), s = *reinterpret_cast<const float4*>(angle + half + 4 * j);
+        const float co[4] = {c.x, c.y, c.z, c.w}, si[4] = {s.x, s.y, s.z, s.w};
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          u[k] = fmaf(ru[k], co[k], -(rv[k] * si[k]));
+          v[k] = fmaf(rv[k], co[k], ru[k] * si[k]);
+        }
+      } else {
+        const float4 c = *reinterpret_cast<const float4*>(angle + 4 * j), s = *reinterpret_cast<const float4*>(angle + half + 4 * j);
+        u[0] = fmaf(ru[0], c.x, -(ru[1] * s.x));
+        u[1] = fmaf(ru[1], c.x, ru[0] * s.x);
+        u[2] = fmaf(ru[2], c.y, -(ru[3] * s.y));
+        u[3] = fmaf(ru[3], c.y, ru[2] * s.y);
+        v[0] = fmaf(rv[0], c.z, -(rv[1] * s.z));
+        v[1] = fmaf(rv[1], c.z, rv[0] * s.z);
+        v[2] = fmaf(rv[2], c.w, -(rv[3] * s.w));
+        v[3] = fmaf(rv[3], c.w, rv[2] * s.w);
+      }
+    }
+    step();
+    if (tok < nt) fetch();
+    if (p.unit_norm) {
+      float ss = 0.f;
+#pragma unroll
+      for (int k = 0; k < 4; ++k) ss = fmaf(u[k], u[k], fmaf(v[k], v[k], ss));
+#pragma unroll
+      for (int o = LPH / 2; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+      const float r = 1.0f / sqrtf(ss / static_cast<float>(kDim) + p.eps);
+#pragma unroll
+      for (int k = 0; k < 4; ++k) u[k] *= r, v[k] *= r;
+    }
+    if (!live) continue;
+    const float* nw = is_q ? p.q_norm_w : p.k_norm_w;
+    if (nw) {
+#pragma unroll
+      for (int k = 0; k < 4; ++k) u[k] *= nw[c0 + k], v[k] *= nw[c1 + k];
+    }
+    if (is_q) {
+      const size_t q = (static_cast<size_t>(t) * HQ + hh) * kDim;
+      store_four(p.q_out, VILA_DT_F32, q + c0, u);
+      store_four(p.q_out, VILA_DT_F32, q + c1, v);
+    } else {
+      const size_t kd = static_cast<size_t>(p.cache_rows[t]) * width + (hh - HQ) * kDim;
+      store_four(p.pool, p.pool_dtype, kd + c0, u);
+      store_four(p.pool, p.pool_dtype, kd + c1, v);
+      if (p.v_from_k) {   // the value is the key as it came in
+        store_four(p.pool, p.pool_dtype, kd + koff + c0, ru);
+        store_four(p.pool, p.pool_dtype, kd + koff + c1, rv);
+      }
+    }
+  }
+  if (p.v_from_k) return;
+  const int per = V >> 2;
+  for (int c = tid; c < nt * per; c += kThreads) {
+    const int at = TOK == 1 ? 0 : c / per, i = (c - at * per) * 4, t = t0 + at;
+    Four<BF16> in;
+    in.load(p.qkv, static_cast<size_t>(t) * p.ldq + heads * kDim + i);
+    float v[4];
+    in.get(v);
+    if (p.v_first)   // part of the value comes from another layer's value of the same token
+#pragma unroll
+      for (int k = 0; k < 4; ++k)
+        v[k] = fmaf(p.v_mix, ld_any(p.v_first, p.v_first_dtype, static_cast<size_t>(t) * p.ld_vf + i + k), (1.0f - p.v_mix) * v[k]);
+    store_four(p.pool, p.pool_dtype, static_cast<size_t>(p.cache_rows[t]) * width + koff + i, v);
+  }
+}
+
 // ---- attention -----------------------------------------------------------------------------------------
 struct AttnShape {
   int BQ;      // query rows per CTA
@@ -925,6 +1077,33 @@ int rope_append(const vila_rope_append_params& p, cudaStream_t stream) {
            "rope_append: H=%d G=%d dim=%d vdim=%d rot_dims=%d v_from_k=%d", p.H, p.G, p.dim, p.vdim, p.rot_dims,
            p.v_from_k);
   const size_t cs_bytes = sizeof(float) * (p.rot_dims + 2);
+  // four columns at a time: every run of four starts on 8 bytes (bf16) or 16 (fp32)
+  const bool fours = (p.dim == 64 || p.dim == 128 || p.dim == 256) && p.rot_dims % 8 == 0 && p.vdim % 4 == 0 && p.ldq % 4 == 0 &&
+                     (reinterpret_cast<uintptr_t>(p.qkv) & (p.qkv_dtype == VILA_DT_BF16 ? 7 : 15)) == 0 &&
+                     (reinterpret_cast<uintptr_t>(p.pool) & (p.pool_dtype == VILA_DT_BF16 ? 7 : 15)) == 0 &&
+                     (reinterpret_cast<uintptr_t>(p.q_out) & 15) == 0;
+  if (fours) {
+    const size_t angles = sizeof(float) * p.rot_dims;
+#define VB_ROPE_TOK(LPH, TOK)                                                                                                     \
+  do {                                                                                                                            \
+    const dim3 grid((p.T + TOK - 1) / TOK);                                                                                       \
+    if (p.qkv_dtype == VILA_DT_BF16)                                                                                              \
+      VB_CUDA(launch_serial(rope_append_vec_kernel<true, LPH, TOK>, grid, dim3(kThreads), TOK * angles, stream, p));              \
+    else                                                                                                                          \
+      VB_CUDA(launch_serial(rope_append_vec_kernel<false, LPH, TOK>, grid, dim3(kThreads), TOK * angles, stream, p));             \
+  } while (0)
+#define VB_ROPE_VEC(LPH)                         \
+  do {                                           \
+    if (p.T > 4 * num_sms()) VB_ROPE_TOK(LPH, 2); \
+    else VB_ROPE_TOK(LPH, 1);                    \
+  } while (0)
+    if (p.dim == 64) VB_ROPE_VEC(8);
+    else if (p.dim == 128) VB_ROPE_VEC(16);
+    else VB_ROPE_VEC(32);
+#undef VB_ROPE_VEC
+#undef VB_ROPE_TOK
+    return 0;
+  }
   if (p.dim % 2 == 0 && p.dim <= 256) {
 #define VB_ROPE(NP)                                                                                                    \
   do {                                                                                                                 \
