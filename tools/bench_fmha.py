@@ -1,4 +1,4 @@
-"""GPU micro-benchmark: tcgen05 FMHA one-tile (v1) vs two-tile (v2) kernels on the NVILA shapes (warm,
+"""GPU micro-benchmark: tcgen05 FMHA with units of one (v1) and two (v2) query tiles on the NVILA shapes (warm,
 CUDA events).  Usage: python tools/bench_fmha.py"""
 import sys, os, json, math
 from pathlib import Path
@@ -15,7 +15,7 @@ def timeit(fn, reps=20):
     e1.record(); torch.cuda.synchronize()
     return e0.elapsed_time(e1) * 1e3 / reps
 res = {}
-for variant, tag in ((1, "v1"), (2, "v2"), (3, "v2_poly4")):
+for variant, tag in ((1, "v1"), (2, "v2")):
   for name, (B, S, H, Hkv, D, causal) in {"vit_1tile": (1, 1024, 16, 16, 72, False), "vit_64": (64, 1024, 16, 16, 72, False),
                                         "llm_279": (1, 279, 28, 4, 128, True), "llm_4k": (1, 4096, 28, 4, 128, True),
                                         "llm_16k": (1, 16470, 28, 4, 128, True),
