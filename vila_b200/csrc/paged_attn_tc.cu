@@ -20,6 +20,10 @@
 //
 // As in fmha2_tcgen05.cu a row's reference maximum moves only when a score exceeds it by 5.5 (a weight of 2^8): exact, since
 // weights, sums and l use the same.
+//
+// Relative error against float64, fp32 out, last 64 rows of 64 / 2048 / 16384 keys: 1.5e-7 / 2.95e-7 / 4.1e-7 (mma.sync 1.5e-7 /
+// 2.95e-7 / 3.9e-7; 3.0e-7 and 4.4e-7 before l kept what its additions lose); values of one sign 9.1e-8 / 1.27e-7 / 2.5e-7 (9.1e-8 /
+// 1.14e-7 / 1.9e-7: there a row's sums are in more accumulators).
 #include "../../include/vila_b200.h"
 #include "common.cuh"
 #include "kernels.h"
@@ -246,6 +250,7 @@ paged_attn_tc_kernel(const __grid_constant__ vila_paged_attn_params p, int tiles
     const int lo = first_key(p, max(pos, 0)), wlo = p.window > 0 ? pos - p.window + 1 : 0, keep = p.window > 0 ? p.keep_first : 0;
     const float cap_inv = cap_inverse(p);
     float m = kNegBig, l = 0.f;
+    float l_lost = 0.f;   // what l's additions rounded away: one sum over all keys of a row weighs on every column
     if (p.sink != nullptr) {
       const float z = p.sink[h];
       if (z >= kNegBig) {   // a sink below every score (-inf: switched off) weighs nothing
@@ -340,6 +345,7 @@ paged_attn_tc_kernel(const __grid_constant__ vila_paged_attn_params p, int tiles
           const float mn = mx > m + kLead ? mx : m;
           const float alpha = ex2(__fsub_rn(log2_units(m), log2_units(mn)));
           l *= alpha;
+          l_lost *= alpha;
 #pragma unroll
           for (int c = 0; c < 64; ++c) o[c] *= alpha;
           m = mn;
@@ -362,7 +368,9 @@ paged_attn_tc_kernel(const __grid_constant__ vila_paged_attn_params p, int tiles
           tmem_st_32x32b_x8(at + 16 + 8 * k, part[1]);
           tmem_st_32x32b_x8(at + 64 + 8 * k, part[2]);
         }
-        l += (l4[0] + l4[1]) + (l4[2] + l4[3]);
+        const float lb = (l4[0] + l4[1]) + (l4[2] + l4[3]), ls = __fadd_rn(l, lb), lt = __fsub_rn(ls, l);
+        l_lost += __fadd_rn(__fsub_rn(l, __fsub_rn(ls, lt)), __fsub_rn(lb, lt));
+        l = ls;
         tmem_st_wait();
         tc_fence_before();
         __syncwarp();
@@ -373,6 +381,7 @@ paged_attn_tc_kernel(const __grid_constant__ vila_paged_attn_params p, int tiles
     }
     if (pending) take(n - 1);
     // ---- rows
+    l += l_lost;
     float z = l * 0.f;
 #pragma unroll
     for (int c = 0; c < 64; ++c) z = fmaf(o[c], 0.f, z);
