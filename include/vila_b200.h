@@ -120,7 +120,8 @@ int vila_fmha(const vila_fmha_params* p, void* stream);
  *   0 heuristic; 1 one query tile at a time; 2 two query tiles, whose softmax and products alternate (one where Sq <= 128);
  *   3 / 4: as 2 */
 int vila_fmha_cfg(int variant, const vila_fmha_params* p, void* stream);
-/* the same with waits that end after `tries` tries (test hook: 0 gives up at once, see vila_wait_status). */
+/* the same with waits that end after `tries` tries (test hook: 0 gives up at once, see vila_wait_status; -2 - r: those of
+ * role r at once, the others as ever; 0 loads, 1 stores, 2 products, 3 softmax). */
 int vila_fmha_tries(int variant, const vila_fmha_params* p, int tries, void* stream);
 
 /* im2col for Conv2d(3,1152,k=14,s=14) (modeling_siglip.py:269-275): pixels [B,C,H,W] ->

@@ -476,6 +476,30 @@ def test_fmha_waits_that_run_out_are_reported(cuda, monkeypatch, variant):
     assert torch.equal(limited(1 << 20), want)
 
 
+@pytest.mark.parametrize("role", [0, 1, 2, 3])
+@pytest.mark.parametrize("D", [72, 128])
+def test_fmha_gives_up_behind_work_in_flight(cuda, D, role):
+    """one role of the CTAs gives up at its first wait while the others' waits hold: loads of a unit of one key block, which wait
+    for nothing, and products behind which nobody looks are drained all the same; the launch ends and the next ones are right"""
+    from vila_b200 import _lib
+    ops, lib = _ops(), _lib.load()
+    g = torch.Generator(device="cuda").manual_seed(role)
+    for (B, S) in ((40, 64), (2, 300), (3, 1000)):
+        q, k, v = (bf(torch.randn(B * S, 16, D, device=cuda, generator=g)) for _ in range(3))
+        for variant in (1, 2):
+            kw = dict(B=B, Sq=S, Sk=S, causal=True, scale=0.1, variant=variant)
+            want = ops.fmha(q, k, v, **kw)
+            for _ in range(3):
+                with pytest.MonkeyPatch.context() as m:
+                    m.setattr(lib, "vila_fmha_cfg", lambda n, p, stream: lib.vila_fmha_tries(n, p, -2 - role, stream))
+                    ops.fmha(q, k, v, **kw)
+                torch.cuda.synchronize()
+                with pytest.raises(RuntimeError, match="ran out"):
+                    ops.check_waits()
+                assert torch.equal(ops.fmha(q, k, v, **kw), want)
+    ops.check_waits()
+
+
 # ------------------------------------------------------------------------------------------------
 # data movement (bit-exact unless averaged)
 # ------------------------------------------------------------------------------------------------

@@ -173,7 +173,8 @@ __device__ __forceinline__ void mbar_wait(uint64_t* bar, uint32_t parity) {
 
 // An mbarrier wait that ends: a lost arrival must not leave the GPU spinning.  The first wait of a CTA that runs out of
 // tries sets `gave_up`, which ends the other warps' waits; a warp whose wait failed leaves its loop for the CTA's last
-// barrier (or, where warps meet at other barriers on the way, runs it to its end without waiting).
+// barrier (or, where warps meet at other barriers on the way, runs it to its end without waiting).  Behind that barrier every
+// warp that has asked for copies or products drains them if `gave_up` is set, whichever warp set it.
 constexpr int kTries = 1 << 20;        // of a wait, then the launch gives up
 constexpr int kDrainTries = 1 << 14;   // of a wait for what is still in flight after that
 __device__ __forceinline__ bool mbar_wait_limited(uint64_t* bar, uint32_t parity, volatile int* gave_up, int tries) {
@@ -184,6 +185,8 @@ __device__ __forceinline__ bool mbar_wait_limited(uint64_t* bar, uint32_t parity
   *gave_up = 1;
   return false;
 }
+// Tries of the waits of a kernel's role: `tries`, or (tests: -2 - r) none for role r and the limit for the others.
+__device__ __forceinline__ int tries_of(int tries, int role) { return tries >= 0 ? tries : tries == -2 - role ? 0 : kTries; }
 __device__ __forceinline__ void mbar_drain(uint64_t* bar, uint32_t parity) {
   for (int i = 0; i < kDrainTries; ++i)
     if (mbar_try_wait(bar, parity)) return;

@@ -201,10 +201,12 @@ fmha_pipe_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
     return true;
   };
   const int rounds = (total + static_cast<int>(gridDim.x) - 1) / static_cast<int>(gridDim.x);
+  int items = 0, qn[2] = {0, 0};   // producer: tiles asked for, of the ring and of the queries
 
   // The producer and the issuers run as whole warps whose values are the same in all lanes (they stay in uniform registers) and
   // elect a lane for what is issued.
-  auto wait = [&](uint64_t* bar, int phase) { return __all_sync(0xffffffffu, mbar_wait_limited(bar, phase & 1, gave_up, tries)); };
+  const int limit = tries_of(tries, warp == C::kProducer ? 0 : warp == C::kStore ? 1 : warp >= C::kMma ? 2 : 3);
+  auto wait = [&](uint64_t* bar, int phase) { return __all_sync(0xffffffffu, mbar_wait_limited(bar, phase & 1, gave_up, limit)); };
   if (warp == C::kProducer) {
     // ===================== TMA producer =====================
     if (elect_one()) {
@@ -212,7 +214,7 @@ fmha_pipe_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
       tma_prefetch_desc(&tm_k);
       tma_prefetch_desc(&tm_v);
     }
-    int slot = 0, ph = 1, items = 0, qn[2] = {0, 0};
+    int slot = 0, ph = 1;
     bool ok = true;
     Unit w;
     for (int r = 0; ok && r < rounds; ++r) {
@@ -257,11 +259,6 @@ fmha_pipe_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
         }
         if (ok) load(&tm_v, tok, page);
       }
-    }
-    if (!ok) {   // copies in flight land before the CTA ends
-      for (int k = max(0, items - R); k < items; ++k) mbar_drain(&r_full[k % R], (k / R) & 1);
-      for (int t = 0; t < TILES; ++t)
-        for (int k = max(0, qn[t] - C::kQ); k < qn[t]; ++k) mbar_drain(&q_full[t * C::kQ + k % C::kQ], (k / C::kQ) & 1);
     }
   } else if (warp == C::kStore) {
     // ===================== rows of O =====================
@@ -373,10 +370,6 @@ fmha_pipe_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
       }
       if (!ok) break;
       units += n > 0;
-    }
-    if (!ok) {   // products in flight end before their operands and TMEM go
-      if (elect_one()) umma_commit(&fin[t]);
-      mbar_drain(&fin[t], 0);
     }
   } else {
     // ===================== softmax =====================
@@ -503,6 +496,21 @@ fmha_pipe_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
 
   tc_fence_before();
   __syncthreads();
+  if (*gave_up) {
+    // Copies and products in flight end before shared memory and TMEM go, also those of warps whose own waits all held: a
+    // producer or an issuer that was through with its work before another warp gave up.
+    if (warp == C::kProducer) {
+      for (int k = max(0, items - R); k < items; ++k) mbar_drain(&r_full[k % R], (k / R) & 1);
+#pragma unroll
+      for (int t = 0; t < TILES; ++t)
+        for (int k = max(0, qn[t] - C::kQ); k < qn[t]; ++k) mbar_drain(&q_full[t * C::kQ + k % C::kQ], (k / C::kQ) & 1);
+    } else if (warp >= C::kMma) {
+      uint64_t* done = &fin[warp - C::kMma];
+      if (elect_one()) umma_commit(done);
+      mbar_drain(done, 0);
+    }
+    __syncthreads();
+  }
   if (warp == C::kMma) {
     tc_fence_after();
     tmem_dealloc<512>(tmem_base);
@@ -577,7 +585,7 @@ int launch_tiles(const FmhaParams& p, int tiles, cudaStream_t stream, int tries)
 
 int fmha_prefill(const FmhaParams& p, cudaStream_t stream) { return fmha_prefill_cfg(0, p, stream); }
 
-// variant: 0 by size, 1 one query tile at a time, 2 (3, 4) two; tries >= 0: of every wait (tests)
+// variant: 0 by size, 1 one query tile at a time, 2 (3, 4) two; tries: of every wait (tests, see tries_of), -1 the kernel's limit
 int fmha_prefill_cfg(int variant, const FmhaParams& p, cudaStream_t stream, int tries) {
   VB_CHECK(variant >= 0 && variant <= 4, "fmha: unknown variant %d", variant);
   VB_CHECK(p.B > 0 && p.Sq > 0 && p.Sk > 0, "fmha: empty problem");
@@ -588,7 +596,7 @@ int fmha_prefill_cfg(int variant, const FmhaParams& p, cudaStream_t stream, int 
            "fmha: strides must be multiples of 8 elements (16 bytes)");
   VB_CHECK(!p.causal || p.Sk >= p.Sq, "fmha: causal needs Sk >= Sq");
   if (wait_status()) return 1;   // an earlier launch gave up: nothing is built on its output
-  if (tries < 0) tries = kTries;
+  if (tries == -1) tries = kTries;
   // Two tiles at a time take 1.6 times as long per key block as one (13 x 16 heads of 1024 keys, head size 72: 23.5 and 14.5
   // us a round of units).  Key blocks per CTA: whole rounds of equal units, or (causal, dealt evenly) the mean, but no less
   // than the longest unit.  1 / 2 / 3 / 4 / 7 / 13 images: one 17, 31, 39, 56, 84, 167 us, two 25, 26, 46, 46, 76, 121; causal,

@@ -71,7 +71,7 @@ struct FmhaParams {
   float scale;      // softmax scale (1/sqrt(D))
 };
 int fmha_prefill(const FmhaParams& p, cudaStream_t stream);
-// variant: 0 by size, 1 one query tile at a time, 2 .. 4 two; tries >= 0: of every wait (tests), otherwise the kernel's limit
+// variant: 0 by size, 1 one query tile at a time, 2 .. 4 two; tries: of every wait (tests), -1: the kernel's limit
 int fmha_prefill_cfg(int variant, const FmhaParams& p, cudaStream_t stream, int tries = -1);
 // split-KV attention for decode at long context (see fmha_tcgen05.cu)
 // counters != nullptr ([Hq] ints, zero-initialised once): the last split CTA of a head combines into p.o
