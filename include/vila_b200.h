@@ -375,7 +375,8 @@ int vila_stalled_waits(void);
  * of host memory and does not synchronise: after a synchronisation it speaks for everything launched before.  vila_glinear
  * and vila_fmha return the same error before they launch anything. */
 int vila_wait_status(void);
-/* vila_glinear on its tensor-core kernel with waits that end after `tries` tries (test hook: 0 gives up at once). */
+/* vila_glinear on its tensor-core kernel with waits that end after `tries` tries (test hook: 0 gives up at once; -2 - r: those
+ * of role r at once, the others as ever; 0 loads, 1 products, 2 gathered rows, 3 epilogue). */
 int vila_glinear_tries(const vila_glinear_params* p, int tries, void* stream);
 
 /* vila_latent_attention — causal attention of H query heads over ONE shared latent per token

@@ -167,6 +167,38 @@ def test_glinear_waits_that_run_out_are_reported(ops, monkeypatch, rows, routed)
     assert torch.equal(limited(1 << 20), want)
 
 
+@pytest.mark.parametrize("role", [0, 1, 2, 3])
+@pytest.mark.parametrize("rows,routed", [(40, False), (9, True), (200, True), (600, True), (600, False)])
+def test_glinear_gives_up_behind_work_in_flight(ops, rows, routed, role):
+    """one role of the CTAs gives up at its first wait while the others' waits hold: tiles that are still landing and products behind
+    which nobody looks are drained all the same; the launch ends and the next ones are right.  K of fewer stages than the ring has"""
+    from vila_b200 import _lib
+    lib, g, N, E = _lib.load(), gen(rows + role), 300, 4
+    if role == 2 and not routed:
+        return   # no rows are gathered
+    for K in (128, 1024):
+        a, w, kw = randn(g, rows, K), randn(g, *((E, N, K) if routed else (N, K))), {}
+        if routed:
+            seg, srt = ops.moe_group(torch.randint(0, E, (rows, 1), generator=g, device="cuda", dtype=torch.int32), E)
+            kw = dict(groups=E, seg=seg, a_rows=srt, a_row_div=1)
+
+        def limited(tries):
+            with pytest.MonkeyPatch.context() as m:
+                m.setattr(lib, "vila_glinear", lambda p, stream: lib.vila_glinear_tries(p, tries, stream))
+                out = ops.glinear(a, w, out_dtype=F32, **kw)
+            torch.cuda.synchronize()
+            return out
+
+        want = limited(1 << 20)
+        ops.check_waits()
+        for _ in range(3):
+            limited(-2 - role)
+            with pytest.raises(RuntimeError, match="ran out"):
+                ops.check_waits()
+            assert torch.equal(limited(1 << 20), want)
+    ops.check_waits()
+
+
 def test_engine_reports_a_step_that_gave_up_before_a_second_one_builds_on_it(ops):
     """a step whose logits nobody reads gives up behind a second of other work: the step after next raises"""
     from vila_b200 import _lib

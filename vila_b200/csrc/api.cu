@@ -378,7 +378,7 @@ int vila_wait_status(void) { return vb::wait_status(); }
 
 int vila_glinear_tries(const vila_glinear_params* p, int tries, void* stream) {
   VB_REQUIRE_DEVICE();
-  return vb::glinear(*p, st(stream), nullptr, tries < 0 ? 0 : tries);
+  return vb::glinear(*p, st(stream), nullptr, tries == -1 ? 0 : tries);
 }
 
 int vila_glinear(const vila_glinear_params* p, void* stream) {

@@ -345,9 +345,9 @@ int glinear(const vila_glinear_params& p, cudaStream_t stream, const vila_glinea
   VB_CHECK(p.act >= VILA_ACT_NONE && p.act <= VILA_ACT_SOFTCAP && (p.act != VILA_ACT_SOFTCAP || x.act_pos > 0.f),
            "glinear: act=%d (cap %f)", p.act, x.act_pos);
   VB_CHECK(p.a_rows == nullptr || p.a_row_div >= 1, "glinear: a_row_div=%d", p.a_row_div);
-  if (tries < 0 && glinear_rows_takes(p)) return glinear_rows(p, stream, x);
+  if (tries == -1 && glinear_rows_takes(p)) return glinear_rows(p, stream, x);
   if (glinear_tc_takes(p)) return glinear_tc(p, stream, x, tries);
-  VB_CHECK(tries < 0, "glinear: the kernel with limited waits does not take this layer");
+  VB_CHECK(tries == -1, "glinear: the kernel with limited waits does not take this layer");
   const bool small = p.M <= 16;
   // few rows: stream the weights once per 16-row chunk instead of tiling
   if ((p.mode == 0 && p.M <= 2 * kSmallRows) || (p.mode == 1 && p.M <= 8 * kSmallRows)) {

@@ -191,10 +191,11 @@ glinear_tc_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
   const uint32_t tmem = *tmem_ptr;
   const int total = p.mode == 0 ? tiles_of(p.M, BT) * n_blocks * p.groups : first[p.groups] * n_blocks;
   bool ok = true;
+  int s = 0, rounds = 0;                  // of the thread that loads: next stage, rounds through all of them
+  const int limit = tries_of(tries, warp == kTma ? 0 : warp == kMma ? 1 : warp >= kGather ? 2 : 3);
 
   if (warp == kTma) {
     if (lane == 0) {
-      int s = 0, rounds = 0;              // rounds: through all the stages
       uint32_t ph = 1;                    // parity to wait for on an empty barrier: the first round passes
       for (int it = blockIdx.x; it < total && ok; it += gridDim.x) {
         const Tile t = tile_at(p, BT, it, n_blocks, first);
@@ -203,7 +204,7 @@ glinear_tc_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
         const int col0 = p.mode == 0 ? t.g * static_cast<int>(p.a_group_off) : 0;
         const uint32_t bytes = kWBytes + boxes * box * kDepth * 2;
         for (int kb = 0; kb < nkb; ++kb) {
-          ok = mbar_wait_limited(&empty_bar[s], ph, gave_up, tries);
+          ok = mbar_wait_limited(&empty_bar[s], ph, gave_up, limit);
           if (!ok) break;
           uint8_t* st = smem + s * S::kStage;
           mbar_arrive_expect_tx(&full_bar[s], bytes);
@@ -217,27 +218,21 @@ glinear_tc_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
           }
         }
       }
-      // requested tiles land before the CTA's memory is given back: stages below s in this round, the others in the last
-      if (!ok)
-        for (int i = 0; i < ST; ++i) {
-          const int round = i < s ? rounds : rounds - 1;
-          if (round >= 0) mbar_drain(&full_bar[i], round & 1);
-        }
     }
   } else if (warp == kMma) {
     if (lane == 0) {
-      int s = 0, k = 0;
+      int k = 0;
       uint32_t ph = 0;
       for (int it = blockIdx.x; it < total && ok; it += gridDim.x) {
         const Tile t = tile_at(p, BT, it, n_blocks, first);
         if (t.count <= 0) continue;
         const uint32_t idesc = make_idesc_bf16(kRowsW, (t.count + 15) & ~15, 0, 0), acc = tmem + (k & 1) * S::kAcc * BT;
-        ok = mbar_wait_limited(&acc_free[k & 1], ((k >> 1) & 1) ^ 1, gave_up, tries);
+        ok = mbar_wait_limited(&acc_free[k & 1], ((k >> 1) & 1) ^ 1, gave_up, limit);
         tc_fence_after();
         int part = 0, left = per_acc;
         uint32_t more = 0;                                // 0: first product of an accumulator
         for (int kb = 0; kb < nkb && ok; ++kb) {
-          ok = mbar_wait_limited(&full_bar[s], ph, gave_up, tries);
+          ok = mbar_wait_limited(&full_bar[s], ph, gave_up, limit);
           if (!ok) break;
           if (gathered) fence_proxy_async_smem();        // the copies that arrived here, before the products below
           tc_fence_after();
@@ -265,10 +260,6 @@ glinear_tc_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
         if (ok) umma_commit(&acc_full[k & 1]);
         ++k;
       }
-      if (!ok) {                          // products under way end before TMEM and the CTA's memory are given back
-        umma_commit(drain_bar);
-        mbar_drain(drain_bar, 0);
-      }
     }
   } else if (warp >= kGather) {
     if (gathered) {
@@ -276,7 +267,6 @@ glinear_tc_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
       const int gt = tid - 32 * kGather, r0 = gt >> 3, c = gt & 7;
       const __nv_bfloat16* A = static_cast<const __nv_bfloat16*>(p.a);
       const uint32_t base = smem_u32(smem) + kWBytes + r0 * 128 + ((c ^ (r0 & 7)) << 4);
-      int s = 0;
       uint32_t ph = 1;
       // the next tile's row indices are on their way while this tile's rows are fetched
       Tile t, next = {0, 0, 0, 0};
@@ -297,7 +287,7 @@ glinear_tc_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
         look(it + gridDim.x);
         if (t.count <= 0) continue;
         for (int kb = 0; kb < nkb; ++kb) {
-          ok = mbar_wait_limited(&empty_bar[s], ph, gave_up, tries);
+          ok = mbar_wait_limited(&empty_bar[s], ph, gave_up, limit);
           if (!ok) break;
           const bool in_k = kb * kDepth + c * 8 < p.K;
 #pragma unroll
@@ -350,8 +340,8 @@ glinear_tc_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
       __syncwarp();
       if (lane == 0) mbar_arrive(meta_bar);
       // all lanes or none: the TMEM loads need the whole warp
-      ok = __all_sync(0xffffffffu, mbar_wait_limited(meta_bar, k & 1, gave_up, tries) &&
-                                       mbar_wait_limited(&acc_full[k & 1], (k >> 1) & 1, gave_up, tries));
+      ok = __all_sync(0xffffffffu, mbar_wait_limited(meta_bar, k & 1, gave_up, limit) &&
+                                       mbar_wait_limited(&acc_full[k & 1], (k >> 1) & 1, gave_up, limit));
       if (!ok) break;
       tc_fence_after();
       const int n = t.n0 + quad * 32 + lane;             // this thread's weight row
@@ -415,6 +405,20 @@ glinear_tc_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
     tc_fence_before();
   }
   __syncthreads();
+  if (*gave_up) {
+    // requested tiles land and products under way end before the CTA's memory and TMEM are given back, also those of a warp that
+    // was through before another one gave up
+    if (warp == kTma && lane == 0) {
+      for (int i = 0; i < ST; ++i) {      // stages below s in this round, the others in the last
+        const int round = i < s ? rounds : rounds - 1;
+        if (round >= 0) mbar_drain(&full_bar[i], round & 1);
+      }
+    } else if (warp == kMma && lane == 0) {
+      umma_commit(drain_bar);
+      mbar_drain(drain_bar, 0);
+    }
+    __syncthreads();
+  }
   if (warp == kMma) {
     tc_fence_after();
     tmem_dealloc<S::kCols>(tmem);
@@ -492,7 +496,7 @@ int glinear_tc(const vila_glinear_params& p, cudaStream_t stream, const vila_gli
   const bool grouped = p.mode == 0 && p.groups > 1;
   const uint64_t a_cols = grouped ? (p.groups - 1) * static_cast<uint64_t>(p.a_group_off) + p.K : p.K;
   if (int rc = make_tmap_2d_bf16(&ta, p.a, p.M, a_cols, p.lda, bt < kBox ? bt : kBox, kDepth, 128)) return rc;
-  if (tries < 0) tries = kTries;
+  if (tries == -1) tries = kTries;
   if (bt == 16) return launch<16>(tm, ta, p, x, tries, stream);
   if (bt == 64) return launch<64>(tm, ta, p, x, tries, stream);
   return launch<256>(tm, ta, p, x, tries, stream);

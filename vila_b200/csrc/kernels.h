@@ -323,7 +323,7 @@ int glinear_tc(const vila_glinear_params& p, cudaStream_t stream, const vila_gli
 // few rows of bf16 operands: fp32 multiply-adds over the streamed weights (glinear_rows.cu)
 bool glinear_rows_takes(const vila_glinear_params& p);
 int glinear_rows(const vila_glinear_params& p, cudaStream_t stream, const vila_glinear_ext& x);
-// tries >= 0: of every wait of the tcgen05 kernel (tests); otherwise its own limit
+// tries: of every wait of the tcgen05 kernel (tests), -1: its own limit
 int glinear(const vila_glinear_params& p, cudaStream_t stream, const vila_glinear_ext* ext = nullptr, int tries = -1);
 int latent_attention(const vila_latent_attn_params& p, cudaStream_t stream);
 int latent_rope_append(const vila_latent_rope_params& p, cudaStream_t stream);
