@@ -626,6 +626,10 @@ typedef struct vila_paged_attn_params {
   float diff_lambda, diff_scale, diff_eps;
 } vila_paged_attn_params;
 int vila_paged_attention(const vila_paged_attn_params* p, void* stream);
+/* the same for prompt portions on its tcgen05 kernel (bf16 pool, 128 | 128 columns, heads not mixed) with waits that end after
+ * `tries` tries (test hook: 0 gives up at once; -2 - r: those of role r at once, the others as ever; 0 loads, 1 products, 2
+ * softmax).  A launch that gives up leaves its output incomplete and is reported by vila_wait_status. */
+int vila_paged_attention_tries(const vila_paged_attn_params* p, int tries, void* stream);
 
 /* Router with sigmoid scores and group-limited choice: s = sigmoid(w_router x) (fp32), choice = s +
  * correction; the experts form `groups` equal groups of neighbours, a group's score is the sum of its

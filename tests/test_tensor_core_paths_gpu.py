@@ -462,6 +462,32 @@ def test_paged_attention_prompt_infinite_entries(ops, form, rep):
             assert int(seen.sum()) > T - 3 and rel(got[seen], ref[seen]) < 3e-6
 
 
+@pytest.mark.parametrize("tries", [0, 1, 3, 30, -2, -3, -4])
+@pytest.mark.parametrize("seqs", [[(9, 0)], [(40, 300), (64, 1)], [(200, 0)]])
+def test_paged_attention_prompt_waits_that_run_out(ops, tries, seqs):
+    """all waits give up at once or somewhere under way, or (negative) those of one role do while the others' hold, so that products
+    are in flight behind which nobody looks: the launch ends, the next status says so once, and the kernel works as before"""
+    from vila_b200 import _lib
+    lib = _lib.load()
+    for form in (dict(softcap=30.0, gate=True), dict(dist_bias=11, chunk=100)):
+        want, ref, (q, pool, tables, tiles, o) = attention_case(ops, form, 8, 2, 128, 128, 64, seqs, seed=3)
+        kw = dict(heads=8, kv_heads=2, dim=128, vdim=128, page=64, scale=0.1, out_dtype=F32, max_rows=16, **o)
+        assert rel(want, ref) < 3e-6
+        ops.check_waits()
+        for _ in range(3):
+            with pytest.MonkeyPatch.context() as m:
+                m.setattr(lib, "vila_paged_attention", lambda p, stream: lib.vila_paged_attention_tries(p, tries, stream))
+                out = ops.paged_attention(q, pool, tables, tiles, **kw)
+            torch.cuda.synchronize()
+            if tries <= 0 or not torch.equal(out, want):
+                with pytest.raises(RuntimeError, match="ran out"):
+                    ops.check_waits()
+            else:
+                lib.vila_wait_status()
+            assert torch.equal(ops.paged_attention(q, pool, tables, tiles, **kw), want)
+    ops.check_waits()
+
+
 MIX_FORMS = {"talk": dict(talk=True), "sink": dict(talk=True, sink=True, softcap=5.0, gate=True), "chunk": dict(talk=True, chunk=24, dist_bias=30),
              "after": dict(talk=True, talk_after=True), "after_window": dict(talk=True, talk_after=True, window=21, keep_first=3, head_scale=True, gate=True)}
 

@@ -313,6 +313,7 @@ SIGNATURES = {
                              c_int, c_void_p],
     "vila_short_conv_state": [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_void_p],
     "vila_rope_append": [C.POINTER(RopeAppendParams), c_void_p],
+    "vila_paged_attention_tries": [C.POINTER(PagedAttnParams), c_int, c_void_p],
     "vila_paged_attention": [C.POINTER(PagedAttnParams), c_void_p],
     "vila_moe_route_sigmoid": [c_void_p, c_int, c_i64, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int,
                                c_int, c_int, c_int, c_void_p],

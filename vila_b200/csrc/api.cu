@@ -473,6 +473,11 @@ int vila_rope_append(const vila_rope_append_params* p, void* stream) {
   return vb::rope_append(*p, st(stream));
 }
 
+int vila_paged_attention_tries(const vila_paged_attn_params* p, int tries, void* stream) {
+  VB_REQUIRE_DEVICE();
+  return vb::paged_attention(*p, st(stream), tries == -1 ? 0 : tries);
+}
+
 int vila_paged_attention(const vila_paged_attn_params* p, void* stream) {
   VB_REQUIRE_DEVICE();
   return vb::paged_attention(*p, st(stream));

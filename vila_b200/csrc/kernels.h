@@ -305,13 +305,14 @@ int rope_append(const vila_rope_append_params& p, cudaStream_t stream);
 bool paged_attention_mix_takes(const vila_paged_attn_params& p);   // prompt portions of mixed heads
 int paged_attention_mix(const vila_paged_attn_params& p, cudaStream_t stream);
 bool paged_attention_tc_takes(const vila_paged_attn_params& p);    // prompt portions, 128 columns
-int paged_attention_tc(const vila_paged_attn_params& p, cudaStream_t stream);
+int paged_attention_tc(const vila_paged_attn_params& p, cudaStream_t stream, int tries);
 bool paged_attention_mma_takes(const vila_paged_attn_params& p);
 int paged_attention_mma(const vila_paged_attn_params& p, cudaStream_t stream);
 // decoded tokens over a bf16 pool, 128 key and value columns, heads not mixed (paged_attn_decode.cu)
 bool paged_attention_decode_takes(const vila_paged_attn_params& p);
 int paged_attention_decode(const vila_paged_attn_params& p, cudaStream_t stream);
-int paged_attention(const vila_paged_attn_params& p, cudaStream_t stream);
+// tries: of every wait of the tcgen05 kernel (tests), -1: its own limit
+int paged_attention(const vila_paged_attn_params& p, cudaStream_t stream, int tries = -1);
 int sink_attention(const vila_sink_attn_params& p, cudaStream_t stream);
 int gather_rows(const void* src, const int32_t* rows, void* dst, int n_rows, int row_bytes, cudaStream_t stream);
 // bf16 operands on 16-byte boundaries with at least 128 weight rows: tcgen05 tiles (glinear_tcgen05.cu)

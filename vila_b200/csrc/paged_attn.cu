@@ -1122,7 +1122,7 @@ int rope_append(const vila_rope_append_params& p, cudaStream_t stream) {
   return 0;
 }
 
-int paged_attention(const vila_paged_attn_params& p, cudaStream_t stream) {
+int paged_attention(const vila_paged_attn_params& p, cudaStream_t stream, int tries) {
   if (p.ntiles <= 0) return 0;
   VB_CHECK(p.H >= 1 && p.G >= 1 && p.H % p.G == 0 && p.dim >= 1 && p.vdim >= 1 && p.page >= 1 && p.nsplit >= 1 &&
                p.nsplit <= 64 && (p.nsplit == 1 || p.partial != nullptr),
@@ -1138,7 +1138,8 @@ int paged_attention(const vila_paged_attn_params& p, cudaStream_t stream) {
            "paged_attention: maps=%d (two maps per head take no head mixing, sink, distance bias or head scale)", p.maps);
   VB_CHECK(p.max_rows >= 1 && p.max_rows <= 16 && (p.nsplit == 1 || p.max_rows == 1),
            "paged_attention: max_rows=%d nsplit=%d (key splitting serves one-row tiles)", p.max_rows, p.nsplit);
-  if (paged_attention_tc_takes(p)) return paged_attention_tc(p, stream);
+  if (paged_attention_tc_takes(p)) return paged_attention_tc(p, stream, tries);
+  VB_CHECK(tries == -1, "paged_attention: the kernel with limited waits does not take this call");
   if (paged_attention_mma_takes(p)) return paged_attention_mma(p, stream);
   if (paged_attention_mix_takes(p)) return paged_attention_mix(p, stream);
   if (paged_attention_decode_takes(p)) return paged_attention_decode(p, stream);

@@ -133,7 +133,8 @@ paged_attn_tc_kernel(const __grid_constant__ vila_paged_attn_params p, int tiles
     r.bl = visible_blocks(p, first_pos, r.nkeys, kBK);
     return true;
   };
-  auto wait = [&](uint64_t* bar, int phase) { return __all_sync(0xffffffffu, mbar_wait_limited(bar, phase & 1, gave_up, tries)); };
+  const int limit = tries_of(tries, warp < 8 ? 2 : warp == kMma ? 1 : 0);
+  auto wait = [&](uint64_t* bar, int phase) { return __all_sync(0xffffffffu, mbar_wait_limited(bar, phase & 1, gave_up, limit)); };
   Run run;
 
   if (warp >= 8 && warp < kMma) {
@@ -233,10 +234,6 @@ paged_attn_tc_kernel(const __grid_constant__ vila_paged_attn_params p, int tiles
         st1 = 0;
         ph1 ^= 1;
       }
-    }
-    if (!ok) {   // products in flight end before their operands and TMEM go
-      if (elect_one()) umma_commit(fin);
-      mbar_drain(fin, 0);
     }
   } else {
     // ===================== softmax =====================
@@ -432,6 +429,13 @@ paged_attn_tc_kernel(const __grid_constant__ vila_paged_attn_params p, int tiles
   }
   tc_fence_before();
   __syncthreads();
+  if (*gave_up) {   // products in flight end before their operands and TMEM go, whichever warp gave up (the loaders' copies have landed)
+    if (warp == kMma) {
+      if (elect_one()) umma_commit(fin);
+      mbar_drain(fin, 0);
+    }
+    __syncthreads();
+  }
   if (warp == kMma) {
     tc_fence_after();
     tmem_dealloc<512>(tmem);
@@ -443,7 +447,7 @@ paged_attn_tc_kernel(const __grid_constant__ vila_paged_attn_params p, int tiles
 }
 
 template <bool CAP>
-int launch(const vila_paged_attn_params& p, cudaStream_t stream) {
+int launch(const vila_paged_attn_params& p, cudaStream_t stream, int tries) {
   volatile unsigned int* failed = failed_word();
   VB_CHECK(failed != nullptr, "paged_attention: no pinned host memory for the status word");
   auto kernel = paged_attn_tc_kernel<CAP>;
@@ -455,7 +459,7 @@ int launch(const vila_paged_attn_params& p, cudaStream_t stream) {
   const bool staged = bias_bytes > 0 && bias_bytes <= kBiasBytes;
   const long ctas = static_cast<long>((p.ntiles + tpc - 1) / tpc) * p.G;
   VB_CHECK(ctas < (1L << 31), "paged_attention: too many tiles");
-  VB_CUDA(launch_serial(kernel, dim3(static_cast<unsigned>(ctas)), dim3(kThreads), kSmem + (staged ? bias_bytes : 0), stream, p, tpc, staged ? p.dist_rows : 0, kTries, failed));
+  VB_CUDA(launch_serial(kernel, dim3(static_cast<unsigned>(ctas)), dim3(kThreads), kSmem + (staged ? bias_bytes : 0), stream, p, tpc, staged ? p.dist_rows : 0, tries, failed));
   return 0;
 }
 
@@ -468,8 +472,9 @@ bool paged_attention_tc_takes(const vila_paged_attn_params& p) {
          p.H / p.G <= 8 && p.G <= 65535 && aligned(p.pool, 16) && aligned(p.q, 16) && aligned(p.out, 16);
 }
 
-int paged_attention_tc(const vila_paged_attn_params& p, cudaStream_t stream) {
-  return p.softcap > 0.f ? launch<true>(p, stream) : launch<false>(p, stream);
+int paged_attention_tc(const vila_paged_attn_params& p, cudaStream_t stream, int tries) {
+  if (tries == -1) tries = kTries;
+  return p.softcap > 0.f ? launch<true>(p, stream, tries) : launch<false>(p, stream, tries);
 }
 
 }  // namespace vb
