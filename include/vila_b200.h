@@ -371,9 +371,10 @@ int vila_glinear(const vila_glinear_params* p, void* stream);
 /* CTAs of vila_glinear's tensor-core kernel that gave up a wait since the process started on the current device (0 in a
  * correct run; the launch's output is then incomplete).  Synchronises; -1: could not be read. */
 int vila_stalled_waits(void);
-/* 0, or 1 once after a launch of that kernel or of vila_fmha which had to give up (vila_last_error says so).  Reads a word
- * of host memory and does not synchronise: after a synchronisation it speaks for everything launched before.  vila_glinear
- * and vila_fmha return the same error before they launch anything. */
+/* 0, or 1 once after a launch of that kernel, of vila_fmha or of vila_paged_attention's tcgen05 kernel which had to give up
+ * (vila_last_error says so).  Reads a word of host memory and does not synchronise: after a synchronisation it speaks for
+ * everything launched before, replays of captured graphs included.  vila_glinear, vila_fmha and vila_paged_attention (where
+ * that kernel serves the call) return the same error before they launch anything; a replay does not ask. */
 int vila_wait_status(void);
 /* vila_glinear on its tensor-core kernel with waits that end after `tries` tries (test hook: 0 gives up at once; -2 - r: those
  * of role r at once, the others as ever; 0 loads, 1 products, 2 gathered rows, 3 epilogue). */

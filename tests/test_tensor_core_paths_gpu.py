@@ -488,6 +488,24 @@ def test_paged_attention_prompt_waits_that_run_out(ops, tries, seqs):
     ops.check_waits()
 
 
+def test_paged_attention_prompt_refuses_to_build_on_a_launch_that_gave_up(ops):
+    """a prompt's attention behind an incomplete one, or behind an incomplete linear layer, raises before it launches anything"""
+    from vila_b200 import _lib
+    lib, g = _lib.load(), gen(2)
+    want, _, (q, pool, tables, tiles, o) = attention_case(ops, {}, 8, 2, 128, 128, 64, [(40, 30)], seed=2)
+    kw = dict(heads=8, kv_heads=2, dim=128, vdim=128, page=64, scale=0.1, out_dtype=F32, max_rows=16)
+    a, w = randn(g, 40, 256), randn(g, 256, 256)
+    for name, call in (("vila_paged_attention", lambda: ops.paged_attention(q, pool, tables, tiles, **kw)), ("vila_glinear", lambda: ops.glinear(a, w))):
+        with pytest.MonkeyPatch.context() as m:
+            m.setattr(lib, name, lambda p, stream: getattr(lib, name + "_tries")(p, 0, stream))
+            call()
+        torch.cuda.synchronize()
+        with pytest.raises(RuntimeError, match="vila_paged_attention.*ran out"):
+            ops.paged_attention(q, pool, tables, tiles, **kw)
+        assert torch.equal(ops.paged_attention(q, pool, tables, tiles, **kw), want)
+    ops.check_waits()
+
+
 MIX_FORMS = {"talk": dict(talk=True), "sink": dict(talk=True, sink=True, softcap=5.0, gate=True), "chunk": dict(talk=True, chunk=24, dist_bias=30),
              "after": dict(talk=True, talk_after=True), "after_window": dict(talk=True, talk_after=True, window=21, keep_first=3, head_scale=True, gate=True)}
 

@@ -473,6 +473,7 @@ bool paged_attention_tc_takes(const vila_paged_attn_params& p) {
 }
 
 int paged_attention_tc(const vila_paged_attn_params& p, cudaStream_t stream, int tries) {
+  if (wait_status()) return 1;   // an earlier launch gave up: nothing is built on its output
   if (tries == -1) tries = kTries;
   return p.softcap > 0.f ? launch<true>(p, stream, tries) : launch<false>(p, stream, tries);
 }

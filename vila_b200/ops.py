@@ -497,9 +497,10 @@ def gated_norm_residual(x: torch.Tensor, part: torch.Tensor, *, n_partials: int 
 
 
 def check_waits() -> None:
-    """Raise if a launch of glinear's tensor-core kernel gave up (a wait of its pipeline ran out of tries) since the last
-    check: its output is incomplete.  Costs a read of host memory; after a synchronisation it speaks for all launches so far."""
-    check(_lib.load().vila_wait_status(), "vila_glinear")
+    """Raise if a launch of a tensor-core kernel with limited waits (glinear, fmha, prompts of paged_attention) gave up since the
+    last check: its output is incomplete.  Costs a read of host memory; after a synchronisation it speaks for all launches so
+    far, replays of captured graphs included."""
+    check(_lib.load().vila_wait_status(), "an earlier launch")
 
 
 def glinear(a: torch.Tensor, w: torch.Tensor, *, out: Optional[torch.Tensor] = None, out_dtype=None,
