@@ -106,6 +106,57 @@ def test_generate_greedy_matches_oracle(cuda, decoder, monkeypatch):
     assert torch.equal(out, out3)
 
 
+@pytest.mark.parametrize("part,call", [("image", "generate"), ("image", "stream"), ("prompt", "generate"), ("prompt", "sample"), ("prompt", "batch")])
+def test_tokens_of_a_launch_that_gave_up_are_not_returned(cuda, part, call):
+    """the attention of a captured graph (image, prompt) or of an eager prompt gives up: whoever reads the tokens raises"""
+    from vila_b200 import _lib
+    from vila_b200.model import tiny_test_config
+    from vila_b200.serving import generate_batch
+    lib = _lib.load()
+    real, limited = lib.vila_fmha, lib.vila_fmha_tries
+    model = build(tiny_test_config(llm_layers=1), seed=6)
+    ids, images = synth_inputs(model.config, n_images=1, n_text=12)
+    px = images[0].cuda()
+    llm = model.llm
+
+    def embed():
+        return model._embed(ids, {"image": [px]}, None, None, None)[0][0]
+
+    def tokens(emb, eos=None):
+        if call == "stream":
+            return [t for chunk in llm.stream_greedy(emb, max_new_tokens=6) for t in chunk]
+        if call == "batch":
+            return generate_batch(llm, [emb], 6, slots=2, max_tokens_per_slot=512)
+        return llm.generate(emb[None], max_new_tokens=6, eos_token_id=eos, do_sample=call == "sample", top_k=1).tolist()
+
+    def clear():
+        torch.cuda.synchronize()
+        lib.vila_wait_status()
+        model._vision_graphs.clear()
+        llm._prefill_graphs.clear()
+
+    emb = embed().clone()
+    want = tokens(emb)
+    eos = want[0][0] if call == "sample" else None   # its first token ends it: no launch follows that would ask
+    clear()
+    with pytest.MonkeyPatch.context() as m:
+        m.setattr(lib, "vila_fmha", lambda p, stream: limited(0, p, 0, stream) if torch.cuda.is_current_stream_capturing() or call in ("sample", "batch")
+                  else real(p, stream))
+        if part == "image":
+            model.encode_images(px[None])
+            torch.cuda.synchronize()
+        else:
+            with pytest.raises(RuntimeError, match="ran out"):
+                tokens(emb, eos)
+    if part == "image":
+        lib.vila_wait_status()
+        with pytest.raises(RuntimeError, match="ran out"):
+            tokens(embed())   # the image's graph is there, the prompt's is made now
+    clear()
+    assert tokens(embed()) == want
+    clear()
+
+
 def test_decode_logits_match_prefill(cuda):
     """KV-cached decode (GEMV + split-KV attention path) must agree with re-running the prefill
     (GEMM + FMHA path) on the extended sequence."""

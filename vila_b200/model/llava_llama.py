@@ -321,6 +321,7 @@ class LlavaLlamaModel(nn.Module):
                 self._vision_graphs[key] = ent
             g, static_in, static_out = ent
             static_in.copy_(images, non_blocking=True)
+            ops.check_waits()   # a replay does not ask by itself whether a launch before it gave up
             g.replay()
             return static_out
         feats = tower(images)  # [n_tiles, N, C]

@@ -208,6 +208,7 @@ class Qwen2ForCausalLM(nn.Module):
             self._prefill_graphs[key] = ent
         g, static_in, static_out, _ = ent
         static_in.copy_(inputs_embeds)
+        ops.check_waits()   # a replay does not ask by itself whether a launch before it gave up
         g.replay()
         cache.length = S
         return static_out
@@ -488,6 +489,7 @@ class Qwen2ForCausalLM(nn.Module):
             e = self.model.embed_tokens(torch.tensor([tok], device=self.device))
             hid = self.prefill_hidden(e, cache)
             logits = self.logits_from_hidden(hid)[0]
+        ops.check_waits()   # the tokens have been read from the device: they are of complete launches
         return ids
 
 
@@ -634,7 +636,9 @@ class GraphDecoder:
         self.cache.length += n
 
     def tokens(self, n: int) -> List[int]:
-        return self.hist[:n].tolist()
+        ids = self.hist[:n].tolist()
+        ops.check_waits()   # everything that these tokens come from has run: none of it gave up
+        return ids
 
 
 class MegaDecoder(GraphDecoder):

@@ -189,7 +189,9 @@ class BatchedDecoder:
 
     def generated(self, slot: int) -> List[int]:
         n = int(self.step_idx[slot, 0])
-        return self.hist[slot, :n].tolist()
+        ids = self.hist[slot, :n].tolist()
+        ops.check_waits()   # everything that these tokens come from has run: none of it gave up
+        return ids
 
 
 @torch.inference_mode()
