@@ -506,6 +506,28 @@ def test_paged_attention_prompt_refuses_to_build_on_a_launch_that_gave_up(ops):
     ops.check_waits()
 
 
+@pytest.mark.parametrize("keys", [64, 128, 192, 256, 512, 704, 2048, 3008])
+@pytest.mark.parametrize("form", ["signs", "one", "chunk"])
+def test_paged_attention_prompt_error_does_not_grow_with_the_keys(ops, keys, form):
+    """rounding of fp32 sums over up to 3008 keys.  Values of one sign: a block's four truncated additions of 16 weights' first
+    parts are 2^-24 each of what they add to, half that on average and all one way (0.8e-7), a row's value is rounded once (0.3e-7
+    rms) and its quotient once; 1.2e-7 holds them, while a plain sum of the blocks adds 1e-8 sqrt(blocks) and is past it from 1000
+    keys on.  Both signs: the weights' own error, of scores whose 128 products are added in two sums of 64, on top: 2.4e-7"""
+    e = []
+    for seed in range(6):
+        g, R, H, G, D = gen(seed), 64, 16, 4, 128
+        q, kv = torch.randn(R, H * D, generator=g, device="cuda"), torch.randn(keys, 2 * G * D, generator=g, device="cuda")
+        if form != "signs":
+            kv[:, G * D:] = kv[:, G * D:].abs()
+        pool, o = kv.to(BF), dict(chunk=512) if form == "chunk" else {}
+        tables = torch.arange(keys // 64, dtype=torch.int32, device="cuda")[None].contiguous()
+        tiles = torch.tensor([(r, 16, keys - R + r, 0) for r in range(0, R, 16)], dtype=torch.int32, device="cuda")
+        got = ops.paged_attention(q, pool, tables, tiles, heads=H, kv_heads=G, dim=D, vdim=D, page=64, scale=D ** -0.5, out_dtype=F32, max_rows=16, **o)
+        want = attention_reference(q, pool, tables, [(0, R, keys - R, 0)], H, G, D, D, 64, D ** -0.5, o)
+        e.append(rel(got, want))
+    assert sum(e) / len(e) < (2.4e-7 if form == "signs" else 1.2e-7)
+
+
 MIX_FORMS = {"talk": dict(talk=True), "sink": dict(talk=True, sink=True, softcap=5.0, gate=True), "chunk": dict(talk=True, chunk=24, dist_bias=30),
              "after": dict(talk=True, talk_after=True), "after_window": dict(talk=True, talk_after=True, window=21, keep_first=3, head_scale=True, gate=True)}
 

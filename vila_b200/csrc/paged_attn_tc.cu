@@ -1,18 +1,20 @@
 // vila_paged_attention for prompt portions over a bf16 pool, 128 key and value columns, on tcgen05 in fp32 precision.
 //
 // What is computed is paged_attn_mma.cu's: queries and weights in three bf16 parts, whose products with bf16 keys and values are
-// exact; the queries' first parts in sums apart from the others; a block's 64 keys in fresh sums of a value column, the parts in
-// ascending size, which join the row's by rounded additions (the tensor core truncates, tcgen05 as mma.sync does); rows that come
-// out infinite or NaN again, key by key.  A row's numbers depend on its own keys only, by blocks at multiples of 64.
+// exact; a score in two sums, of the first 64 columns' first parts and of the rest, small parts first; a block's 64 keys in fresh
+// sums of a value column, the parts in ascending size, which join the row's by rounded additions (the tensor core truncates, tcgen05
+// as mma.sync does), in registers for up to four blocks, which then join those before them in TMEM (a quarter of the roundings
+// of a long sum); rows that come out infinite or NaN again, key by key.  A row's numbers depend on its own keys only, by blocks at
+// multiples of 64.
 //
 // A CTA: 128 rows = 8 groups of a 16-row tile and one of the query heads that share the key / value head.
 //   warps 0 - 7    softmax, two threads a row (keys 0 - 31 and 32 - 63 of a block); the row's sums in their registers (64 columns each)
 //   warps 8, 9     keys and values by cp.async into a ring of 64-key blocks (K-major and MN-major operands, 128-byte swizzle)
 //   warp 10        tcgen05.mma issuer, TMEM
 // (three warps a scheduler: the softmax needs 168 registers a thread)
-// TMEM: two score buffers of 128 columns (64 keys: first parts | other parts), over which the weights' parts come back as the A
-// operand; two buffers of 128 columns for a block's sums.  S(j + 1) is computed under block j's softmax, PV(j) under block
-// j + 1's, whose end takes it in.
+// TMEM: two score buffers of 128 columns (the two sums of 64 keys), over which the weights' parts come back as the A operand; 128
+// columns for a block's sums and 128 for the rows'.  S(j + 1) is computed under block j's softmax, PV(j) under block j + 1's, whose
+// end takes it in before PV(j + 1) may begin.
 //
 // A block takes 2800 clocks without the cap: scores 1200 (24 products of 64 keys, 50 clocks each), sums 800, the issuer's turns; 3400
 // with it (maxima, cap, exponentials and parts 2800, taking in the last block's sums 450).  2048 causal rows of 16 heads over 4: 70
@@ -21,9 +23,10 @@
 // As in fmha2_tcgen05.cu a row's reference maximum moves only when a score exceeds it by 5.5 (a weight of 2^8): exact, since
 // weights, sums and l use the same.
 //
-// Relative error against float64, fp32 out, last 64 rows of 64 / 2048 / 16384 keys: 1.5e-7 / 2.95e-7 / 4.1e-7 (mma.sync 1.5e-7 /
-// 2.95e-7 / 3.9e-7; 3.0e-7 and 4.4e-7 before l kept what its additions lose); values of one sign 9.1e-8 / 1.27e-7 / 2.5e-7 (9.1e-8 /
-// 1.14e-7 / 1.9e-7: there a row's sums are in more accumulators).
+// Relative error against float64 (2-norm, fp32 out, rows on 64 / 512 / 2048 / 3072 keys; mma.sync in brackets), values of both signs:
+// 1.2 / 2.0 / 2.1 / 2.15e-7 (1.5 / 2.8 / 3.0 / 3.05e-7); of one sign: 0.88 / 1.02 / 1.05 / 1.08e-7 (0.92 / 1.04 / 1.14 / 1.21e-7).  With
+// one sum of all first parts and one of all blocks (l compensated as below): 1.5 / 2.8 / 3.0 / 3.05e-7 and 0.92 / 1.06 / 1.27 /
+// 1.40e-7; the two sums of a score cost nothing, a row's groups of four blocks 2 % (2048 capped rows 74.1 -> 75.7 us).
 #include "../../include/vila_b200.h"
 #include "common.cuh"
 #include "kernels.h"
@@ -39,7 +42,7 @@ constexpr int kLoaders = 2, kMma = 8 + kLoaders, kThreads = 32 * (kMma + 1);
 constexpr int kQPart = kM * D * 2;                 // bytes of a part of the queries
 constexpr int kStage = 2 * kBK * D * 2;            // keys, then values
 constexpr int kStages = 3;
-constexpr int kNumBars = 2 * kStages + 7;
+constexpr int kNumBars = 2 * kStages + 6;
 constexpr int kSmem = 3 * kQPart + kStages * kStage + 3 * 2 * kM * 4 + kNumBars * 8 + 16 + 1024;
 constexpr int kBiasBytes = (227 * 1024 - kSmem) / 16 * 16;
 static_assert(kBiasBytes >= 16 * 1024, "paged_attn_tc: shared memory");
@@ -51,6 +54,10 @@ __device__ __forceinline__ bool pair_any(int id, bool v) {   // the two warps of
   return r != 0;
 }
 __device__ __forceinline__ void pair_sync(int id) { asm volatile("bar.sync %0, 64;" ::"r"(id) : "memory"); }
+
+// A row's sums join those in TMEM behind every fourth block of its sequence, and behind the second and the last kept one of a window:
+// by position, so that a row's numbers do not depend on its launch.
+__device__ __forceinline__ bool joins(int block, int kept_blocks) { return (block & 3) == 3 || block == 1 || block == kept_blocks - 1; }
 
 template <bool CAP>
 __global__ void __launch_bounds__(kThreads, 1)
@@ -64,10 +71,10 @@ paged_attn_tc_kernel(const __grid_constant__ vila_paged_attn_params p, int tiles
   int* xodd = reinterpret_cast<int*>(xl + 2 * kM);
   uint64_t* kv_full = reinterpret_cast<uint64_t*>(xodd + 2 * kM);
   uint64_t* kv_empty = kv_full + kStages;
-  uint64_t* s_full = kv_empty + kStages;           // [2], as those below
-  uint64_t* p_full = s_full + 2;
+  uint64_t* s_full = kv_empty + kStages;           // [2]
+  uint64_t* p_full = s_full + 2;                   // [2]
   uint64_t* o_full = p_full + 2;
-  uint64_t* fin = o_full + 2;
+  uint64_t* fin = o_full + 1;
   uint32_t* tmem_ptr = reinterpret_cast<uint32_t*>(fin + 1);
   volatile int* gave_up = reinterpret_cast<int*>(tmem_ptr + 1);
   float* bias_s = reinterpret_cast<float*>(tmem_ptr + 4);   // [head][bias_rows]: the heads' biases by distance, if there is room
@@ -84,8 +91,8 @@ paged_attn_tc_kernel(const __grid_constant__ vila_paged_attn_params p, int tiles
     for (int i = 0; i < 2; ++i) {
       mbar_init(&s_full[i], 1);
       mbar_init(&p_full[i], 8);
-      mbar_init(&o_full[i], 1);
     }
+    mbar_init(o_full, 1);
     mbar_init(fin, 1);
     *gave_up = 0;
     fence_barrier_init();
@@ -196,7 +203,7 @@ paged_attn_tc_kernel(const __grid_constant__ vila_paged_attn_params p, int tiles
         for (int part = 2; part >= 0; --part)
 #pragma unroll
           for (int k = 0; k < D / 16; ++k)
-            umma_f16(d + (part ? 64 : 0), qd + ((part * kQPart + (k >> 2) * (kM * 128) + (k & 3) * 32) >> 4),
+            umma_f16(d + (part || k >= D / 32 ? 64 : 0), qd + ((part * kQPart + (k >> 2) * (kM * 128) + (k & 3) * 32) >> 4),
                      kd + (((k >> 2) * (kBK * 128) + (k & 3) * 32) >> 4), idesc_s, k != 0 || part == 1 ? 1u : 0u);
         umma_commit(&s_full[n & 1]);
       }
@@ -213,19 +220,19 @@ paged_attn_tc_kernel(const __grid_constant__ vila_paged_attn_params p, int tiles
         if (!ok) break;
         issue_s(n + 1, st1);
       }
-      ok = wait(&p_full[n & 1], n >> 1);   // behind it the sums of block n - 2 have been taken in, too
+      ok = wait(&p_full[n & 1], n >> 1);   // behind it the sums of block n - 1 have been taken in, too
       if (!ok) break;
       tc_fence_after();
       if (elect_one()) {
         const uint64_t vd = vd0 + static_cast<uint32_t>(st * (kStage >> 4));
-        const uint32_t a = tmem + (n & 1) * 128, d = tmem + 256 + (n & 1) * 128;
+        const uint32_t a = tmem + (n & 1) * 128, d = tmem + 256;
 #pragma unroll
         for (int part = 2; part >= 0; --part)
 #pragma unroll
           for (int k = 0; k < kBK / 16; ++k)   // keys 16 k ..: of half k / 2, whose parts stand over its own scores
             umma_f16_ts(d, a + (k >> 1) * 32 + (part == 2 ? 64 : 16 * part) + (k & 1) * 8, vd + k * (16 * 128 >> 4), idesc_o,
                         part != 2 || k != 0 ? 1u : 0u);
-        umma_commit(&o_full[n & 1]);
+        umma_commit(o_full);
         umma_commit(&kv_empty[st]);
       }
       __syncwarp();
@@ -260,10 +267,32 @@ paged_attn_tc_kernel(const __grid_constant__ vila_paged_attn_params p, int tiles
     for (int c = 0; c < 64; ++c) o[c] = 0.f;
     int n = 0;            // blocks so far
     bool pending = false; // the sums of block n - 1 have not been taken in
+    int last = 0;         // that block's place in its sequence
+    const uint32_t sums = lanes + 384 + half * 64;
+    bool kept = false;    // there are sums in TMEM
+    // o joins the row's sums in TMEM.  With nothing in o it changes nothing, so that it does not matter whether a row's CTA goes on
+    // over blocks that the row does not see.
+    auto keep_sums = [&]() {
+#pragma unroll
+      for (int c = 0; c < 64; c += 32) {
+        uint32_t t[32];
+        if (kept) {
+          tmem_ld_32x32b_x32(sums + c, t);
+          tmem_ld_wait();
+#pragma unroll
+          for (int e = 0; e < 32; e += 2) add2(o[c + e], o[c + e + 1], __uint_as_float(t[e]), __uint_as_float(t[e + 1]));
+        }
+        tmem_st_32x32b_x32(sums + c, reinterpret_cast<uint32_t*>(o + c));
+#pragma unroll
+        for (int e = 0; e < 32; ++e) o[c + e] = 0.f;
+      }
+      tmem_st_wait();
+      kept = true;
+    };
     auto take = [&](int b) {
-      wait(&o_full[b & 1], b >> 1);
+      wait(o_full, b);
       tc_fence_after();
-      const uint32_t at = lanes + 256 + (b & 1) * 128 + half * 64;
+      const uint32_t at = lanes + 256 + half * 64;
 #pragma unroll
       for (int c = 0; c < 64; c += 32) {
         uint32_t t[32];
@@ -345,6 +374,18 @@ paged_attn_tc_kernel(const __grid_constant__ vila_paged_attn_params p, int tiles
           l_lost *= alpha;
 #pragma unroll
           for (int c = 0; c < 64; ++c) o[c] *= alpha;
+          if (kept) {
+#pragma unroll 1
+            for (int c = 0; c < 64; c += 8) {   // rare: few registers
+              uint32_t t[8];
+              tmem_ld_32x32b_x8(sums + c, t);
+              tmem_ld_wait();
+#pragma unroll
+              for (int e = 0; e < 8; ++e) t[e] = __float_as_uint(__uint_as_float(t[e]) * alpha);
+              tmem_st_32x32b_x8(sums + c, t);
+            }
+            tmem_st_wait();
+          }
           m = mn;
         }
         const float ml = log2_units(m);
@@ -369,14 +410,26 @@ paged_attn_tc_kernel(const __grid_constant__ vila_paged_attn_params p, int tiles
         l_lost += __fadd_rn(__fsub_rn(l, __fsub_rn(ls, lt)), __fsub_rn(lb, lt));
         l = ls;
         tmem_st_wait();
+        if (pending) take(n - 1);   // before this block's product, which goes where these sums are
+        if (n > 0 && joins(last, (keep + kBK - 1) / kBK)) keep_sums();
+        pending = true;
+        last = run.bl.block(v);
         tc_fence_before();
         __syncwarp();
         if (lane == 0) mbar_arrive(&p_full[n & 1]);
-        if (pending) take(n - 1);
-        pending = true;
       }
     }
     if (pending) take(n - 1);
+    if (kept) {
+#pragma unroll
+      for (int c = 0; c < 64; c += 32) {
+        uint32_t t[32];
+        tmem_ld_32x32b_x32(sums + c, t);
+        tmem_ld_wait();
+#pragma unroll
+        for (int e = 0; e < 32; e += 2) add2(o[c + e], o[c + e + 1], __uint_as_float(t[e]), __uint_as_float(t[e + 1]));
+      }
+    }
     // ---- rows
     l += l_lost;
     float z = l * 0.f;
