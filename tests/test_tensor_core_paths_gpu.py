@@ -506,6 +506,21 @@ def test_paged_attention_prompt_refuses_to_build_on_a_launch_that_gave_up(ops):
     ops.check_waits()
 
 
+@pytest.mark.parametrize("form", [dict(), dict(softcap=5.0, sink=True), dict(window=300, keep_first=70), dict(window=90, keep_first=130, dist_bias=40), dict(chunk=200, dist_bias=250)])
+@pytest.mark.parametrize("H,G", [(32, 32), (12, 4), (32, 8), (16, 2)])
+def test_paged_attention_prompt_rows_do_not_depend_on_their_cta(ops, form, H, G):
+    """tiles of several sequences and positions side by side in a CTA, whose other rows see other blocks, against launches of one
+    tile: the same bits, and CTAs of one tile (few rows, heads that do not divide 8) are as right as full ones"""
+    seqs = [(16, 700), (40, 0), (3, 900), (64, 500), (1, 65), (17, 250), (33, 1000), (2, 0), (50, 333), (5, 64)] * (2 if G < 8 else 1)
+    got, want, (q, pool, tables, tiles, o) = attention_case(ops, form, H, G, 128, 128, 64, seqs, seed=H)
+    assert rel(got, want) < 3e-6
+    for t in tiles:
+        r0, n = int(t[0]), int(t[1])
+        alone = ops.paged_attention(q, pool, tables, t[None].contiguous(), heads=H, kv_heads=G, dim=128, vdim=128, page=64, scale=0.1, out_dtype=F32,
+                                    max_rows=16, **o)
+        assert torch.equal(alone[r0:r0 + n], got[r0:r0 + n])
+
+
 @pytest.mark.parametrize("keys", [64, 128, 192, 256, 512, 704, 2048, 3008])
 @pytest.mark.parametrize("form", ["signs", "one", "chunk"])
 def test_paged_attention_prompt_error_does_not_grow_with_the_keys(ops, keys, form):

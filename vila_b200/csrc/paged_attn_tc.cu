@@ -8,8 +8,10 @@
 // multiples of 64.
 //
 // A CTA: 128 rows = 8 groups of a 16-row tile and one of the query heads that share the key / value head.
-//   warps 0 - 7    softmax, two threads a row (keys 0 - 31 and 32 - 63 of a block); the row's sums in their registers (64 columns each)
-//   warps 8, 9     keys and values by cp.async into a ring of 64-key blocks (K-major and MN-major operands, 128-byte swizzle)
+//   warps 0 - 7    queries; softmax, two threads a row (keys 0 - 31 and 32 - 63 of a block); the row's sums in their registers (64
+//                  columns each).  Those whose 32 rows belong to no tile only count the blocks.
+//   warps 8, 9     keys and values by cp.async into a ring of 64-key blocks (K-major and MN-major operands, 128-byte swizzle); the
+//                  first ones come while the queries do
 //   warp 10        tcgen05.mma issuer, TMEM
 // (three warps a scheduler: the softmax needs 168 registers a thread)
 // TMEM: two score buffers of 128 columns (the two sums of 64 keys), over which the weights' parts come back as the A operand; 128
@@ -17,8 +19,10 @@
 // end takes it in before PV(j + 1) may begin.
 //
 // A block takes 2800 clocks without the cap: scores 1200 (24 products of 64 keys, 50 clocks each), sums 800, the issuer's turns; 3400
-// with it (maxima, cap, exponentials and parts 2800, taking in the last block's sums 450).  2048 causal rows of 16 heads over 4: 70
-// us, capped 79 (mma.sync: 186, 193); 1024 rows on 500 keys of 32 heads over 32, capped / chunks of 512 with a bias 240 / 116 -> 104 / 75.
+// with it (maxima, cap, exponentials and parts 2800, taking in the last block's sums 450); a launch of one block 8 - 9 us.  2048
+// causal rows of 16 heads over 4: 60 us, capped 71 (mma.sync: 171, 187); 700 rows on 300 keys of 32 heads over 32, capped / chunks of
+// 512 with a bias 121 / 80 -> 55 / 47; 2 / 33 / 200 rows of 16 over 4 8.4 / 9.2 / 15.8 -> 8.3 / 8.7 / 14.2.  When a warp after the
+// other brought its queries, before the first keys and for rows of no tile too: 9.8 / 12.8 / 15.5.
 //
 // As in fmha2_tcgen05.cu a row's reference maximum moves only when a score exceeds it by 5.5 (a weight of 2^8): exact, since
 // weights, sums and l use the same.
@@ -83,7 +87,7 @@ paged_attn_tc_kernel(const __grid_constant__ vila_paged_attn_params p, int tiles
   // CTAs of late positions, which see most keys, start first, those of all heads
   const int rep = p.H / p.G, g = blockIdx.x % p.G;
   const int tile0 = (static_cast<int>(gridDim.x) / p.G - 1 - static_cast<int>(blockIdx.x) / p.G) * tiles_per_cta, ntile = min(tiles_per_cta, p.ntiles - tile0);
-  if (tid == 0) {
+  if (warp == kMma && lane == 0) {
     for (int i = 0; i < kStages; ++i) {
       mbar_init(&kv_full[i], 32 * kLoaders);
       mbar_init(&kv_empty[i], 1);
@@ -98,28 +102,43 @@ paged_attn_tc_kernel(const __grid_constant__ vila_paged_attn_params p, int tiles
     fence_barrier_init();
   }
   if (warp == kMma) tmem_alloc<512>(tmem_ptr);
-  // queries, scaled, in three parts: row r is row r & 15 of tile (r >> 4) / rep, head (r >> 4) % rep
-  for (int x = tid; x < kM * (D / 4); x += kThreads) {
-    const int r = x / (D / 4), c = 4 * (x % (D / 4)), mt = (r >> 4) / rep, h = g * rep + (r >> 4) % rep;
-    float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (mt < ntile) {
-      const int* t = p.tiles + 4 * (tile0 + mt);
-      if ((r & 15) < t[1]) v = *reinterpret_cast<const float4*>(p.q + (static_cast<size_t>(t[0] + (r & 15)) * p.H + h) * D + c);
-    }
-    const float sc = head_scale(p, h);
-    uint2 part[3];
-    split3(v.x * sc, v.y * sc, part[0].x, part[1].x, part[2].x);
-    split3(v.z * sc, v.w * sc, part[0].y, part[1].y, part[2].y);
-    uint8_t* at = q_s + (c >> 6) * (kM * 128) + r * 128 + ((((c & 63) >> 3) ^ (r & 7)) << 4) + (c & 7) * 2;
-#pragma unroll
-    for (int k = 0; k < 3; ++k) *reinterpret_cast<uint2*>(at + k * kQPart) = part[k];
-  }
-  for (int x = tid; x < rep * bias_rows; x += kThreads) bias_s[x] = p.dist_bias[static_cast<size_t>(x % bias_rows) * p.H + g * rep + x / bias_rows];
-  fence_proxy_async_smem();
   tc_fence_before();
-  __syncthreads();
+  __syncthreads();   // the loaders go ahead, the others meet again behind the queries
   tc_fence_after();
   const uint32_t tmem = *tmem_ptr;
+  if (warp < 8) {
+    // queries, scaled, in three parts: row r is row r & 15 of tile (r >> 4) / rep, head (r >> 4) % rep.  A warp brings a row at a time
+    // and asks for eight before it writes: one after the other their latency was 5 us.  Whole 32 rows of no
+    // tile hold what was there: their warps leave them alone.
+    constexpr int kAhead = 8;
+    for (int r0 = warp; r0 < (16 * rep * ntile + 31) / 32 * 32; r0 += 8 * kAhead) {
+      float4 v[kAhead];
+      float sc[kAhead];
+#pragma unroll
+      for (int u = 0; u < kAhead; ++u) {
+        const int r = r0 + 8 * u, mt = (r >> 4) / rep, h = g * rep + (r >> 4) % rep;
+        v[u] = make_float4(0.f, 0.f, 0.f, 0.f);
+        sc[u] = 0.f;
+        if (mt < ntile) {
+          const int* t = p.tiles + 4 * (tile0 + mt);
+          if ((r & 15) < t[1]) v[u] = *reinterpret_cast<const float4*>(p.q + (static_cast<size_t>(t[0] + (r & 15)) * p.H + h) * D + 4 * lane);
+          sc[u] = head_scale(p, h);
+        }
+      }
+      uint8_t* at = q_s + (lane >> 4) * (kM * 128) + (lane & 1) * 8;
+#pragma unroll
+      for (int u = 0; u < kAhead; ++u) {
+        const int r = r0 + 8 * u;
+        uint2 part[3];
+        split3(v[u].x * sc[u], v[u].y * sc[u], part[0].x, part[1].x, part[2].x);
+        split3(v[u].z * sc[u], v[u].w * sc[u], part[0].y, part[1].y, part[2].y);
+#pragma unroll
+        for (int k = 0; k < 3; ++k) *reinterpret_cast<uint2*>(at + k * kQPart + r * 128 + ((((lane & 15) >> 1) ^ (r & 7)) << 4)) = part[k];
+      }
+    }
+    fence_proxy_async_smem();
+  }
+  if (warp < 8 || warp == kMma) asm volatile("bar.sync 5, 288;" ::: "memory");
 
   // the CTA's tiles in runs of one sequence (nearly always a single run)
   struct Run {
@@ -242,6 +261,14 @@ paged_attn_tc_kernel(const __grid_constant__ vila_paged_attn_params p, int tiles
         ph1 ^= 1;
       }
     }
+  } else if ((warp & 3) * 32 >= 16 * rep * ntile) {
+    // no rows: the weights that stand there reach sums that nobody reads
+    int n = 0;
+    for (int b = 0; next_run(run, b); b = run.end)
+      for (int v = 0; v < run.bl.count; ++v, ++n) {
+        wait(&s_full[n & 1], n >> 1);
+        if (lane == 0) mbar_arrive(&p_full[n & 1]);
+      }
   } else {
     // ===================== softmax =====================
     const int half = warp >> 2, quad = warp & 3, r = quad * 32 + lane, id = 1 + quad;
@@ -253,6 +280,27 @@ paged_attn_tc_kernel(const __grid_constant__ vila_paged_attn_params p, int tiles
     const int pos = i < nrows ? tile[2] + i : -1;
     const int lo = first_key(p, max(pos, 0)), wlo = p.window > 0 ? pos - p.window + 1 : 0, keep = p.window > 0 ? p.keep_first : 0;
     const float cap_inv = cap_inverse(p);
+    if (bias_rows > 0) {   // under the first block's scores
+      // the heads' biases, neighbours in global memory, by the distances that occur
+      int far = 0;
+      for (int mt = 0; mt < ntile; ++mt) far = max(far, p.tiles[4 * (tile0 + mt) + 2] + p.tiles[4 * (tile0 + mt) + 1]);
+      if (p.chunk > 0) far = min(far, p.chunk);
+      const int nbias = rep * min(far, bias_rows), nq = (16 * rep * ntile + 31) / 32;   // pairs of warps that have rows
+      for (int x0 = half * 32 * nq + quad * 32 + lane; x0 < nbias; x0 += 4 * 64 * nq) {
+        float b[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          const int x = x0 + u * 64 * nq;
+          if (x < nbias) b[u] = p.dist_bias[static_cast<size_t>(x / rep) * p.H + g * rep + x % rep];
+        }
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          const int x = x0 + u * 64 * nq;
+          if (x < nbias) bias_s[(x % rep) * bias_rows + x / rep] = b[u];
+        }
+      }
+      asm volatile("bar.sync 6, %0;" ::"r"(64 * nq) : "memory");
+    }
     float m = kNegBig, l = 0.f;
     float l_lost = 0.f;   // what l's additions rounded away: one sum over all keys of a row weighs on every column
     if (p.sink != nullptr) {
@@ -506,7 +554,13 @@ int launch(const vila_paged_attn_params& p, cudaStream_t stream, int tries) {
   auto kernel = paged_attn_tc_kernel<CAP>;
   static PerDeviceOnce once;
   if (once.first()) VB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem + kBiasBytes));
-  const int rep = p.H / p.G, tpc = 8 / rep;
+  // Tiles of a CTA: as few as leave no CTA without an SM, otherwise as many as its 128 rows hold.  A CTA of one tile takes as long
+  // as one of several tiles of a sequence, and tiles of other sequences wait for each other there: 8 sequences of 16 rows on 100 keys,
+  // capped, 16 heads over 4 / over 16 / 32 over 32 19.8 / 48 / 49 us as full as they get and 11.2 / 11.6 / 16.9 so (mma.sync 12.1 / 29 /
+  // 29); 16 of 3 rows on 900 74 / 274 / 274 and 40 / 77 / 145 (50 / 171 / 172).
+  const int rep = p.H / p.G;
+  int tpc = 1;
+  while (tpc < 8 / rep && static_cast<long>((p.ntiles + tpc - 1) / tpc) * p.G > num_sms()) ++tpc;
   // a lookup of every score in global memory, a line apart from row to row, cost more than the rest of a block's softmax
   const long bias_bytes = p.dist_bias ? 4L * rep * p.dist_rows : 0;
   const bool staged = bias_bytes > 0 && bias_bytes <= kBiasBytes;
