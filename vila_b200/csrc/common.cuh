@@ -185,8 +185,13 @@ __device__ __forceinline__ bool mbar_wait_limited(uint64_t* bar, uint32_t parity
   *gave_up = 1;
   return false;
 }
-// Tries of the waits of a kernel's role: `tries`, or (tests: -2 - r) none for role r and the limit for the others.
-__device__ __forceinline__ int tries_of(int tries, int role) { return tries >= 0 ? tries : tries == -2 - role ? 0 : kTries; }
+// Tries of a kernel's waits: `tries` (-1: the limit), or (tests: -2 - r) the limit, and role r gives up before its first wait.
+// A kernel parameter, read from constant memory where a warp waits: as a register of each role it cost vila_fmha's two-tile form,
+// which has none to spare, 10 % of its time.
+struct WaitLimit {
+  int tries, quits;
+};
+inline WaitLimit wait_limit(int tries) { return {tries >= 0 ? tries : kTries, tries < -1 ? -2 - tries : -1}; }
 __device__ __forceinline__ void mbar_drain(uint64_t* bar, uint32_t parity) {
   for (int i = 0; i < kDrainTries; ++i)
     if (mbar_try_wait(bar, parity)) return;

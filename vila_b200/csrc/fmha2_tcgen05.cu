@@ -108,7 +108,7 @@ struct Args {
 template <int DP, int CW, int TILES>
 __global__ void __launch_bounds__(Shape<DP, CW, TILES>::kThreads, 1)
 fmha_pipe_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
-                 const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_o, const Args a, int tries, volatile unsigned int* failed) {
+                 const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_o, const Args a, const WaitLimit limit, volatile unsigned int* failed) {
   using C = Shape<DP, CW, TILES>;
   constexpr int R = C::kRing;
   extern __shared__ uint8_t smem_raw[];
@@ -205,8 +205,8 @@ fmha_pipe_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
 
   // The producer and the issuers run as whole warps whose values are the same in all lanes (they stay in uniform registers) and
   // elect a lane for what is issued.
-  const int limit = tries_of(tries, warp == C::kProducer ? 0 : warp == C::kStore ? 1 : warp >= C::kMma ? 2 : 3);
-  auto wait = [&](uint64_t* bar, int phase) { return __all_sync(0xffffffffu, mbar_wait_limited(bar, phase & 1, gave_up, limit)); };
+  if (limit.quits == (warp == C::kProducer ? 0 : warp == C::kStore ? 1 : warp >= C::kMma ? 2 : 3)) *gave_up = 1;
+  auto wait = [&](uint64_t* bar, int phase) { return __all_sync(0xffffffffu, mbar_wait_limited(bar, phase & 1, gave_up, limit.tries)); };
   if (warp == C::kProducer) {
     // ===================== TMA producer =====================
     if (elect_one()) {
@@ -215,7 +215,7 @@ fmha_pipe_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
       tma_prefetch_desc(&tm_v);
     }
     int slot = 0, ph = 1;
-    bool ok = true;
+    bool ok = limit.quits != 0;
     Unit w;
     for (int r = 0; ok && r < rounds; ++r) {
       if (!unit(r, w)) continue;
@@ -263,7 +263,7 @@ fmha_pipe_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
   } else if (warp == C::kStore) {
     // ===================== rows of O =====================
     int un[2] = {0, 0};
-    bool ok = true;
+    bool ok = limit.quits != 1;
     Unit w;
     for (int r = 0; ok && r < rounds; ++r) {
       if (!unit(r, w)) continue;
@@ -294,7 +294,7 @@ fmha_pipe_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
     const uint64_t kd0 = make_smem_desc(smem_u32(ring_s), 16, C::kSBO, C::kLayout);
     const uint64_t vd0 = make_smem_desc(smem_u32(ring_s), C::kChunkBytes, C::kSBO, C::kLayout);
     const uint32_t o_tmem = tmem_base + 256 + t * 128;
-    bool ok = true;
+    bool ok = limit.quits != 2;
     int slot = 0, ph = 0, g = 0, units = 0;   // ring; blocks and units of the tile so far
     auto advance = [&]() {
       if (++slot == R) {
@@ -572,7 +572,7 @@ int launch(const FmhaParams& p, cudaStream_t stream, int tries) {
   const long total = static_cast<long>(a.units) * p.Hq * p.B;
   VB_CHECK(total < (1L << 30), "fmha: too many query tiles");
   const int grid = static_cast<int>(total < num_sms() ? total : num_sms());
-  VB_CUDA(launch_pdl(kern, dim3(grid), dim3(C::kThreads), C::kSmem, stream, tq, tk, tv, to, a, tries, failed));
+  VB_CUDA(launch_pdl(kern, dim3(grid), dim3(C::kThreads), C::kSmem, stream, tq, tk, tv, to, a, wait_limit(tries), failed));
   return 0;
 }
 
@@ -585,7 +585,7 @@ int launch_tiles(const FmhaParams& p, int tiles, cudaStream_t stream, int tries)
 
 int fmha_prefill(const FmhaParams& p, cudaStream_t stream) { return fmha_prefill_cfg(0, p, stream); }
 
-// variant: 0 by size, 1 one query tile at a time, 2 (3, 4) two; tries: of every wait (tests, see tries_of), -1 the kernel's limit
+// variant: 0 by size, 1 one query tile at a time, 2 (3, 4) two; tries: of every wait (tests, see wait_limit), -1 the kernel's limit
 int fmha_prefill_cfg(int variant, const FmhaParams& p, cudaStream_t stream, int tries) {
   VB_CHECK(variant >= 0 && variant <= 4, "fmha: unknown variant %d", variant);
   VB_CHECK(p.B > 0 && p.Sq > 0 && p.Sk > 0, "fmha: empty problem");
@@ -596,7 +596,6 @@ int fmha_prefill_cfg(int variant, const FmhaParams& p, cudaStream_t stream, int 
            "fmha: strides must be multiples of 8 elements (16 bytes)");
   VB_CHECK(!p.causal || p.Sk >= p.Sq, "fmha: causal needs Sk >= Sq");
   if (wait_status()) return 1;   // an earlier launch gave up: nothing is built on its output
-  if (tries == -1) tries = kTries;
   // Two tiles at a time take 1.6 times as long per key block as one (13 x 16 heads of 1024 keys, head size 72: 23.5 and 14.5
   // us a round of units).  Key blocks per CTA: whole rounds of equal units, or (causal, dealt evenly) the mean, but no less
   // than the longest unit.  1 / 2 / 3 / 4 / 7 / 13 images: one 17, 31, 39, 56, 84, 167 us, two 25, 26, 46, 46, 76, 121; causal,

@@ -128,7 +128,7 @@ constexpr int kGatedEpi = 64;
 template <int BT, int EPI>
 __global__ void __launch_bounds__(Shape<BT>::kThreads, Shape<BT>::kPerSm)
 glinear_tc_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_a,
-                  const vila_glinear_params p, const vila_glinear_ext x, int tries, volatile unsigned int* failed) {
+                  const vila_glinear_params p, const vila_glinear_ext x, const WaitLimit limit, volatile unsigned int* failed) {
   using S = Shape<BT>;
   constexpr int ST = S::kStages, kGather = S::kEpi, kTma = kGather + kGatherWarps, kMma = kTma + 1;
   extern __shared__ uint8_t smem_raw[];
@@ -190,9 +190,10 @@ glinear_tc_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
   tc_fence_after();
   const uint32_t tmem = *tmem_ptr;
   const int total = p.mode == 0 ? tiles_of(p.M, BT) * n_blocks * p.groups : first[p.groups] * n_blocks;
-  bool ok = true;
+  const int role = warp == kTma ? 0 : warp == kMma ? 1 : warp >= kGather ? 2 : 3;
+  bool ok = limit.quits != role;
+  if (!ok) *gave_up = 1;
   int s = 0, rounds = 0;                  // of the thread that loads: next stage, rounds through all of them
-  const int limit = tries_of(tries, warp == kTma ? 0 : warp == kMma ? 1 : warp >= kGather ? 2 : 3);
 
   if (warp == kTma) {
     if (lane == 0) {
@@ -204,7 +205,7 @@ glinear_tc_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
         const int col0 = p.mode == 0 ? t.g * static_cast<int>(p.a_group_off) : 0;
         const uint32_t bytes = kWBytes + boxes * box * kDepth * 2;
         for (int kb = 0; kb < nkb; ++kb) {
-          ok = mbar_wait_limited(&empty_bar[s], ph, gave_up, limit);
+          ok = mbar_wait_limited(&empty_bar[s], ph, gave_up, limit.tries);
           if (!ok) break;
           uint8_t* st = smem + s * S::kStage;
           mbar_arrive_expect_tx(&full_bar[s], bytes);
@@ -227,12 +228,12 @@ glinear_tc_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
         const Tile t = tile_at(p, BT, it, n_blocks, first);
         if (t.count <= 0) continue;
         const uint32_t idesc = make_idesc_bf16(kRowsW, (t.count + 15) & ~15, 0, 0), acc = tmem + (k & 1) * S::kAcc * BT;
-        ok = mbar_wait_limited(&acc_free[k & 1], ((k >> 1) & 1) ^ 1, gave_up, limit);
+        ok = mbar_wait_limited(&acc_free[k & 1], ((k >> 1) & 1) ^ 1, gave_up, limit.tries);
         tc_fence_after();
         int part = 0, left = per_acc;
         uint32_t more = 0;                                // 0: first product of an accumulator
         for (int kb = 0; kb < nkb && ok; ++kb) {
-          ok = mbar_wait_limited(&full_bar[s], ph, gave_up, limit);
+          ok = mbar_wait_limited(&full_bar[s], ph, gave_up, limit.tries);
           if (!ok) break;
           if (gathered) fence_proxy_async_smem();        // the copies that arrived here, before the products below
           tc_fence_after();
@@ -287,7 +288,7 @@ glinear_tc_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
         look(it + gridDim.x);
         if (t.count <= 0) continue;
         for (int kb = 0; kb < nkb; ++kb) {
-          ok = mbar_wait_limited(&empty_bar[s], ph, gave_up, limit);
+          ok = mbar_wait_limited(&empty_bar[s], ph, gave_up, limit.tries);
           if (!ok) break;
           const bool in_k = kb * kDepth + c * 8 < p.K;
 #pragma unroll
@@ -340,8 +341,8 @@ glinear_tc_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
       __syncwarp();
       if (lane == 0) mbar_arrive(meta_bar);
       // all lanes or none: the TMEM loads need the whole warp
-      ok = __all_sync(0xffffffffu, mbar_wait_limited(meta_bar, k & 1, gave_up, limit) &&
-                                       mbar_wait_limited(&acc_full[k & 1], (k >> 1) & 1, gave_up, limit));
+      ok = __all_sync(0xffffffffu, mbar_wait_limited(meta_bar, k & 1, gave_up, limit.tries) &&
+                                       mbar_wait_limited(&acc_full[k & 1], (k >> 1) & 1, gave_up, limit.tries));
       if (!ok) break;
       tc_fence_after();
       const int n = t.n0 + quad * 32 + lane;             // this thread's weight row
@@ -440,7 +441,7 @@ int launch_epi(const CUtensorMap& tm, const CUtensorMap& ta, const vila_glinear_
   const long long tiles = tok * ((p.N + kRowsW - 1) / kRowsW) * (p.mode == 0 ? p.groups : 1);
   VB_CHECK(tiles < (1LL << 31), "glinear: too many tiles (M=%d N=%d groups=%d)", p.M, p.N, p.groups);
   const int grid = static_cast<int>(tiles < S::kPerSm * num_sms() ? tiles : S::kPerSm * num_sms());
-  VB_CUDA(launch_serial(glinear_tc_kernel<BT, EPI>, dim3(grid), dim3(S::kThreads), S::smem(p.mode == 1 ? p.groups : 0), stream, tm, ta, p, x, tries, failed_word()));
+  VB_CUDA(launch_serial(glinear_tc_kernel<BT, EPI>, dim3(grid), dim3(S::kThreads), S::smem(p.mode == 1 ? p.groups : 0), stream, tm, ta, p, x, wait_limit(tries), failed_word()));
   return 0;
 }
 template <int BT>
@@ -496,7 +497,6 @@ int glinear_tc(const vila_glinear_params& p, cudaStream_t stream, const vila_gli
   const bool grouped = p.mode == 0 && p.groups > 1;
   const uint64_t a_cols = grouped ? (p.groups - 1) * static_cast<uint64_t>(p.a_group_off) + p.K : p.K;
   if (int rc = make_tmap_2d_bf16(&ta, p.a, p.M, a_cols, p.lda, bt < kBox ? bt : kBox, kDepth, 128)) return rc;
-  if (tries == -1) tries = kTries;
   if (bt == 16) return launch<16>(tm, ta, p, x, tries, stream);
   if (bt == 64) return launch<64>(tm, ta, p, x, tries, stream);
   return launch<256>(tm, ta, p, x, tries, stream);

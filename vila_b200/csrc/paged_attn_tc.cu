@@ -65,7 +65,7 @@ __device__ __forceinline__ bool joins(int block, int kept_blocks) { return (bloc
 
 template <bool CAP>
 __global__ void __launch_bounds__(kThreads, 1)
-paged_attn_tc_kernel(const __grid_constant__ vila_paged_attn_params p, int tiles_per_cta, int bias_rows, int tries, volatile unsigned int* failed) {
+paged_attn_tc_kernel(const __grid_constant__ vila_paged_attn_params p, int tiles_per_cta, int bias_rows, const WaitLimit limit, volatile unsigned int* failed) {
   extern __shared__ uint8_t raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(raw) + 1023) & ~static_cast<uintptr_t>(1023));
   uint8_t* q_s = smem;                             // [part][64-column chunk][128 rows]
@@ -159,8 +159,8 @@ paged_attn_tc_kernel(const __grid_constant__ vila_paged_attn_params p, int tiles
     r.bl = visible_blocks(p, first_pos, r.nkeys, kBK);
     return true;
   };
-  const int limit = tries_of(tries, warp < 8 ? 2 : warp == kMma ? 1 : 0);
-  auto wait = [&](uint64_t* bar, int phase) { return __all_sync(0xffffffffu, mbar_wait_limited(bar, phase & 1, gave_up, limit)); };
+  if (limit.quits == (warp < 8 ? 2 : warp == kMma ? 1 : 0)) *gave_up = 1;
+  auto wait = [&](uint64_t* bar, int phase) { return __all_sync(0xffffffffu, mbar_wait_limited(bar, phase & 1, gave_up, limit.tries)); };
   Run run;
 
   if (warp >= 8 && warp < kMma) {
@@ -174,7 +174,7 @@ paged_attn_tc_kernel(const __grid_constant__ vila_paged_attn_params p, int tiles
     const size_t off = (static_cast<size_t>(lane < 16 ? 0 : p.G) + g) * D + 8 * c;
     const uint32_t dst = smem_u32(ring) + (lane < 16 ? 0 : kBK * D * 2) + (c >> 3) * (kBK * 128) + k0 * 128;
     int stage = 0, ph = 1;
-    bool ok = true;
+    bool ok = limit.quits != 0;
     for (int b = 0; ok && next_run(run, b); b = run.end) {
       const int32_t* pt = p.page_tables + static_cast<size_t>(run.slot) * p.pt_stride;
       auto look = [&](int v) {   // rows of this warp's keys of block v, -1 behind the last
@@ -212,7 +212,7 @@ paged_attn_tc_kernel(const __grid_constant__ vila_paged_attn_params p, int tiles
     const uint64_t qd = make_smem_desc(smem_u32(q_s), 16, 1024, kLayoutSW128);
     const uint64_t kd0 = make_smem_desc(smem_u32(ring), 16, 1024, kLayoutSW128);
     const uint64_t vd0 = make_smem_desc(smem_u32(ring) + kBK * D * 2, kBK * 128, 1024, kLayoutSW128);
-    bool ok = true;
+    bool ok = limit.quits != 1;
     auto issue_s = [&](int n, int stage) {
       tc_fence_after();
       if (elect_one()) {
@@ -228,7 +228,7 @@ paged_attn_tc_kernel(const __grid_constant__ vila_paged_attn_params p, int tiles
       }
       __syncwarp();
     };
-    if (total > 0) {
+    if (ok && total > 0) {
       ok = wait(&kv_full[0], 0);
       if (ok) issue_s(0, 0);
     }
@@ -566,7 +566,7 @@ int launch(const vila_paged_attn_params& p, cudaStream_t stream, int tries) {
   const bool staged = bias_bytes > 0 && bias_bytes <= kBiasBytes;
   const long ctas = static_cast<long>((p.ntiles + tpc - 1) / tpc) * p.G;
   VB_CHECK(ctas < (1L << 31), "paged_attention: too many tiles");
-  VB_CUDA(launch_serial(kernel, dim3(static_cast<unsigned>(ctas)), dim3(kThreads), kSmem + (staged ? bias_bytes : 0), stream, p, tpc, staged ? p.dist_rows : 0, tries, failed));
+  VB_CUDA(launch_serial(kernel, dim3(static_cast<unsigned>(ctas)), dim3(kThreads), kSmem + (staged ? bias_bytes : 0), stream, p, tpc, staged ? p.dist_rows : 0, wait_limit(tries), failed));
   return 0;
 }
 
@@ -581,7 +581,6 @@ bool paged_attention_tc_takes(const vila_paged_attn_params& p) {
 
 int paged_attention_tc(const vila_paged_attn_params& p, cudaStream_t stream, int tries) {
   if (wait_status()) return 1;   // an earlier launch gave up: nothing is built on its output
-  if (tries == -1) tries = kTries;
   return p.softcap > 0.f ? launch<true>(p, stream, tries) : launch<false>(p, stream, tries);
 }
 
