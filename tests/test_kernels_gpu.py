@@ -476,6 +476,27 @@ def test_fmha_waits_that_run_out_are_reported(cuda, monkeypatch, variant):
     assert torch.equal(limited(1 << 20), want)
 
 
+@pytest.mark.parametrize("D,Sq,Sk,H,variant", [(128, 1024, 16384, 4, 1), (72, 1024, 16384, 4, 1), (64, 1024, 16384, 4, 1), (128, 300, 9000, 16, 0),
+                                               (64, 2304, 9000, 16, 0)])
+def test_fmha_one_tile_sums_are_rounded(cuda, D, Sq, Sk, H, variant):
+    """values of one sign: what the tensor core truncates goes one way and grows with every product that joins a sum (5e-9 of it:
+    4e-5 at 9000 keys, 8e-5 at 16384), rounded additions of blocks of 128 keys have no such mean.  Against the exact result rounded
+    to bf16 the rounding of the output is common to both sides.  What is left does not grow with the keys: 2e-6 - 3.3e-6 at 1024 -
+    16384 of them (eight products of a block, exponentials), whose noise at 5e5 values is 4e-7; 8e-6 lies between the two"""
+    ops = _ops()
+    g = torch.Generator(device="cuda").manual_seed(D + Sk)
+    q, k = (bf(torch.randn(S, H, D, device=cuda, generator=g)) for S in (Sq, Sk))
+    v = bf(torch.rand(Sk, H, D, device=cuda, generator=g) + 0.5)
+    got = ops.fmha(q, k, v, B=1, Sq=Sq, Sk=Sk, causal=False, scale=D ** -0.5, variant=variant)
+    want = torch.empty(Sq, H, D, device=cuda, dtype=torch.float64)
+    for h in range(H):
+        want[:, h] = (q[:, h].double() @ k[:, h].double().T * D ** -0.5).softmax(-1) @ v[:, h].double()
+    bias = float(((got.double() - want.to(torch.bfloat16).double()) / want).mean())
+    assert abs(bias) < 8e-6
+    if variant == 0:   # long keys whose units of two tiles would not fill the card, or of 64 columns
+        assert torch.equal(got, ops.fmha(q, k, v, B=1, Sq=Sq, Sk=Sk, causal=False, scale=D ** -0.5, variant=1))
+
+
 @pytest.mark.parametrize("role", [0, 1, 2, 3])
 @pytest.mark.parametrize("D", [72, 128])
 def test_fmha_gives_up_behind_work_in_flight(cuda, D, role):
