@@ -248,6 +248,18 @@ def test_moe_group_is_a_stable_sort(ops, pairs, E):
     assert torch.equal(srt[:int(seg[-1])].long(), torch.cat(want))
 
 
+@pytest.mark.parametrize("pairs", [257, 512, 2049, 8192, 8193])
+@pytest.mark.parametrize("E", [1, 4, 63, 64, 65, 128, 256, 4096])
+def test_moe_group_at_the_ends_of_its_forms(ops, pairs, E):
+    """scanned and walked counts, lanes kept and found again, one to 32 warps, tables that just fit shared memory and do not"""
+    idx = torch.randint(-1, E + 1, (pairs,), generator=gen(pairs + E), device="cuda", dtype=torch.int32)
+    seg, srt = ops.moe_group(idx, E)
+    order = torch.argsort(torch.where((idx >= 0) & (idx < E), idx, E), stable=True)
+    n = torch.bincount(idx[(idx >= 0) & (idx < E)].long(), minlength=E)
+    assert torch.equal(seg[1:].long(), n.cumsum(0)) and int(seg[0]) == 0
+    assert torch.equal(srt[:int(seg[-1])].long(), order[:int(seg[-1])])
+
+
 @pytest.mark.parametrize("rows", [1, 256, 257, 1184, 1191])
 @pytest.mark.parametrize("cols", [256, 1030])
 def test_moe_route_forms_agree(ops, rows, cols):

@@ -229,19 +229,22 @@ moe_group_kernel(const int32_t* __restrict__ idx, int32_t* __restrict__ seg, int
 // The same grouping with the pairs dealt to the warps instead of the experts: every pair is read twice in all, not once
 // per expert and pass.  A warp owns a run of consecutive pairs; the lanes of one expert find each other with a ballot per
 // bit of the index, so the ranks stay those of the pairs' order (__match_any_sync does the same in one instruction, but
-// its 512 uses were 10 of 16 us).  cnt_s [warps][experts]: first the counts, then the warp's next position.
-// 8192 pairs, 32 experts: 59 -> 12 us, 11 since scans took the place of a thread's walk over the warps' counts; the loop over experts is kept for few pairs (32: 1.9 against 5.1 us) and for
-// tables that do not fit shared memory.
+// its 512 uses were 10 of 16 us).  cnt_s [warps][stride]: first the counts, then the warp's next position.
+// 8192 pairs, 32 experts: 59 -> 11 us; the loop over experts is kept for few pairs (32: 1.9 against 5.1 us) and for tables that do
+// not fit shared memory.
+template <bool SCAN, bool KEEP>   // KEEP: a warp has at most kBatch steps, whose lanes of one expert it keeps
 __global__ void __launch_bounds__(1024)
 moe_group_pairs_kernel(const int32_t* __restrict__ idx, int32_t* __restrict__ seg, int32_t* __restrict__ sorted,
-                       int pairs, int experts) {
-  extern __shared__ int cnt_s[];   // then total_s [experts]
+                       int pairs, int experts, int stride) {
+  extern __shared__ __align__(16) int total_s[];      // SCAN: [experts, whole fours]; then cnt_s [warps][stride]
+  __shared__ int carry_s[32];
   const int wid = threadIdx.x >> 5, lane = lane_id(), nw = blockDim.x >> 5;
-  int* total_s = cnt_s + nw * experts;
+  int* cnt_s = total_s + (SCAN ? (experts + 3) / 4 * 4 : 0);
   const int per = (pairs + 32 * nw - 1) / (32 * nw) * 32, p_begin = wid * per, p_end = min(pairs, p_begin + per);
-  for (int i = threadIdx.x; i < nw * experts; i += blockDim.x) cnt_s[i] = 0;
+  for (int i = threadIdx.x; i < nw * stride; i += blockDim.x) cnt_s[i] = 0;
+  if (SCAN && threadIdx.x < 4) total_s[(experts - 1) / 4 * 4 + threadIdx.x] = 0;
   __syncthreads();
-  int* mine = cnt_s + wid * experts;
+  int* mine = cnt_s + wid * stride;
   const int bits = 32 - __clz(experts);
   auto peers = [&](int e) {                           // lanes with the same e in -1 .. experts - 1
     unsigned m = 0xffffffffu;
@@ -266,49 +269,92 @@ moe_group_pairs_kernel(const int32_t* __restrict__ idx, int32_t* __restrict__ se
     fetch(p0);
 #pragma unroll
     for (int j = 0; j < kBatch; ++j) {
-      const unsigned m = mv[j] = peers(ev[j]);
+      const unsigned m = peers(ev[j]);
+      if (KEEP) mv[j] = m;
       if (ev[j] >= 0 && lane == __ffs(m) - 1) mine[ev[j]] += __popc(m);
       __syncwarp();
     }
   }
   __syncthreads();
-  // exclusive prefix over (expert, warp): a warp per expert scans the warps' counts, the first warp the experts' totals
-  for (int e = wid; e < experts; e += nw) {
-    const int n = lane < nw ? cnt_s[lane * experts + e] : 0;
-    int end = n;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const int v = __shfl_up_sync(0xffffffffu, end, o);
-      if (lane >= o) end += v;
+  // exclusive prefix over (expert, warp)
+  if constexpr (SCAN) {
+    // as many lanes per expert as there are warps (a power of two) scan their counts, which an odd stride keeps in different banks;
+    // then the first warp the experts' totals, four a lane
+    const int span = 1 << (32 - __clz(nw - 1)), sub = lane & (span - 1), at_once = 32 / span;
+    for (int e0 = wid * at_once; e0 < experts; e0 += nw * at_once) {
+      const int e = e0 + lane / span;
+      const bool in = sub < nw && e < experts;
+      const int n = in ? cnt_s[sub * stride + e] : 0;
+      int end = n;
+      for (int o = 1; o < span; o <<= 1) {
+        const int v = __shfl_up_sync(0xffffffffu, end, o, span);
+        if (sub >= o) end += v;
+      }
+      if (in) cnt_s[sub * stride + e] = end - n;
+      if (sub == nw - 1 && in) total_s[e] = end;
     }
-    if (lane < nw) cnt_s[lane * experts + e] = end - n;
-    if (lane == 31) total_s[e] = end;
-  }
-  __syncthreads();
-  if (wid == 0) {
+    __syncthreads();
+    if (wid == 0) {
+      int at = 0;
+      for (int e = 4 * lane; e - 4 * lane < experts; e += 128) {
+        int4 v = e < experts ? *reinterpret_cast<const int4*>(total_s + e) : make_int4(0, 0, 0, 0);
+        const int n = v.x + v.y + v.z + v.w;
+        int end = n;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+          const int u = __shfl_up_sync(0xffffffffu, end, o);
+          if (lane >= o) end += u;
+        }
+        const int x = at + end - n, y = x + v.x, z = y + v.y, w = z + v.z;
+        if (e < experts) *reinterpret_cast<int4*>(total_s + e) = make_int4(x, y, z, w);
+        at += __shfl_sync(0xffffffffu, end, 31);
+      }
+      if (lane == 0) seg[experts] = at;
+    }
+    __syncthreads();
+    for (int e = threadIdx.x; e < experts; e += blockDim.x) seg[e] = total_s[e];
+  } else {
+    // a thread per expert walks the warps' counts, before and after a scan over the threads of the CTA
     int at = 0;
-    for (int e0 = 0; e0 < experts; e0 += 32) {
-      const int e = e0 + lane, n = e < experts ? total_s[e] : 0;
+    for (int e0 = 0; e0 < experts; e0 += blockDim.x) {
+      const int e = e0 + threadIdx.x;
+      int n = 0;
+      if (e < experts)
+        for (int w = 0; w < nw; ++w) n += cnt_s[w * stride + e];
       int end = n;
 #pragma unroll
       for (int o = 1; o < 32; o <<= 1) {
         const int v = __shfl_up_sync(0xffffffffu, end, o);
         if (lane >= o) end += v;
       }
-      if (e < experts) total_s[e] = seg[e] = at + end - n;
-      at += __shfl_sync(0xffffffffu, end, 31);
+      if (lane == 31) carry_s[wid] = end;
+      __syncthreads();
+      int before = at, all = 0;
+      for (int w = 0; w < nw; ++w) {
+        if (w < wid) before += carry_s[w];
+        all += carry_s[w];
+      }
+      if (e < experts) {
+        int pos = before + end - n;
+        seg[e] = pos;
+        for (int w = 0; w < nw; ++w) {
+          const int c = cnt_s[w * stride + e];
+          cnt_s[w * stride + e] = pos;
+          pos += c;
+        }
+        if (e == experts - 1) seg[experts] = pos;
+      }
+      at += all;
+      __syncthreads();
     }
-    if (lane == 0) seg[experts] = at;
   }
-  __syncthreads();
   for (int p0 = p_begin; p0 < p_end; p0 += 32 * kBatch) {
-    const bool again = per > 32 * kBatch;             // otherwise they are still there
-    if (again) fetch(p0);
+    if (!KEEP) fetch(p0);                             // otherwise they are still there
 #pragma unroll
     for (int j = 0; j < kBatch; ++j) {
       const int e = ev[j];
-      const unsigned m = again ? peers(e) : mv[j];
-      const int first = e >= 0 ? total_s[e] : 0, pos = e >= 0 ? mine[e] : 0;
+      const unsigned m = KEEP ? mv[j] : peers(e);
+      const int first = SCAN && e >= 0 ? total_s[e] : 0, pos = e >= 0 ? mine[e] : 0;
       __syncwarp();
       if (e >= 0) sorted[first + pos + __popc(m & ((1u << lane) - 1u))] = p0 + 32 * j + lane;
       if (e >= 0 && lane == __ffs(m) - 1) mine[e] = pos + __popc(m);
@@ -1159,8 +1205,16 @@ int moe_group(const int32_t* idx, int32_t* seg, int32_t* sorted, int pairs, int 
   VB_CHECK(experts >= 1 && experts <= 8192 && pairs >= 0, "moe_group: experts=%d pairs=%d", experts, pairs);
   const int warps = pairs >= 32 * 256 ? 32 : (pairs + 255) / 256;   // a warp per 256 pairs up to 32
   const size_t table = sizeof(int) * static_cast<size_t>(warps) * experts;
-  if (warps > 1 && table <= 32 * 1024)
-    VB_CUDA(launch_serial(moe_group_pairs_kernel, dim3(1), dim3(32 * warps), table + sizeof(int) * experts, stream, idx, seg, sorted, pairs, experts));
+  if (warps > 1 && table <= 32 * 1024) {
+    // Counts scanned up to 64 experts, walked above; lanes of one expert kept where a warp has few steps.  us, 512 / 2048 / 8192 pairs
+    // of 32 experts 4.3 / 5.2 / 10.9 (walked, lanes found twice: 5.3 / 5.9 / 11.6); 512 of 128, 2048 of 512, 8192 of 256 experts walked
+    // 5.5 / 7.0 / 14.1, scanned (an expert a warp, all of a lane's counts in one bank) 15.9 / 20.6 / 22.5.
+    const bool scan = experts <= 64, keep = pairs <= (scan ? 32 * 256 : 16 * 256);
+    const int stride = scan ? experts | 1 : experts, totals = scan ? (experts + 3) / 4 * 4 : 0;
+    const auto kernel = scan ? (keep ? moe_group_pairs_kernel<true, true> : moe_group_pairs_kernel<true, false>)
+                             : (keep ? moe_group_pairs_kernel<false, true> : moe_group_pairs_kernel<false, false>);
+    VB_CUDA(launch_serial(kernel, dim3(1), dim3(32 * warps), sizeof(int) * (totals + warps * stride), stream, idx, seg, sorted, pairs, experts, stride));
+  }
   else
     VB_CUDA(launch_serial(moe_group_kernel, dim3(1), dim3(1024), sizeof(int) * (experts + 1), stream, idx, seg,
                        sorted, pairs, experts));
