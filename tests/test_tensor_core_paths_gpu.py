@@ -285,6 +285,17 @@ def test_moe_route_tiles_give_the_bits_of_one_token(ops, rows, cols, pad, E, gro
         assert torch.equal(one[0][0], idx[r]) and torch.equal(one[1][0], wt[r])
 
 
+@pytest.mark.parametrize("rows,cols,E,groups", [(1185, 2048, 32, 4), (2049, 1028, 64, 4), (1200, 4096, 128, 8), (3601, 132, 33, 3), (2368, 64, 97, 1)])
+def test_moe_route_tiles_of_many_tokens(ops, rows, cols, E, groups):
+    """sizes that go to tiles of 16 tokens x 32 experts whichever number of SMs up to 148 holds them: the bits of a token alone"""
+    g = gen(rows)
+    x, w, c = randn(g, rows, cols + (-cols) % 8)[:, :cols], randn(g, E, cols, dtype=F32) * cols ** -0.5, randn(g, E, dtype=F32) * 0.05
+    idx, wt = ops.moe_route_sigmoid(x, w, c, 3, groups, max(1, groups // 2))
+    for r in sorted({0, 15, 16, rows // 2, rows - 2, rows - 1}):
+        one = ops.moe_route_sigmoid(x[r:r + 1].contiguous(), w, c, 3, groups, max(1, groups // 2))
+        assert torch.equal(one[0][0], idx[r]) and torch.equal(one[1][0], wt[r])
+
+
 @pytest.mark.parametrize("rows,cols,np_", [(1, 4, 1), (3, 1028, 2), (300, 2048, 4), (5, 136, 7)])
 @pytest.mark.parametrize("a_dt", [None, BF, F32])
 def test_residual_add_vec_equals_the_general_form(ops, rows, cols, np_, a_dt):

@@ -1186,10 +1186,19 @@ int moe_route_scores(const vila_moe_route_params& p, cudaStream_t stream) {
     else if (p.x_dtype == VILA_DT_F32) VB_ROUTE_K(NT, NU, TH, true, true);                                              \
     else VB_ROUTE_K(NT, NU, TH, true, false);                                                                           \
   } while (0)
-  // Few tokens (or very many experts): one per CTA of 32 warps, otherwise four.  From half a round of tiles of 16 on (bf16 rows on 16
-  // bytes, no gate) those: 32 experts of 2048 columns, 1000 / 2048 tokens 19 / 19 us, four at a time 14 / 28; 64 of 4096, 1000 tokens 51, 37
+  // Few tokens (or very many experts): one per CTA of 32 warps, otherwise four, or 16 with bf16 rows on 16 bytes and no gate.  Four a
+  // CTA take (us) 2 and 4 + 0.21 an expert of 2048 columns for every 8 tokens an SM has; 16 take 5 (9 from the third on) and 10.3 for
+  // every 16 tokens an SM has and 32 experts of 2048 columns, those in part too, 1.2 more for the first.  Measured, four | 16: 32 x
+  // 2048 on 1184 / 2048 / 4096 tokens 11.4 | 17.3, 20.9 | 17.4, 39.8 | 26.5; 8 x 2048 8.3 | 17.3, 14.6 | 17.4, 27.1 | 26.5; 64 x 4096
+  // on 1184 / 2048 / 2800 29.6 | 50.9, 56.9 | 51.1, 83.8 | 86.0; 100 x 4096 on 2400 140 | 167.
+  auto tiles_ahead = [&]() {
+    const long sms = num_sms(), eights = (p.rows + 8 * sms - 1) / (8 * sms), sixteens = (p.rows + 16 * sms - 1) / (16 * sms);
+    const float w = static_cast<float>(p.cols) / 2048.f, blocks = static_cast<float>((p.experts + kRouteExp - 1) / kRouteExp);
+    const float four = 2.f + eights * (4.f + 0.21f * p.experts * w), sixteen = (sixteens > 2 ? 9.4f : 5.3f) + blocks * w * (10.3f * sixteens + 1.2f);
+    return eights > 1 && sixteen < 0.97f * four;
+  };
   if (p.rows <= 256 || 4 * per_tok > 48 * 1024) VB_ROUTE(1, 1, 1024);
-  else if (p.rows >= 8 * num_sms() && vec && p.x_dtype == VILA_DT_BF16 && p.ldx % 8 == 0 && aligned_to(p.x, 16) && !p.gate_w && kRouteStages * kRouteStage + kRouteTok * per_tok <= 200 * 1024) {
+  else if (vec && p.x_dtype == VILA_DT_BF16 && p.ldx % 8 == 0 && aligned_to(p.x, 16) && !p.gate_w && kRouteStages * kRouteStage + kRouteTok * per_tok <= 200 * 1024 && tiles_ahead()) {
     const size_t smem = kRouteStages * kRouteStage + kRouteTok * per_tok;
     static PerDeviceOnce once;
     if (once.first()) VB_CUDA(cudaFuncSetAttribute(moe_route_tiles_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
