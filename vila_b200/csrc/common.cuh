@@ -173,8 +173,9 @@ __device__ __forceinline__ void mbar_wait(uint64_t* bar, uint32_t parity) {
 
 // An mbarrier wait that ends: a lost arrival must not leave the GPU spinning.  The first wait of a CTA that runs out of
 // tries sets `gave_up`, which ends the other warps' waits; a warp whose wait failed leaves its loop for the CTA's last
-// barrier (or, where warps meet at other barriers on the way, runs it to its end without waiting).  Behind that barrier every
-// warp that has asked for copies or products drains them if `gave_up` is set, whichever warp set it.
+// barrier (or, where warps meet at other barriers on the way, runs it to its end without waiting).  Whoever has
+// asked for copies or products waits for them before shared memory and TMEM go, whichever warp gave up: at its own end, or
+// behind that barrier.
 constexpr int kTries = 1 << 20;        // of a wait, then the launch gives up
 constexpr int kDrainTries = 1 << 14;   // of a wait for what is still in flight after that
 __device__ __forceinline__ bool mbar_wait_limited(uint64_t* bar, uint32_t parity, volatile int* gave_up, int tries) {

@@ -190,13 +190,15 @@ glinear_tc_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
   tc_fence_after();
   const uint32_t tmem = *tmem_ptr;
   const int total = p.mode == 0 ? tiles_of(p.M, BT) * n_blocks * p.groups : first[p.groups] * n_blocks;
-  const int role = warp == kTma ? 0 : warp == kMma ? 1 : warp >= kGather ? 2 : 3;
-  bool ok = limit.quits != role;
-  if (!ok) *gave_up = 1;
-  int s = 0, rounds = 0;                  // of the thread that loads: next stage, rounds through all of them
+  bool ok = true;
+  if (limit.quits >= 0) {
+    ok = limit.quits != (warp == kTma ? 0 : warp == kMma ? 1 : warp >= kGather ? 2 : 3);
+    if (!ok) *gave_up = 1;
+  }
 
   if (warp == kTma) {
     if (lane == 0) {
+      int s = 0, rounds = 0;              // rounds: through all the stages
       uint32_t ph = 1;                    // parity to wait for on an empty barrier: the first round passes
       for (int it = blockIdx.x; it < total && ok; it += gridDim.x) {
         const Tile t = tile_at(p, BT, it, n_blocks, first);
@@ -219,10 +221,16 @@ glinear_tc_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
           }
         }
       }
+      // Requested tiles land before the CTA's memory is given back, whichever warp gave up (if none did they have long): stages below
+      // s in this round, the others in the last.  Behind the CTA's last barrier instead this took 2 % of a large layer's time.
+      for (int i = 0; i < ST; ++i) {
+        const int round = i < s ? rounds : rounds - 1;
+        if (round >= 0) mbar_drain(&full_bar[i], round & 1);
+      }
     }
   } else if (warp == kMma) {
     if (lane == 0) {
-      int k = 0;
+      int s = 0, k = 0;
       uint32_t ph = 0;
       for (int it = blockIdx.x; it < total && ok; it += gridDim.x) {
         const Tile t = tile_at(p, BT, it, n_blocks, first);
@@ -261,6 +269,8 @@ glinear_tc_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
         if (ok) umma_commit(&acc_full[k & 1]);
         ++k;
       }
+      umma_commit(drain_bar);             // products under way end before TMEM and the CTA's memory are given back, too
+      mbar_drain(drain_bar, 0);
     }
   } else if (warp >= kGather) {
     if (gathered) {
@@ -268,6 +278,7 @@ glinear_tc_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
       const int gt = tid - 32 * kGather, r0 = gt >> 3, c = gt & 7;
       const __nv_bfloat16* A = static_cast<const __nv_bfloat16*>(p.a);
       const uint32_t base = smem_u32(smem) + kWBytes + r0 * 128 + ((c ^ (r0 & 7)) << 4);
+      int s = 0;
       uint32_t ph = 1;
       // the next tile's row indices are on their way while this tile's rows are fetched
       Tile t, next = {0, 0, 0, 0};
@@ -406,20 +417,6 @@ glinear_tc_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
     tc_fence_before();
   }
   __syncthreads();
-  if (*gave_up) {
-    // requested tiles land and products under way end before the CTA's memory and TMEM are given back, also those of a warp that
-    // was through before another one gave up
-    if (warp == kTma && lane == 0) {
-      for (int i = 0; i < ST; ++i) {      // stages below s in this round, the others in the last
-        const int round = i < s ? rounds : rounds - 1;
-        if (round >= 0) mbar_drain(&full_bar[i], round & 1);
-      }
-    } else if (warp == kMma && lane == 0) {
-      umma_commit(drain_bar);
-      mbar_drain(drain_bar, 0);
-    }
-    __syncthreads();
-  }
   if (warp == kMma) {
     tc_fence_after();
     tmem_dealloc<S::kCols>(tmem);

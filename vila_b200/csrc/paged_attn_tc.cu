@@ -261,6 +261,9 @@ paged_attn_tc_kernel(const __grid_constant__ vila_paged_attn_params p, int tiles
         ph1 ^= 1;
       }
     }
+    // products in flight end before their operands and TMEM go, whichever warp gave up (the loaders' copies have landed)
+    if (elect_one()) umma_commit(fin);
+    mbar_drain(fin, 0);
   } else if ((warp & 3) * 32 >= 16 * rep * ntile) {
     // no rows: the weights that stand there reach sums that nobody reads
     int n = 0;
@@ -530,13 +533,6 @@ paged_attn_tc_kernel(const __grid_constant__ vila_paged_attn_params p, int tiles
   }
   tc_fence_before();
   __syncthreads();
-  if (*gave_up) {   // products in flight end before their operands and TMEM go, whichever warp gave up (the loaders' copies have landed)
-    if (warp == kMma) {
-      if (elect_one()) umma_commit(fin);
-      mbar_drain(fin, 0);
-    }
-    __syncthreads();
-  }
   if (warp == kMma) {
     tc_fence_after();
     tmem_dealloc<512>(tmem);
