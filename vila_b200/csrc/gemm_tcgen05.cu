@@ -762,6 +762,9 @@ int gemm_bf16(const __nv_bfloat16* A, int lda, const __nv_bfloat16* W, int ldw, 
     // Weights of a round of CTA pairs and more (18944 outputs) go to the swap-AB kernel's pairs, whole blocks of 256 in turn: 6 us +
     // 0.04 a row + 0.118 a MB, 0.0002 more per row.  40 / 100 / 279 / 384 rows x 37888 x 3584 gated 43 / 46 / 64 / 81 (one CTA a
     // block 43 / 47 / 71 / 92, tiles 46 / 48 / 82 / 92), 22016 x 2048 20.5 / 21 / 32 / 45 (22 / 24 / 35 / 47 and 22 / 23 / 33 / 34).
+    // An activation of every output is more of an epilogue than that estimate knows: with one the tiles stay where they were ahead
+    // (GELU, 279 rows x 22016 x 2048 37 and 70, 384 x 27392 x 2048 48 and 90), and up to 256 rows one round of single CTAs too (40 x
+    // 18944 x 2048 18 and 23); the others take pairs (279 x 20480 x 3584 80, one CTA a block 111).
     // A projection with a bias and no more onto whole 128-column heads may be the other half of vila_linear_qkv_rope: it
     // stays where that has the same bits (rows that fill their tiles: K halved, as ever).  Without a bias it goes by the
     // time, and the header says so (1024 x 1024 on 279 rows 6.4, there 13.0).
@@ -769,10 +772,10 @@ int gemm_bf16(const __nv_bfloat16* A, int lda, const __nv_bfloat16* W, int ldw, 
     const bool heads = plain && epi.residual == nullptr && epi.bias != nullptr && N % 128 == 0;
     const bool one_round = mb * nb <= sms || mb2 * nb2 <= sms / 2;
     const double t_swap = 6.0 + 0.027 * M + (0.20 + 0.0003 * M) * mbytes;
-    const bool whole = (nb + 1) / 2 >= sms / 2;
+    const bool whole = (nb + 1) / 2 >= sms / 2 && (epi.act == ACT_NONE || nb > sms || M > 256);
     const double t_whole = 6.0 + 0.04 * M + (0.118 + 0.0002 * M) * mbytes;
     const bool ahead = M > 56 && N <= 8192 && (t_half < 1.05 * t_swap || (one_round && fmax(t_tiles, 4.0 + 0.21 * mbytes) < 0.95 * t_swap));
-    const bool tiles = M <= 16 ? false : heads ? t_half < 1e30 && M * 10 >= mb * 128 * 9 : plain ? ahead : whole ? fmax(1.25 * t_tiles, 4.0 + 0.18 * mbytes) < t_whole : mbytes < 16 || t_half < t_swap || t_tiles < 0.7 * t_swap;
+    const bool tiles = M <= 16 ? false : heads ? t_half < 1e30 && M * 10 >= mb * 128 * 9 : plain ? ahead : whole && epi.swiglu != 0 ? fmax(1.25 * t_tiles, 4.0 + 0.18 * mbytes) < t_whole : mbytes < 16 || t_half < t_swap || t_tiles < 0.7 * t_swap;
     if (!tiles) {
       const int rc = gemm_skinny_bf16(A, lda, W, ldw, C, ldc, M, N, K, epi, whole && M > 16 ? 1 : 0, stream);
       if (rc >= 0) return rc;
