@@ -63,6 +63,69 @@ def test_linear_plain(cuda, M, N, K, block_n):
     assert rel_err(out, ref) < 8e-3, rel_err(out, ref)
 
 
+def _near(got, want, what, addend=torch.zeros(())):
+    """elementwise: a few roundings to bf16 of numbers no larger than 1 + |result|, and than that plus what was added to it where the
+    sum may be the smaller one, 2^-9 of them each"""
+    bad = (got.double() - want).abs() > 2.0 ** -6 * (want.abs() + addend.to(want).abs() + 1)
+    assert not bool(bad.any()), (what, int(bad.sum()), bad.nonzero()[:4].tolist())
+
+
+@pytest.mark.parametrize("N,K", [(18952, 64), (19072, 1024), (37888, 200), (38016, 72), (38016, 1024), (57352, 64)])
+@pytest.mark.parametrize("epi", ["plain", "act", "gated"])
+def test_linear_walks_weight_blocks(cuda, N, K, epi):
+    """two to four weight blocks of 128 rows per CTA, or pair of CTAs, in turn: accumulators side by side (up to 256 rows) and sharing
+    columns (above), an odd number of blocks, so that the last pair's second one lies behind N, and a last block in part"""
+    if epi == "gated":
+        N = N // 32 * 32
+    ops = _ops()
+    g = torch.Generator(device="cuda").manual_seed(N + K)
+    w = bf(torch.randn(N, K, device=cuda, generator=g) / math.sqrt(K))
+    b = bf(torch.randn(N, device=cuda, generator=g))
+    for M in (17, 64, 256, 257, 279, 384, 512):
+        x = bf(torch.randn(M, K, device=cuda, generator=g))
+        z = x.double() @ w.double().t()
+        kw = {}
+        if epi == "act":
+            kw = dict(bias=b, act=ops.ACT_GELU_TANH, residual=bf(torch.randn(M, N, device=cuda, generator=g)))
+            want = rb(F.gelu(rb((z + b.double()).float()), approximate="tanh")).double() + kw["residual"].double()
+        elif epi == "gated":
+            kw = dict(swiglu=True)
+            zr = rb(z.float()).double()
+            want = F.silu(zr[:, 0::2]) * zr[:, 1::2]
+        else:
+            want = z
+        for form in (None, 3000, 3001):
+            out = ops.linear(x, w, block_n=form, static_w=True, **kw)
+            _near(out, want, (M, form), kw.get("residual", torch.zeros((), device=cuda)))
+            for _ in range(2):
+                assert torch.equal(out, ops.linear(x, w, block_n=form, static_w=True, **kw))
+
+
+@pytest.mark.parametrize("N,K", [(8200, 1024), (9472, 520), (4608, 1024), (2048, 2056)])
+@pytest.mark.parametrize("gated", [False, True])
+def test_linear_cluster_partials_and_residual(cuda, N, K, gated):
+    """K over clusters of two to eight CTAs: the own partial from shared memory and the peers' over the cluster, residual rows asked for
+    before the sums (also in place and by row modulus), tokens that do not fill a warp's four"""
+    ops = _ops()
+    g = torch.Generator(device="cuda").manual_seed(N + K)
+    N = N // 32 * 32 if gated else N
+    w = bf(torch.randn(N, K, device=cuda, generator=g) / math.sqrt(K))
+    n = N // 2 if gated else N
+    for M in (17, 33, 130, 279, 384):
+        x, res = bf(torch.randn(M, K, device=cuda, generator=g)), bf(torch.randn(M, N, device=cuda, generator=g))
+        z = rb((x.double() @ w.double().t()).float()).double()
+        want = F.silu(z[:, 0::2]) * z[:, 1::2] if gated else z + res.double()
+        kw = dict(swiglu=True) if gated else dict(residual=res)
+        out = ops.linear(x, w, block_n=3000, **kw)
+        assert out.shape == (M, n)
+        _near(out, want, M, torch.zeros((), device=cuda) if gated else res)
+        if not gated:
+            again = res.clone()
+            ops.linear(x, w, block_n=3000, residual=again, out=again)
+            assert torch.equal(out, again)
+            _near(ops.linear(x, w, block_n=3000, residual=res[:5], res_row_mod=5), z + res.double()[torch.arange(M, device=cuda) % 5], (M, "mod"), res)
+
+
 @pytest.mark.parametrize("act", [0, 1, 2])
 @pytest.mark.parametrize("with_res", [False, True])
 def test_linear_epilogues(cuda, act, with_res):
