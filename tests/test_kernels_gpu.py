@@ -607,6 +607,16 @@ def test_space_to_depth(cuda, h, w, r):
     assert torch.equal(out, ref.reshape(2, -1, ref.shape[-1]))
 
 
+@pytest.mark.parametrize("B,C,H,W,P,pad", [(1, 3, 378, 378, 14, 4), (1, 3, 448, 448, 14, 52), (1, 3, 434, 462, 14, 4), (2, 3, 56, 84, 28, 0), (3, 3, 64, 96, 16, 0),
+                                           (2, 1, 40, 24, 8, 8), (2, 5, 6, 10, 2, 4), (40, 3, 224, 224, 16, 0)])
+def test_patch_im2col_of_any_patch(cuda, B, C, H, W, P, pad):
+    """patches of 14 below, at and above 1024 rows, patches of other sizes, padded columns"""
+    px = bf(torch.randn(B, C, H, W, device=cuda, generator=torch.Generator(device="cuda").manual_seed(H + W)))
+    out = _ops().patch_im2col(px, P, C * P * P + pad)
+    assert torch.equal(out[:, :C * P * P].float(), F.unfold(px.float(), kernel_size=P, stride=P).transpose(1, 2).reshape(-1, C * P * P))
+    assert int(out[:, C * P * P:].count_nonzero()) == 0
+
+
 @pytest.mark.parametrize("idx", [-1, 0, 1])
 def test_s2_merge_and_chessboard(cuda, idx):
     ops = _ops()

@@ -18,20 +18,44 @@ inline int grid_for(long total_items, int threads, int items_per_thread = 1) {
 // im2col for the 14x14/s14 patch-embed conv (modeling_siglip.py:269-275,322): row = (b, py, px),
 // col = (c, ky, kx) matching Conv2d weight.view(1152, 588); columns [588, k_pad) are zero.
 // ------------------------------------------------------------------------------------------------
-// A warp per output row, a lane per 32-bit word: writes are whole lines, a strip's reads (28 bytes at P = 14) lie in
-// neighbouring lanes, the row is divided up once and, for P14, a word by constants: 13 x 3 x 448 x 448 20 -> 13 us (a thread per
-// strip, or per word with divisions of its own: 200 instructions a word).
-template <bool P14>
-__global__ void im2col_kernel(const __nv_bfloat16* __restrict__ pix, __nv_bfloat16* __restrict__ out,
-                              int B, int C, int H, int W, int patch, int k_pad) {
+// Any patch: a thread copies a (row, c, ky) strip of P contiguous pixels, as 32-bit pairs (P and W are even).
+__global__ void im2col_strips_kernel(const __nv_bfloat16* __restrict__ pix, __nv_bfloat16* __restrict__ out, int B, int C, int H, int W,
+                                     int P, int k_pad) {
   griddep_launch_dependents();
   griddep_wait();
-  const int P = P14 ? 14 : patch, half = P / 2, gh = H / P, gw = W / P, words = k_pad / 2, used = C * P * half, lane = threadIdx.x & 31;
+  const int gh = H / P, gw = W / P, used = C * P * P;
+  const long strips = static_cast<long>(B) * gh * gw * C * P;
+  for (long s = blockIdx.x * static_cast<long>(blockDim.x) + threadIdx.x; s < strips; s += static_cast<long>(gridDim.x) * blockDim.x) {
+    const int ky = s % P;
+    long t = s / P;
+    const int c = t % C;
+    t /= C;
+    const int px = t % gw;
+    t /= gw;
+    const int py = t % gh, b = t / gh;
+    const uint32_t* src = reinterpret_cast<const uint32_t*>(pix + ((static_cast<long>(b) * C + c) * H + (py * P + ky)) * W + px * P);
+    const long row = (static_cast<long>(b) * gh + py) * gw + px;
+    uint32_t* dst = reinterpret_cast<uint32_t*>(out + row * k_pad + (c * P + ky) * P);
+#pragma unroll 7
+    for (int i = 0; i < P / 2; ++i) dst[i] = src[i];
+    if (c == C - 1 && ky == P - 1)
+      for (int i = used; i < k_pad; ++i) out[row * k_pad + i] = __float2bfloat16(0.f);
+  }
+}
+// Patches of 14, 1024 rows and more: a warp per output row, a lane per 32-bit word.  Writes are whole lines, a strip's reads (28
+// bytes) lie in neighbouring lanes, the row is divided up once and a word by constants: 13 x 3 x 448 x 448 20 -> 13 us.  Fewer rows are
+// too few warps (729 rows 3.6 and 4.4 us), and with divisions by a number that is not known a word costs 200 instructions (2 x 3 x
+// 512 x 512 in patches of 32 14.7 and 17.6, 1 x 3 x 224 x 224 of 16 3.0 and 5.5).
+__global__ void im2col_rows14_kernel(const __nv_bfloat16* __restrict__ pix, __nv_bfloat16* __restrict__ out, int B, int C, int H, int W,
+                                     int k_pad) {
+  griddep_launch_dependents();
+  griddep_wait();
+  constexpr int P = 14, half = P / 2;
+  const int gh = H / P, gw = W / P, words = k_pad / 2, used = C * P * half, lane = threadIdx.x & 31;
   const long rows = static_cast<long>(B) * gh * gw, warps = static_cast<long>(gridDim.x) * (blockDim.x >> 5);
   for (long row = blockIdx.x * static_cast<long>(blockDim.x >> 5) + (threadIdx.x >> 5); row < rows; row += warps) {
     const long t = row / gw, b = t / gh;
     const int px = static_cast<int>(row - t * gw), py = static_cast<int>(t - b * gh);
-    // P and W are even: strips of whole words
     const uint32_t* src = reinterpret_cast<const uint32_t*>(pix) + (b * C * H + py * P) * (W / 2) + px * half;
     uint32_t* dst = reinterpret_cast<uint32_t*>(out) + row * words;
 #pragma unroll 5
@@ -457,8 +481,10 @@ int im2col_patch14(const __nv_bfloat16* pixels, __nv_bfloat16* out, int B, int C
   VB_CHECK(k_pad >= C * patch * patch && k_pad % 8 == 0, "im2col: bad k_pad %d", k_pad);
   const long rows = (long)B * (H / patch) * (W / patch);
   if (rows == 0 || C == 0) return 0;
-  VB_CUDA(launch_pdl(patch == 14 ? im2col_kernel<true> : im2col_kernel<false>, dim3(grid_for(rows, 8)), dim3(256), 0, stream, pixels, out, B,
-                     C, H, W, patch, k_pad));
+  if (patch == 14 && rows >= 1024)
+    VB_CUDA(launch_pdl(im2col_rows14_kernel, dim3(grid_for(rows, 8)), dim3(256), 0, stream, pixels, out, B, C, H, W, k_pad));
+  else
+    VB_CUDA(launch_pdl(im2col_strips_kernel, dim3(grid_for(rows * C * patch, 256)), dim3(256), 0, stream, pixels, out, B, C, H, W, patch, k_pad));
   return 0;
 }
 
