@@ -508,6 +508,16 @@ def test_fmha_edges_of_tiles(cuda, D, variant):
         assert torch.equal(out, ops.fmha(q, k, v, B=B, Sq=Sq, Sk=Sk, causal=causal, scale=D ** -0.5, variant=variant))
 
 
+def test_fmha_one_row_of_64_columns(cuda):
+    """a single query row asked for in two tiles, of which there is one"""
+    ops = _ops()
+    g = torch.Generator(device="cuda").manual_seed(65)
+    q, k, v = (bf(torch.randn(S, 3, 64, device=cuda, generator=g)) for S in (1, 77, 77))
+    out = ops.fmha(q, k, v, B=1, Sq=1, Sk=77, causal=False, scale=0.125, variant=2)
+    assert rel_err(out[None], ref_attention(q[None], k[None], v[None], False, 0.125)) < 1.5e-2
+    assert torch.equal(out, ops.fmha(q, k, v, B=1, Sq=1, Sk=77, causal=False, scale=0.125, variant=1))
+
+
 @pytest.mark.parametrize("variant", [1, 2])
 def test_fmha_waits_that_run_out_are_reported(cuda, monkeypatch, variant):
     """waits of 0 tries give up at once, few tries somewhere under way: the launch ends, the next status says so once"""
@@ -597,16 +607,6 @@ def test_patch_im2col(cuda):
     assert out[:, 588:].abs().max() == 0
 
 
-@pytest.mark.parametrize("h,w,r", [(32, 32, 2), (27, 27, 2), (32, 32, 3), (27, 27, 3), (5, 7, 2)])
-def test_space_to_depth(cuda, h, w, r):
-    ops = _ops()
-    g = torch.Generator(device="cuda").manual_seed(h * w + r)
-    x = bf(torch.randn(2, h * w, 64, device=cuda, generator=g))
-    out = ops.space_to_depth(x, h, w, r)
-    ref = O.flat_square(x.view(2, h, w, 64), r)
-    assert torch.equal(out, ref.reshape(2, -1, ref.shape[-1]))
-
-
 @pytest.mark.parametrize("B,C,H,W,P,pad", [(1, 3, 378, 378, 14, 4), (1, 3, 448, 448, 14, 52), (1, 3, 434, 462, 14, 4), (2, 3, 56, 84, 28, 0), (3, 3, 64, 96, 16, 0),
                                            (2, 1, 40, 24, 8, 8), (2, 5, 6, 10, 2, 4), (40, 3, 224, 224, 16, 0)])
 def test_patch_im2col_of_any_patch(cuda, B, C, H, W, P, pad):
@@ -615,6 +615,16 @@ def test_patch_im2col_of_any_patch(cuda, B, C, H, W, P, pad):
     out = _ops().patch_im2col(px, P, C * P * P + pad)
     assert torch.equal(out[:, :C * P * P].float(), F.unfold(px.float(), kernel_size=P, stride=P).transpose(1, 2).reshape(-1, C * P * P))
     assert int(out[:, C * P * P:].count_nonzero()) == 0
+
+
+@pytest.mark.parametrize("h,w,r", [(32, 32, 2), (27, 27, 2), (32, 32, 3), (27, 27, 3), (5, 7, 2)])
+def test_space_to_depth(cuda, h, w, r):
+    ops = _ops()
+    g = torch.Generator(device="cuda").manual_seed(h * w + r)
+    x = bf(torch.randn(2, h * w, 64, device=cuda, generator=g))
+    out = ops.space_to_depth(x, h, w, r)
+    ref = O.flat_square(x.view(2, h, w, 64), r)
+    assert torch.equal(out, ref.reshape(2, -1, ref.shape[-1]))
 
 
 @pytest.mark.parametrize("idx", [-1, 0, 1])

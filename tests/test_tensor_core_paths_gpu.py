@@ -529,6 +529,14 @@ def test_paged_attention_prompt_refuses_to_build_on_a_launch_that_gave_up(ops):
     ops.check_waits()
 
 
+@pytest.mark.parametrize("rows", [1900, 2100])
+def test_paged_attention_prompt_bias_of_many_distances(ops, rows):
+    """tables by distance that just fit beside the operands in shared memory and that do not; distances past their end"""
+    for seqs in ([(33, 300), (64, 1)], [(20, 2300)]):
+        got, want, _ = attention_case(ops, dict(dist_bias=rows, gate=True), 8, 2, 128, 128, 64, seqs, seed=rows)
+        assert rel(got, want) < 3e-6
+
+
 @pytest.mark.parametrize("form", [dict(), dict(softcap=5.0, sink=True), dict(window=300, keep_first=70), dict(window=90, keep_first=130, dist_bias=40), dict(chunk=200, dist_bias=250)])
 @pytest.mark.parametrize("H,G", [(32, 32), (12, 4), (32, 8), (16, 2)])
 def test_paged_attention_prompt_rows_do_not_depend_on_their_cta(ops, form, H, G):

@@ -202,7 +202,7 @@ __device__ __forceinline__ void finish_cluster(const float* dump, int warp, int 
   const uint32_t at = smem_u32(dump) + 16u * lane;
   for (int m0 = split * 8 + warp; m0 < a.M; m0 += U * step) {
     // The residual, or the angles and the page, are asked for before the sums (without branches: of tokens past the last one, its
-    // own): behind each token's stores they were waited for token by token.  384 rows x 9472 x 4096 with a residual 43 -> 34 us, 64
+    // own): behind each token's stores they were waited for token by token.  384 rows x 9472 x 4096 with a residual 43 -> 35 us, 64
     // heads over 4 of 1024 columns with their rotation 25 -> 20.5.
     auto token = [&](int u) { return min(m0 + u * step, a.M - 1); };
     uint2 res[U], sines[U];   // with a rope_table: cosines, sines
