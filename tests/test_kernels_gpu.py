@@ -553,9 +553,9 @@ def test_fmha_waits_that_run_out_are_reported(cuda, monkeypatch, variant):
                                                (64, 2304, 9000, 16, 0)])
 def test_fmha_one_tile_sums_are_rounded(cuda, D, Sq, Sk, H, variant):
     """values of one sign: what the tensor core truncates goes one way and grows with every product that joins a sum (5e-9 of it:
-    4e-5 at 9000 keys, 8e-5 at 16384), rounded additions of blocks of 128 keys have no such mean.  Against the exact result rounded
-    to bf16 the rounding of the output is common to both sides.  What is left does not grow with the keys: 2e-6 - 3.3e-6 at 1024 -
-    16384 of them (eight products of a block, exponentials), whose noise at 5e5 values is 4e-7; 8e-6 lies between the two"""
+    4e-5 at 9000 keys, 8e-5 at 16384), rounded additions of 256 keys' sums have no such mean.  Against the exact result rounded
+    to bf16 the rounding of the output is common to both sides.  What is left does not grow with the keys: 2e-6 - 3.5e-6 at 1024 -
+    16384 of them (sixteen products of two blocks, exponentials), whose noise at 5e5 values is 4e-7; 8e-6 lies between the two"""
     ops = _ops()
     g = torch.Generator(device="cuda").manual_seed(D + Sk)
     q, k = (bf(torch.randn(S, H, D, device=cuda, generator=g)) for S in (Sq, Sk))

@@ -5,27 +5,28 @@
 //                             the exponentials; with one thread a row the exponential unit was busy for 40 % of the time
 //   next two warps            TMA: Q tiles, and ONE ring over the sequence K0, V0, K1, V1, ...; rows of O
 //   last one or two warps     a tile's tcgen05.mma issuer (one issuer for both tiles was what the kernel waited for)
-//   TMEM: scores at 0 and 128 (fp32 128 x 128 each); at 256 / 384 O of tile 0 / 1, or (one tile) the sums of even / odd key blocks
+//   TMEM: scores at 0 and 128 (fp32 128 x 128 each); at 256 / 384 O of tile 0 / 1, or (one tile) the sums of two key
+//   blocks and of the next two
 //
 // The weights go back to TMEM as bf16 over the scores that they come from and are the A operand of the PV product from
 // there: in shared memory they cost its port 48 KB a block beside the 64 KB of the operands and the 32 KB that arrive.
 //   two tiles: each PV(j) S(j+1) in turn: the tensor pipe works on one tile under the other's softmax
-//   one tile:  S(j+1) PV(j): two score buffers, taken in turn; a block's sums join the row's in registers, under the next PV
+//   one tile:  S(j+1) PV(j): two score buffers, taken in turn; the sums of two blocks join the row's in registers, under the next PV
 // The products of one thread execute in order, so scores may follow the weights that a product issued before still reads.
 // Descriptors are a base plus constants: made anew for every instruction, the issue alone took 85 clocks of the 64 that a
 // product of 128 x 128 x 16 needs.
 //
 // Bound by the chain of a tile (two tiles: scores 500 clocks at 128 columns, maxima and exponentials 1500, product 500) and by
 // the exponential unit (1024 a tile and block).  Before (four softmax warps a tile, weights through shared memory, one CTA a
-// pair of tiles): 16 heads of 72 columns, 1024 x 1024, 1 / 4 / 13 images 20.4 / 46.8 / 136.8 us, now 16.6 / 42.2 / 108.3; causal,
-// 28 heads of 128 over 4, 279 / 1024 / 2500 / 8000 / 16470 rows 9.8 / 33 / 91 / 550 / 1955, now 8.0 / 15.1 / 49.7 / 382 / 1530 (1270 TFLOP/s).
-// Registers: two tiles have 96 a thread and spill 44 - 68 bytes of their softmax, one tile (168) 24 - 88, at 128 columns most.
+// pair of tiles): 16 heads of 72 columns, 1024 x 1024, 1 / 4 / 13 images 20.4 / 46.8 / 136.8 us, now 17.0 / 42.1 / 107; causal,
+// 28 heads of 128 over 4, 279 / 1024 / 2500 / 8000 / 16470 rows 9.8 / 33 / 91 / 550 / 1955, now 7.8 / 15.0 / 49.7 / 385 / 1530 (1270 TFLOP/s).
+// Registers: two tiles have 96 a thread and spill 44 - 68 bytes of their softmax, one tile (168) up to 72, at 128 columns.
 //
 // S = QK^T in fp32, online softmax in fp32 with exp2, P rounded to bf16 for PV, a lazy (exact) rescale when a row maximum moves
-// by more than 2^8.  The tensor core truncates as it accumulates: one tile adds each block's sums by rounded additions; two tiles,
-// which have no registers for them, let O grow in TMEM.  Mean signed error of values of one sign, 1024 / 4096 / 16384 keys, against
-// the exact result rounded to bf16: -2.7 / -3.3 / -2.1e-6 and -4.3 / -16 / -78e-6.  With O in TMEM one tile was 5 % faster at 128
-// columns (1024 rows), 1 % at 72.  D = 65 .. 96 zero-padded by TMA fill (SW64
+// by more than 2^8.  The tensor core truncates as it accumulates: one tile adds the sums of two blocks, 16 products, by rounded
+// additions; two tiles, which have no registers for them, let O grow in TMEM.  Mean signed error of values of one sign, 1024 / 4096 /
+// 16384 keys, against the exact result rounded to bf16: -2.9 / -3.5 / -2.2e-6 (-2.7 / -3.3 / -2.1e-6 a block at a time) and -4.3 / -16 /
+// -78e-6.  With O in TMEM one tile was 5 % faster at 128 columns (1024 rows 14.2; a block at a time 15.2), 3 % at 72.  D = 65 .. 96 zero-padded by TMA fill (SW64
 // chunks of 32 columns; up to 80 columns products stop there), D = 64 and 128 as SW128 chunks, V the MN-major B operand.
 //
 // Replaces flash_attn_func in SiglipFlashAttention2 (modeling_siglip.py:583-585, non-causal, scale 72^-0.5) and HF
@@ -130,7 +131,7 @@ fmha_pipe_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
   uint64_t* q_empty = q_full + 2 * C::kQ;               // [tile][buffer]
   uint64_t* s_full = q_empty + 2 * C::kQ;               // [2]: by score buffer
   uint64_t* p_full = s_full + 2;                        // [2]
-  uint64_t* o_full = p_full + 2;                        // [2]: by tile, or (one tile) by buffer of a block's sums
+  uint64_t* o_full = p_full + 2;                        // [2]: by tile, or (one tile) of even and odd blocks
   uint64_t* o_free = o_full + 2;                        // [2]
   uint64_t* o_ready = o_free + 2;                       // [tile][buffer]: rows stand in the Q buffer
   uint64_t* fin = o_ready + 2 * C::kQ;                  // [2]
@@ -301,7 +302,7 @@ fmha_pipe_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
     const uint64_t vd0 = make_smem_desc(smem_u32(ring_s), C::kChunkBytes, C::kSBO, C::kLayout);
     const uint32_t o_tmem = tmem_base + 256 + t * 128;
     bool ok = limit.quits != 2;
-    int slot = 0, ph = 0, g = 0, units = 0;   // ring; blocks and units of the tile so far
+    int slot = 0, ph = 0, g = 0, units = 0, pairs = 0;   // ring; blocks, units and (one tile) pairs of blocks of the tile so far
     auto advance = [&]() {
       if (++slot == R) {
         slot = 0;
@@ -333,7 +334,7 @@ fmha_pipe_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
         const uint32_t p = tmem_base + sb * BKV;
 #pragma unroll
         for (int k = 0; k < BKV / 16; ++k)   // weights of keys 16 k ..: 8 columns, each half's from its own scores' first on
-          umma_f16_ts(o_tmem + (TILES == 2 ? 0 : sb * 128), p + (k >> 2) * 64 + (k & 3) * 8, vd + k * (16 * CW * 2 >> 4), idesc_o,
+          umma_f16_ts(o_tmem + (TILES == 2 ? 0 : (pairs & 1) * 128), p + (k >> 2) * 64 + (k & 3) * 8, vd + k * (16 * CW * 2 >> 4), idesc_o,
                       k != 0 || !first ? 1u : 0u);
         umma_commit(&o_full[sb]);
         umma_commit(&r_empty[slot_v]);
@@ -362,11 +363,12 @@ fmha_pipe_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
           if (!ok) break;
           issue_s(g + 1, slot_k);
         }
-        // the weights: also orders this PV after any rescale of block j and (one tile) after block g - 2's sums have been taken in
+        // the weights: also orders this PV after any rescale of block j and (one tile) after the sums that were here have been taken in
         ok = wait(&r_full[slot_v], ph_v) && (TILES == 1 || ((!more || wait(&r_full[slot_k], ph_k)) && (j > 0 || wait(&o_free[t], units + 1)))) &&
              wait(&p_full[TILES == 2 ? t : g & 1], TILES == 2 ? g : g >> 1);
         if (!ok) break;
-        issue_pv(g, slot_v, TILES == 1 || j == 0);
+        issue_pv(g, slot_v, TILES == 1 ? (j & 1) == 0 : j == 0);
+        if (TILES == 1 && ((j & 1) != 0 || !more)) ++pairs;
         if (TILES == 2 && more) issue_s(g + 1, slot_k);
         if (more) advance();
       }
@@ -387,8 +389,9 @@ fmha_pipe_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
     const uint32_t o_addr = lane_addr + 256 + t * 128 + half * C::kHalf;
     float *xm_t = xm + t * 2 * BQ + row, *xl_t = xl + t * 2 * BQ + row;
     int g = 0, units = 0;   // blocks and units of the tile so far
-    // One tile: a row's sums, to which a block's are added from TMEM under the next block's product
+    // One tile: a row's sums, to which those of two blocks, up to block b, are added from TMEM under the next block's product
     uint32_t o[C::kHalf];
+    int pairs = 0;          // that have been taken in
     auto take = [&](int b, auto columns) {   // of so many at a time
       constexpr int N = decltype(columns)::value;
       wait(&o_full[b & 1], b >> 1);
@@ -396,7 +399,7 @@ fmha_pipe_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
 #pragma unroll
       for (int c = 0; c < C::kHalf; c += N) {
         uint32_t x[N];
-        const uint32_t from = o_addr + (b & 1) * 128 + c;
+        const uint32_t from = o_addr + (pairs & 1) * 128 + c;
 #pragma unroll
         for (int i = 0; i + 32 <= N; i += 32) tmem_ld_32x32b_x32(from + i, x + i);
 #pragma unroll
@@ -410,6 +413,7 @@ fmha_pipe_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
           o[c + i + 1] = __float_as_uint(y1);
         }
       }
+      ++pairs;
     };
     using Few = std::integral_constant<int, 8>;
     using All = std::integral_constant<int, C::kHalf>;
@@ -448,7 +452,7 @@ fmha_pipe_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
 #pragma unroll
           for (int q = 0; q < 4; ++q) m4[q] = fmax3(m4[q], __uint_as_float(s[i + 2 * q]), __uint_as_float(s[i + 2 * q + 1]));
         float mx = fmaxf(fmaxf(m4[0], m4[1]), fmaxf(m4[2], m4[3])) * a.scale_log2;
-        bool taken = j == 0;   // block j - 1's sums
+        bool taken = j == 0 || (j & 1) != 0;   // no two blocks' sums are complete and still in TMEM
         if (pair_any(id, j == 0 || mx > m_ref + 8.0f)) {
           xm_t[half * BQ] = mx;
           pair_sync(id);
@@ -459,23 +463,28 @@ fmha_pipe_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
             const float m_new = mx > m_ref + 8.0f ? mx : m_ref;
             const float alpha = ex2f(m_ref - m_new);                      // 1 for rows that keep their reference
             // rare: few registers rather than few round trips
-            if constexpr (TILES == 1) {
+            if (TILES == 1 && !taken) {
               take(g - 1, Few());
-#pragma unroll
-              for (int i = 0; i < C::kHalf; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * alpha);
               taken = true;
             } else {
-              wait(&o_full[t], g - 1);   // PV(j - 1) has landed
+              // PV(j - 1) has landed
+              if (TILES == 1) wait(&o_full[(g - 1) & 1], (g - 1) >> 1);
+              else wait(&o_full[t], g - 1);
               tc_fence_after();
+              const uint32_t sums = o_addr + (TILES == 1 ? (pairs & 1) * 128 : 0);
 #pragma unroll 1
               for (int c = 0; c < C::kHalf / 8; ++c) {
                 uint32_t o8[8];
-                tmem_ld_32x32b_x8(o_addr + c * 8, o8);
+                tmem_ld_32x32b_x8(sums + c * 8, o8);
                 tmem_ld_wait();
 #pragma unroll
                 for (int i = 0; i < 8; ++i) o8[i] = __float_as_uint(__uint_as_float(o8[i]) * alpha);
-                tmem_st_32x32b_x8(o_addr + c * 8, o8);
+                tmem_st_32x32b_x8(sums + c * 8, o8);
               }
+            }
+            if (TILES == 1) {
+#pragma unroll
+              for (int i = 0; i < C::kHalf; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * alpha);
             }
             l *= alpha;
             m_ref = m_new;
@@ -649,7 +658,7 @@ int fmha_prefill_cfg(int variant, const FmhaParams& p, cudaStream_t stream, int 
   // Two tiles at a time take 1.6 times as long per key block as one (13 x 16 heads of 1024 keys, head size 72: 23.5 and 14.5
   // us a round of units).  Key blocks per CTA: whole rounds of equal units, or (causal, dealt evenly) the mean, but no less
   // than the longest unit.  1 / 2 / 3 / 4 / 7 / 13 images: one 17, 31, 39, 56, 84, 167 us, two 25, 26, 46, 46, 76, 121; causal,
-  // 28 heads of 128, 600 / 1024 / 1500 / 2500 / 8000 rows: 10.9, 15.1, 27, 57, 465 and 14, 21, 29, 50, 382.
+  // 28 heads of 128, 600 / 1024 / 1500 / 2500 / 8000 rows: 10.8, 15.0, 27, 55, 445 and 14, 21, 29, 50, 385.
   // More than 2560 keys keep rounded sums (see above) where two tiles would not fill the SMs once, and at 64 columns; up to there
   // the two forms' errors are the same (rms 1.7958e-3 at 1024 keys, both; 1.7676e-3 and 1.7694e-3 at 16384).
   const int q_tiles = (p.Sq + BQ - 1) / BQ;
