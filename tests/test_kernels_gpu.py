@@ -421,7 +421,7 @@ def test_fmha_paged(cuda):
 
 
 # ---- one and two query tiles at a time (fmha_pipe_kernel: O in TMEM with lazy rescale)
-# forced through vila_fmha_cfg(variant=2); the heuristic only picks it once 256-row CTAs fill 148 SMs --
+# forced through vila_fmha_cfg(variant=2); by itself it is chosen where its key blocks per CTA take less time --
 @pytest.mark.parametrize("B", [1, 8, 64])
 def test_fmha2_noncausal_siglip(cuda, B):
     from tests.helpers import report_rel

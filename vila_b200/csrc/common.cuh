@@ -198,6 +198,31 @@ __device__ __forceinline__ void mbar_drain(uint64_t* bar, uint32_t parity) {
     if (mbar_try_wait(bar, parity)) return;
 }
 
+// packed fp32: d = a b + c of two numbers, d += a of two
+__device__ __forceinline__ void ffma2(float& d0, float& d1, float a0, float a1, float b, float c) {
+  asm("{.reg .b64 ra, rb, rc, rd; mov.b64 ra, {%2,%3}; mov.b64 rb, {%4,%4}; mov.b64 rc, {%5,%5}; "
+      "fma.rn.f32x2 rd, ra, rb, rc; mov.b64 {%0,%1}, rd;}"
+      : "=f"(d0), "=f"(d1)
+      : "f"(a0), "f"(a1), "f"(b), "f"(c));
+}
+__device__ __forceinline__ void fadd2(float& d0, float& d1, float a0, float a1) {
+  asm("{.reg .b64 ra, rd; mov.b64 ra, {%2,%3}; mov.b64 rd, {%0,%1}; add.rn.f32x2 rd, rd, ra; "
+      "mov.b64 {%0,%1}, rd;}"
+      : "+f"(d0), "+f"(d1)
+      : "f"(a0), "f"(a1));
+}
+// the two warps that share 32 rows meet at barrier id; true if any of their threads says so
+__device__ __forceinline__ bool pair_any(int id, bool v) {
+  uint32_t r;
+  asm volatile(
+      "{.reg .pred p, q; setp.ne.b32 p, %1, 0; bar.red.or.pred q, %2, 64, p; selp.u32 %0, 1, 0, q;}"
+      : "=r"(r)
+      : "r"(v ? 1u : 0u), "r"(id)
+      : "memory");
+  return r != 0;
+}
+__device__ __forceinline__ void pair_sync(int id) { asm volatile("bar.sync %0, 64;" ::"r"(id) : "memory"); }
+
 // ----------------------------------------------------------------------------------------------
 // TMA (cp.async.bulk.tensor) — loads arrive on an mbarrier with complete_tx::bytes
 // ----------------------------------------------------------------------------------------------

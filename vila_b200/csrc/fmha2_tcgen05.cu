@@ -67,33 +67,11 @@ __device__ __forceinline__ float ex2f(float x) {
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
   return y;
 }
-// packed fp32 and 3-input maximum: half the instructions of the softmax
-__device__ __forceinline__ void ffma2(float& d0, float& d1, float a0, float a1, float b, float c) {
-  asm("{.reg .b64 ra, rb, rc, rd; mov.b64 ra, {%2,%3}; mov.b64 rb, {%4,%4}; mov.b64 rc, {%5,%5}; "
-      "fma.rn.f32x2 rd, ra, rb, rc; mov.b64 {%0,%1}, rd;}"
-      : "=f"(d0), "=f"(d1)
-      : "f"(a0), "f"(a1), "f"(b), "f"(c));
-}
-__device__ __forceinline__ void fadd2(float& d0, float& d1, float a0, float a1) {
-  asm("{.reg .b64 ra, rd; mov.b64 ra, {%2,%3}; mov.b64 rd, {%0,%1}; add.rn.f32x2 rd, rd, ra; "
-      "mov.b64 {%0,%1}, rd;}"
-      : "+f"(d0), "+f"(d1)
-      : "f"(a0), "f"(a1));
-}
+// 3-input maximum: half the instructions
 __device__ __forceinline__ float fmax3(float a, float b, float c) {
   float d;
   asm("max.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
   return d;
-}
-// the two warps that share 32 rows meet at barrier id; true if any of their threads says so
-__device__ __forceinline__ bool pair_any(int id, bool v) {
-  uint32_t r;
-  asm volatile(
-      "{.reg .pred p, q; setp.ne.b32 p, %1, 0; bar.red.or.pred q, %2, 64, p; selp.u32 %0, 1, 0, q;}"
-      : "=r"(r)
-      : "r"(v ? 1u : 0u), "r"(id)
-      : "memory");
-  return r != 0;
 }
 // a chunk of O from shared memory; the tensor's ends are not written past
 __device__ __forceinline__ void store_chunk(const CUtensorMap* m, uint32_t src, int c0, int h, int row, int b) {
@@ -102,7 +80,6 @@ __device__ __forceinline__ void store_chunk(const CUtensorMap* m, uint32_t src, 
                "r"(src), "r"(c0), "r"(h), "r"(row), "r"(b)
                : "memory");
 }
-__device__ __forceinline__ void pair_sync(int id) { asm volatile("bar.sync %0, 64;" ::"r"(id) : "memory"); }
 
 struct Args {
   const int32_t* page_table;

@@ -47,19 +47,6 @@ __device__ __forceinline__ float ex2(float x) {
   return y;
 }
 
-__device__ __forceinline__ void ffma2(float& d0, float& d1, float a0, float a1, float b, float c) {
-  asm("{.reg .b64 ra, rb, rc, rd; mov.b64 ra, {%2,%3}; mov.b64 rb, {%4,%4}; mov.b64 rc, {%5,%5}; "
-      "fma.rn.f32x2 rd, ra, rb, rc; mov.b64 {%0,%1}, rd;}"
-      : "=f"(d0), "=f"(d1)
-      : "f"(a0), "f"(a1), "f"(b), "f"(c));
-}
-__device__ __forceinline__ void fadd2(float& d0, float& d1, float a0, float a1) {
-  asm("{.reg .b64 ra, rd; mov.b64 ra, {%2,%3}; mov.b64 rd, {%0,%1}; add.rn.f32x2 rd, rd, ra; "
-      "mov.b64 {%0,%1}, rd;}"
-      : "+f"(d0), "+f"(d1)
-      : "f"(a0), "f"(a1));
-}
-
 struct FmhaKernelArgs {
   __nv_bfloat16* o;
   int64_t o_tok_stride, o_head_stride;

@@ -17,7 +17,8 @@
 // key by key: zero parts meet an infinite number where the number itself does not.
 //
 // Bound by latency: a block of 16 heads takes 9100 clocks, of which the tensor pipe works 1540 and shared memory's 2000; the
-// loads of a stage and the barrier of a block are what the 16 warps wait for.
+// loads of a stage and the barrier of a block are what the 16 warps wait for.  Two heads of 128 columns a warp (17 heads and more) do
+// not fit its 128 registers: 150 - 200 bytes are stored and 360 - 500 loaded a block besides.
 // The tiles on the CUDA cores (paged_attn_tile4_kernel) hold whole key blocks of all heads in shared memory, 32 keys of 4
 // heads, 4 of 32.  Scores mixed / weights mixed there and here: 2048 causal rows of 16 heads over 4 1923 / 2115 -> 532 / 620 us,
 // 1024 rows on 500 keys of 32 heads over 32 21700 / 24500 -> 1007 / 963, 40 rows on 300 keys 163 / 240 -> 106 / 139.

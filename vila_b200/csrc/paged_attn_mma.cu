@@ -459,7 +459,7 @@ bool paged_attention_mma_takes(const vila_paged_attn_params& p) {
   return p.max_rows > 1 && p.nsplit == 1 && p.pool_dtype == VILA_DT_BF16 && p.talk == nullptr && p.H / p.G * maps <= kMaxWarps &&
          ((maps == 1 && p.dim == 128 && p.vdim == 128) || (maps == 2 && p.dim == 64 && p.vdim == 128) ||
           (maps == 1 && p.dim == 64 && p.vdim == 64)) &&
-         p.G <= 65535 && aligned(p.pool, 16) && aligned(p.q, 8) && aligned(p.out, 8);
+         aligned(p.pool, 16) && aligned(p.q, 8) && aligned(p.out, 8);
 }
 
 int paged_attention_mma(const vila_paged_attn_params& p, cudaStream_t stream) {

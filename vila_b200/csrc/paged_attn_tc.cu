@@ -52,13 +52,6 @@ constexpr int kBiasBytes = (227 * 1024 - kSmem) / 16 * 16;
 static_assert(kBiasBytes >= 16 * 1024, "paged_attn_tc: shared memory");
 constexpr float kLead = 5.5f;
 
-__device__ __forceinline__ bool pair_any(int id, bool v) {   // the two warps of 32 rows
-  uint32_t r;
-  asm volatile("{.reg .pred p, q; setp.ne.b32 p, %1, 0; bar.red.or.pred q, %2, 64, p; selp.u32 %0, 1, 0, q;}" : "=r"(r) : "r"(v ? 1u : 0u), "r"(id) : "memory");
-  return r != 0;
-}
-__device__ __forceinline__ void pair_sync(int id) { asm volatile("bar.sync %0, 64;" ::"r"(id) : "memory"); }
-
 // A row's sums join those in TMEM behind every fourth block of its sequence, and behind the second and the last kept one of a window:
 // by position, so that a row's numbers do not depend on its launch.
 __device__ __forceinline__ bool joins(int block, int kept_blocks) { return (block & 3) == 3 || block == 1 || block == kept_blocks - 1; }
@@ -572,7 +565,7 @@ bool aligned(const void* p, size_t n) { return reinterpret_cast<uintptr_t>(p) % 
 
 bool paged_attention_tc_takes(const vila_paged_attn_params& p) {
   return p.max_rows > 1 && p.nsplit == 1 && p.pool_dtype == VILA_DT_BF16 && p.talk == nullptr && maps_of(p.maps) == 1 && p.dim == D && p.vdim == D &&
-         p.H / p.G <= 8 && p.G <= 65535 && aligned(p.pool, 16) && aligned(p.q, 16) && aligned(p.out, 16);
+         p.H / p.G <= 8 && aligned(p.pool, 16) && aligned(p.q, 16) && aligned(p.out, 16);
 }
 
 int paged_attention_tc(const vila_paged_attn_params& p, cudaStream_t stream, int tries) {
