@@ -627,6 +627,25 @@ def test_space_to_depth(cuda, h, w, r):
     assert torch.equal(out, ref.reshape(2, -1, ref.shape[-1]))
 
 
+def test_space_to_depth_past_32_bits(cuda):
+    """more pieces of 16 bytes than 32-bit indices count: 69 GB of rows, of which the first, the middle and the last images are looked at"""
+    torch.cuda.empty_cache()
+    if torch.cuda.mem_get_info()[0] < 90e9:
+        pytest.skip("two operands of 34 GB")
+    ops, B, side = _ops(), 513, 2048
+    x = torch.zeros(B, side * side, 8, device=cuda, dtype=torch.bfloat16)
+    look = (0, 255, 256, 511, 512)
+    g = torch.Generator(device="cuda").manual_seed(3)
+    for b in look:
+        x[b] = torch.randn(side * side, 8, device=cuda, generator=g)
+    out = ops.space_to_depth(x, side, side, 2)
+    for b in look:
+        assert torch.equal(out[b], O.flat_square(x[b].view(1, side, side, 8), 2).reshape(-1, 32))
+    assert int(out[254].count_nonzero()) == 0 and int(out[510].count_nonzero()) == 0
+    del x, out
+    torch.cuda.empty_cache()
+
+
 @pytest.mark.parametrize("idx", [-1, 0, 1])
 def test_s2_merge_and_chessboard(cuda, idx):
     ops = _ops()
