@@ -89,7 +89,8 @@ struct Args {
   float scale_log2;
 };
 
-template <int DP, int CW, int TILES>
+// ADD: one tile whose rows have more than two key blocks; what two blocks sum to stays in TMEM otherwise
+template <int DP, int CW, int TILES, bool ADD>
 __global__ void __launch_bounds__(Shape<DP, CW, TILES>::kThreads, 1)
 fmha_pipe_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                  const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_o, const Args a, const WaitLimit limit, volatile unsigned int* failed) {
@@ -368,7 +369,7 @@ fmha_pipe_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
     int g = 0, units = 0;   // blocks and units of the tile so far
     // One tile: a row's sums, to which those of two blocks, up to block b, are added from TMEM under the next block's product
     uint32_t o[C::kHalf];
-    int pairs = 0;          // that have been taken in
+    int pairs = 0;          // that have been taken in, or (one tile, not ADD) units before this one
     auto take = [&](int b, auto columns) {   // of so many at a time
       constexpr int N = decltype(columns)::value;
       wait(&o_full[b & 1], b >> 1);
@@ -397,7 +398,7 @@ fmha_pipe_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
     Unit w;
     for (int r = 0; r < rounds; ++r) {
       if (!unit(r, w) || w.n[t] == 0) continue;
-      if (TILES == 1) {
+      if (ADD) {
 #pragma unroll
         for (int i = 0; i < C::kHalf; ++i) o[i] = 0u;
       }
@@ -429,7 +430,7 @@ fmha_pipe_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
 #pragma unroll
           for (int q = 0; q < 4; ++q) m4[q] = fmax3(m4[q], __uint_as_float(s[i + 2 * q]), __uint_as_float(s[i + 2 * q + 1]));
         float mx = fmaxf(fmaxf(m4[0], m4[1]), fmaxf(m4[2], m4[3])) * a.scale_log2;
-        bool taken = j == 0 || (j & 1) != 0;   // no two blocks' sums are complete and still in TMEM
+        bool taken = !ADD || j == 0 || (j & 1) != 0;   // no two blocks' sums are complete and still in TMEM
         if (pair_any(id, j == 0 || mx > m_ref + 8.0f)) {
           xm_t[half * BQ] = mx;
           pair_sync(id);
@@ -440,7 +441,7 @@ fmha_pipe_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
             const float m_new = mx > m_ref + 8.0f ? mx : m_ref;
             const float alpha = ex2f(m_ref - m_new);                      // 1 for rows that keep their reference
             // rare: few registers rather than few round trips
-            if (TILES == 1 && !taken) {
+            if (ADD && !taken) {
               take(g - 1, Few());
               taken = true;
             } else {
@@ -459,7 +460,7 @@ fmha_pipe_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
                 tmem_st_32x32b_x8(sums + c * 8, o8);
               }
             }
-            if (TILES == 1) {
+            if (ADD) {
 #pragma unroll
               for (int i = 0; i < C::kHalf; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * alpha);
             }
@@ -487,7 +488,7 @@ fmha_pipe_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
         tc_fence_before();
         __syncwarp();
         if (lane == 0) mbar_arrive(&p_full[sb]);
-        if constexpr (TILES == 1) {
+        if constexpr (ADD) {
           if (!taken) take(g - 1, All());
         }
       }
@@ -495,17 +496,19 @@ fmha_pipe_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
       xl_t[half * BQ] = l;
       pair_sync(id);
       l += xl_t[(half ^ 1) * BQ];
-      if constexpr (TILES == 1) {
+      if constexpr (ADD) {
         take(g - 1, All());
       } else {
-        wait(&o_full[t], g - 1);
+        if (TILES == 1) wait(&o_full[(g - 1) & 1], (g - 1) >> 1);
+        else wait(&o_full[t], g - 1);
         tc_fence_after();
+        const uint32_t sums = o_addr + (TILES == 1 ? (pairs++ & 1) * 128 : 0);
 #pragma unroll
-        for (int c = 0; c < C::kHalf / 8; ++c) tmem_ld_32x32b_x8(o_addr + c * 8, o + c * 8);
+        for (int c = 0; c < C::kHalf / 8; ++c) tmem_ld_32x32b_x8(sums + c * 8, o + c * 8);
         tmem_ld_wait();
         tc_fence_before();
         __syncwarp();
-        if (lane == 0) mbar_arrive(&o_free[t]);
+        if (TILES == 2 && lane == 0) mbar_arrive(&o_free[t]);
       }
       // Rows go out by TMA from the unit's Q tile, which its last scores have left: 16-byte stores of a row per lane held the
       // load / store unit for 2500 clocks a unit, and the softmax warps that issued the copies waited as long for TMA's queue.
@@ -557,7 +560,7 @@ fmha_pipe_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
   }
 }
 
-template <int DP, int CW, int TILES>
+template <int DP, int CW, int TILES, bool ADD>
 int launch(const FmhaParams& p, cudaStream_t stream, int tries) {
   using C = Shape<DP, CW, TILES>;
   static_assert(C::kSmem <= 227 * 1024, "fmha: shared memory");
@@ -600,7 +603,7 @@ int launch(const FmhaParams& p, cudaStream_t stream, int tries) {
   a.paged = paged ? 1 : 0;
   a.units = (p.Sq + TILES * BQ - 1) / (TILES * BQ);
   a.scale_log2 = p.scale * 1.4426950408889634f;
-  auto kern = fmha_pipe_kernel<DP, CW, TILES>;
+  auto kern = fmha_pipe_kernel<DP, CW, TILES, ADD>;
   static PerDeviceOnce attr_once;
   if (attr_once.first()) {
     VB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kSmem));
@@ -614,7 +617,9 @@ int launch(const FmhaParams& p, cudaStream_t stream, int tries) {
 
 template <int DP, int CW>
 int launch_tiles(const FmhaParams& p, int tiles, cudaStream_t stream, int tries) {
-  return tiles == 2 ? launch<DP, CW, 2>(p, stream, tries) : launch<DP, CW, 1>(p, stream, tries);
+  if (tiles == 2) return launch<DP, CW, 2, false>(p, stream, tries);
+  // up to two key blocks there is nothing to add, and the registers for it cost 0.4 of 5.8 us (64 rows, 128 columns); the same bits
+  return p.Sk > 2 * BKV ? launch<DP, CW, 1, true>(p, stream, tries) : launch<DP, CW, 1, false>(p, stream, tries);
 }
 
 }  // namespace
